@@ -119,8 +119,9 @@ struct sphgb_ctx {
     bool inSweep = false, sweepPrepared = false;
     // within one sweep: the EOS ran in the gradh epilogue / the per-particle quotients are formed
     bool eosFused = false, auxReady = false;
-    // packed neighbour-side records of the mixed pair passes (float4 x 4 per particle)
-    sphgb::DBuf pack;
+    // packed neighbour-side records of the mixed pair passes and of the pair-once momentum-energy pass
+    // (96 bytes per particle), and that pass's FP32 copy of rho
+    sphgb::DBuf pack, rhof;
     // forward tape of the VE adjoint: with tapeOn the FP64 VE passes over all particles keep the
     // per-particle sums the adjoint needs (kTape* sections x n doubles); tapeMask tells which passes
     // wrote theirs on the lists of epoch tapeEpoch for tapeN particles
@@ -150,6 +151,8 @@ struct sphgb_ctx {
     sphgb::DBuf whS64, whdS64;
     bool smoothKernel = false;
     sphgb::DBuf whx32;  // FP32 linear table (the mixed adjoint)
+    // e^(k/1024), e^(-k/1024), k/1024, |k| <= kExpNodes (the Atwood ramp of the pair-once passes)
+    sphgb::DBuf expTab;
     sphgb::DBuf whH32, whdH32;  // mixed passes: cubic pieces of W and dW/dv (kHermIntervals float4)
 
     // mixed precision grid-local coordinates: packed cell (21 bits per axis) + float4 {dx,dy,dz,1/h}

@@ -570,6 +570,8 @@ __global__ void __launch_bounds__(kPairBlock) avKernel(ListView lv, CoordFp64 cf
 }
 
 // ---------------------------------------------------------------- momentum and energy (VE)
+struct Rec4d;
+
 struct MeVeArgs {
     const void *vx, *vy, *vz, *h, *m, *prho, *c, *kx, *xm, *alpha;
     const void *c11, *c12, *c13, *c22, *c23, *c33;
@@ -595,6 +597,10 @@ struct MeVeArgs {
     const Rec8* pack;
     // FP64: the energy sums (en, avE before max(0, .)) for the VE adjoint, or null
     double *tapeEn, *tapeAvE;
+    // pair-once form: the neighbour side of a pair (meVeRec64Kernel) and rho in FP32
+    const Rec4d* rec64;
+    const float* rhof;
+    const double4* expTab;  // e^(k/1024), e^(-k/1024), k/1024 for |k| <= kExpNodes
 };
 
 template<class T>
@@ -1186,6 +1192,103 @@ __global__ void avOnceFinish(int64_t first, int64_t last, int64_t n, AvArgs a, c
                avAlpha<double>(a, ld<double>(a.alpha, i), hi, ci, divvi, __longlong_as_double(vb), gx, gy, gz));
 }
 
+// neighbour-side fields of the pair-once momentum-energy pass, 96 bytes per particle in three 32-byte
+// loads: A = m h^-3 c_ab (six entries), c, m, prho, 1/rho, xm, alpha / 8; and rho in FP32.  m and
+// h^-3 enter every use of c, so they are folded in once per particle instead of per pair.
+struct alignas(32) Rec4d {
+    double v[4];
+};
+
+__device__ __forceinline__ Rec4d ldRec4d(const Rec4d* p)
+{
+    Rec4d r;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.v[0]), "=d"(r.v[1]), "=d"(r.v[2]), "=d"(r.v[3]) : "l"(p));
+    return r;
+}
+
+// Aux: also forms the quotients rho, ln xm and 1/rho (outside a sweep, which has them already)
+template<bool Aux>
+__global__ void meVeRec64Kernel(int64_t n, MeVeArgs a, double* __restrict__ aux, Rec4d* __restrict__ rec,
+                                float* __restrict__ rhof)
+{
+    const int64_t j = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (j >= n) return;
+    const double m = ld<double>(a.m, j), xm = ld<double>(a.xm, j), f = m * a.hInv64[n + j];
+    double rho, rhoInv;
+    if constexpr (Aux) {
+        rho = ld<double>(a.kx, j) * m / xm;
+        rhoInv = 1.0 / rho;
+        aux[j] = rho;
+        aux[4 * n + j] = log(xm);
+    } else {
+        rho = aux[j];
+        rhoInv = aux[5 * n + j];
+    }
+    rec[3 * j] = {f * ld<double>(a.c11, j), f * ld<double>(a.c12, j), f * ld<double>(a.c13, j), f * ld<double>(a.c22, j)};
+    rec[3 * j + 1] = {f * ld<double>(a.c23, j), f * ld<double>(a.c33, j), ld<double>(a.c, j), m};
+    rec[3 * j + 2] = {ld<double>(a.prho, j), rhoInv, xm, 0.125 * ld<double>(a.alpha, j)};
+    rhof[j] = float(rho);
+}
+
+// Atwood weights a_mom, b_mom of a pair (momentum_energy_kern.hpp:160-190) in FP64: the exact decision
+// of |rho_i - rho_j| / (rho_i + rho_j) against 0.1 and 0.2 and, between them, the ramp
+// xm_i^(2-s) xm_j^s = xm_i^2 q and xm_j^(2-s) xm_i^s = xm_j^2 / q, q = (xm_j / xm_i)^s.  For the pairs
+// atwoodWeights leaves open: sums near a threshold, arguments beyond the table.
+__device__ __noinline__ double2 atwoodExact(double rhoi, double rhoj, double dln, double xmi, double xmj)
+{
+    constexpr double Atmin = 0.1, Atmax = 0.2, ramp = 1.0 / (Atmax - Atmin);
+    const double dr = fabs(rhoi - rhoj), sr = rhoi + rhoj;
+    if (lessNonNeg(dr, Atmin * sr)) return make_double2(xmi * xmi, xmj * xmj);
+    if (lessNonNeg(Atmax * sr, dr)) return make_double2(xmi * xmj, xmi * xmj);
+    const double s = ramp * (dr / sr - Atmin);
+    const double q = exp(s * dln);
+    return make_double2(xmi * xmi * q, xmj * xmj / q);
+}
+
+// the same weights with few FP64 instructions: the two flat branches are taken where FP32 copies of rho
+// decide safely (1e-6 of the sum beside a threshold, and sums FP32 cannot hold, go to atwoodExact).
+// On the ramp (a quarter of the pairs of a jittered lattice or a clustered sphere, so nearly every warp
+// is there for some lane) the quotient comes from a 20-bit reciprocal by two Newton corrections, and
+// q = e^a and 1 / q = e^-a, |a| <= 1/2, together from a table of e^(+-k/1024) and the even and odd parts
+// of the series of the rest, |rest| <= 2^-11: 21 FP64 instructions instead of two divisions and an exp.
+__device__ __forceinline__ void atwoodWeights(const double* __restrict__ rho, const double* __restrict__ lnxm,
+                                              const double4* __restrict__ expTab, int64_t i, int64_t j, float rhofi,
+                                              float rhofj, double xmi, double xmj, double& am, double& bm)
+{
+    const float dr = fabsf(rhofi - rhofj), sr = rhofi + rhofj;
+    am = xmi * xmi;
+    bm = xmj * xmj;
+    if (sr > 1e-30f && dr < (0.1f - 1e-6f) * sr) return;
+    if (sr > 1e-30f && dr > (0.2f + 1e-6f) * sr && dr < 1e38f) {
+        am = bm = xmi * xmj;
+        return;
+    }
+    const double rhoi = rho[i], rhoj = __ldg(rho + j), dln = __ldg(lnxm + j) - lnxm[i];
+    const double d = fabs(rhoi - rhoj), t = rhoi + rhoj;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(t));
+    double at = d * y;
+    at = fma(fma(-t, at, d), y, at);
+    at = fma(fma(-t, at, d), y, at);
+    const double a = fma(10.0, at, -1.0) * dln;
+    // |a| from the high word, truncated to 20 bits, as a float: the nearest table node to within 2^-20
+    const unsigned hi = unsigned(__double2hiint(a)), mag = hi & 0x7fffffffu;
+    const bool onRamp = sr > 1e-30f && dr > (0.1f + 1e-6f) * sr && dr < (0.2f - 1e-6f) * sr && mag < 0x3fe00000u;
+    if (!onRamp) {
+        const double2 ab = atwoodExact(rhoi, rhoj, dln, xmi, xmj);
+        am = ab.x;
+        bm = ab.y;
+        return;
+    }
+    int k = mag < 0x3f300000u ? 0 : __float2int_rn(__uint_as_float((mag - (896u << 20)) << 3) * 1024.f);
+    k = (hi >> 31) ? -k : k;
+    const double4 e = expTab[kExpNodes + k];  // e^(k/1024), e^(-k/1024), k/1024
+    const double r = a - e.z, r2 = r * r;
+    const double even = r2 * fma(r2, 1.0 / 24.0, 0.5), odd = fma(r * r2, 1.0 / 6.0, r);
+    am *= fma(e.x, even + odd, e.x);
+    bm *= fma(e.y, even - odd, e.y);
+}
+
 // FP64 VE momentum-energy with one evaluation per mutual pair, for lists that cover every particle.
 // i walks its owned list: every pair of its list that j does not list back, and half of the
 // mutual pairs (the other half is in the owned lists of the other ends).  The two ends' terms follow from one
@@ -1194,7 +1297,17 @@ __global__ void avOnceFinish(int64_t first, int64_t last, int64_t n, AvArgs a, c
 // 1/rho_i and 1/rho_j trade places; the viscosity and the signal velocity are symmetric.  i's terms
 // stay in registers; j's go to its accumulators with FP64 atomics (the signal-velocity maximum as an
 // integer maximum of non-negative bit patterns).
-template<bool Smooth>
+//
+// Bound by the FP64 pipe (2 lanes per cycle and SM), so the pair terms are arranged for few FP64
+// instructions: 54 per mutual pair, 21 more on the Atwood ramp (atwoodWeights).  The sums are forces: with A = m h^-3 c at each end (per particle),
+// w_i' = m_j w_i and w_j' = m_i w_j, hv = visc / 2, t = hv / rho, P_i = w_i' (prho_i am + t_i) and
+// P_j = w_j' (prho_j bm + t_j), both ends add the same V = P_i A_i r + P_j A_j r, with opposite signs,
+// and the same Q = t_i w_i' s_i + t_j w_j' s_j (s = v_ij . A r); the finishing kernel divides by the
+// particle's mass.  vsig is kept doubled, alpha divided by 8 (both exact).  With the per-pair exp and
+// divisions of the ramp and the terms factored by m_j and m_i the kernel ran 109 FP64 instructions per
+// pair: 89.8 ms at 8M (jittered Sedov), now 82 and 65.2 ms, the FP64 pipe 87 % busy in both.
+// Geo: arrays of the pair-geometry cache to read (5, 2), or 0 to form the geometry here.
+template<bool Smooth, int Geo>
 __global__ void __launch_bounds__(kPairBlock) meVeOnceKernel(ListView lv, CoordFp64 cf, MeVeArgs a, PairGeo geo)
 {
     using T = double;
@@ -1203,114 +1316,92 @@ __global__ void __launch_bounds__(kPairBlock) meVeOnceKernel(ListView lv, CoordF
     const int64_t ii = i - lv.first;
     const unsigned nOwned = __ldg(a.ownedCount + ii);
     const KTab<Smooth> tabX{a.w64};
-    const T* aux = static_cast<const T*>(a.aux);
-    const T *auxRho = aux, *auxLnXm = aux + 4 * a.n, *auxRhoInv = aux + 5 * a.n;
-    const double* hInv3 = a.hInv64 + a.n;
+    const double* aux = static_cast<const double*>(a.aux);
     const double* hInvDx = a.hInv64 + 2 * a.n;
-    const T *vxA = static_cast<const T*>(a.vx), *vyA = static_cast<const T*>(a.vy),
-            *vzA = static_cast<const T*>(a.vz), *prhoA = static_cast<const T*>(a.prho);
-    constexpr T Atmin = 0.1, Atmax = 0.2, ramp = 1.0 / (Atmax - Atmin);
+    const T *vxA = static_cast<const T*>(a.vx), *vyA = static_cast<const T*>(a.vy), *vzA = static_cast<const T*>(a.vz);
 
-    const T hi = ld<T>(a.h, i), mi = ld<T>(a.m, i), ci = ld<T>(a.c, i), ai = ld<T>(a.alpha, i);
-    const T xmi = ld<T>(a.xm, i), prhoi = prhoA[i];
-    const T rhoi = auxRho[i], lnxmi = auxLnXm[i], rhoiInv = auxRhoInv[i];
-    const T vxi = vxA[i], vyi = vyA[i], vzi = vzA[i];
-    const T c11i = ld<T>(a.c11, i), c12i = ld<T>(a.c12, i), c13i = ld<T>(a.c13, i);
-    const T c22i = ld<T>(a.c22, i), c23i = ld<T>(a.c23, i), c33i = ld<T>(a.c33, i);
-    const T xmi2 = xmi * xmi;
-    auto t = cf.target(i);
-    const T hiInv3 = hInv3[i], hiInvDx = hInvDx[i], twoH = 2.0 * hi;
-    const bool wrap = cf.needsWrap(t, twoH);
-    const int64_t gb = geo.base(ii);
+    const Rec4d i0 = a.rec64[3 * i], i1 = a.rec64[3 * i + 1], i2 = a.rec64[3 * i + 2];
+    const float rhofi = a.rhof[i];
+    typename CoordFp64::Target t{};
+    T vxi = 0, vyi = 0, vzi = 0, hiInvDx = 0, twoH = 0;
+    bool wrap = false;
+    if constexpr (Geo != 5) {
+        t = cf.target(i);
+        twoH = 2.0 * ld<T>(a.h, i);
+        wrap = cf.needsWrap(t, twoH);
+        vxi = vxA[i], vyi = vyA[i], vzi = vzA[i];
+        hiInvDx = hInvDx[i];
+    }
+    int64_t g = 0;
+    if constexpr (Geo != 0) g = geo.base(ii);
     T mx = 0, my = 0, mz = 0, en = 0, avE = 0;
     long long maxvBits = 0;
     double *accX = a.acc, *accY = a.acc + a.n, *accZ = a.acc + 2 * a.n, *accE = a.acc + 3 * a.n,
            *accV = a.acc + 4 * a.n;
     long long* accS = reinterpret_cast<long long*>(a.acc + 5 * a.n);
-    for (unsigned k = 0; k < nOwned; ++k) {
+    for (unsigned k = 0; k < nOwned; ++k, g += 32) {
         const uint32_t e = __ldg(a.owned + listSlot(ii, k, lv.stride));
         const uint32_t j = e & 0x7fffffffu;
         const bool mutual = (e >> 31) != 0;
+        const Rec4d j0 = ldRec4d(a.rec64 + 3 * int64_t(j)), j1 = ldRec4d(a.rec64 + 3 * int64_t(j) + 1),
+                    j2 = ldRec4d(a.rec64 + 3 * int64_t(j) + 2);
+        const float rhofj = __ldg(a.rhof + j);
         T rx, ry, rz, rinv, Wi, Wj, vxij, vyij, vzij;
-        if (geo.g) {
-            const int64_t e = gb + 32 * int64_t(k);
-            const double2 gd = __ldg(geo.g + e), wv = __ldg(geo.w + e);
-            rinv = gd.y;
-            Wi = hiInv3 * wv.x;
-            Wj = __ldg(hInv3 + j) * wv.y;
-            if (geo.x) {  // v_ij = v_i - v_j = -dv exactly
-                const double2 a0 = __ldg(geo.x + e), a1 = __ldg(geo.x + geo.plane + e),
-                              a2 = __ldg(geo.x + 2 * geo.plane + e);
-                rx = a0.x, ry = a0.y, rz = a1.x;
-                vxij = -a1.y, vyij = -a2.x, vzij = -a2.y;
-            } else {
-                cf.diffFast(t, j, twoH, wrap, rx, ry, rz);
-                vxij = vxi - vxA[j], vyij = vyi - vyA[j], vzij = vzi - vzA[j];
-            }
+        if constexpr (Geo != 0) {
+            const double2 wv = __ldg(geo.w + g);
+            rinv = __ldg(geo.g + g).y;
+            Wi = j1.v[3] * wv.x;
+            Wj = i1.v[3] * wv.y;
+        }
+        if constexpr (Geo == 5) {  // v_ij = v_i - v_j = -dv exactly
+            const double2 a0 = __ldg(geo.x + g), a1 = __ldg(geo.x + geo.plane + g), a2 = __ldg(geo.x + 2 * geo.plane + g);
+            rx = a0.x, ry = a0.y, rz = a1.x;
+            vxij = -a1.y, vyij = -a2.x, vzij = -a2.y;
         } else {
             cf.diffFast(t, j, twoH, wrap, rx, ry, rz);
+            vxij = vxi - vxA[j], vyij = vyi - vyA[j], vzij = vzi - vzA[j];
+        }
+        if constexpr (Geo == 0) {
             const T r2 = dist2(rx, ry, rz);
             rinv = invDist(r2);
             const T dist = r2 * rinv;
-            Wi = hiInv3 * lookupX(tabX, dist * hiInvDx);
-            Wj = __ldg(hInv3 + j) * lookupX(tabX, dist * __ldg(hInvDx + j));
-            vxij = vxi - vxA[j], vyij = vyi - vyA[j], vzij = vzi - vzA[j];
+            Wi = j1.v[3] * lookupX(tabX, dist * hiInvDx);
+            Wj = i1.v[3] * lookupX(tabX, dist * __ldg(hInvDx + j));
         }
-        T gix = c11i * rx + c12i * ry + c13i * rz;
-        T giy = c12i * rx + c22i * ry + c23i * rz;
-        T giz = c13i * rx + c23i * ry + c33i * rz;
-        T c11j = ld<T>(a.c11, j), c12j = ld<T>(a.c12, j), c13j = ld<T>(a.c13, j);
-        T c22j = ld<T>(a.c22, j), c23j = ld<T>(a.c23, j), c33j = ld<T>(a.c33, j);
-        T gjx = c11j * rx + c12j * ry + c13j * rz;
-        T gjy = c12j * rx + c22j * ry + c23j * rz;
-        T gjz = c13j * rx + c23j * ry + c33j * rz;
-        T mj = ld<T>(a.m, j), cj = ld<T>(a.c, j), xmj = ld<T>(a.xm, j);
-        T rhoj = __ldg(auxRho + j);
-        T rv = fma(rz, vzij, fma(ry, vyij, rx * vxij));
-        T wij = rv * rinv;
-        T visc = artificialViscosity<T>(ai, ld<T>(a.alpha, j), ci, cj, wij);
-        const T vsig = fma(T(-2), wij, T(0.5) * (ci + cj));
-        maxvBits = maxBitsNonNeg(maxvBits, vsig);
-        T dr = fabs(rhoi - rhoj), sr = rhoi + rhoj;
+        const T gix = i0.v[0] * rx + i0.v[1] * ry + i0.v[2] * rz;
+        const T giy = i0.v[1] * rx + i0.v[3] * ry + i1.v[0] * rz;
+        const T giz = i0.v[2] * rx + i1.v[0] * ry + i1.v[1] * rz;
+        const T gjx = j0.v[0] * rx + j0.v[1] * ry + j0.v[2] * rz;
+        const T gjy = j0.v[1] * rx + j0.v[3] * ry + j1.v[0] * rz;
+        const T gjz = j0.v[2] * rx + j1.v[0] * ry + j1.v[1] * rz;
+        const T wij = fma(rz, vzij, fma(ry, vyij, rx * vxij)) * rinv;
+        const T cs = i1.v[2] + j1.v[2];
+        const T vsig2 = fma(T(-4), wij, cs);  // twice the reference's 0.5 (c_i + c_j) - 2 w_ij
+        maxvBits = maxBitsNonNeg(maxvBits, vsig2);
         T am, bm;
-        if (lessNonNeg(dr, Atmin * sr)) {
-            am = xmi2;
-            bm = xmj * xmj;
-        } else if (lessNonNeg(Atmax * sr, dr)) {
-            am = xmi * xmj;
-            bm = am;
-        } else {
-            T s = ramp * (dr / sr - Atmin);
-            T q = exp(s * (__ldg(auxLnXm + j) - lnxmi));
-            am = xmi2 * q;
-            bm = xmj * xmj / q;
+        atwoodWeights(aux, aux + 4 * a.n, a.expTab, i, j, rhofi, rhofj, i2.v[2], j2.v[2], am, bm);
+        const T wsi = Wi * (vxij * gix + vyij * giy + vzij * giz), wsj = Wj * (vxij * gjx + vyij * gjy + vzij * gjz);
+        T ti = 0, tj = 0, Q = 0;
+        if (negative(wij)) {  // approaching: hv = -((alpha_i + alpha_j) / 8 (c_i + c_j) - w_ij) w_ij
+            const T hv = fma(i2.v[3] + j2.v[3], cs, -wij) * -wij;
+            ti = i2.v[1] * hv;
+            tj = j2.v[1] * hv;
+            Q = fma(ti, wsi, tj * wsj);
         }
-        T si = vxij * gix + vyij * giy + vzij * giz;
-        T sj = vxij * gjx + vyij * gjy + vzij * gjz;
-        // the reference's terms, factored: with hv = visc / 2, t_i = hv / rho_i and t_j = hv / rho_j,
-        // P_i = W_i (prho_i am + t_i) and P_j = W_j (prho_j bm + t_j), i's momentum term momi a_i +
-        // momj a_j + (av a_i + bv a_j) / 2 is m_j V with V = P_i G_i + P_j G_j and its viscous work
-        // m_j Q with Q = t_i W_i s_i + t_j W_j s_j; j's terms of the same pair are m_i V and m_i Q
-        // (i and j trade places, G and v_ij change sign); the energy terms m_j am W_i s_i and
-        // m_i bm W_j s_j stay apart
-        const T hv = T(0.5) * visc;
-        const T wsi = Wi * si, wsj = Wj * sj;
-        const T ti = rhoiInv * hv, tj = __ldg(auxRhoInv + j) * hv;
-        const T Pi = Wi * fma(prhoi, am, ti), Pj = Wj * fma(prhoA[j], bm, tj);
+        const T Pi = Wi * fma(i2.v[0], am, ti), Pj = Wj * fma(j2.v[0], bm, tj);
         const T Vx = fma(Pi, gix, Pj * gjx), Vy = fma(Pi, giy, Pj * gjy), Vz = fma(Pi, giz, Pj * gjz);
-        const T Q = fma(ti, wsi, tj * wsj);
-        mx = fma(-mj, Vx, mx);
-        my = fma(-mj, Vy, my);
-        mz = fma(-mj, Vz, mz);
-        en = fma(-(mj * am), wsi, en);
-        avE = fma(-mj, Q, avE);
+        mx -= Vx;
+        my -= Vy;
+        mz -= Vz;
+        en = fma(-am, wsi, en);
+        avE -= Q;
         if (mutual) {
-            atomicAdd(accX + j, mi * Vx);
-            atomicAdd(accY + j, mi * Vy);
-            atomicAdd(accZ + j, mi * Vz);
-            atomicAdd(accE + j, -(mi * bm) * wsj);
-            atomicAdd(accV + j, -mi * Q);
-            atomicMax(accS + j, __double_as_longlong(vsig));
+            atomicAdd(accX + j, Vx);
+            atomicAdd(accY + j, Vy);
+            atomicAdd(accZ + j, Vz);
+            atomicAdd(accE + j, -bm * wsj);
+            atomicAdd(accV + j, -Q);
+            atomicMax(accS + j, __double_as_longlong(vsig2));
         }
     }
     atomicAdd(accX + i, mx);
@@ -1328,18 +1419,20 @@ __global__ void __launch_bounds__(kPairBlock) meVeOnceFinish(ListView lv, MeVeAr
     double dt = INFINITY;
     if (valid) {
         const int64_t i = i0;
-        const double prhoi = ld<double>(a.prho, i);
+        const double prhoi = ld<double>(a.prho, i), mInv = 1.0 / ld<double>(a.m, i);
+        const double en = a.acc[3 * a.n + i] * mInv, avSum = a.acc[4 * a.n + i] * mInv;
         if (a.tapeEn) {
-            a.tapeEn[i] = a.acc[3 * a.n + i];
-            a.tapeAvE[i] = a.acc[4 * a.n + i];
+            a.tapeEn[i] = en;
+            a.tapeAvE[i] = avSum;
         }
-        const double avE = fmax(0.0, a.acc[4 * a.n + i]);
-        a.du[i] = a.K * (prhoi * a.acc[3 * a.n + i] + 0.5 * avE);
-        st<double>(a.ax, i, -a.K * a.acc[i]);
-        st<double>(a.ay, i, -a.K * a.acc[a.n + i]);
-        st<double>(a.az, i, -a.K * a.acc[2 * a.n + i]);
+        const double avE = fmax(0.0, avSum);
+        a.du[i] = a.K * (prhoi * en + 0.5 * avE);
+        const double km = -a.K * mInv;
+        st<double>(a.ax, i, km * a.acc[i]);
+        st<double>(a.ay, i, km * a.acc[a.n + i]);
+        st<double>(a.az, i, km * a.acc[2 * a.n + i]);
         const long long mb = reinterpret_cast<const long long*>(a.acc + 5 * a.n)[i];
-        dt = courantDt(__longlong_as_double(mb), ld<double>(a.h, i), ld<double>(a.c, i), a.Kcour);
+        dt = courantDt(0.5 * __longlong_as_double(mb), ld<double>(a.h, i), ld<double>(a.c, i), a.Kcour);
     }
     if (a.groupDt) {
         double g = dt;
@@ -1592,7 +1685,10 @@ int passMomentumEnergyVe(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_
     if (avClean && !(p->dV11 && p->dV12 && p->dV13 && p->dV22 && p->dV23 && p->dV33)) return SPHGB_ERR_ARG;
     SPHGB_TRY(checkPass(c, p, first, last));
     const bool mixed = p->precision == SPHGB_MIXED;
-    SPHGB_TRY(launchVeAux<kAuxMe>(c, p));
+    // one evaluation per mutual pair when the lists cover all particles and the order may vary
+    const bool once = !mixed && !avClean && pairOnce(c, p, first, last);
+    if (once) SPHGB_TRY(c->aux.ensure(sizeof(double) * 6 * size_t(p->n)));
+    else SPHGB_TRY(launchVeAux<kAuxMe>(c, p));
     ListView lv = listView(c);
     lv.first = first;
     lv.last = last;
@@ -1651,17 +1747,31 @@ int passMomentumEnergyVe(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_
             a.tapeEn = tape + int64_t(kTapeEn) * p->n;
             a.tapeAvE = tape + int64_t(kTapeAvE) * p->n;
         }
-        // one evaluation per mutual pair when the lists cover all particles and the order may vary
-        const bool once = !avClean && pairOnce(c, p, first, last);
         if (once) {
             SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * 6 * size_t(p->n)));
             SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * 6 * size_t(p->n), c->stream));
             a.owned = c->owned.as<uint32_t>();
             a.ownedCount = c->ownedCount.as<uint32_t>();
             a.acc = c->pairAcc.as<double>();
+            SPHGB_TRY(c->pack.ensure(sizeof(Rec4d) * 3 * size_t(p->n)));
+            SPHGB_TRY(c->rhof.ensure(sizeof(float) * size_t(p->n)));
+            const unsigned rb = gridFor(p->n, 256);
+            if (c->inSweep && c->auxReady)
+                meVeRec64Kernel<false><<<rb, 256, 0, c->stream>>>(p->n, a, c->aux.as<double>(), c->pack.as<Rec4d>(),
+                                                                  c->rhof.as<float>());
+            else
+                meVeRec64Kernel<true><<<rb, 256, 0, c->stream>>>(p->n, a, c->aux.as<double>(), c->pack.as<Rec4d>(),
+                                                                 c->rhof.as<float>());
+            SPHGB_TRY(launched(c, "meVeRec64Kernel"));
+            a.rec64 = c->pack.as<Rec4d>();
+            a.rhof = c->rhof.as<float>();
+            a.expTab = c->expTab.as<double4>();
+            const PairGeo geo = pairGeoRead(c);
             SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
-                meVeOnceKernel<decltype(smooth)::value><<<blocks, kPairBlock, 0, c->stream>>>(lv, cf, a,
-                                                                                              pairGeoRead(c));
+                constexpr bool S = decltype(smooth)::value;
+                if (geo.x) meVeOnceKernel<S, 5><<<blocks, kPairBlock, 0, c->stream>>>(lv, cf, a, geo);
+                else if (geo.g) meVeOnceKernel<S, 2><<<blocks, kPairBlock, 0, c->stream>>>(lv, cf, a, geo);
+                else meVeOnceKernel<S, 0><<<blocks, kPairBlock, 0, c->stream>>>(lv, cf, a, geo);
                 return launched(c, "meVeOnceKernel");
             }));
             meVeOnceFinish<<<blocks, kPairBlock, 0, c->stream>>>(lv, a);

@@ -118,6 +118,17 @@ int buildTables(sphgb_ctx* c)
         SPHGB_CUDA(cudaMemcpy(c->whS64.p, sw.data(), sizeof(double) * sw.size(), cudaMemcpyHostToDevice));
         SPHGB_CUDA(cudaMemcpy(c->whdS64.p, sd.data(), sizeof(double) * sd.size(), cudaMemcpyHostToDevice));
     }
+    {
+        std::vector<double> e(4 * (2 * kExpNodes + 1));
+        for (int k = -kExpNodes; k <= kExpNodes; ++k) {
+            double* q = &e[4 * (k + kExpNodes)];
+            q[0] = std::exp(k / 1024.0);
+            q[1] = std::exp(-k / 1024.0);
+            q[2] = k / 1024.0;
+        }
+        SPHGB_TRY(c->expTab.ensure(sizeof(double) * e.size()));
+        SPHGB_CUDA(cudaMemcpy(c->expTab.p, e.data(), sizeof(double) * e.size(), cudaMemcpyHostToDevice));
+    }
     SPHGB_TRY(c->whx64.ensure(sizeof(double) * 2 * kTableSize));
     SPHGB_TRY(c->whdx64.ensure(sizeof(double) * 2 * kTableSize));
     SPHGB_CUDA(cudaMemcpy(c->whx64.p, wx.data(), sizeof(double) * 2 * kTableSize, cudaMemcpyHostToDevice));

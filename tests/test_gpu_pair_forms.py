@@ -1,0 +1,33 @@
+"""The FP64 pass variants chosen by size, list form or field values, against the CPU oracle at the sizes
+and values where their branches change.  Bars as in test_gpu_parity.py: 1e-12 of the field's magnitude,
+scaled by the conditioning of gradh for the fields downstream of it."""
+
+import numpy as np
+import pytest
+
+from test_gpu_parity import field_scale, fp64_tol, run_gpu
+
+pytestmark = pytest.mark.gpu
+
+VE_FIELDS = ("rho", "p", "c", "xm", "kx", "gradh", "prho", "c11", "c12", "c13", "c22", "c23", "c33", "divv", "curlv",
+             "alpha", "ax", "ay", "az", "du")
+
+
+def check_fields(r, ref, variant, fields, what):
+    for f in fields:
+        err = np.max(np.abs(r[f] - ref[f])) / field_scale(ref, f)
+        assert err <= fp64_tol(ref, f, variant), f"{what} {f}: {err:.3e}"
+
+
+@pytest.mark.parametrize("spread", [0.02, 0.2, 1.0])
+def test_atwood_branches_match_oracle(gpu_ctx, port, spread):
+    """Masses spread by 10^(+-spread): pairs on the flat Atwood branches, on the ramp, and (spread 1) on
+    the ramp with |ln xm_j - ln xm_i| s beyond the exponential table's range."""
+    from sphexa_gb300 import workloads as W
+    wl = W.fourier(14, seed=71, rho_seed=72, v_seed=73)
+    rng = np.random.Generator(np.random.PCG64(74))
+    wl.fields["m"] = (wl.fields["m"] * 10.0 ** rng.uniform(-spread, spread, wl.n)).astype(np.float32).astype(np.float64)
+    gpu_ctx.set_deterministic(False)
+    r = run_gpu(gpu_ctx, wl, "ve", False)
+    ref = port.sweep(wl, "ve", False)
+    check_fields(r, ref, "ve", VE_FIELDS, f"spread {spread}")
