@@ -108,10 +108,11 @@ struct sphgb_ctx {
     // per-particle accumulators of the pair-once passes (up to 6 x n doubles)
     bool deterministic = false;
     sphgb::DBuf pairAcc;
-    // within one sweep: |r|, 1/|r| and the kernel function at both ends of every owned entry, stored
+    // within one sweep: |r|, w_ij and the kernel function at both ends of every owned entry, stored
     // by the pair-once xmass pass and read by the later pair-once passes of the same sweep (PairGeo in
     // pairs.cuh); geoRows: per warp of 32 targets its longest owned list, then its first row
-    sphgb::DBuf pairGeo, geoRows;
+    // rho0Sum: the xmass pass's sum w m_j per particle, for gradh
+    sphgb::DBuf pairGeo, geoRows, rho0Sum;
     size_t geoRowCount = 0;
     int geoArrays = 0;  // 5: with the difference and velocity-difference vectors, 2: without
     bool geoValid = false;

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(kPairBlock) xmassOnceKernel(ListView lv, Owned
     const double hi = h[i], mi = m[i], twoH = 2.0 * hi, hiInvDx = hInvDx[i];
     const bool wrap = cf.needsWrap(t, twoH);
     const int64_t gb = geo.base(ii);
-    const double vxi = geo.x ? vx[i] : 0.0, vyi = geo.x ? vy[i] : 0.0, vzi = geo.x ? vz[i] : 0.0;
+    const double vxi = geo.g ? vx[i] : 0.0, vyi = geo.g ? vy[i] : 0.0, vzi = geo.g ? vz[i] : 0.0;
     double rho0 = 0.0;
     for (unsigned k = 0; k < no; ++k) {
         bool mutual;
@@ -116,10 +116,11 @@ __global__ void __launch_bounds__(kPairBlock) xmassOnceKernel(ListView lv, Owned
         if (geo.g) {  // the sweep's later pair-once passes load the geometry and both kernel values
             const double wj = lookupX(tab, dist * __ldg(hInvDx + j));
             const int64_t e = gb + 32 * int64_t(k);
-            geo.g[e] = make_double2(dist, rinv);
+            const double dvx = __ldg(vx + j) - vxi, dvy = __ldg(vy + j) - vyi, dvz = __ldg(vz + j) - vzi;
+            // w_ij = (r . v_ij) / |r| with v_ij = -dv, in the order of every FP64 pass
+            geo.g[e] = make_double2(dist, -fma(rz, dvz, fma(ry, dvy, rx * dvx)) * rinv);
             geo.w[e] = make_double2(wi, wj);
             if (geo.x) {
-                const double dvx = __ldg(vx + j) - vxi, dvy = __ldg(vy + j) - vyi, dvz = __ldg(vz + j) - vzi;
                 geo.x[e] = make_double2(rx, ry);
                 geo.x[geo.plane + e] = make_double2(rz, dvx);
                 geo.x[2 * geo.plane + e] = make_double2(dvy, dvz);
@@ -132,15 +133,17 @@ __global__ void __launch_bounds__(kPairBlock) xmassOnceKernel(ListView lv, Owned
     atomicAdd(acc + i, rho0);
 }
 
+// sums: where the pass keeps sum w m_j for gradh (with the geometry cache), or null
 template<bool StoreRho>
 __global__ void xmassOnceFinish(int64_t first, int64_t last, const double* h, const double* m, double K,
-                                const double* acc, double* out)
+                                const double* acc, double* out, double* sums)
 {
     const int64_t i = first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (i >= last) return;
     const double hi = h[i], mi = m[i];
     const double hInv = 1.0 / hi, h3Inv = hInv * hInv * hInv;
     const double xm = mi / ((mi + acc[i]) * K * h3Inv);
+    if (sums) sums[i] = acc[i];
     out[i] = StoreRho ? mi / xm : xm;
 }
 
@@ -418,8 +421,13 @@ int launchXmass(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, v
         const int64_t n = p->n;
         SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * size_t(n)));
         SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * size_t(n), c->stream));
-        PairGeo geo;
-        SPHGB_TRY(pairGeoStore(c, &geo));
+        PairGeo geo{};
+        if (p->vx && p->vy && p->vz) SPHGB_TRY(pairGeoStore(c, &geo));
+        double* sums = nullptr;
+        if (geo.g) {
+            SPHGB_TRY(c->rho0Sum.ensure(sizeof(double) * size_t(n)));
+            sums = c->rho0Sum.as<double>();
+        }
         SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
             constexpr bool S = decltype(smooth)::value;
             xmassOnceKernel<S><<<blocks, kPairBlock, 0, c->stream>>>(
@@ -433,11 +441,11 @@ int launchXmass(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, v
         if (storeRho)
             xmassOnceFinish<true><<<eb, 256, 0, c->stream>>>(first, last, static_cast<const double*>(p->h),
                                                               static_cast<const double*>(p->m), c->K,
-                                                              c->pairAcc.as<double>(), static_cast<double*>(out));
+                                                              c->pairAcc.as<double>(), static_cast<double*>(out), sums);
         else
             xmassOnceFinish<false><<<eb, 256, 0, c->stream>>>(first, last, static_cast<const double*>(p->h),
                                                                static_cast<const double*>(p->m), c->K,
-                                                               c->pairAcc.as<double>(), static_cast<double*>(out));
+                                                               c->pairAcc.as<double>(), static_cast<double*>(out), sums);
         return launched(c, "xmassOnceFinish");
     }
     const Rec8* rec = nullptr;

@@ -14,7 +14,7 @@
 // |r| and rv/|r|; the Atwood-number branches are decided by comparison, and the ramp's four
 // pow() calls become one exp() of the precomputed ln xm difference; the periodic wrap tests run
 // only for targets whose 2h box touches a periodic face; inside a sweep the pair-once passes read
-// r, v_j - v_i, |r|, 1/|r| and both kernel values from the cache the xmass pass fills (PairGeo).
+// r, v_j - v_i, |r|, w_ij and both kernel values from the cache the xmass pass fills (PairGeo).
 // Results agree with the reference to rounding (<= 1e-12 relative).  The mixed form runs the same
 // loops in FP32 on grid-local offsets with Kahan sums.
 #include "pairs.cuh"
@@ -871,11 +871,17 @@ __global__ void __launch_bounds__(kPairBlock) meVeKernel(ListView lv, CoordFp64 
     if (a.minDt) blockMinDt(dt, a.minDt);
 }
 
-// FP64 gradh with one evaluation per mutual pair over the owned lists.  i adds w_i xm_j,
-// dterh_i xm_j and dterh_i m_j (veDefGradhJLoop, ve_def_gradh_kern.hpp:64-78); a mutual pair also
-// gives j its terms at v_j = d / h_j with xm_i and m_i, by FP64 atomics.  The self terms and the
-// epilogue (ve_def_gradh_kern.hpp:60-62, 80-88) run in gradhOnceFinish.
-template<bool Smooth>
+// FP64 gradh with one evaluation per mutual pair over the owned lists.  With x = v / dx (table units)
+// and D = x dW, the reference's dterh = -(3 w + v dW) (veDefGradhJLoop, ve_def_gradh_kern.hpp:64-78)
+// is -(3 w + dx D), so its sums follow from sum w xm_j (which kx needs), sum D xm_j, and either sum w m_j
+// of the xmass pass and sum D m_j (Geo: within a sweep, where that sum is of the same geometry), or
+// sum (3 w / dx + D) m_j.  A mutual pair also gives j its terms at v_j = d / h_j with xm_i and m_i, by
+// FP64 atomics.  The self terms and the epilogue (ve_def_gradh_kern.hpp:60-62, 80-88) run in the
+// finishing kernels.  FP64-pipe bound: 12 instructions per mutual pair with the cache (18 with v and
+// dterh per pair, 14.7 ms at 8M; now 11.3 ms).
+constexpr double kTabDx = 1.0 / kTabInvDx;
+
+template<bool Smooth, bool Geo>
 __global__ void __launch_bounds__(kPairBlock) gradhOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf,
                                                                const double* h, const double* m, const double* xm,
                                                                KTab<Smooth> tw, KTab<Smooth> tdw,
@@ -886,22 +892,27 @@ __global__ void __launch_bounds__(kPairBlock) gradhOnceKernel(ListView lv, Owned
     if (i >= lv.last) return;
     const int64_t ii = i - lv.first;
     const unsigned no = ov.size(ii);
-    const double* hInv = hInv64;
     const double* hInvDx = hInv64 + 2 * n;
-    auto t = cf.target(i);
-    const double hi = h[i], mi = m[i], xmi = xm[i], twoH = 2.0 * hi, hiInv = hInv[i], hiInvDx = hInvDx[i];
-    const bool wrap = cf.needsWrap(t, twoH);
-    const int64_t gb = geo.base(ii);
-    double kx = 0.0, whom = 0.0, wr0 = 0.0;
-    for (unsigned k = 0; k < no; ++k) {
+    const double mi = m[i], xmi = xm[i], hiInvDx = hInvDx[i];
+    typename CoordFp64::Target t{};
+    double twoH = 0.0;
+    bool wrap = false;
+    int64_t g = 0;
+    if constexpr (Geo) g = geo.base(ii);
+    else {
+        t = cf.target(i);
+        twoH = 2.0 * h[i];
+        wrap = cf.needsWrap(t, twoH);
+    }
+    double kx = 0.0, dxm = 0.0, dm = 0.0;
+    for (unsigned k = 0; k < no; ++k, g += 32) {
         bool mutual;
         const uint32_t j = ov.at(ii, k, mutual);
         double dist;
         double2 wv = make_double2(0.0, 0.0);
-        if (geo.g) {
-            const int64_t e = gb + 32 * int64_t(k);
-            dist = __ldg(geo.g + e).x;
-            wv = __ldg(geo.w + e);
+        if constexpr (Geo) {
+            dist = __ldg(geo.g + g).x;
+            wv = __ldg(geo.w + g);
         } else {
             double rx, ry, rz;
             cf.diffFast(t, j, twoH, wrap, rx, ry, rz);
@@ -909,42 +920,39 @@ __global__ void __launch_bounds__(kPairBlock) gradhOnceKernel(ListView lv, Owned
             dist = r2 * invDist(r2);
         }
         {
-            const double v = dist * hiInv;
-            const TabSlot sl = tabSlot(dist * hiInvDx);
-            const double w = geo.g ? wv.x : lookupX(tw, sl), dw = lookupX(tdw, sl);
-            const double dterh = -(3.0 * w + v * dw);
+            const double x = dist * hiInvDx;
+            const TabSlot sl = tabSlot(x);
+            const double w = Geo ? wv.x : lookupX(tw, sl), D = x * lookupX(tdw, sl);
             const double xmj = __ldg(xm + j);
-            kx += w * xmj;
-            whom += dterh * xmj;
-            wr0 += dterh * __ldg(m + j);
+            kx = fma(w, xmj, kx);
+            dxm = fma(D, xmj, dxm);
+            dm = fma(Geo ? D : fma(3.0 * kTabInvDx, w, D), __ldg(m + j), dm);
         }
         if (mutual) {
-            const double v = dist * __ldg(hInv + j);
-            const TabSlot sl = tabSlot(dist * __ldg(hInvDx + j));
-            const double w = geo.g ? wv.y : lookupX(tw, sl), dw = lookupX(tdw, sl);
-            const double dterh = -(3.0 * w + v * dw);
+            const double x = dist * __ldg(hInvDx + j);
+            const TabSlot sl = tabSlot(x);
+            const double w = Geo ? wv.y : lookupX(tw, sl), D = x * lookupX(tdw, sl);
             atomicAdd(acc + j, w * xmi);
-            atomicAdd(acc + n + j, dterh * xmi);
-            atomicAdd(acc + 2 * n + j, dterh * mi);
+            atomicAdd(acc + n + j, D * xmi);
+            atomicAdd(acc + 2 * n + j, (Geo ? D : fma(3.0 * kTabInvDx, w, D)) * mi);
         }
     }
     atomicAdd(acc + i, kx);
-    atomicAdd(acc + n + i, whom);
-    atomicAdd(acc + 2 * n + i, wr0);
+    atomicAdd(acc + n + i, dxm);
+    atomicAdd(acc + 2 * n + i, dm);
 }
 
-__global__ void gradhOnceFinish(int64_t first, int64_t last, int64_t n, const double* h, const double* m,
-                                const double* xm, double K, const double* acc, double* kxOut, double* gradhOut,
-                                double* tapeWom, double* tapeWr0)
+// kx and gradh of particle i from the sums of gradhOnceKernel (sums: the xmass pass's sum w m_j, or
+// null where that is part of the third sum)
+__device__ __forceinline__ void gradhEpilogue(int64_t i, int64_t n, double hi, double mi, double xmi, double K,
+                                              const double* acc, const double* sums, double* tapeWom, double* tapeWr0,
+                                              double& kxi, double& gradhi)
 {
-    const int64_t i = first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-    if (i >= last) return;
-    const double hi = h[i], mi = m[i], xmi = xm[i];
     const double hInv = 1.0 / hi, h3Inv = hInv * hInv * hInv;
-    double kxi = xmi + acc[i], whomega = -3.0 * xmi + acc[n + i], wrho0 = -3.0 * mi + acc[2 * n + i];
-    kxi *= K * h3Inv;
-    whomega *= K * h3Inv * hInv;
-    wrho0 *= K * h3Inv * hInv;
+    const double sx = acc[i], sm = sums ? sums[i] : 0.0;
+    kxi = (xmi + sx) * (K * h3Inv);
+    double whomega = fma(-kTabDx, acc[n + i], -3.0 * (xmi + sx)) * (K * h3Inv * hInv);
+    const double wrho0 = fma(-kTabDx, acc[2 * n + i], -3.0 * (mi + sm)) * (K * h3Inv * hInv);
     if (tapeWom) {
         tapeWom[i] = whomega;
         tapeWr0[i] = wrho0;
@@ -952,32 +960,32 @@ __global__ void gradhOnceFinish(int64_t first, int64_t last, int64_t n, const do
     whomega = whomega * mi / xmi + (kxi - K * xmi * h3Inv) * wrho0;
     const double rhoi = kxi * mi / xmi;
     const double dhdrho = -hi / (rhoi * 3.0);
+    gradhi = 1.0 - dhdrho * whomega;
+}
+
+__global__ void gradhOnceFinish(int64_t first, int64_t last, int64_t n, const double* h, const double* m,
+                                const double* xm, double K, const double* acc, const double* sums, double* kxOut,
+                                double* gradhOut, double* tapeWom, double* tapeWr0)
+{
+    const int64_t i = first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (i >= last) return;
+    double kxi, gradhi;
+    gradhEpilogue(i, n, h[i], m[i], xm[i], K, acc, sums, tapeWom, tapeWr0, kxi, gradhi);
     kxOut[i] = kxi;
-    gradhOut[i] = 1.0 - dhdrho * whomega;
+    gradhOut[i] = gradhi;
 }
 
 // the same epilogue fused with the EOS and the quotients of the later passes (inside a sweep)
 __global__ void gradhEosFinish(int64_t n, const double* h, const double* m, const double* xm, double K,
-                               const double* acc, double* kxOut, double* gradhOut, const double* u, double gamma,
-                               void* prho, void* c, void* rho, void* p, double* aux, double* tapeWom,
+                               const double* acc, const double* sums, double* kxOut, double* gradhOut, const double* u,
+                               double gamma, void* prho, void* c, void* rho, void* p, double* aux, double* tapeWom,
                                double* tapeWr0)
 {
     const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (i >= n) return;
-    const double hi = h[i], mi = m[i], xmi = xm[i];
-    const double hInv = 1.0 / hi, h3Inv = hInv * hInv * hInv;
-    double kxi = xmi + acc[i], whomega = -3.0 * xmi + acc[n + i], wrho0 = -3.0 * mi + acc[2 * n + i];
-    kxi *= K * h3Inv;
-    whomega *= K * h3Inv * hInv;
-    wrho0 *= K * h3Inv * hInv;
-    if (tapeWom) {
-        tapeWom[i] = whomega;
-        tapeWr0[i] = wrho0;
-    }
-    whomega = whomega * mi / xmi + (kxi - K * xmi * h3Inv) * wrho0;
-    const double rhoi = kxi * mi / xmi;
-    const double dhdrho = -hi / (rhoi * 3.0);
-    const double gradhi = 1.0 - dhdrho * whomega;
+    const double mi = m[i], xmi = xm[i];
+    double kxi, gradhi;
+    gradhEpilogue(i, n, h[i], mi, xmi, K, acc, sums, tapeWom, tapeWr0, kxi, gradhi);
     kxOut[i] = kxi;
     gradhOut[i] = gradhi;
     const double prhoi = eosVe<double>(i, u[i], mi, kxi, xmi, gradhi, gamma, prho, c, rho, p);
@@ -1096,7 +1104,10 @@ __global__ void iadOnceFinish(int64_t first, int64_t last, int64_t n, IadDivvArg
 // S_i = sum vol_j (divv_i - divv_j) W_i r (r = x_i - x_j; c_i is applied after the walk), j's term of
 // the same pair is vol_i (divv_i - divv_j) W_j r (r and the divv difference both change sign);
 // the signal-velocity candidate c_i + c_j - 3 (r.v) / |r| of approaching pairs is symmetric.
-template<bool Smooth>
+//
+// Bound by the FP64 pipe (13 instructions per mutual pair with the cache's w_ij, 17 with r . v and 1/|r|:
+// 15.7 -> 12.5 ms at 8M).  Geo: arrays of the pair-geometry cache (5, 2), or 0 to form the geometry.
+template<bool Smooth, int Geo>
 __global__ void __launch_bounds__(kPairBlock) avOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf, AvArgs a,
                                                             const double* hInv64, int64_t n, double* acc, PairGeo geo)
 {
@@ -1109,54 +1120,57 @@ __global__ void __launch_bounds__(kPairBlock) avOnceKernel(ListView lv, OwnedVie
     const double *vx = static_cast<const double*>(a.vx), *vy = static_cast<const double*>(a.vy),
                  *vz = static_cast<const double*>(a.vz), *c = static_cast<const double*>(a.c),
                  *divv = static_cast<const double*>(a.divv), *vol = static_cast<const double*>(a.vol);
-    auto t = cf.target(i);
-    const double hi = ld<double>(a.h, i), ci = c[i], divvi = divv[i], voli = vol[i];
-    const double vxi = vx[i], vyi = vy[i], vzi = vz[i], twoH = 2.0 * hi, hiInvDx = hInvDx[i];
-    const bool wrap = cf.needsWrap(t, twoH);
-    const int64_t gb = geo.base(ii);
+    const double ci = c[i], divvi = divv[i], voli = vol[i];
+    typename CoordFp64::Target t{};
+    double vxi = 0, vyi = 0, vzi = 0, twoH = 0, hiInvDx = 0;
+    bool wrap = false;
+    int64_t g = 0;
+    if constexpr (Geo != 0) g = geo.base(ii);
+    if constexpr (Geo != 5) {
+        t = cf.target(i);
+        twoH = 2.0 * ld<double>(a.h, i);
+        wrap = cf.needsWrap(t, twoH);
+        vxi = vx[i], vyi = vy[i], vzi = vz[i];
+        hiInvDx = hInvDx[i];
+    }
     double Sx = 0, Sy = 0, Sz = 0;
     long long vsigBits = 0;
     long long* accV = reinterpret_cast<long long*>(acc + 3 * n);
-    for (unsigned k = 0; k < no; ++k) {
+    for (unsigned k = 0; k < no; ++k, g += 32) {
         bool mutual;
         const uint32_t j = ov.at(ii, k, mutual);
-        double rx, ry, rz, rinv, dist, rv;
-        double2 wv = make_double2(0.0, 0.0);
-        if (geo.g) {
-            const int64_t e = gb + 32 * int64_t(k);
-            const double2 gd = __ldg(geo.g + e);
-            dist = gd.x;
-            rinv = gd.y;
-            wv = __ldg(geo.w + e);
-            if (geo.x) {  // v_i - v_j = -dv exactly
-                const double2 a0 = __ldg(geo.x + e), a1 = __ldg(geo.x + geo.plane + e),
-                              a2 = __ldg(geo.x + 2 * geo.plane + e);
-                rx = a0.x, ry = a0.y, rz = a1.x;
-                rv = fma(rz, -a2.y, fma(ry, -a2.x, rx * -a1.y));
-            } else {
-                cf.diffFast(t, j, twoH, wrap, rx, ry, rz);
-                rv = fma(rz, vzi - vz[j], fma(ry, vyi - vy[j], rx * (vxi - vx[j])));
-            }
+        double rx, ry, rz, wij;
+        double2 wv;
+        if constexpr (Geo != 0) {
+            wij = __ldg(geo.g + g).y;
+            wv = __ldg(geo.w + g);
+        }
+        if constexpr (Geo == 5) {
+            const double2 a0 = __ldg(geo.x + g);
+            rx = a0.x, ry = a0.y, rz = __ldg(geo.x + geo.plane + g).x;
         } else {
             cf.diffFast(t, j, twoH, wrap, rx, ry, rz);
-            const double r2 = dist2(rx, ry, rz);
-            rinv = invDist(r2);
-            dist = r2 * rinv;
-            rv = fma(rz, vzi - vz[j], fma(ry, vyi - vy[j], rx * (vxi - vx[j])));
         }
-        const bool approaching = negative(rv);
+        if constexpr (Geo == 0) {
+            const double r2 = dist2(rx, ry, rz);
+            const double rinv = invDist(r2), dist = r2 * rinv;
+            wij = fma(rz, vzi - vz[j], fma(ry, vyi - vy[j], rx * (vxi - vx[j]))) * rinv;
+            wv.x = lookupX(tabX, dist * hiInvDx);
+            wv.y = lookupX(tabX, dist * __ldg(hInvDx + j));
+        }
+        const bool approaching = negative(wij);
         double vs = 0.0;
         if (approaching) {
-            vs = fma(-3.0 * rv, rinv, ci + c[j]);
+            vs = fma(-3.0, wij, ci + c[j]);
             vsigBits = maxBitsNonNeg(vsigBits, vs);
         }
         const double dd = divvi - divv[j];
-        const double fw = vol[j] * dd * (geo.g ? wv.x : lookupX(tabX, dist * hiInvDx));
+        const double fw = vol[j] * dd * wv.x;
         Sx += fw * rx;
         Sy += fw * ry;
         Sz += fw * rz;
         if (mutual) {
-            const double fwj = voli * dd * (geo.g ? wv.y : lookupX(tabX, dist * __ldg(hInvDx + j)));
+            const double fwj = voli * dd * wv.y;
             atomicAdd(acc + j, fwj * rx);
             atomicAdd(acc + n + j, fwj * ry);
             atomicAdd(acc + 2 * n + j, fwj * rz);
@@ -1299,13 +1313,13 @@ __device__ __forceinline__ void atwoodWeights(const double* __restrict__ rho, co
 // integer maximum of non-negative bit patterns).
 //
 // Bound by the FP64 pipe (2 lanes per cycle and SM), so the pair terms are arranged for few FP64
-// instructions: 54 per mutual pair, 21 more on the Atwood ramp (atwoodWeights).  The sums are forces: with A = m h^-3 c at each end (per particle),
+// instructions: 50 per mutual pair, 21 more on the Atwood ramp (atwoodWeights).  The sums are forces: with A = m h^-3 c at each end (per particle),
 // w_i' = m_j w_i and w_j' = m_i w_j, hv = visc / 2, t = hv / rho, P_i = w_i' (prho_i am + t_i) and
 // P_j = w_j' (prho_j bm + t_j), both ends add the same V = P_i A_i r + P_j A_j r, with opposite signs,
 // and the same Q = t_i w_i' s_i + t_j w_j' s_j (s = v_ij . A r); the finishing kernel divides by the
 // particle's mass.  vsig is kept doubled, alpha divided by 8 (both exact).  With the per-pair exp and
 // divisions of the ramp and the terms factored by m_j and m_i the kernel ran 109 FP64 instructions per
-// pair: 89.8 ms at 8M (jittered Sedov), now 82 and 65.2 ms, the FP64 pipe 87 % busy in both.
+// pair: 89.8 ms at 8M (jittered Sedov), now 78 and 62.1 ms, the FP64 pipe 87 % busy.
 // Geo: arrays of the pair-geometry cache to read (5, 2), or 0 to form the geometry here.
 template<bool Smooth, int Geo>
 __global__ void __launch_bounds__(kPairBlock) meVeOnceKernel(ListView lv, CoordFp64 cf, MeVeArgs a, PairGeo geo)
@@ -1346,10 +1360,10 @@ __global__ void __launch_bounds__(kPairBlock) meVeOnceKernel(ListView lv, CoordF
         const Rec4d j0 = ldRec4d(a.rec64 + 3 * int64_t(j)), j1 = ldRec4d(a.rec64 + 3 * int64_t(j) + 1),
                     j2 = ldRec4d(a.rec64 + 3 * int64_t(j) + 2);
         const float rhofj = __ldg(a.rhof + j);
-        T rx, ry, rz, rinv, Wi, Wj, vxij, vyij, vzij;
+        T rx, ry, rz, wij, Wi, Wj, vxij, vyij, vzij;
         if constexpr (Geo != 0) {
             const double2 wv = __ldg(geo.w + g);
-            rinv = __ldg(geo.g + g).y;
+            wij = __ldg(geo.g + g).y;
             Wi = j1.v[3] * wv.x;
             Wj = i1.v[3] * wv.y;
         }
@@ -1363,8 +1377,9 @@ __global__ void __launch_bounds__(kPairBlock) meVeOnceKernel(ListView lv, CoordF
         }
         if constexpr (Geo == 0) {
             const T r2 = dist2(rx, ry, rz);
-            rinv = invDist(r2);
+            const T rinv = invDist(r2);
             const T dist = r2 * rinv;
+            wij = fma(rz, vzij, fma(ry, vyij, rx * vxij)) * rinv;
             Wi = j1.v[3] * lookupX(tabX, dist * hiInvDx);
             Wj = i1.v[3] * lookupX(tabX, dist * __ldg(hInvDx + j));
         }
@@ -1374,7 +1389,6 @@ __global__ void __launch_bounds__(kPairBlock) meVeOnceKernel(ListView lv, CoordF
         const T gjx = j0.v[0] * rx + j0.v[1] * ry + j0.v[2] * rz;
         const T gjy = j0.v[1] * rx + j0.v[3] * ry + j1.v[0] * rz;
         const T gjz = j0.v[2] * rx + j1.v[0] * ry + j1.v[1] * rz;
-        const T wij = fma(rz, vzij, fma(ry, vyij, rx * vxij)) * rinv;
         const T cs = i1.v[2] + j1.v[2];
         const T vsig2 = fma(T(-4), wij, cs);  // twice the reference's 0.5 (c_i + c_j) - 2 w_ij
         maxvBits = maxBitsNonNeg(maxvBits, vsig2);
@@ -1460,26 +1474,32 @@ int passGradh(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last)
         const int64_t n = p->n;
         SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * 3 * size_t(n)));
         SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * 3 * size_t(n), c->stream));
+        const PairGeo geo = pairGeoRead(c);
+        const double* sums = geo.g ? c->rho0Sum.as<double>() : nullptr;
         SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
             constexpr bool S = decltype(smooth)::value;
-            gradhOnceKernel<S><<<blocks, kPairBlock, 0, c->stream>>>(
-                lv, ownedView(c), coordFp64(c, p), static_cast<const double*>(p->h), static_cast<const double*>(p->m),
-                static_cast<const double*>(p->xm), KTab<S>{tabW64(c)}, KTab<S>{tabDW64(c)}, c->hInv64.as<double>(),
-                n, c->pairAcc.as<double>(), pairGeoRead(c));
+            auto run = [&](auto kernel) {
+                kernel<<<blocks, kPairBlock, 0, c->stream>>>(
+                    lv, ownedView(c), coordFp64(c, p), static_cast<const double*>(p->h),
+                    static_cast<const double*>(p->m), static_cast<const double*>(p->xm), KTab<S>{tabW64(c)},
+                    KTab<S>{tabDW64(c)}, c->hInv64.as<double>(), n, c->pairAcc.as<double>(), geo);
+            };
+            if (geo.g) run(gradhOnceKernel<S, true>);
+            else run(gradhOnceKernel<S, false>);
             return launched(c, "gradhOnceKernel");
         }));
         if (c->inSweep && p->u && p->prho && p->c) {  // EOS and quotients fused into the epilogue
             SPHGB_TRY(c->aux.ensure(sizeof(double) * 6 * n));
             gradhEosFinish<<<gridFor(n, 256), 256, 0, c->stream>>>(
                 n, static_cast<const double*>(p->h), static_cast<const double*>(p->m), static_cast<const double*>(p->xm),
-                c->K, c->pairAcc.as<double>(), static_cast<double*>(p->kx), static_cast<double*>(p->gradh), p->u,
+                c->K, c->pairAcc.as<double>(), sums, static_cast<double*>(p->kx), static_cast<double*>(p->gradh), p->u,
                 c->prm.gamma, p->prho, p->c, p->rho, p->p, c->aux.as<double>(), tWom, tWr0);
             c->eosFused = c->auxReady = true;
             return launched(c, "gradhEosFinish");
         }
         gradhOnceFinish<<<gridFor(last - first, 256), 256, 0, c->stream>>>(
             first, last, n, static_cast<const double*>(p->h), static_cast<const double*>(p->m),
-            static_cast<const double*>(p->xm), c->K, c->pairAcc.as<double>(), static_cast<double*>(p->kx),
+            static_cast<const double*>(p->xm), c->K, c->pairAcc.as<double>(), sums, static_cast<double*>(p->kx),
             static_cast<double*>(p->gradh), tWom, tWr0);
         return launched(c, "gradhOnceFinish");
     }
@@ -1657,9 +1677,15 @@ int passAVswitches(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last
         SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * 4 * size_t(n)));
         SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * 4 * size_t(n), c->stream));
         SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
-            avOnceKernel<decltype(smooth)::value><<<blocks, kPairBlock, 0, c->stream>>>(
-                lv, ownedView(c), coordFp64(c, p), a, c->hInv64.as<double>(), n, c->pairAcc.as<double>(),
-                pairGeoRead(c));
+            constexpr bool S = decltype(smooth)::value;
+            const PairGeo geo = pairGeoRead(c);
+            auto run = [&](auto kernel) {
+                kernel<<<blocks, kPairBlock, 0, c->stream>>>(lv, ownedView(c), coordFp64(c, p), a,
+                                                             c->hInv64.as<double>(), n, c->pairAcc.as<double>(), geo);
+            };
+            if (geo.x) run(avOnceKernel<S, 5>);
+            else if (geo.g) run(avOnceKernel<S, 2>);
+            else run(avOnceKernel<S, 0>);
             return launched(c, "avOnceKernel");
         }));
         avOnceFinish<<<gridFor(last - first, 256), 256, 0, c->stream>>>(first, last, n, a, c->pairAcc.as<double>());

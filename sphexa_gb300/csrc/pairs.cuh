@@ -125,16 +125,16 @@ inline bool pairOnce(const sphgb_ctx* c, const sphgb_particles* p, int64_t first
 }
 
 // ---- pair geometry shared by the pair-once passes of one sweep ----
-// Inside one sweep positions, velocities and h stay put, so an owned entry's |r| and 1/|r| (the FP64
-// difference, its square and the reciprocal square root: about a dozen FP64-pipe instructions), the
-// kernel function at both ends, w(|r| / h_i) and w(|r| / h_j), and, where the memory is there, the
-// difference vector r = x_i - x_j and the velocity difference dv = v_j - v_i are formed once by the
-// xmass pass and loaded by gradh, IAD, AV and momentum-energy.  Layout: the 32 targets of a warp own
+// Inside one sweep positions, velocities and h stay put, so an owned entry's |r| (the FP64 difference,
+// its square and the reciprocal square root: about a dozen FP64-pipe instructions), the approach
+// velocity w_ij = r . v_ij / |r|, the kernel function at both ends, w(|r| / h_i) and w(|r| / h_j), and,
+// where the memory is there, the difference vector r = x_i - x_j and the velocity difference dv =
+// v_j - v_i are formed once by the xmass pass and loaded by gradh, IAD, AV and momentum-energy.  Layout: the 32 targets of a warp own
 // rows rowOff[w] .. rowOff[w] + (their longest owned list) - 1, a row holding entry k of all 32 side
 // by side, so a warp reads 512 contiguous bytes per entry and array.
 struct PairGeo {
     const uint32_t* rowOff;  // first row of each warp of 32 targets
-    double2* g;              // {|r|, 1/|r|}; null: the pass forms the geometry itself
+    double2* g;              // {|r|, w_ij}; null: the pass forms the geometry itself
     double2* w;              // {w(|r| / h_i), w(|r| / h_j)}
     double2* x;              // {rx, ry}, {rz, dvx}, {dvy, dvz} at x, x + plane, x + 2 plane; or null
     int64_t plane;           // entries per array
