@@ -517,8 +517,10 @@ __global__ void exportKernel(const uint32_t* __restrict__ nbr, const uint32_t* _
 // the margin or crossing a periodic face take the exact FP64 test.
 // i owns every non-mutual entry and half of its mutual ones: the mutual pair {i, j} belongs to the
 // smaller index when i + j is odd and to the larger when it is even, so each particle owns about
-// half of its mutual pairs wherever it sits in the SFC order.  The owned entries are written
-// compacted in the granule layout of the lists, entry = j | mutual << 31, with their count per particle.
+// half of its mutual pairs wherever it sits in the SFC order; pairs within one warp of 32 targets
+// (about 25 of a particle's 96) go to whichever end owns fewer (ownWithinWarp).  The owned entries are
+// written compacted in the granule layout of the lists, entry = j | mutual << 31, the warp's own
+// pairs last, with their count per particle.
 struct MutualArgs {
     const double *x, *y, *z;
     const void* h;
@@ -622,41 +624,91 @@ __device__ bool mutualPair(const MutualArgs& a, int64_t i, int ci[3], float4 li,
     return mutualExact(a, i, j, loadH(a.h, a.hIsFloat, j));
 }
 
+// the lanes among `intra` (the lane's mutual neighbours within its warp) that this lane owns: every
+// pair of lanes meets in one of 31 steps and goes to the lane that owns fewer entries so far (on a tie
+// by index parity).  The pair-once passes walk a warp's owned lists in step, so they take as long as
+// the longest of the 32: with the parity rule alone that was 55 entries against a mean of 48.
+__device__ __forceinline__ unsigned ownWithinWarp(unsigned intra, unsigned cnt, int lane)
+{
+    unsigned own = 0;
+#pragma unroll 1
+    for (int s = 1; s < kWarp; ++s) {
+        const int p = lane ^ s;
+        const unsigned theirs = __shfl_xor_sync(0xffffffffu, intra, s), theirCnt = __shfl_xor_sync(0xffffffffu, cnt, s);
+        const bool odd = (s & 1) != 0, lower = lane < p;
+        if ((intra >> p) & (theirs >> lane) & 1u) {
+            const bool take = cnt < theirCnt || (cnt == theirCnt && odd == lower);
+            own |= unsigned(take) << p;
+            cnt += take;
+        }
+    }
+    return own;
+}
+
+// one target's owned list: entries are offered in list order; mutual ones within the warp are kept
+// back until the warp has shared them out in finish()
+struct OwnedWriter {
+    GranuleWriter out;
+    int64_t ii, first;
+    unsigned cnt = 0, intra = 0;
+    __device__ __forceinline__ OwnedWriter(uint32_t* base, int64_t ii_, int64_t first_, int64_t stride, uint32_t ngmax)
+        : out(base, ii_, stride, ngmax), ii(ii_), first(first_)
+    {
+    }
+    __device__ __forceinline__ void offer(uint32_t j, bool mutual)
+    {
+        const int64_t jj = int64_t(j) - first;
+        if (mutual && (jj >> 5) == (ii >> 5)) {
+            intra |= 1u << (jj & 31);
+            return;
+        }
+        const bool own = !mutual || ((((ii ^ jj) & 1) != 0) == (ii < jj));
+        if (own) out.put(cnt++, j | (mutual ? 0x80000000u : 0u));
+    }
+    // all 32 lanes of the warp together
+    __device__ __forceinline__ unsigned finish()
+    {
+        unsigned own = ownWithinWarp(intra, cnt, int(ii & 31));
+        const uint32_t base = uint32_t(first + (ii & ~int64_t(31)));
+        for (; own != 0; own &= own - 1u) out.put(cnt++, (base + unsigned(__ffs(own) - 1)) | 0x80000000u);
+        out.finish(cnt);
+        return cnt;
+    }
+};
+
 __global__ void __launch_bounds__(128) ownedListKernel(MutualArgs a)
 {
     const int64_t i = a.first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-    if (i >= a.last) return;
+    const bool valid = i < a.last;
     const int64_t ii = i - a.first;
-    const unsigned nc = min(__ldg(a.count + ii), a.ngmax);
-    int ci[3];
-    unpackCell(__ldg(a.cell + i), ci);
-    const float4 li = __ldg(a.loc + i);
-    unsigned cnt = 0;
-    GranuleWriter out(a.owned, ii, a.stride, a.ngmax);
-    for (unsigned k = 0; k < nc; ++k) {
-        const uint32_t j = __ldg(a.nbr + listSlot(ii, k, a.stride));
-        const bool m = mutualPair(a, i, ci, li, j);
-        const bool own = !m || ((((i ^ int64_t(j)) & 1) != 0) == (i < int64_t(j)));
-        if (own) out.put(cnt++, j | (m ? 0x80000000u : 0u));
+    OwnedWriter w(a.owned, ii, a.first, a.stride, a.ngmax);
+    if (valid) {
+        const unsigned nc = min(__ldg(a.count + ii), a.ngmax);
+        int ci[3];
+        unpackCell(__ldg(a.cell + i), ci);
+        const float4 li = __ldg(a.loc + i);
+        for (unsigned k = 0; k < nc; ++k) {
+            const uint32_t j = __ldg(a.nbr + listSlot(ii, k, a.stride));
+            w.offer(j, mutualPair(a, i, ci, li, j));
+        }
     }
-    out.finish(cnt);
-    a.ownedCount[ii] = cnt;
+    const unsigned cnt = w.finish();
+    if (valid) a.ownedCount[ii] = cnt;
 }
 
 // owned lists from list membership alone: (i, j) is mutual when i is in j's (capped, ascending)
 // list, found by binary search, so the decision holds whatever the positions are now (frozen lists
-// after moved particles).  Ownership of a mutual pair as in ownedListKernel (index parity).
+// after moved particles).  Ownership of a mutual pair as in ownedListKernel.
 __global__ void __launch_bounds__(128) ownedByListKernel(const uint32_t* __restrict__ nbr,
                                                          const uint32_t* __restrict__ count, int64_t first, int64_t last,
                                                          int64_t stride, uint32_t ngmax, uint32_t* __restrict__ owned,
                                                          uint32_t* __restrict__ ownedCount)
 {
     const int64_t i = first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-    if (i >= last) return;
+    const bool valid = i < last;
     const int64_t ii = i - first;
-    const unsigned nc = min(__ldg(count + ii), ngmax);
-    unsigned cnt = 0;
-    GranuleWriter out(owned, ii, stride, ngmax);
+    const unsigned nc = valid ? min(__ldg(count + ii), ngmax) : 0u;
+    OwnedWriter w(owned, ii, first, stride, ngmax);
     for (unsigned k = 0; k < nc; ++k) {
         const uint32_t j = __ldg(nbr + listSlot(ii, k, stride));
         bool m = false;
@@ -671,11 +723,10 @@ __global__ void __launch_bounds__(128) ownedByListKernel(const uint32_t* __restr
             }
             m = lo < min(__ldg(count + jj), ngmax) && int64_t(__ldg(nbr + listSlot(jj, lo, stride))) == i;
         }
-        const bool own = !m || ((((i ^ int64_t(j)) & 1) != 0) == (i < int64_t(j)));
-        if (own) out.put(cnt++, j | (m ? 0x80000000u : 0u));
+        w.offer(j, m);
     }
-    out.finish(cnt);
-    ownedCount[ii] = cnt;
+    const unsigned cnt = w.finish();
+    if (valid) ownedCount[ii] = cnt;
 }
 
 // longest owned list of each warp of 32 targets
