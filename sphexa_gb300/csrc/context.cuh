@@ -152,7 +152,7 @@ struct sphgb_ctx {
     sphgb::DBuf whS64, whdS64;
     bool smoothKernel = false;
     sphgb::DBuf whx32;  // FP32 linear table (the mixed adjoint)
-    // e^(k/1024), e^(-k/1024), k/1024, |k| <= kExpNodes (the Atwood ramp of the pair-once passes)
+    // e^(k/1024), e^(-k/1024), k/1024, |k| <= kExpNodes, then e^-n (the pair-once momentum-energy pass)
     sphgb::DBuf expTab;
     sphgb::DBuf whH32, whdH32;  // mixed passes: cubic pieces of W and dW/dv (kHermIntervals float4)
 

@@ -1208,7 +1208,9 @@ __global__ void avOnceFinish(int64_t first, int64_t last, int64_t n, AvArgs a, c
 
 // neighbour-side fields of the pair-once momentum-energy pass, 96 bytes per particle in three 32-byte
 // loads: A = m h^-3 c_ab (six entries), c, m, prho, 1/rho, xm, alpha / 8; and rho in FP32.  m and
-// h^-3 enter every use of c, so they are folded in once per particle instead of per pair.
+// h^-3 enter every use of c, so they are folded in once per particle instead of per pair.  With the
+// viscosity cleaning two more: the symmetric velocity gradient (six entries), 1/h, and eta_crit of the
+// particle's neighbour count (momentum_energy_kern.hpp:43-63).
 struct alignas(32) Rec4d {
     double v[4];
 };
@@ -1221,10 +1223,11 @@ __device__ __forceinline__ Rec4d ldRec4d(const Rec4d* p)
 }
 
 // Aux: also forms the quotients rho, ln xm and 1/rho (outside a sweep, which has them already)
-template<bool Aux>
-__global__ void meVeRec64Kernel(int64_t n, MeVeArgs a, double* __restrict__ aux, Rec4d* __restrict__ rec,
+template<bool Aux, bool AvClean>
+__global__ void meVeRec64Kernel(int64_t n, MeVeArgs a, ListView lv, double* __restrict__ aux, Rec4d* __restrict__ rec,
                                 float* __restrict__ rhof)
 {
+    constexpr int R = AvClean ? 5 : 3;
     const int64_t j = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (j >= n) return;
     const double m = ld<double>(a.m, j), xm = ld<double>(a.xm, j), f = m * a.hInv64[n + j];
@@ -1238,9 +1241,15 @@ __global__ void meVeRec64Kernel(int64_t n, MeVeArgs a, double* __restrict__ aux,
         rho = aux[j];
         rhoInv = aux[5 * n + j];
     }
-    rec[3 * j] = {f * ld<double>(a.c11, j), f * ld<double>(a.c12, j), f * ld<double>(a.c13, j), f * ld<double>(a.c22, j)};
-    rec[3 * j + 1] = {f * ld<double>(a.c23, j), f * ld<double>(a.c33, j), ld<double>(a.c, j), m};
-    rec[3 * j + 2] = {ld<double>(a.prho, j), rhoInv, xm, 0.125 * ld<double>(a.alpha, j)};
+    rec[R * j] = {f * ld<double>(a.c11, j), f * ld<double>(a.c12, j), f * ld<double>(a.c13, j), f * ld<double>(a.c22, j)};
+    rec[R * j + 1] = {f * ld<double>(a.c23, j), f * ld<double>(a.c33, j), ld<double>(a.c, j), m};
+    rec[R * j + 2] = {ld<double>(a.prho, j), rhoInv, xm, 0.125 * ld<double>(a.alpha, j)};
+    if constexpr (AvClean) {
+        const unsigned nc = lv.capped(j - lv.first);
+        rec[R * j + 3] = {ld<double>(a.dV11, j), ld<double>(a.dV12, j), ld<double>(a.dV13, j), ld<double>(a.dV22, j)};
+        rec[R * j + 4] = {ld<double>(a.dV23, j), ld<double>(a.dV33, j), a.hInv64[j],
+                          cbrt(32.0 * M_PI / 3.0 / double(nc + 1))};
+    }
     rhof[j] = float(rho);
 }
 
@@ -1303,6 +1312,47 @@ __device__ __forceinline__ void atwoodWeights(const double* __restrict__ rho, co
     bm *= fma(e.y, even - odd, e.y);
 }
 
+// num / den by a 20-bit reciprocal and two Newton corrections of the quotient (five FP64 instructions,
+// within an ulp); den beyond 2^+-1000 takes the division
+__device__ __forceinline__ double quotient(double num, double den)
+{
+    const unsigned e = (unsigned(__double2hiint(den)) >> 20) & 0x7ffu;
+    if (e - 23u > 2000u) return num / den;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(den));
+    double q = num * y;
+    q = fma(fma(-den, q, num), y, q);
+    return fma(fma(-den, q, num), y, q);
+}
+
+// e^-x for x >= 0: below 16 from e^-n, n = round(x), and the table of e^(k/1024) (x reaches 16 only with
+// a handful of neighbours)
+__device__ __forceinline__ double expNegSmall(double x, const double4* __restrict__ expTab)
+{
+    if (!(x < 16.0)) return exp(-x);
+    const int n = __float2int_rn(float(x));
+    const double4 en = expTab[2 * kExpNodes + 1 + n];  // e^-n, -, n
+    const double a = en.z - x;                         // |a| <= 1/2
+    const int k = __float2int_rn(float(a) * 1024.f);
+    const double4 e = expTab[kExpNodes + k];
+    const double r = a - e.z, r2 = r * r;
+    const double y = fma(r2, fma(r2, 1.0 / 24.0, fma(r, 1.0 / 6.0, 0.5)), r);
+    return en.x * fma(e.x, y, e.x);
+}
+
+// avRvCorrection (hydro_ve/momentum_energy_kern.hpp:43-63) over |r|, without d3: with d1 and d2 the
+// velocity gradients' quadratic forms at both ends and A = d1 / d2, the limiter 4 A / (1 + A)^2 lies in
+// [0, 1] for A >= 0 and is cut to 0 below, so that -phi (d1 + d2) = -d3 2 d1 d2 / (d1 + d2) where d1 and
+// d2 have one sign, else 0: one quotient instead of two divisions, shared by the two ends.
+__device__ __forceinline__ double avRvShared(double d1, double d2, double dist)
+{
+    const long long b1 = __double_as_longlong(d1), b2 = __double_as_longlong(d2);
+    constexpr long long inf = 0x7ff0000000000000LL, mag = 0x7fffffffffffffffLL;
+    const bool finite = (b1 & mag) < inf && (b2 & mag) < inf;
+    if (finite && ((b1 ^ b2) < 0 || (b1 & mag) == 0 || (b2 & mag) == 0)) return 0.0;
+    return 2.0 * d1 * quotient(d2, (d1 + d2) * dist);
+}
+
 // FP64 VE momentum-energy with one evaluation per mutual pair, for lists that cover every particle.
 // i walks its owned list: every pair of its list that j does not list back, and half of the
 // mutual pairs (the other half is in the owned lists of the other ends).  The two ends' terms follow from one
@@ -1320,8 +1370,12 @@ __device__ __forceinline__ void atwoodWeights(const double* __restrict__ rho, co
 // particle's mass.  vsig is kept doubled, alpha divided by 8 (both exact).  With the per-pair exp and
 // divisions of the ramp and the terms factored by m_j and m_i the kernel ran 109 FP64 instructions per
 // pair: 89.8 ms at 8M (jittered Sedov), now 78 and 62.1 ms, the FP64 pipe 87 % busy.
+// AvClean: the cleaned approach velocity differs between the ends by d3, the cut-off of close pairs at
+// the owner's eta_crit (a few per cent of the pairs), so the viscous terms of the neighbour's end are
+// formed again where it does; everything else is shared.  300k-particle sphere: 12.1 ms with every
+// directed pair evaluated, now 4.3 ms.
 // Geo: arrays of the pair-geometry cache to read (5, 2), or 0 to form the geometry here.
-template<bool Smooth, int Geo>
+template<bool AvClean, bool Smooth, int Geo>
 __global__ void __launch_bounds__(kPairBlock) meVeOnceKernel(ListView lv, CoordFp64 cf, MeVeArgs a, PairGeo geo)
 {
     using T = double;
@@ -1334,7 +1388,10 @@ __global__ void __launch_bounds__(kPairBlock) meVeOnceKernel(ListView lv, CoordF
     const double* hInvDx = a.hInv64 + 2 * a.n;
     const T *vxA = static_cast<const T*>(a.vx), *vyA = static_cast<const T*>(a.vy), *vzA = static_cast<const T*>(a.vz);
 
-    const Rec4d i0 = a.rec64[3 * i], i1 = a.rec64[3 * i + 1], i2 = a.rec64[3 * i + 2];
+    constexpr int R = AvClean ? 5 : 3;
+    const Rec4d i0 = a.rec64[R * i], i1 = a.rec64[R * i + 1], i2 = a.rec64[R * i + 2];
+    Rec4d i3{}, i4{};
+    if constexpr (AvClean) i3 = a.rec64[R * i + 3], i4 = a.rec64[R * i + 4];
     const float rhofi = a.rhof[i];
     typename CoordFp64::Target t{};
     T vxi = 0, vyi = 0, vzi = 0, hiInvDx = 0, twoH = 0;
@@ -1357,13 +1414,14 @@ __global__ void __launch_bounds__(kPairBlock) meVeOnceKernel(ListView lv, CoordF
         const uint32_t e = __ldg(a.owned + listSlot(ii, k, lv.stride));
         const uint32_t j = e & 0x7fffffffu;
         const bool mutual = (e >> 31) != 0;
-        const Rec4d j0 = ldRec4d(a.rec64 + 3 * int64_t(j)), j1 = ldRec4d(a.rec64 + 3 * int64_t(j) + 1),
-                    j2 = ldRec4d(a.rec64 + 3 * int64_t(j) + 2);
+        const Rec4d* recj = a.rec64 + R * int64_t(j);
+        const Rec4d j0 = ldRec4d(recj), j1 = ldRec4d(recj + 1), j2 = ldRec4d(recj + 2);
         const float rhofj = __ldg(a.rhof + j);
-        T rx, ry, rz, wij, Wi, Wj, vxij, vyij, vzij;
+        T rx, ry, rz, dist, wij, Wi, Wj, vxij, vyij, vzij;
         if constexpr (Geo != 0) {
-            const double2 wv = __ldg(geo.w + g);
-            wij = __ldg(geo.g + g).y;
+            const double2 wv = __ldg(geo.w + g), gd = __ldg(geo.g + g);
+            dist = gd.x;
+            wij = gd.y;
             Wi = j1.v[3] * wv.x;
             Wj = i1.v[3] * wv.y;
         }
@@ -1378,7 +1436,7 @@ __global__ void __launch_bounds__(kPairBlock) meVeOnceKernel(ListView lv, CoordF
         if constexpr (Geo == 0) {
             const T r2 = dist2(rx, ry, rz);
             const T rinv = invDist(r2);
-            const T dist = r2 * rinv;
+            dist = r2 * rinv;
             wij = fma(rz, vzij, fma(ry, vyij, rx * vxij)) * rinv;
             Wi = j1.v[3] * lookupX(tabX, dist * hiInvDx);
             Wj = i1.v[3] * lookupX(tabX, dist * __ldg(hInvDx + j));
@@ -1389,33 +1447,65 @@ __global__ void __launch_bounds__(kPairBlock) meVeOnceKernel(ListView lv, CoordF
         const T gjx = j0.v[0] * rx + j0.v[1] * ry + j0.v[2] * rz;
         const T gjy = j0.v[1] * rx + j0.v[3] * ry + j1.v[0] * rz;
         const T gjz = j0.v[2] * rx + j1.v[0] * ry + j1.v[1] * rz;
+        T wji = wij;  // the approach velocity as j's directed term sees it
+        if constexpr (AvClean) {
+            const Rec4d j3 = ldRec4d(recj + 3), j4 = ldRec4d(recj + 4);
+            const T gi[6] = {i3.v[0], i3.v[1], i3.v[2], i3.v[3], i4.v[0], i4.v[1]};
+            const T gj[6] = {j3.v[0], j3.v[1], j3.v[2], j3.v[3], j4.v[0], j4.v[1]};
+            const T share = avRvShared(quadForm(rx, ry, rz, gi), quadForm(rx, ry, rz, gj), dist);
+            const T eta = dist * (lessNonNeg(j4.v[2], i4.v[2]) ? j4.v[2] : i4.v[2]);  // min of |r|/h
+            T ci = share, cj = share;
+            if (lessNonNeg(eta, i4.v[3])) {
+                const T e = 5.0 * (eta - i4.v[3]);
+                ci *= expNegSmall(e * e, a.expTab);
+            }
+            if (lessNonNeg(eta, j4.v[3])) {
+                const T e = 5.0 * (eta - j4.v[3]);
+                cj *= expNegSmall(e * e, a.expTab);
+            }
+            wji = wij - cj;
+            wij = wij - ci;
+        }
         const T cs = i1.v[2] + j1.v[2];
         const T vsig2 = fma(T(-4), wij, cs);  // twice the reference's 0.5 (c_i + c_j) - 2 w_ij
         maxvBits = maxBitsNonNeg(maxvBits, vsig2);
         T am, bm;
         atwoodWeights(aux, aux + 4 * a.n, a.expTab, i, j, rhofi, rhofj, i2.v[2], j2.v[2], am, bm);
         const T wsi = Wi * (vxij * gix + vyij * giy + vzij * giz), wsj = Wj * (vxij * gjx + vyij * gjy + vzij * gjz);
-        T ti = 0, tj = 0, Q = 0;
-        if (negative(wij)) {  // approaching: hv = -((alpha_i + alpha_j) / 8 (c_i + c_j) - w_ij) w_ij
-            const T hv = fma(i2.v[3] + j2.v[3], cs, -wij) * -wij;
-            ti = i2.v[1] * hv;
-            tj = j2.v[1] * hv;
-            Q = fma(ti, wsi, tj * wsj);
-        }
-        const T Pi = Wi * fma(i2.v[0], am, ti), Pj = Wj * fma(j2.v[0], bm, tj);
-        const T Vx = fma(Pi, gix, Pj * gjx), Vy = fma(Pi, giy, Pj * gjy), Vz = fma(Pi, giz, Pj * gjz);
+        // V and Q of the directed term that sees the approach velocity w
+        T Vx, Vy, Vz, Q;
+        auto terms = [&](T w) {
+            T ti = 0, tj = 0;
+            Q = 0;
+            if (negative(w)) {  // approaching: hv = -((alpha_i + alpha_j) / 8 (c_i + c_j) - w) w
+                const T hv = fma(i2.v[3] + j2.v[3], cs, -w) * -w;
+                ti = i2.v[1] * hv;
+                tj = j2.v[1] * hv;
+                Q = fma(ti, wsi, tj * wsj);
+            }
+            const T Pi = Wi * fma(i2.v[0], am, ti), Pj = Wj * fma(j2.v[0], bm, tj);
+            Vx = fma(Pi, gix, Pj * gjx), Vy = fma(Pi, giy, Pj * gjy), Vz = fma(Pi, giz, Pj * gjz);
+        };
+        terms(wij);
         mx -= Vx;
         my -= Vy;
         mz -= Vz;
         en = fma(-am, wsi, en);
         avE -= Q;
         if (mutual) {
+            T vsigj = vsig2;
+            if constexpr (AvClean) {
+                if (__double_as_longlong(wji) != __double_as_longlong(wij)) {
+                    terms(wji);
+                    vsigj = fma(T(-4), wji, cs);
+                }
+            }
             atomicAdd(accX + j, Vx);
             atomicAdd(accY + j, Vy);
             atomicAdd(accZ + j, Vz);
             atomicAdd(accE + j, -bm * wsj);
             atomicAdd(accV + j, -Q);
-            atomicMax(accS + j, __double_as_longlong(vsig2));
+            atomicMax(accS + j, __double_as_longlong(vsigj));
         }
     }
     atomicAdd(accX + i, mx);
@@ -1712,7 +1802,7 @@ int passMomentumEnergyVe(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_
     SPHGB_TRY(checkPass(c, p, first, last));
     const bool mixed = p->precision == SPHGB_MIXED;
     // one evaluation per mutual pair when the lists cover all particles and the order may vary
-    const bool once = !mixed && !avClean && pairOnce(c, p, first, last);
+    const bool once = !mixed && pairOnce(c, p, first, last);
     if (once) SPHGB_TRY(c->aux.ensure(sizeof(double) * 6 * size_t(p->n)));
     else SPHGB_TRY(launchVeAux<kAuxMe>(c, p));
     ListView lv = listView(c);
@@ -1779,15 +1869,15 @@ int passMomentumEnergyVe(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_
             a.owned = c->owned.as<uint32_t>();
             a.ownedCount = c->ownedCount.as<uint32_t>();
             a.acc = c->pairAcc.as<double>();
-            SPHGB_TRY(c->pack.ensure(sizeof(Rec4d) * 3 * size_t(p->n)));
+            SPHGB_TRY(c->pack.ensure(sizeof(Rec4d) * (avClean ? 5 : 3) * size_t(p->n)));
             SPHGB_TRY(c->rhof.ensure(sizeof(float) * size_t(p->n)));
-            const unsigned rb = gridFor(p->n, 256);
-            if (c->inSweep && c->auxReady)
-                meVeRec64Kernel<false><<<rb, 256, 0, c->stream>>>(p->n, a, c->aux.as<double>(), c->pack.as<Rec4d>(),
+            const bool haveAux = c->inSweep && c->auxReady;
+            auto records = [&](auto kernel) {
+                kernel<<<gridFor(p->n, 256), 256, 0, c->stream>>>(p->n, a, lv, c->aux.as<double>(), c->pack.as<Rec4d>(),
                                                                   c->rhof.as<float>());
-            else
-                meVeRec64Kernel<true><<<rb, 256, 0, c->stream>>>(p->n, a, c->aux.as<double>(), c->pack.as<Rec4d>(),
-                                                                 c->rhof.as<float>());
+            };
+            if (avClean) haveAux ? records(meVeRec64Kernel<false, true>) : records(meVeRec64Kernel<true, true>);
+            else haveAux ? records(meVeRec64Kernel<false, false>) : records(meVeRec64Kernel<true, false>);
             SPHGB_TRY(launched(c, "meVeRec64Kernel"));
             a.rec64 = c->pack.as<Rec4d>();
             a.rhof = c->rhof.as<float>();
@@ -1795,9 +1885,16 @@ int passMomentumEnergyVe(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_
             const PairGeo geo = pairGeoRead(c);
             SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
                 constexpr bool S = decltype(smooth)::value;
-                if (geo.x) meVeOnceKernel<S, 5><<<blocks, kPairBlock, 0, c->stream>>>(lv, cf, a, geo);
-                else if (geo.g) meVeOnceKernel<S, 2><<<blocks, kPairBlock, 0, c->stream>>>(lv, cf, a, geo);
-                else meVeOnceKernel<S, 0><<<blocks, kPairBlock, 0, c->stream>>>(lv, cf, a, geo);
+                auto run = [&](auto kernel) { kernel<<<blocks, kPairBlock, 0, c->stream>>>(lv, cf, a, geo); };
+                if (avClean) {
+                    if (geo.x) run(meVeOnceKernel<true, S, 5>);
+                    else if (geo.g) run(meVeOnceKernel<true, S, 2>);
+                    else run(meVeOnceKernel<true, S, 0>);
+                } else {
+                    if (geo.x) run(meVeOnceKernel<false, S, 5>);
+                    else if (geo.g) run(meVeOnceKernel<false, S, 2>);
+                    else run(meVeOnceKernel<false, S, 0>);
+                }
                 return launched(c, "meVeOnceKernel");
             }));
             meVeOnceFinish<<<blocks, kPairBlock, 0, c->stream>>>(lv, a);

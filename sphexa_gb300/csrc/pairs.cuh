@@ -26,7 +26,8 @@ struct MixedTag {
 };
 
 constexpr int kPairBlock = 128;
-constexpr int kExpNodes = 512;  // table of e^(k/1024), |k| <= kExpNodes
+constexpr int kExpNodes = 512;  // table of e^(k/1024), |k| <= kExpNodes, then of e^-n, n < kExpWhole
+constexpr int kExpWhole = 17;
 
 // ---- neighbour list layout ----
 // Lists are stored in granules of kListGran entries, transposed per granule: entries 4g .. 4g+3 of

@@ -119,12 +119,17 @@ int buildTables(sphgb_ctx* c)
         SPHGB_CUDA(cudaMemcpy(c->whdS64.p, sd.data(), sizeof(double) * sd.size(), cudaMemcpyHostToDevice));
     }
     {
-        std::vector<double> e(4 * (2 * kExpNodes + 1));
+        std::vector<double> e(4 * (2 * kExpNodes + 1 + kExpWhole));
         for (int k = -kExpNodes; k <= kExpNodes; ++k) {
             double* q = &e[4 * (k + kExpNodes)];
             q[0] = std::exp(k / 1024.0);
             q[1] = std::exp(-k / 1024.0);
             q[2] = k / 1024.0;
+        }
+        for (int k = 0; k < kExpWhole; ++k) {
+            double* q = &e[4 * (2 * kExpNodes + 1 + k)];
+            q[0] = std::exp(-double(k));
+            q[2] = k;
         }
         SPHGB_TRY(c->expTab.ensure(sizeof(double) * e.size()));
         SPHGB_CUDA(cudaMemcpy(c->expTab.p, e.data(), sizeof(double) * e.size(), cudaMemcpyHostToDevice));

@@ -31,3 +31,25 @@ def test_atwood_branches_match_oracle(gpu_ctx, port, spread):
     r = run_gpu(gpu_ctx, wl, "ve", False)
     ref = port.sweep(wl, "ve", False)
     check_fields(r, ref, "ve", VE_FIELDS, f"spread {spread}")
+
+
+@pytest.mark.parametrize("name", ["fourier", "sphere", "few_neighbours"])
+def test_avclean_once_matches_oracle(gpu_ctx, port, name):
+    """Viscosity cleaning, one evaluation per mutual pair: lattice and clustered sets, and a set whose
+    lists are short (wide eta_crit)."""
+    from sphexa_gb300 import workloads as W
+    wl = {"fourier": lambda: W.fourier(13, seed=75, rho_seed=76, v_seed=77),
+          "sphere": lambda: W.sphere(4001, seed=78),
+          "few_neighbours": lambda: W.random_cube(1500, seed=79)}[name]()
+    rng = np.random.Generator(np.random.PCG64(80))
+    for k in ("vx", "vy", "vz"):
+        wl.fields[k] = rng.normal(0.0, 0.2, wl.n).astype(np.float32).astype(np.float64)
+    if name == "few_neighbours":
+        wl.params["ng0"], wl.params["ngmax"] = 40, 90
+        wl.fields["h"] = (wl.fields["h"] * 0.7).astype(np.float32).astype(np.float64)
+    gpu_ctx.set_deterministic(False)
+    r = run_gpu(gpu_ctx, wl, "ve", True)
+    ref = port.sweep(wl, "ve", True)
+    np.testing.assert_array_equal(r["nc"], ref["nc"])
+    check_fields(r, ref, "ve", VE_FIELDS, name)
+    assert r["minDt"] == pytest.approx(float(ref["minDtCourant"]), rel=1e-12)
