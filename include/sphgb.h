@@ -104,8 +104,8 @@ int sphgb_create(sphgb_ctx** ctx, int device);
 int sphgb_destroy(sphgb_ctx* ctx);
 int sphgb_set_stream(sphgb_ctx* ctx, void* cuda_stream);
 int sphgb_set_params(sphgb_ctx* ctx, const sphgb_params* params);
-/* Summation order of the FP64 VE passes xmass, gradh, IAD + divv/curlv, AV switches and
- * momentum-energy (no reference counterpart; the reference's GPU passes are order-fixed, e.g.
+/* Summation order of the FP64 passes: VE xmass, gradh, IAD + divv/curlv, AV switches and
+ * momentum-energy, std density, IAD and momentum-energy (no reference counterpart; the reference's GPU passes are order-fixed, e.g.
  * hydro_ve/momentum_energy_gpu.cu:53-144).  on = 0 (default): when the lists cover every particle,
  * each pair whose two ends list each other is evaluated once and the neighbour's share is added
  * with FP64 atomics, so the last bits of those passes' outputs can differ from run to run.
@@ -246,8 +246,8 @@ int sphgb_compute_momentum_energy(sphgb_ctx* ctx, sphgb_particles* p, int64_t fi
 
 /* ---- whole sweep: sync + neighbours + the pair passes of one propagator step
  *      (main/src/propagator/std_hydro.hpp:124-168, ve_hydro.hpp:130-204) ----
- * Positions, velocities and h cannot change between the passes of one call, so the FP64 VE sweep
- * (default mode) forms each owned pair's geometry and kernel values once, in the xmass pass, and
+ * Positions, velocities and h cannot change between the passes of one call, so the FP64 sweep
+ * (default mode) forms each owned pair's geometry and kernel values once, in the xmass or density pass, and
  * the later passes read them: a context-owned buffer of up to 80 bytes per owned pair (8M
  * particles: 35 GB), taken only when it fits in half of the free device memory, kept between
  * calls, given back when larger neighbour lists need the space.  The pass entry points above form

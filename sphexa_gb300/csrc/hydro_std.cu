@@ -8,8 +8,10 @@
 //   ME       -> momentumAndEnergyJLoop + tsKCourant (hydro_std/momentum_energy_kern.hpp:12-134,
 //               momentum_energy.hpp:41-101)
 // FP64 form: per-particle quotients (m/rho, p/rho, p/rho^2, 1/h, 1/h^3) are formed once per
-// particle, 1/|r| comes from rsqrt, periodic wrap tests run only where they can fire; results
-// agree with the reference to rounding.  Mixed form: FP32 pair arithmetic on grid-local
+// particle, 1/|r| comes from rsqrt, periodic wrap tests run only where they can fire; where the lists
+// cover every particle a mutual pair is evaluated once (owned lists, FP64 atomics; set_deterministic
+// selects the order-fixed walks), and inside a sweep IAD and momentum-energy read the pair geometry
+// that the density pass stored.  Results agree with the reference to rounding.  Mixed form: FP32 pair arithmetic on grid-local
 // offsets, Kahan sums, per-particle epilogues (normalisation, 3x3 inverse factor) in FP64.
 #include "pairs.cuh"
 
@@ -261,6 +263,78 @@ __global__ void __launch_bounds__(kPairBlock) iadKernel(ListView lv, CoordFp64 c
     }
 }
 
+// FP64 IAD with one evaluation per mutual pair over the owned lists: i adds vol_j W_i r r^T, and a mutual
+// pair gives j vol_i W_j r r^T by FP64 atomics.  Geo: arrays of the pair-geometry cache (5, 2), or 0.
+template<bool Smooth, int Geo>
+__global__ void __launch_bounds__(kPairBlock) iadStdOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf,
+                                                               const double* h, const double* vol,
+                                                               KTab<Smooth> tab, const double* hInv64, int64_t n,
+                                                               double* acc, PairGeo geo)
+{
+    const int64_t i = lv.first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (i >= lv.last) return;
+    const int64_t ii = i - lv.first;
+    const unsigned no = ov.size(ii);
+    const double* hInvDx = hInv64 + 2 * n;
+    const double voli = vol[i];
+    typename CoordFp64::Target t{};
+    double twoH = 0, hiInvDx = 0;
+    bool wrap = false;
+    int64_t g = 0;
+    if constexpr (Geo != 0) g = geo.base(ii);
+    if constexpr (Geo != 5) {
+        t = cf.target(i);
+        twoH = 2.0 * h[i];
+        wrap = cf.needsWrap(t, twoH);
+        hiInvDx = hInvDx[i];
+    }
+    double tau[6] = {0, 0, 0, 0, 0, 0};
+    for (unsigned k = 0; k < no; ++k, g += 32) {
+        bool mutual;
+        const uint32_t j = ov.at(ii, k, mutual);
+        double rx, ry, rz;
+        double2 wv;
+        if constexpr (Geo != 0) wv = __ldg(geo.w + g);
+        if constexpr (Geo == 5) {
+            const double2 a0 = __ldg(geo.x + g);
+            rx = a0.x, ry = a0.y, rz = __ldg(geo.x + geo.plane + g).x;
+        } else {
+            cf.diffFast(t, j, twoH, wrap, rx, ry, rz);
+        }
+        if constexpr (Geo == 0) {
+            const double r2 = dist2(rx, ry, rz);
+            const double dist = r2 * invDist(r2);
+            wv.x = lookupX(tab, dist * hiInvDx);
+            wv.y = lookupX(tab, dist * __ldg(hInvDx + j));
+        }
+        const double s[6] = {rx * rx, rx * ry, rx * rz, ry * ry, ry * rz, rz * rz};
+        const double vw = __ldg(vol + j) * wv.x;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) tau[q] = fma(vw, s[q], tau[q]);
+        if (mutual) {
+            const double vwj = voli * wv.y;
+#pragma unroll
+            for (int q = 0; q < 6; ++q) atomicAdd(acc + q * n + j, vwj * s[q]);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 6; ++q) atomicAdd(acc + q * n + i, tau[q]);
+}
+
+__global__ void iadStdOnceFinish(int64_t n, const double* h, double K, const double* acc, IadOut o)
+{
+    const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (i >= n) return;
+    double cc[6];
+    iadInvert<double>(acc[i], acc[n + i], acc[2 * n + i], acc[3 * n + i], acc[4 * n + i], acc[5 * n + i], h[i], K, cc);
+    st<double>(o.c11, i, cc[0]);
+    st<double>(o.c12, i, cc[1]);
+    st<double>(o.c13, i, cc[2]);
+    st<double>(o.c22, i, cc[3]);
+    st<double>(o.c23, i, cc[4]);
+    st<double>(o.c33, i, cc[5]);
+}
+
 // ---------------------------------------------------------------- momentum and energy (std)
 struct MeStdArgs {
     const void *vx, *vy, *vz, *h, *m, *rho, *p, *c;
@@ -405,6 +479,139 @@ __global__ void __launch_bounds__(kPairBlock) meStdKernel(ListView lv, CoordFp64
     if (a.minDt) blockMinDt(dt, a.minDt);
 }
 
+// neighbour-side fields of the pair-once momentum-energy pass in three 32-byte loads: A = h^-3 c_ab (six
+// entries), c, m, q = p / rho^2 and s = m / rho
+__global__ void meStdRec64Kernel(int64_t n, MeStdArgs a, Rec4d* __restrict__ rec)
+{
+    const int64_t j = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (j >= n) return;
+    const double f = a.hInv64[n + j], rho = ld<double>(a.rho, j), m = ld<double>(a.m, j);
+    rec[3 * j] = {f * ld<double>(a.c11, j), f * ld<double>(a.c12, j), f * ld<double>(a.c13, j), f * ld<double>(a.c22, j)};
+    rec[3 * j + 1] = {f * ld<double>(a.c23, j), f * ld<double>(a.c33, j), ld<double>(a.c, j), m};
+    rec[3 * j + 2] = {ld<double>(a.p, j) / (rho * rho), m / rho, 0.0, 0.0};
+}
+
+// FP64 std momentum-energy with one evaluation per mutual pair over the owned lists.  With W A r = w A r
+// at each end (A = h^-3 c) and t = visc s, i's directed term of momentum_energy_kern.hpp:60-134 is
+// V_i = w_i (m_j q_i + t_i) A_i r + w_j (m_j q_j + t_j) A_j r, since m_j / rho_j (p_j / rho_j) = m_j q_j;
+// j's is -V_j with m_i in place of m_j (the same where the masses are equal).  Energy: 2 m_j q_i w_i s_i +
+// Q with s = v_ij . A r and Q = t_i w_i s_i + t_j w_j s_j; j's is 2 m_i q_j w_j s_j + Q.  Bound by the
+// FP64 pipe: 1M particles 15.3 ms with every directed pair evaluated, now 5.4 ms (IAD 5.7 -> 2.1,
+// density 3.5 -> 2.8, which also fills the geometry cache).
+// Geo: arrays of the pair-geometry cache (5, 2), or 0 to form the geometry here.
+template<bool Smooth, int Geo>
+__global__ void __launch_bounds__(kPairBlock) meStdOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf, MeStdArgs a,
+                                                              const Rec4d* __restrict__ rec, double* __restrict__ acc,
+                                                              PairGeo geo)
+{
+    using T = double;
+    const int64_t i = lv.first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (i >= lv.last) return;
+    const int64_t ii = i - lv.first, n = a.n;
+    const unsigned no = ov.size(ii);
+    const KTab<Smooth> tabX{a.w64};
+    const double* hInvDx = a.hInv64 + 2 * n;
+    const T *vxA = static_cast<const T*>(a.vx), *vyA = static_cast<const T*>(a.vy), *vzA = static_cast<const T*>(a.vz);
+    const Rec4d i0 = rec[3 * i], i1 = rec[3 * i + 1], i2 = rec[3 * i + 2];
+    const T mi = i1.v[3];
+    typename CoordFp64::Target t{};
+    T vxi = 0, vyi = 0, vzi = 0, twoH = 0, hiInvDx = 0;
+    bool wrap = false;
+    int64_t g = 0;
+    if constexpr (Geo != 0) g = geo.base(ii);
+    if constexpr (Geo != 5) {
+        t = cf.target(i);
+        twoH = 2.0 * ld<T>(a.h, i);
+        wrap = cf.needsWrap(t, twoH);
+        vxi = vxA[i], vyi = vyA[i], vzi = vzA[i];
+        hiInvDx = hInvDx[i];
+    }
+    T mx = 0, my = 0, mz = 0, en = 0;
+    long long maxvBits = 0;
+    long long* accS = reinterpret_cast<long long*>(acc + 4 * n);
+    for (unsigned k = 0; k < no; ++k, g += 32) {
+        bool mutual;
+        const uint32_t j = ov.at(ii, k, mutual);
+        const Rec4d j0 = ldRec4d(rec + 3 * int64_t(j)), j1 = ldRec4d(rec + 3 * int64_t(j) + 1),
+                    j2 = ldRec4d(rec + 3 * int64_t(j) + 2);
+        T rx, ry, rz, wij, vxij, vyij, vzij;
+        double2 wv;
+        if constexpr (Geo != 0) {
+            wij = __ldg(geo.g + g).y;
+            wv = __ldg(geo.w + g);
+        }
+        if constexpr (Geo == 5) {  // v_ij = v_i - v_j = -dv exactly
+            const double2 a0 = __ldg(geo.x + g), a1 = __ldg(geo.x + geo.plane + g), a2 = __ldg(geo.x + 2 * geo.plane + g);
+            rx = a0.x, ry = a0.y, rz = a1.x;
+            vxij = -a1.y, vyij = -a2.x, vzij = -a2.y;
+        } else {
+            cf.diffFast(t, j, twoH, wrap, rx, ry, rz);
+            vxij = vxi - vxA[j], vyij = vyi - vyA[j], vzij = vzi - vzA[j];
+        }
+        if constexpr (Geo == 0) {
+            const T r2 = dist2(rx, ry, rz);
+            const T rinv = invDist(r2), dist = r2 * rinv;
+            wij = fma(rz, vzij, fma(ry, vyij, rx * vxij)) * rinv;
+            wv.x = lookupX(tabX, dist * hiInvDx);
+            wv.y = lookupX(tabX, dist * __ldg(hInvDx + j));
+        }
+        const T gix = i0.v[0] * rx + i0.v[1] * ry + i0.v[2] * rz;
+        const T giy = i0.v[1] * rx + i0.v[3] * ry + i1.v[0] * rz;
+        const T giz = i0.v[2] * rx + i1.v[0] * ry + i1.v[1] * rz;
+        const T gjx = j0.v[0] * rx + j0.v[1] * ry + j0.v[2] * rz;
+        const T gjy = j0.v[1] * rx + j0.v[3] * ry + j1.v[0] * rz;
+        const T gjz = j0.v[2] * rx + j1.v[0] * ry + j1.v[1] * rz;
+        const T cs = i1.v[2] + j1.v[2], mj = j1.v[3];
+        const T vsig = fma(T(-3), wij, cs);
+        maxvBits = maxBitsNonNeg(maxvBits, vsig);
+        const T wsi = wv.x * (vxij * gix + vyij * giy + vzij * giz), wsj = wv.y * (vxij * gjx + vyij * gjy + vzij * gjz);
+        T ti = 0, tj = 0, Q = 0;
+        if (negative(wij)) {  // approaching: half of artificial_viscosity(1, 1, c_i, c_j, w_ij)
+            const T visc = fma(T(0.25), cs, -wij) * -wij;
+            ti = i2.v[1] * visc;
+            tj = j2.v[1] * visc;
+            Q = fma(ti, wsi, tj * wsj);
+        }
+        T Pi = wv.x * fma(mj, i2.v[0], ti), Pj = wv.y * fma(mj, j2.v[0], tj);
+        T Vx = fma(Pi, gix, Pj * gjx), Vy = fma(Pi, giy, Pj * gjy), Vz = fma(Pi, giz, Pj * gjz);
+        mx += Vx;
+        my += Vy;
+        mz += Vz;
+        en += fma(mj * (2.0 * i2.v[0]), wsi, Q);
+        if (mutual) {
+            if (__double_as_longlong(mi) != __double_as_longlong(mj)) {
+                Pi = wv.x * fma(mi, i2.v[0], ti), Pj = wv.y * fma(mi, j2.v[0], tj);
+                Vx = fma(Pi, gix, Pj * gjx), Vy = fma(Pi, giy, Pj * gjy), Vz = fma(Pi, giz, Pj * gjz);
+            }
+            atomicAdd(acc + j, -Vx);
+            atomicAdd(acc + n + j, -Vy);
+            atomicAdd(acc + 2 * n + j, -Vz);
+            atomicAdd(acc + 3 * n + j, fma(mi * (2.0 * j2.v[0]), wsj, Q));
+            atomicMax(accS + j, __double_as_longlong(vsig));
+        }
+    }
+    atomicAdd(acc + i, mx);
+    atomicAdd(acc + n + i, my);
+    atomicAdd(acc + 2 * n + i, mz);
+    atomicAdd(acc + 3 * n + i, en);
+    atomicMax(accS + i, maxvBits);
+}
+
+__global__ void __launch_bounds__(kPairBlock) meStdOnceFinish(MeStdArgs a, const double* __restrict__ acc)
+{
+    const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    double dt = INFINITY;
+    if (i < a.n) {
+        a.du[i] = -a.K * 0.5 * acc[3 * a.n + i];
+        st<double>(a.ax, i, a.K * acc[i]);
+        st<double>(a.ay, i, a.K * acc[a.n + i]);
+        st<double>(a.az, i, a.K * acc[2 * a.n + i]);
+        const long long mb = reinterpret_cast<const long long*>(acc + 4 * a.n)[i];
+        dt = courantDt(__longlong_as_double(mb), ld<double>(a.h, i), ld<double>(a.c, i), a.Kcour);
+    }
+    if (a.minDt) blockMinDt(dt, a.minDt);
+}
+
 template<class P>
 int launchXmass(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, void* out, bool storeRho)
 {
@@ -416,8 +623,7 @@ int launchXmass(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, v
     CoordMixed cm = coordMixed(c);
     const void* wh = std::is_same_v<P, Fp64Tag> ? c->whx64.p : c->whH32.p;
     unsigned blocks = gridFor(last - first, kPairBlock);
-    // pair-once for the VE xmass; the std density keeps the order-fixed walk
-    if (std::is_same_v<P, Fp64Tag> && !storeRho && pairOnce(c, p, first, last)) {
+    if (std::is_same_v<P, Fp64Tag> && pairOnce(c, p, first, last)) {
         const int64_t n = p->n;
         SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * size_t(n)));
         SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * size_t(n), c->stream));
@@ -476,6 +682,28 @@ int launchIad(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last)
     lv.first = first;
     lv.last = last;
     const void* wh = std::is_same_v<P, Fp64Tag> ? c->whx64.p : c->whH32.p;
+    if (std::is_same_v<P, Fp64Tag> && pairOnce(c, p, first, last)) {
+        const int64_t n = p->n;
+        SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * 6 * size_t(n)));
+        SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * 6 * size_t(n), c->stream));
+        const PairGeo geo = pairGeoRead(c);
+        const double* h = static_cast<const double*>(p->h);
+        SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
+            constexpr bool S = decltype(smooth)::value;
+            auto run = [&](auto kernel) {
+                kernel<<<gridFor(n, kPairBlock), kPairBlock, 0, c->stream>>>(
+                    lv, ownedView(c), coordFp64(c, p), h, c->aux.as<double>(), KTab<S>{tabW64(c)},
+                    c->hInv64.as<double>(), n, c->pairAcc.as<double>(), geo);
+            };
+            if (geo.x) run(iadStdOnceKernel<S, 5>);
+            else if (geo.g) run(iadStdOnceKernel<S, 2>);
+            else run(iadStdOnceKernel<S, 0>);
+            return launched(c, "iadStdOnceKernel");
+        }));
+        iadStdOnceFinish<<<gridFor(n, 256), 256, 0, c->stream>>>(n, h, c->K, c->pairAcc.as<double>(),
+                                                                 IadOut{p->c11, p->c12, p->c13, p->c22, p->c23, p->c33});
+        return launched(c, "iadStdOnceFinish");
+    }
     return withKernelForm(c, [&](auto smooth) {
         constexpr bool S = std::is_same_v<P, Fp64Tag> && decltype(smooth)::value;
         iadKernel<P, S><<<gridFor(last - first, kPairBlock), kPairBlock, 0, c->stream>>>(
@@ -488,7 +716,8 @@ int launchIad(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last)
 template<class P>
 int launchMeStd(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, double* minDt)
 {
-    SPHGB_TRY(launchStdAux<P>(c, p, true));
+    const bool once = std::is_same_v<P, Fp64Tag> && pairOnce(c, p, first, last);
+    if (!once) SPHGB_TRY(launchStdAux<P>(c, p, true));
     ListView lv = listView(c);
     lv.first = first;
     lv.last = last;
@@ -519,6 +748,30 @@ int launchMeStd(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, d
     a.az = p->az;
     a.du = p->du;
     SPHGB_TRY(beginDtReduction(c, &a.minDt));
+    if (once) {
+        const int64_t n = p->n;
+        SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * 5 * size_t(n)));
+        SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * 5 * size_t(n), c->stream));
+        SPHGB_TRY(c->pack.ensure(sizeof(Rec4d) * 3 * size_t(n)));
+        meStdRec64Kernel<<<gridFor(n, 256), 256, 0, c->stream>>>(n, a, c->pack.as<Rec4d>());
+        SPHGB_TRY(launched(c, "meStdRec64Kernel"));
+        const PairGeo geo = pairGeoRead(c);
+        const unsigned blocks = gridFor(n, kPairBlock);
+        SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
+            constexpr bool S = decltype(smooth)::value;
+            auto run = [&](auto kernel) {
+                kernel<<<blocks, kPairBlock, 0, c->stream>>>(lv, ownedView(c), coordFp64(c, p), a, c->pack.as<Rec4d>(),
+                                                             c->pairAcc.as<double>(), geo);
+            };
+            if (geo.x) run(meStdOnceKernel<S, 5>);
+            else if (geo.g) run(meStdOnceKernel<S, 2>);
+            else run(meStdOnceKernel<S, 0>);
+            return launched(c, "meStdOnceKernel");
+        }));
+        meStdOnceFinish<<<blocks, kPairBlock, 0, c->stream>>>(a, c->pairAcc.as<double>());
+        SPHGB_TRY(launched(c, "meStdOnceFinish"));
+        return endDtReduction(c, a.minDt, minDt);
+    }
     SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
         constexpr bool S = std::is_same_v<P, Fp64Tag> && decltype(smooth)::value;
         meStdKernel<P, S><<<gridFor(last - first, kPairBlock), kPairBlock, 0, c->stream>>>(lv, coordFp64(c, p),

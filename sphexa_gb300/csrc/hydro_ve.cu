@@ -570,8 +570,6 @@ __global__ void __launch_bounds__(kPairBlock) avKernel(ListView lv, CoordFp64 cf
 }
 
 // ---------------------------------------------------------------- momentum and energy (VE)
-struct Rec4d;
-
 struct MeVeArgs {
     const void *vx, *vy, *vz, *h, *m, *prho, *c, *kx, *xm, *alpha;
     const void *c11, *c12, *c13, *c22, *c23, *c33;
@@ -1211,17 +1209,6 @@ __global__ void avOnceFinish(int64_t first, int64_t last, int64_t n, AvArgs a, c
 // h^-3 enter every use of c, so they are folded in once per particle instead of per pair.  With the
 // viscosity cleaning two more: the symmetric velocity gradient (six entries), 1/h, and eta_crit of the
 // particle's neighbour count (momentum_energy_kern.hpp:43-63).
-struct alignas(32) Rec4d {
-    double v[4];
-};
-
-__device__ __forceinline__ Rec4d ldRec4d(const Rec4d* p)
-{
-    Rec4d r;
-    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.v[0]), "=d"(r.v[1]), "=d"(r.v[2]), "=d"(r.v[3]) : "l"(p));
-    return r;
-}
-
 // Aux: also forms the quotients rho, ln xm and 1/rho (outside a sweep, which has them already)
 template<bool Aux, bool AvClean>
 __global__ void meVeRec64Kernel(int64_t n, MeVeArgs a, ListView lv, double* __restrict__ aux, Rec4d* __restrict__ rec,

@@ -450,6 +450,18 @@ __device__ __forceinline__ void packGridBlock(float4* q, u64 cell, float4 loc, f
     q[1] = make_float4(loc.z, f5, f6, f7);
 }
 
+// neighbour record of the FP64 pair-once passes: four doubles, one 256-bit load
+struct alignas(32) Rec4d {
+    double v[4];
+};
+
+__device__ __forceinline__ Rec4d ldRec4d(const Rec4d* p)
+{
+    Rec4d r;
+    asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.v[0]), "=d"(r.v[1]), "=d"(r.v[2]), "=d"(r.v[3]) : "l"(p));
+    return r;
+}
+
 // W and dW/dv at the same v
 __device__ __forceinline__ void lookupH32Pair(const float4* __restrict__ tw, const float4* __restrict__ tdw, float v,
                                               float& w, float& dw)

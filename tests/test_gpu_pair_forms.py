@@ -53,3 +53,31 @@ def test_avclean_once_matches_oracle(gpu_ctx, port, name):
     np.testing.assert_array_equal(r["nc"], ref["nc"])
     check_fields(r, ref, "ve", VE_FIELDS, name)
     assert r["minDt"] == pytest.approx(float(ref["minDtCourant"]), rel=1e-12)
+
+
+@pytest.mark.parametrize("n", [33, 640, 1331])
+@pytest.mark.parametrize("masses", ["equal", "spread"])
+def test_std_once_matches_oracle(gpu_ctx, port, n, masses):
+    """The std chain with one evaluation per mutual pair, in a sweep (cached geometry) and pass by pass
+    (geometry formed in every pass): partly filled warps and blocks, equal and unequal masses."""
+    from sphexa_gb300 import sph, workloads as W
+    wl = W.random_cube(n, seed=81 + n, periodic=n > 600)
+    rng = np.random.Generator(np.random.PCG64(82))
+    m = np.full(n, 1.0 / n) if masses == "equal" else 10.0 ** rng.uniform(-0.5, 0.5, n) / n
+    wl.fields["m"] = m.astype(np.float32).astype(np.float64)
+    fields = ("rho", "p", "c", "c11", "c12", "c13", "c22", "c23", "c33", "ax", "ay", "az", "du")
+    gpu_ctx.set_deterministic(False)
+    r = run_gpu(gpu_ctx, wl, "std", False)
+    ref = port.sweep(wl, "std", False)
+    check_fields(r, ref, "std", fields, f"sweep {n} {masses}")
+    assert r["minDt"] == pytest.approx(float(ref["minDtCourant"]), rel=1e-12)
+    d = sph.ParticlesData.from_workload(wl, "fp64", "cuda:0")
+    box = sph.Box(wl.box.copy(), wl.bc.copy())
+    sph.Domain(gpu_ctx, box).sync(d)
+    sph.find_neighbors_sfc(gpu_ctx, 0, wl.n, d)
+    sph.compute_density(gpu_ctx, d)
+    sph.compute_eos_hydro_std(gpu_ctx, d)
+    sph.compute_iad(gpu_ctx, d)
+    sph.compute_momentum_energy_std(gpu_ctx, d)
+    check_fields({f: d.f[f].cpu().numpy() for f in fields}, ref, "std", fields, f"passes {n} {masses}")
+    assert d.minDtCourant == pytest.approx(float(ref["minDtCourant"]), rel=1e-12)
