@@ -151,12 +151,15 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
             gmin[k] = fminf(gmin[k], __shfl_xor_sync(0xffffffffu, gmin[k], o));
             gmax[k] = fmaxf(gmax[k], __shfl_xor_sync(0xffffffffu, gmax[k], o));
         }
-    // absolute position of the origin from its cell (FP32 suffices for pruning, see the pad)
-    bool exactOnly = false;
+    // absolute position of the origin from its cell (FP32 suffices for pruning, see the pad).
+    // foldPairs: on some periodic axis the search box reaches half the box from the origin (sets of a
+    // few thousand particles).  Below that a neighbour's offset, wrapped against the origin, is also
+    // the image nearest to its target (|offset| <= Rg < L/2), so differences of offsets need no fold.
+    bool foldPairs = false;
     float gc[3], gs[3], Rg = 0.f;
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        if (b.pbc[k] && (gmax[k] - gmin[k]) > 0.25f * b.Lf[k]) exactOnly = true;
+        if (b.pbc[k] && fmaxf(fabsf(gmin[k]), fabsf(gmax[k])) > 0.49f * b.Lf[k]) foldPairs = true;
         const float lok = (k == 0) ? lo.x : (k == 1 ? lo.y : lo.z);
         float cAbs = float(b.lo[k]) + fmaf(float(co[k]), a.u[k], lok) + 0.5f * (gmin[k] + gmax[k]);
         if (b.pbc[k]) {
@@ -168,8 +171,9 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
         gs[k] = 0.5f * (gmax[k] - gmin[k]) + pad;
         Rg = fmaxf(Rg, fmaxf(fabsf(gmin[k]), fabsf(gmax[k])));
     }
-    // FP32 decision margin on d2: covers the rounding of cell edge, offsets and the squared sum;
-    // pairs inside the margin get the exact FP64 test (every pair when exactOnly)
+    // FP32 decision margin on d2: covers the rounding of cell edge, offsets and the squared sum (and,
+    // where pairs are folded, of the box length, L <= 2 Rg / 0.98 there); pairs inside the margin get the
+    // exact FP64 test
     const float r2f = float(r2);
     const float margin = 64.f * 0x1p-24f * (Rg + rf) * (Rg + rf);
     const float inBelow = r2f - margin;   // d2f < inBelow: neighbour
@@ -200,16 +204,13 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
         }
     };
 
-    // one chunk of m <= 32 contiguous candidates [ja, ja + m), staged by the warp.  Every target
-    // tests all 32 slots with a fixed trip count; slots >= m hold a far-away sentinel whose FP32
-    // distance is +inf.  Groups that need the exact test for every pair loop over the m slots.
     // Candidates are staged 32 at a time (one per lane, coalesced loads of cell and offset); those
     // outside the group's search box by more than the FP32 rounding of the offsets (cullPad) are
     // dropped and the rest appended, in ascending index order, to the warp's queue by ballot
     // compaction.  A dropped candidate is farther than 2h from every target along one axis, so the
     // reference's FP64 test rejects it too.  Each full queue block of 32 is tested by every target
     // with a fixed trip count; the last, partial block has far-away sentinels in its empty slots.
-    // Groups that need the exact test for every pair keep every candidate and test the filled slots.
+    // Groups that fold their pairs keep every candidate.
     const float cullPad = 32.f * 0x1p-24f * (Rg + fmaxf(a.u[0], fmaxf(a.u[1], a.u[2])));
     const float bxl = gmin[0] - cullPad, bxh = gmax[0] + cullPad;
     const float byl = gmin[1] - cullPad, byh = gmax[1] + cullPad;
@@ -240,15 +241,37 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
         sm.cull[7] = 0.f;
     }
     __syncwarp();
+    // 1/L of the periodic axes (0 leaves an axis unfolded)
+    const float foldL[3] = {b.pbc[0] ? 1.f / b.Lf[0] : 0.f, b.pbc[1] ? 1.f / b.Lf[1] : 0.f, b.pbc[2] ? 1.f / b.Lf[2] : 0.f};
     int qn = 0;  // candidates in the queue
     auto testBlock = [&](int filled) {
         if (valid) tested += unsigned(filled);
-        if (exactOnly) {
-            if (valid)
-                for (int t = 0; t < filled; ++t) {
-                    const uint32_t j = sm.idx[t];
-                    if (exactIn(j)) take(j);
+        uint32_t hit = 0, nearm = 0;
+        if (foldPairs) {
+            // offsets of target and candidate may differ by up to L: the nearest image of the
+            // difference, in FP32.  Where 2h < L/2 there is one image within the radius; beyond,
+            // images at equal distance give the same d2 to rounding.
+#pragma unroll 1
+            for (int t = 0; t < filled; t += 4) {
+                const float4 X = *reinterpret_cast<const float4*>(&sm.nx[t]);
+                const float4 Y = *reinterpret_cast<const float4*>(&sm.ny[t]);
+                const float4 Z = *reinterpret_cast<const float4*>(&sm.nz[t]);
+                const float x[4] = {X.x, X.y, X.z, X.w}, y[4] = {Y.x, Y.y, Y.z, Y.w}, z[4] = {Z.x, Z.y, Z.z, Z.w};
+#pragma unroll
+                for (int s = 0; s < 4; ++s) {
+                    float ex = dxi + x[s], ey = dyi + y[s], ez = dzi + z[s];
+                    ex = fmaf(-b.Lf[0], rintf(ex * foldL[0]), ex);
+                    ey = fmaf(-b.Lf[1], rintf(ey * foldL[1]), ey);
+                    ez = fmaf(-b.Lf[2], rintf(ez * foldL[2]), ez);
+                    const float d2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+                    hit |= (d2 < inBelow ? 1u : 0u) << (t + s);
+                    nearm |= (d2 <= outAbove ? 1u : 0u) << (t + s);
                 }
+            }
+            if (filled < kWarp) {  // the sentinels of a partial block fold to anywhere
+                hit &= (1u << filled) - 1u;
+                nearm &= (1u << filled) - 1u;
+            }
         } else {
             // four slots per step on packed FP32x2 operations: e = d_i + (-r_j) rounds as
             // d_i - r_j, and d2 = fma(ex, ex, fma(ey, ey, ez * ez)) per slot as in scalar form.
@@ -256,7 +279,6 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
             // within it: exact FP64 test), then each lane appends its neighbours slot by slot in
             // ascending order, one loop trip per neighbour instead of a predicated append per slot.
             const float2 dx2 = make_float2(dxi, dxi), dy2 = make_float2(dyi, dyi), dz2 = make_float2(dzi, dzi);
-            uint32_t hit = 0, nearm = 0;
 #pragma unroll
             for (int t = 0; t < kWarp; t += 4) {
                 const float4 X = *reinterpret_cast<const float4*>(&sm.nx[t]);
@@ -277,14 +299,14 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
                     nearm |= (d2[s] <= outAbove ? 1u : 0u) << (t + s);
                 }
             }
-            if (valid) {
-                // a pair within the FP32 margin of the radius (rare): the exact test
-                for (uint32_t band = nearm & ~hit; band != 0; band &= band - 1u) {
-                    const int s = __ffs(band) - 1;
-                    if (exactIn(sm.idx[s])) hit |= 1u << s;
-                }
-                for (; hit != 0; hit &= hit - 1u) take(sm.idx[__ffs(hit) - 1]);
+        }
+        if (valid) {
+            // a pair within the FP32 margin of the radius (rare): the exact test
+            for (uint32_t band = nearm & ~hit; band != 0; band &= band - 1u) {
+                const int s = __ffs(band) - 1;
+                if (exactIn(sm.idx[s])) hit |= 1u << s;
             }
+            for (; hit != 0; hit &= hit - 1u) take(sm.idx[__ffs(hit) - 1]);
         }
         __syncwarp();
     };
@@ -301,7 +323,7 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
             const float ex = fmaxf(fmaxf(cl.x - rj[0], rj[0] - ch.x), 0.f);
             const float ey = fmaxf(fmaxf(cl.y - rj[1], rj[1] - ch.y), 0.f);
             const float ez = fmaxf(fmaxf(cl.z - rj[2], rj[2] - ch.z), 0.f);
-            keep = exactOnly || (rj[0] >= bxl && rj[0] <= bxh && rj[1] >= byl && rj[1] <= byh && rj[2] >= bzl &&
+            keep = foldPairs || (rj[0] >= bxl && rj[0] <= bxh && rj[1] >= byl && rj[1] <= byh && rj[2] >= bzl &&
                                  rj[2] <= bzh && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= cl.w);
         }
         const unsigned km = __ballot_sync(0xffffffffu, keep);

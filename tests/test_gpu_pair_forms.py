@@ -81,3 +81,23 @@ def test_std_once_matches_oracle(gpu_ctx, port, n, masses):
     sph.compute_momentum_energy_std(gpu_ctx, d)
     check_fields({f: d.f[f].cpu().numpy() for f in fields}, ref, "std", fields, f"passes {n} {masses}")
     assert d.minDtCourant == pytest.approx(float(ref["minDtCourant"]), rel=1e-12)
+
+
+@pytest.mark.parametrize("n", [257, 1728, 6000])
+@pytest.mark.parametrize("edges", [(1.0, 1.0, 1.0), (1.0, 0.3, 0.3)])
+def test_search_folds_small_periodic_boxes(gpu_ctx, port, n, edges):
+    """Search boxes that reach half a periodic box (pairs folded one by one) and just stay below (offsets
+    wrapped against the group's origin): neighbour sets against the oracle, cubic and flat boxes."""
+    from sphexa_gb300 import workloads as W
+    from test_gpu_parity import flat_sets
+    h = 0.5 * (3.0 / (4.0 * np.pi) * 100 * np.prod(edges) / n) ** (1.0 / 3.0)
+    wl = W.random_cube(n, seed=90 + n, periodic=True, h=h)
+    for k, f in enumerate(("x", "y", "z")):
+        wl.fields[f] = wl.fields[f] * edges[k]
+        wl.box[2 * k + 1] = edges[k]
+    r = run_gpu(gpu_ctx, wl, "std", False)
+    ref = port.sweep(wl, "std", False)
+    ng = int(wl.params["ngmax"])
+    np.testing.assert_array_equal(r["keys"], ref["keys"])
+    np.testing.assert_array_equal(r["nc"], ref["nc"])
+    np.testing.assert_array_equal(flat_sets(r["nbr"], r["nc"], ng), flat_sets(ref["nbr"], ref["nc"], ng))
