@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kPairBlock) xmassOnceKernel(ListView lv, Owned
     const int64_t gb = geo.base(ii);
     const double vxi = geo.g ? vx[i] : 0.0, vyi = geo.g ? vy[i] : 0.0, vzi = geo.g ? vz[i] : 0.0;
     double rho0 = 0.0;
-    for (unsigned k = 0; k < no; ++k) {
+    for (unsigned k = blockIdx.y; k < no; k += gridDim.y) {
         bool mutual;
         const uint32_t j = ov.at(ii, k, mutual);
         double rx, ry, rz;
@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(kPairBlock) iadStdOnceKernel(ListView lv, Owne
     double twoH = 0, hiInvDx = 0;
     bool wrap = false;
     int64_t g = 0;
-    if constexpr (Geo != 0) g = geo.base(ii);
+    if constexpr (Geo != 0) g = geo.base(ii) + 32 * blockIdx.y;
     if constexpr (Geo != 5) {
         t = cf.target(i);
         twoH = 2.0 * h[i];
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(kPairBlock) iadStdOnceKernel(ListView lv, Owne
         hiInvDx = hInvDx[i];
     }
     double tau[6] = {0, 0, 0, 0, 0, 0};
-    for (unsigned k = 0; k < no; ++k, g += 32) {
+    for (unsigned k = blockIdx.y; k < no; k += gridDim.y, g += 32 * gridDim.y) {
         bool mutual;
         const uint32_t j = ov.at(ii, k, mutual);
         double rx, ry, rz;
@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(kPairBlock) meStdOnceKernel(ListView lv, Owned
     T vxi = 0, vyi = 0, vzi = 0, twoH = 0, hiInvDx = 0;
     bool wrap = false;
     int64_t g = 0;
-    if constexpr (Geo != 0) g = geo.base(ii);
+    if constexpr (Geo != 0) g = geo.base(ii) + 32 * blockIdx.y;
     if constexpr (Geo != 5) {
         t = cf.target(i);
         twoH = 2.0 * ld<T>(a.h, i);
@@ -529,7 +529,7 @@ __global__ void __launch_bounds__(kPairBlock) meStdOnceKernel(ListView lv, Owned
     T mx = 0, my = 0, mz = 0, en = 0;
     long long maxvBits = 0;
     long long* accS = reinterpret_cast<long long*>(acc + 4 * n);
-    for (unsigned k = 0; k < no; ++k, g += 32) {
+    for (unsigned k = blockIdx.y; k < no; k += gridDim.y, g += 32 * gridDim.y) {
         bool mutual;
         const uint32_t j = ov.at(ii, k, mutual);
         const Rec4d j0 = ldRec4d(rec + 3 * int64_t(j)), j1 = ldRec4d(rec + 3 * int64_t(j) + 1),
@@ -636,7 +636,7 @@ int launchXmass(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, v
         }
         SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
             constexpr bool S = decltype(smooth)::value;
-            xmassOnceKernel<S><<<blocks, kPairBlock, 0, c->stream>>>(
+            xmassOnceKernel<S><<<ownedGrid(n), kPairBlock, 0, c->stream>>>(
                 lv, ownedView(c), cf, static_cast<const double*>(p->h), static_cast<const double*>(p->m),
                 KTab<S>{tabW64(c)}, c->hInv64.as<double>() + 2 * n, c->pairAcc.as<double>(), geo,
                 static_cast<const double*>(p->vx), static_cast<const double*>(p->vy),
@@ -691,7 +691,7 @@ int launchIad(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last)
         SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
             constexpr bool S = decltype(smooth)::value;
             auto run = [&](auto kernel) {
-                kernel<<<gridFor(n, kPairBlock), kPairBlock, 0, c->stream>>>(
+                kernel<<<ownedGrid(n), kPairBlock, 0, c->stream>>>(
                     lv, ownedView(c), coordFp64(c, p), h, c->aux.as<double>(), KTab<S>{tabW64(c)},
                     c->hInv64.as<double>(), n, c->pairAcc.as<double>(), geo);
             };
@@ -760,7 +760,7 @@ int launchMeStd(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, d
         SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
             constexpr bool S = decltype(smooth)::value;
             auto run = [&](auto kernel) {
-                kernel<<<blocks, kPairBlock, 0, c->stream>>>(lv, ownedView(c), coordFp64(c, p), a, c->pack.as<Rec4d>(),
+                kernel<<<ownedGrid(n), kPairBlock, 0, c->stream>>>(lv, ownedView(c), coordFp64(c, p), a, c->pack.as<Rec4d>(),
                                                              c->pairAcc.as<double>(), geo);
             };
             if (geo.x) run(meStdOnceKernel<S, 5>);

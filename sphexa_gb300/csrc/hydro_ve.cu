@@ -896,14 +896,14 @@ __global__ void __launch_bounds__(kPairBlock) gradhOnceKernel(ListView lv, Owned
     double twoH = 0.0;
     bool wrap = false;
     int64_t g = 0;
-    if constexpr (Geo) g = geo.base(ii);
+    if constexpr (Geo) g = geo.base(ii) + 32 * blockIdx.y;
     else {
         t = cf.target(i);
         twoH = 2.0 * h[i];
         wrap = cf.needsWrap(t, twoH);
     }
     double kx = 0.0, dxm = 0.0, dm = 0.0;
-    for (unsigned k = 0; k < no; ++k, g += 32) {
+    for (unsigned k = blockIdx.y; k < no; k += gridDim.y, g += 32 * gridDim.y) {
         bool mutual;
         const uint32_t j = ov.at(ii, k, mutual);
         double dist;
@@ -1013,7 +1013,7 @@ __global__ void __launch_bounds__(kPairBlock) iadOnceKernel(ListView lv, OwnedVi
     const double vxi = vx[i], vyi = vy[i], vzi = vz[i], voli = vol[i], xmi = xm[i];
     const int64_t gb = geo.base(ii);
     double tau[6] = {0, 0, 0, 0, 0, 0}, M[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (unsigned k = 0; k < no; ++k) {
+    for (unsigned k = blockIdx.y; k < no; k += gridDim.y) {
         bool mutual;
         const uint32_t j = ov.at(ii, k, mutual);
         double rx, ry, rz, dvx, dvy, dvz, dist;
@@ -1123,7 +1123,7 @@ __global__ void __launch_bounds__(kPairBlock) avOnceKernel(ListView lv, OwnedVie
     double vxi = 0, vyi = 0, vzi = 0, twoH = 0, hiInvDx = 0;
     bool wrap = false;
     int64_t g = 0;
-    if constexpr (Geo != 0) g = geo.base(ii);
+    if constexpr (Geo != 0) g = geo.base(ii) + 32 * blockIdx.y;
     if constexpr (Geo != 5) {
         t = cf.target(i);
         twoH = 2.0 * ld<double>(a.h, i);
@@ -1134,7 +1134,7 @@ __global__ void __launch_bounds__(kPairBlock) avOnceKernel(ListView lv, OwnedVie
     double Sx = 0, Sy = 0, Sz = 0;
     long long vsigBits = 0;
     long long* accV = reinterpret_cast<long long*>(acc + 3 * n);
-    for (unsigned k = 0; k < no; ++k, g += 32) {
+    for (unsigned k = blockIdx.y; k < no; k += gridDim.y, g += 32 * gridDim.y) {
         bool mutual;
         const uint32_t j = ov.at(ii, k, mutual);
         double rx, ry, rz, wij;
@@ -1391,13 +1391,13 @@ __global__ void __launch_bounds__(kPairBlock) meVeOnceKernel(ListView lv, CoordF
         hiInvDx = hInvDx[i];
     }
     int64_t g = 0;
-    if constexpr (Geo != 0) g = geo.base(ii);
+    if constexpr (Geo != 0) g = geo.base(ii) + 32 * blockIdx.y;
     T mx = 0, my = 0, mz = 0, en = 0, avE = 0;
     long long maxvBits = 0;
     double *accX = a.acc, *accY = a.acc + a.n, *accZ = a.acc + 2 * a.n, *accE = a.acc + 3 * a.n,
            *accV = a.acc + 4 * a.n;
     long long* accS = reinterpret_cast<long long*>(a.acc + 5 * a.n);
-    for (unsigned k = 0; k < nOwned; ++k, g += 32) {
+    for (unsigned k = blockIdx.y; k < nOwned; k += gridDim.y, g += 32 * gridDim.y) {
         const uint32_t e = __ldg(a.owned + listSlot(ii, k, lv.stride));
         const uint32_t j = e & 0x7fffffffu;
         const bool mutual = (e >> 31) != 0;
@@ -1556,7 +1556,7 @@ int passGradh(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last)
         SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
             constexpr bool S = decltype(smooth)::value;
             auto run = [&](auto kernel) {
-                kernel<<<blocks, kPairBlock, 0, c->stream>>>(
+                kernel<<<ownedGrid(n), kPairBlock, 0, c->stream>>>(
                     lv, ownedView(c), coordFp64(c, p), static_cast<const double*>(p->h),
                     static_cast<const double*>(p->m), static_cast<const double*>(p->xm), KTab<S>{tabW64(c)},
                     KTab<S>{tabDW64(c)}, c->hInv64.as<double>(), n, c->pairAcc.as<double>(), geo);
@@ -1700,7 +1700,7 @@ int passIadDivvCurlv(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t la
             SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * 15 * size_t(n)));
             SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * 15 * size_t(n), c->stream));
             SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
-                iadOnceKernel<decltype(smooth)::value><<<blocks, kPairBlock, 0, c->stream>>>(
+                iadOnceKernel<decltype(smooth)::value><<<ownedGrid(n), kPairBlock, 0, c->stream>>>(
                     lv, ownedView(c), coordFp64(c, p), a, c->hInv64.as<double>(), n, c->pairAcc.as<double>(),
                     pairGeoRead(c));
                 return launched(c, "iadOnceKernel");
@@ -1757,7 +1757,7 @@ int passAVswitches(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last
             constexpr bool S = decltype(smooth)::value;
             const PairGeo geo = pairGeoRead(c);
             auto run = [&](auto kernel) {
-                kernel<<<blocks, kPairBlock, 0, c->stream>>>(lv, ownedView(c), coordFp64(c, p), a,
+                kernel<<<ownedGrid(n), kPairBlock, 0, c->stream>>>(lv, ownedView(c), coordFp64(c, p), a,
                                                              c->hInv64.as<double>(), n, c->pairAcc.as<double>(), geo);
             };
             if (geo.x) run(avOnceKernel<S, 5>);
@@ -1872,7 +1872,7 @@ int passMomentumEnergyVe(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_
             const PairGeo geo = pairGeoRead(c);
             SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
                 constexpr bool S = decltype(smooth)::value;
-                auto run = [&](auto kernel) { kernel<<<blocks, kPairBlock, 0, c->stream>>>(lv, cf, a, geo); };
+                auto run = [&](auto kernel) { kernel<<<ownedGrid(p->n), kPairBlock, 0, c->stream>>>(lv, cf, a, geo); };
                 if (avClean) {
                     if (geo.x) run(meVeOnceKernel<true, S, 5>);
                     else if (geo.g) run(meVeOnceKernel<true, S, 2>);

@@ -111,6 +111,18 @@ struct OwnedView {
     }
 };
 
+// Grid of a pass over owned lists.  Small sets do not fill the chip with one thread per particle, and a
+// thread's list is a serial chain, so the lists are cut into up to 16 interleaved slices (blockIdx.y
+// walks entries y, y + S, ...; every slice adds its sums to the accumulators with the same atomics).
+// Slices are added until about four waves of warps are in flight (152 SMs x 16 resident warps each);
+// from 311k particles on there is one.
+inline dim3 ownedGrid(int64_t n)
+{
+    const int64_t warps = (n + 31) / 32, want = 4 * 152 * 16;
+    const int64_t s = (want + warps - 1) / warps;
+    return dim3(unsigned((n + kPairBlock - 1) / kPairBlock), unsigned(s < 1 ? 1 : s > 16 ? 16 : s));
+}
+
 inline OwnedView ownedView(const sphgb_ctx* c)
 {
     return OwnedView{c->owned.as<uint32_t>(), c->ownedCount.as<uint32_t>(), c->nbrStride};
