@@ -101,7 +101,7 @@ struct sphgb_ctx {
     bool haveNbr = false;
     // owned pair lists of the pair-once passes, in the granule layout of the lists (listSlot): entry
     // j | mutual << 31 for the pairs i evaluates, ownedCount per particle; valid for epoch ownedEpoch
-    sphgb::DBuf owned, ownedCount, ownedR2;
+    sphgb::DBuf owned, ownedCount;
     int64_t ownedEpoch = -1;
     bool ownedFromLists = false;  // owned lists decided from list membership (mixed adjoint); the FP64 passes skip them
     // summation mode of the FP64 passes (order-fixed, or one evaluation per mutual pair) and the
