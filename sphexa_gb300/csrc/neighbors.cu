@@ -268,10 +268,6 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
                     nearm |= (d2 <= outAbove ? 1u : 0u) << (t + s);
                 }
             }
-            if (filled < kWarp) {  // the sentinels of a partial block fold to anywhere
-                hit &= (1u << filled) - 1u;
-                nearm &= (1u << filled) - 1u;
-            }
         } else {
             // four slots per step on packed FP32x2 operations: e = d_i + (-r_j) rounds as
             // d_i - r_j, and d2 = fma(ex, ex, fma(ey, ey, ez * ez)) per slot as in scalar form.
@@ -299,6 +295,10 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
                     nearm |= (d2[s] <= outAbove ? 1u : 0u) << (t + s);
                 }
             }
+        }
+        if (filled < kWarp) {  // the sentinels of a partial block fold to anywhere, and where r^2 overflows
+            hit &= (1u << filled) - 1u;  // FP32 they are as near as every pair
+            nearm &= (1u << filled) - 1u;
         }
         if (valid) {
             // a pair within the FP32 margin of the radius (rare): the exact test
@@ -651,6 +651,8 @@ __device__ __forceinline__ bool mutualPair(const MutualArgs& a, int64_t i, const
     if (__float_as_uint(bj.v[6]) > a.ngmax &&
         i > int64_t(__ldg(a.nbr + listSlot(j - a.first, a.ngmax - 1, a.stride))))
         return false;
+    const float R2s = bj.v[5], R2j = fabsf(R2s);
+    if (fmaxf(R2j, fabsf(bi.v[5])) > a.wrapSafe2) return false;
     int cj[3];
     unpackCell(u64(__float_as_uint(bj.v[0])) | (u64(__float_as_uint(bj.v[1])) << 32), cj);
     const float lv[3] = {bi.v[2] - bj.v[2], bi.v[3] - bj.v[3], bi.v[4] - bj.v[4]};
@@ -671,14 +673,12 @@ __device__ __forceinline__ bool mutualPair(const MutualArgs& a, int64_t i, const
         }
         r[k] = fmaf(float(d), a.u[k], lv[k]);
     }
-    const float R2s = bj.v[5];
     // across a periodic face only a target that takes the minimum image can list i
     if (wrapped && !(R2s < 0.f)) return false;
-    if (fmaxf(fabsf(R2s), fabsf(bi.v[5])) > a.wrapSafe2) return false;
     const float d2 = fmaf(r[0], r[0], fmaf(r[1], r[1], r[2] * r[2]));
-    const float R2 = fabsf(R2s), eps = 0x1p-17f * R2;
-    if (d2 < R2 - eps) return true;
-    if (d2 > R2 + eps) return false;
+    const float eps = 0x1p-17f * R2j;
+    if (d2 < R2j - eps) return true;
+    if (d2 > R2j + eps) return false;
     return mutualExact(a, i, j, loadH(a.h, a.hIsFloat, j));
 }
 
