@@ -98,6 +98,12 @@ struct WarpSmem {
     alignas(16) float cull[8];
 };
 
+// Fold: groups whose pairs need a fold each do it in FP32 (launched for sets below kFoldBelow, where
+// such groups occur with ordinary h); without it they run the FP64 test for every pair, and the code of the
+// fold does not cost the large sets registers (1 % of the search at 27M).
+constexpr int64_t kFoldBelow = 100000;
+
+template<bool Fold>
 __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
 {
     __shared__ WarpSmem smem[kWarpsPerBlock];
@@ -209,7 +215,7 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
     // dropped and the rest appended, in ascending index order, to the warp's queue by ballot
     // compaction.  A dropped candidate is farther than 2h from every target along one axis, so the
     // reference's FP64 test rejects it too.  Each full queue block of 32 is tested by every target
-    // with a fixed trip count; the last, partial block has far-away sentinels in its empty slots.
+    // with a fixed trip count; the last, partial block has NaN in its empty slots.
     // Groups that fold their pairs keep every candidate.
     const float cullPad = 32.f * 0x1p-24f * (Rg + fmaxf(a.u[0], fmaxf(a.u[1], a.u[2])));
     const float bxl = gmin[0] - cullPad, bxh = gmax[0] + cullPad;
@@ -246,67 +252,71 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
     int qn = 0;  // candidates in the queue
     auto testBlock = [&](int filled) {
         if (valid) tested += unsigned(filled);
-        uint32_t hit = 0, nearm = 0;
-        if (foldPairs) {
-            // offsets of target and candidate may differ by up to L: the nearest image of the
-            // difference, in FP32.  Where 2h < L/2 there is one image within the radius; beyond,
-            // images at equal distance give the same d2 to rounding.
-#pragma unroll 1
-            for (int t = 0; t < filled; t += 4) {
-                const float4 X = *reinterpret_cast<const float4*>(&sm.nx[t]);
-                const float4 Y = *reinterpret_cast<const float4*>(&sm.ny[t]);
-                const float4 Z = *reinterpret_cast<const float4*>(&sm.nz[t]);
-                const float x[4] = {X.x, X.y, X.z, X.w}, y[4] = {Y.x, Y.y, Y.z, Y.w}, z[4] = {Z.x, Z.y, Z.z, Z.w};
-#pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    float ex = dxi + x[s], ey = dyi + y[s], ez = dzi + z[s];
-                    ex = fmaf(-b.Lf[0], rintf(ex * foldL[0]), ex);
-                    ey = fmaf(-b.Lf[1], rintf(ey * foldL[1]), ey);
-                    ez = fmaf(-b.Lf[2], rintf(ez * foldL[2]), ez);
-                    const float d2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
-                    hit |= (d2 < inBelow ? 1u : 0u) << (t + s);
-                    nearm |= (d2 <= outAbove ? 1u : 0u) << (t + s);
+        if (!Fold && foldPairs) {
+            if (valid)
+                for (int t = 0; t < filled; ++t) {
+                    const uint32_t j = sm.idx[t];
+                    if (exactIn(j)) take(j);
                 }
-            }
         } else {
-            // four slots per step on packed FP32x2 operations: e = d_i + (-r_j) rounds as
-            // d_i - r_j, and d2 = fma(ex, ex, fma(ey, ey, ez * ez)) per slot as in scalar form.
-            // The block's decisions go into two 32-bit masks (d2 below the margin: neighbour; d2
-            // within it: exact FP64 test), then each lane appends its neighbours slot by slot in
-            // ascending order, one loop trip per neighbour instead of a predicated append per slot.
-            const float2 dx2 = make_float2(dxi, dxi), dy2 = make_float2(dyi, dyi), dz2 = make_float2(dzi, dzi);
-#pragma unroll
-            for (int t = 0; t < kWarp; t += 4) {
-                const float4 X = *reinterpret_cast<const float4*>(&sm.nx[t]);
-                const float4 Y = *reinterpret_cast<const float4*>(&sm.ny[t]);
-                const float4 Z = *reinterpret_cast<const float4*>(&sm.nz[t]);
-                const float2 ex0 = __fadd2_rn(dx2, make_float2(X.x, X.y));
-                const float2 ex1 = __fadd2_rn(dx2, make_float2(X.z, X.w));
-                const float2 ey0 = __fadd2_rn(dy2, make_float2(Y.x, Y.y));
-                const float2 ey1 = __fadd2_rn(dy2, make_float2(Y.z, Y.w));
-                const float2 ez0 = __fadd2_rn(dz2, make_float2(Z.x, Z.y));
-                const float2 ez1 = __fadd2_rn(dz2, make_float2(Z.z, Z.w));
-                const float2 q0 = __ffma2_rn(ex0, ex0, __ffma2_rn(ey0, ey0, __fmul2_rn(ez0, ez0)));
-                const float2 q1 = __ffma2_rn(ex1, ex1, __ffma2_rn(ey1, ey1, __fmul2_rn(ez1, ez1)));
-                const float d2[4] = {q0.x, q0.y, q1.x, q1.y};
-#pragma unroll
-                for (int s = 0; s < 4; ++s) {
-                    hit |= (d2[s] < inBelow ? 1u : 0u) << (t + s);
-                    nearm |= (d2[s] <= outAbove ? 1u : 0u) << (t + s);
+            uint32_t hit = 0, nearm = 0;
+            if (Fold && foldPairs) {
+                // offsets of target and candidate may differ by up to L: the nearest image of the
+                // difference, in FP32.  Where 2h < L/2 there is one image within the radius; beyond,
+                // images at equal distance give the same d2 to rounding.
+    #pragma unroll 1
+                for (int t = 0; t < filled; t += 4) {
+                    const float4 X = *reinterpret_cast<const float4*>(&sm.nx[t]);
+                    const float4 Y = *reinterpret_cast<const float4*>(&sm.ny[t]);
+                    const float4 Z = *reinterpret_cast<const float4*>(&sm.nz[t]);
+                    const float x[4] = {X.x, X.y, X.z, X.w}, y[4] = {Y.x, Y.y, Y.z, Y.w}, z[4] = {Z.x, Z.y, Z.z, Z.w};
+    #pragma unroll
+                    for (int s = 0; s < 4; ++s) {
+                        float ex = dxi + x[s], ey = dyi + y[s], ez = dzi + z[s];
+                        ex = fmaf(-b.Lf[0], rintf(ex * foldL[0]), ex);
+                        ey = fmaf(-b.Lf[1], rintf(ey * foldL[1]), ey);
+                        ez = fmaf(-b.Lf[2], rintf(ez * foldL[2]), ez);
+                        const float d2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+                        hit |= (d2 < inBelow ? 1u : 0u) << (t + s);
+                        nearm |= (d2 <= outAbove ? 1u : 0u) << (t + s);
+                    }
+                }
+            } else {
+                // four slots per step on packed FP32x2 operations: e = d_i + (-r_j) rounds as
+                // d_i - r_j, and d2 = fma(ex, ex, fma(ey, ey, ez * ez)) per slot as in scalar form.
+                // The block's decisions go into two 32-bit masks (d2 below the margin: neighbour; d2
+                // within it: exact FP64 test), then each lane appends its neighbours slot by slot in
+                // ascending order, one loop trip per neighbour instead of a predicated append per slot.
+                const float2 dx2 = make_float2(dxi, dxi), dy2 = make_float2(dyi, dyi), dz2 = make_float2(dzi, dzi);
+    #pragma unroll
+                for (int t = 0; t < kWarp; t += 4) {
+                    const float4 X = *reinterpret_cast<const float4*>(&sm.nx[t]);
+                    const float4 Y = *reinterpret_cast<const float4*>(&sm.ny[t]);
+                    const float4 Z = *reinterpret_cast<const float4*>(&sm.nz[t]);
+                    const float2 ex0 = __fadd2_rn(dx2, make_float2(X.x, X.y));
+                    const float2 ex1 = __fadd2_rn(dx2, make_float2(X.z, X.w));
+                    const float2 ey0 = __fadd2_rn(dy2, make_float2(Y.x, Y.y));
+                    const float2 ey1 = __fadd2_rn(dy2, make_float2(Y.z, Y.w));
+                    const float2 ez0 = __fadd2_rn(dz2, make_float2(Z.x, Z.y));
+                    const float2 ez1 = __fadd2_rn(dz2, make_float2(Z.z, Z.w));
+                    const float2 q0 = __ffma2_rn(ex0, ex0, __ffma2_rn(ey0, ey0, __fmul2_rn(ez0, ez0)));
+                    const float2 q1 = __ffma2_rn(ex1, ex1, __ffma2_rn(ey1, ey1, __fmul2_rn(ez1, ez1)));
+                    const float d2[4] = {q0.x, q0.y, q1.x, q1.y};
+    #pragma unroll
+                    for (int s = 0; s < 4; ++s) {
+                        hit |= (d2[s] < inBelow ? 1u : 0u) << (t + s);
+                        nearm |= (d2[s] <= outAbove ? 1u : 0u) << (t + s);
+                    }
                 }
             }
-        }
-        if (filled < kWarp) {  // the sentinels of a partial block fold to anywhere, and where r^2 overflows
-            hit &= (1u << filled) - 1u;  // FP32 they are as near as every pair
-            nearm &= (1u << filled) - 1u;
-        }
-        if (valid) {
-            // a pair within the FP32 margin of the radius (rare): the exact test
-            for (uint32_t band = nearm & ~hit; band != 0; band &= band - 1u) {
-                const int s = __ffs(band) - 1;
-                if (exactIn(sm.idx[s])) hit |= 1u << s;
+            if (valid) {
+                // a pair within the FP32 margin of the radius (rare): the exact test
+                for (uint32_t band = nearm & ~hit; band != 0; band &= band - 1u) {
+                    const int s = __ffs(band) - 1;
+                    if (exactIn(sm.idx[s])) hit |= 1u << s;
+                }
+                for (; hit != 0; hit &= hit - 1u) take(sm.idx[__ffs(hit) - 1]);
             }
-            for (; hit != 0; hit &= hit - 1u) take(sm.idx[__ffs(hit) - 1]);
         }
         __syncwarp();
     };
@@ -348,13 +358,12 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
             __syncwarp();
         }
     };
-    // the partial last block: sentinels (FP32 distance +inf) in the empty slots
+    // the partial last block: NaN in the empty slots, so that neither comparison holds (also where r^2
+    // overflows FP32 and every pair is within the margin)
     auto drain = [&]() {
         if (qn == 0) return;
         if (lane >= qn) {
-            sm.nx[lane] = -1e30f;
-            sm.ny[lane] = -1e30f;
-            sm.nz[lane] = -1e30f;
+            sm.nx[lane] = sm.ny[lane] = sm.nz[lane] = __int_as_float(0x7fffffff);
         }
         __syncwarp();
         testBlock(qn);
@@ -858,7 +867,8 @@ int runSearch(sphgb_ctx* c, const double* x, const double* y, const double* z, c
     a.stats = c->counters.as<unsigned long long>();
     int64_t groups = (last - first + kWarp - 1) / kWarp;
     unsigned blocks = unsigned((groups + kWarpsPerBlock - 1) / kWarpsPerBlock);
-    nbrGroupKernel<<<blocks, kNbrBlock, 0, c->stream>>>(a);
+    if (c->n < kFoldBelow) nbrGroupKernel<true><<<blocks, kNbrBlock, 0, c->stream>>>(a);
+    else nbrGroupKernel<false><<<blocks, kNbrBlock, 0, c->stream>>>(a);
     return launched(c, "nbrGroupKernel");
 }
 
