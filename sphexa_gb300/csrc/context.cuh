@@ -228,9 +228,10 @@ int passMomentumEnergyVe(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_
 int buildTranspose(sphgb_ctx* c);
 // owned lists of the current lists from list membership (mixed adjoint)
 int buildOwnedFromLists(sphgb_ctx* c);
-// stable LSD radix sort of 64-bit keys (bits [0, endBit)) with optional 32-bit values, out of place
+// stable LSD radix sort of 64-bit keys (bits [beginBit, endBit), in whole bytes from beginBit) with
+// optional 32-bit values, out of place
 int radixSort(sphgb_ctx* c, const u64* keysIn, u64* keysOut, const uint32_t* valsIn, uint32_t* valsOut, int64_t n,
-              int endBit);
+              int endBit, int beginBit = 0);
 // the radix sort's give-up flag: queue its copy to the host before a stream sync, test it after
 // (SPHGB_ERR_TIMEOUT when a look-back wait gave up; the flag is then cleared)
 int sortStatusAsync(sphgb_ctx* c);

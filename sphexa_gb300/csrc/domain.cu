@@ -57,13 +57,17 @@ __global__ void minmaxPartials(const double* __restrict__ x, const double* __res
     }
 }
 
-__global__ void minmaxFinal(const double* __restrict__ part, int nb, double* __restrict__ out)
+// six warps, one per minimum or maximum
+__global__ void __launch_bounds__(6 * kWarp) minmaxFinal(const double* __restrict__ part, int nb, double* __restrict__ out)
 {
-    int k = threadIdx.x;
-    if (k >= 6) return;
+    const int k = threadIdx.x / kWarp, lane = threadIdx.x % kWarp;
     double r = part[k];
-    for (int b = 1; b < nb; ++b) r = (k & 1) ? fmax(r, part[b * 6 + k]) : fmin(r, part[b * 6 + k]);
-    out[k] = r;
+    for (int b = lane; b < nb; b += kWarp) r = (k & 1) ? fmax(r, part[b * 6 + k]) : fmin(r, part[b * 6 + k]);
+    for (int o = 16; o > 0; o >>= 1) {
+        const double q = __shfl_xor_sync(0xffffffffu, r, o);
+        r = (k & 1) ? fmax(r, q) : fmin(r, q);
+    }
+    if (lane == 0) out[k] = r;
 }
 
 // ---- keys ----
@@ -96,18 +100,35 @@ __global__ void gatherKernel(GatherSet g, const uint32_t* __restrict__ order, in
     }
 }
 
+// the gathered fields back to their arrays, and the sorted keys out: one launch for all
+__global__ void copyBackKernel(GatherSet g, const u64* __restrict__ keys, u64* __restrict__ keysOut, int64_t n)
+{
+    const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (i >= n) return;
+    if (keysOut) keysOut[i] = keys[i];
+#pragma unroll 2
+    for (int f = 0; f < g.count; ++f) {
+        if (g.esz[f] == 8) static_cast<double*>(const_cast<void*>(g.src[f]))[i] = static_cast<const double*>(g.dst[f])[i];
+        else static_cast<float*>(const_cast<void*>(g.src[f]))[i] = static_cast<const float*>(g.dst[f])[i];
+    }
+}
+
 // ---- tree ----
-__global__ void splitCountKernel(const u64* __restrict__ keys, int64_t n, int bucket, uint32_t* __restrict__ cnt)
+// deepest: 1 + the deepest level of a split node (0: none), the depth of the leaves
+__global__ void splitCountKernel(const u64* __restrict__ keys, int64_t n, int bucket, uint32_t* __restrict__ cnt,
+                                 unsigned* __restrict__ deepest)
 {
     int64_t s = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-    if (s > n) return;
-    uint32_t c = 0;
+    uint32_t c = 0, depth = 0;
     if (s + bucket < n) {
         int deep = min(commonPrefixBits(keys[s], keys[s + bucket]) / 3, kMaxLevel - 1);
         int first = (s == 0) ? 0 : commonPrefixBits(keys[s - 1], keys[s]) / 3 + 1;
         c = deep >= first ? uint32_t(deep - first + 1) : 0u;
+        if (c) depth = uint32_t(deep + 1);
     }
-    cnt[s] = c;  // cnt[n] = 0 closes the exclusive scan
+    if (s <= n) cnt[s] = c;  // cnt[n] = 0 closes the exclusive scan
+    depth = __reduce_max_sync(0xffffffffu, depth);
+    if ((threadIdx.x & 31) == 0 && depth > 0 && depth > *deepest) atomicMax(deepest, depth);
 }
 
 __global__ void splitEmitKernel(const u64* __restrict__ keys, int64_t n, int bucket, const uint32_t* __restrict__ off,
@@ -413,7 +434,7 @@ int domainSync(sphgb_ctx* c, sphgb_particles* p, sphgb_box* box)
         double* part = c->minmax.as<double>();
         minmaxPartials<<<nb, kBlock, 0, st>>>(p->x, p->y, p->z, n, part);
         SPHGB_TRY(launched(c, "minmaxPartials"));
-        minmaxFinal<<<1, 32, 0, st>>>(part, nb, part + 6 * nb);
+        minmaxFinal<<<1, 6 * kWarp, 0, st>>>(part, nb, part + 6 * nb);
         SPHGB_TRY(launched(c, "minmaxFinal"));
         double ext[6];
         SPHGB_CUDA(cudaMemcpyAsync(ext, part + 6 * nb, sizeof(ext), cudaMemcpyDeviceToHost, st));
@@ -488,20 +509,30 @@ int domainSync(sphgb_ctx* c, sphgb_particles* p, sphgb_box* box)
     }
     gatherKernel<<<gridFor(n, kBlock), kBlock, 0, st>>>(g, c->order.as<uint32_t>(), n);
     SPHGB_TRY(launched(c, "gatherKernel"));
-    for (int f = 0; f < g.count; ++f)
-        SPHGB_CUDA(cudaMemcpyAsync(const_cast<void*>(g.src[f]), g.dst[f], size_t(g.esz[f]) * n,
-                                   cudaMemcpyDeviceToDevice, st));
-    if (p->keys) SPHGB_CUDA(cudaMemcpyAsync(p->keys, c->keys.p, sizeof(u64) * n, cudaMemcpyDeviceToDevice, st));
+    // one launch instead of eleven copies while launches count; large copies are 4 % faster by the copy
+    // engine's kernels (27M: the sync takes 6.45 ms with copies, 6.65 with the kernel)
+    if (n < (int64_t(1) << 21)) {
+        copyBackKernel<<<gridFor(n, kBlock), kBlock, 0, st>>>(g, c->keys.as<u64>(), reinterpret_cast<u64*>(p->keys), n);
+        SPHGB_TRY(launched(c, "copyBackKernel"));
+    } else {
+        for (int f = 0; f < g.count; ++f)
+            SPHGB_CUDA(cudaMemcpyAsync(const_cast<void*>(g.src[f]), g.dst[f], size_t(g.esz[f]) * n,
+                                       cudaMemcpyDeviceToDevice, st));
+        if (p->keys) SPHGB_CUDA(cudaMemcpyAsync(p->keys, c->keys.p, sizeof(u64) * n, cudaMemcpyDeviceToDevice, st));
+    }
     c->haveSync = true;
     c->haveNbr = false;
     return buildTree(c, rebalance);
 }
 
 // exclusive sum of cnt[0..count) into off[0..count), returns off[count - 1] + cnt[count - 1]
-static int scanCounts(sphgb_ctx* c, uint32_t* cnt, uint32_t* off, int64_t count, int64_t* total)
+// (and, where asked, a device word beside it)
+static int scanCounts(sphgb_ctx* c, uint32_t* cnt, uint32_t* off, int64_t count, int64_t* total,
+                      const unsigned* word = nullptr, unsigned* wordOut = nullptr)
 {
     SPHGB_TRY(exclusiveScan(c, cnt, off, count));
     uint32_t t = 0;
+    if (word) SPHGB_CUDA(cudaMemcpyAsync(wordOut, word, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
     SPHGB_CUDA(cudaMemcpyAsync(&t, off + count - 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
     SPHGB_CUDA(cudaStreamSynchronize(c->stream));
     *total = t;  // cnt[count - 1] is 0 by construction
@@ -518,13 +549,19 @@ int buildTree(sphgb_ctx* c, bool rebalance)
     const int bucket = int(c->prm.bucket);
     const u64* keys = c->keys.as<u64>();
     int64_t S = 0, L = 0;
+    unsigned depth = kMaxLevel;  // of the leaves; known for the converged tree
 
     if (!rebalance) {
         SPHGB_TRY(c->splitCount.ensure(sizeof(uint32_t) * (n + 1)));
         SPHGB_TRY(c->splitOffset.ensure(sizeof(uint32_t) * (n + 1)));
-        splitCountKernel<<<gridFor(n + 1, kBlock), kBlock, 0, st>>>(keys, n, bucket, c->splitCount.as<uint32_t>());
+        SPHGB_TRY(c->levelRangeDev.ensure(sizeof(int32_t) * 2 * (kMaxLevel + 2)));
+        unsigned* deepest = c->levelRangeDev.as<unsigned>();  // filled later: its first word is free here
+        SPHGB_CUDA(cudaMemsetAsync(deepest, 0, sizeof(unsigned), st));
+        splitCountKernel<<<gridFor(n + 1, kBlock), kBlock, 0, st>>>(keys, n, bucket, c->splitCount.as<uint32_t>(),
+                                                                   deepest);
         SPHGB_TRY(launched(c, "splitCountKernel"));
-        SPHGB_TRY(scanCounts(c, c->splitCount.as<uint32_t>(), c->splitOffset.as<uint32_t>(), n + 1, &S));
+        SPHGB_TRY(scanCounts(c, c->splitCount.as<uint32_t>(), c->splitOffset.as<uint32_t>(), n + 1, &S, deepest,
+                             &depth));
         L = 7 * S + 1;
         SPHGB_TRY(c->leafKeysTmp.ensure(sizeof(u64) * (L + 1)));
         SPHGB_TRY(c->leaves.ensure(sizeof(u64) * (L + 1)));
@@ -534,7 +571,9 @@ int buildTree(sphgb_ctx* c, bool rebalance)
                                                                c->leafKeysTmp.as<u64>(), c->internalTmp.as<u64>());
         SPHGB_TRY(launched(c, "splitEmitKernel"));
         if (L > 1) {
-            SPHGB_TRY(radixSort(c, c->leafKeysTmp.as<u64>(), c->leaves.as<u64>(), nullptr, nullptr, L, 63));
+            // leaves of depth d start at multiples of 8^(21 - d): only the bits above differ
+            SPHGB_TRY(radixSort(c, c->leafKeysTmp.as<u64>(), c->leaves.as<u64>(), nullptr, nullptr, L, 63,
+                                3 * (kMaxLevel - int(depth))));
         } else {
             SPHGB_CUDA(cudaMemsetAsync(c->leaves.p, 0, sizeof(u64), st));
         }
@@ -572,7 +611,10 @@ int buildTree(sphgb_ctx* c, bool rebalance)
     c->numInternal = S;
     c->numLeaves = L;
     c->numNodes = L + S;
-    if (S > 0) SPHGB_TRY(radixSort(c, c->internalTmp.as<u64>(), c->internalCodes.as<u64>(), nullptr, nullptr, S, 62));
+    // the code of a split node of level l <= depth - 1 is below 2^(3 l + 1)
+    if (S > 0)
+        SPHGB_TRY(radixSort(c, c->internalTmp.as<u64>(), c->internalCodes.as<u64>(), nullptr, nullptr, S,
+                            3 * (int(depth) - 1) + 1));
     setKey<<<1, 1, 0, st>>>(c->leaves.as<u64>() + L, kKeyEnd);
     SPHGB_TRY(launched(c, "setKey"));
 

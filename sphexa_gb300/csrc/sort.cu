@@ -16,6 +16,7 @@
 //                   look-back stops at the first tile that has).  The tile is staged in shared
 //                   memory grouped by digit and written out in runs: equal digits keep their input
 //                   order, so every pass, and the sort, is stable.
+// Up to kSmallSort items are sorted by one block in shared memory, all digits in one launch.
 // A tile waits only on tiles that drew earlier tickets, which are already resident, so the
 // look-back always ends; its spin is bounded all the same and a give-up raises the context's
 // sort flag (read by sortStatus) instead of hanging.
@@ -65,10 +66,10 @@ __device__ __forceinline__ uint32_t loadRelaxed32(const uint32_t* p)
     return v;
 }
 
-// digit histograms of passes [0, passes) over all keys; a warp whose 32 keys share a digit adds
+// digit histograms of passes [0, passes), pass p the 8 bits from beginBit + 8 p, over all keys; a warp whose 32 keys share a digit adds
 // them with one atomic (sorted or nearly sorted input would otherwise serialise on one counter)
-__global__ void __launch_bounds__(kThreads) allDigitsHist(const u64* __restrict__ keys, int64_t n, int passes,
-                                                          uint32_t* __restrict__ hist)
+__global__ void __launch_bounds__(kThreads) allDigitsHist(const u64* __restrict__ keys, int64_t n, int beginBit,
+                                                          int passes, uint32_t* __restrict__ hist)
 {
     __shared__ uint32_t h[kMaxPasses][kRadix];
     for (int p = 0; p < kMaxPasses; ++p) h[p][threadIdx.x] = 0;
@@ -83,7 +84,7 @@ __global__ void __launch_bounds__(kThreads) allDigitsHist(const u64* __restrict_
 #pragma unroll
         for (int p = 0; p < kMaxPasses; ++p) {
             if (p >= passes) break;
-            const unsigned d = unsigned(key >> (8 * p)) & (kRadix - 1);
+            const unsigned d = unsigned(key >> (beginBit + 8 * p)) & (kRadix - 1);
             const unsigned d0 = __shfl_sync(0xffffffffu, d, 0);
             if (__all_sync(0xffffffffu, !valid || d == d0)) {
                 if (lane == 0) atomicAdd(&h[p][d0], unsigned(__popc(vm)));
@@ -148,7 +149,8 @@ __global__ void __launch_bounds__(kRadix) digitPlan(uint32_t* __restrict__ hist,
 template<bool WithVals>
 __global__ void __launch_bounds__(kThreads, 3) onesweep(const u64* keysIn, const uint32_t* valsIn, u64* keysTmp,
                                                      uint32_t* valsTmp, u64* keysOut, uint32_t* valsOut,
-                                                     int64_t n, int pass, const uint32_t* __restrict__ digitStart,
+                                                     int64_t n, int beginBit, int pass,
+                                                     const uint32_t* __restrict__ digitStart,
                                                      u64* __restrict__ look, uint32_t* __restrict__ state)
 {
     extern __shared__ u64 staged[];  // kTile keys, then kTile values
@@ -165,7 +167,7 @@ __global__ void __launch_bounds__(kThreads, 3) onesweep(const u64* keysIn, const
     const uint32_t* vSrc = srcSel == 0 ? valsIn : srcSel == 1 ? valsTmp : valsOut;
     u64* kDst = dstSel == 1 ? keysTmp : keysOut;
     uint32_t* vDst = dstSel == 1 ? valsTmp : valsOut;
-    const int shift = 8 * pass;
+    const int shift = beginBit + 8 * pass;
     const uint32_t epoch = state[kEpoch + pass];
 
     if (tid == 0) tileSh = atomicAdd(state + kTicket + pass, 1u);
@@ -268,6 +270,85 @@ __global__ void __launch_bounds__(kThreads, 3) onesweep(const u64* keysIn, const
         const uint32_t pos = globalStart[d] + (t - localStart[d]);
         kDst[pos] = k;
         if (WithVals) vDst[pos] = stagedVals[t];
+    }
+}
+
+// Sets of up to kSmallSort items: one block, every digit in shared memory.  Launches and look-back set
+// the time of a sort of one tile (1728 pairs: 10 launches, 150 us; one launch now, 30 us in
+// all), so the tree's key sorts and the smallest syncs come here.  Per digit each warp ranks its 128
+// consecutive items by warp match, the 256 digits' per-warp counts are prefixed, and the items move to
+// their slots; digits that all keys share are skipped.  4096 items fill 88 KB of shared memory.
+constexpr int kSmallThreads = 1024, kSmallItems = 4, kSmallSort = kSmallThreads * kSmallItems;
+constexpr int kSmallWarps = kSmallThreads / 32, kSmallWarpKeys = 32 * kSmallItems;
+constexpr size_t kSmallBytes = (sizeof(u64) + sizeof(uint32_t)) * kSmallSort + sizeof(uint32_t) * kSmallWarps * kRadix;
+
+template<bool WithVals>
+__global__ void __launch_bounds__(kSmallThreads) smallSort(const u64* keysIn, const uint32_t* valsIn, u64* keysOut,
+                                                           uint32_t* valsOut, int n, int beginBit, int passes)
+{
+    extern __shared__ u64 smallKeys[];  // kSmallSort keys, kSmallSort values, per-warp digit counts
+    uint32_t* smallVals = reinterpret_cast<uint32_t*>(smallKeys + kSmallSort);
+    uint32_t(*cnt)[kRadix] = reinterpret_cast<uint32_t(*)[kRadix]>(smallVals + kSmallSort);
+    __shared__ uint32_t sh[32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    const int base = warp * kSmallWarpKeys;
+    for (int i = tid; i < n; i += kSmallThreads) {
+        smallKeys[i] = keysIn[i];
+        if (WithVals) smallVals[i] = valsIn[i];
+    }
+    __syncthreads();
+    u64 key[kSmallItems];
+    uint32_t val[kSmallItems];
+    const u64 first = smallKeys[0];
+    u64 diff = 0;
+    for (int i = tid; i < n; i += kSmallThreads) diff |= smallKeys[i] ^ first;
+    for (int p = 0; p < passes; ++p) {
+        const int shift = beginBit + 8 * p;
+        if (!__syncthreads_or(int((diff >> shift) & (kRadix - 1)))) continue;  // uniform
+        uint32_t rank[kSmallItems];
+        for (int q = lane; q < kRadix; q += 32) cnt[warp][q] = 0;
+        __syncwarp();
+#pragma unroll
+        for (int r = 0; r < kSmallItems; ++r) {
+            const int i = base + r * 32 + lane;
+            const bool valid = i < n;
+            key[r] = valid ? smallKeys[i] : 0;
+            if (WithVals) val[r] = valid ? smallVals[i] : 0u;
+            const unsigned d = valid ? unsigned(key[r] >> shift) & (kRadix - 1) : unsigned(kRadix);
+            const unsigned peers = __match_any_sync(0xffffffffu, d);
+            uint32_t before = 0;
+            if (valid) before = cnt[warp][d];
+            __syncwarp();
+            if (valid && (peers & lt) == 0) cnt[warp][d] = before + __popc(peers);
+            __syncwarp();
+            rank[r] = valid ? (d | ((before + __popc(peers & lt)) << 8)) : 0xffffffffu;
+        }
+        __syncthreads();
+        uint32_t sum = 0;
+        if (tid < kRadix)
+            for (int w = 0; w < kSmallWarps; ++w) {
+                const uint32_t t = cnt[w][tid];
+                cnt[w][tid] = sum;
+                sum += t;
+            }
+        uint32_t total;
+        const uint32_t start = blockExclusiveScan(sum, sh, total);
+        if (tid < kRadix)
+            for (int w = 0; w < kSmallWarps; ++w) cnt[w][tid] += start;
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < kSmallItems; ++r) {
+            if (rank[r] == 0xffffffffu) continue;
+            const uint32_t pos = cnt[warp][rank[r] & (kRadix - 1)] + (rank[r] >> 8);
+            smallKeys[pos] = key[r];
+            if (WithVals) smallVals[pos] = val[r];
+        }
+        __syncthreads();
+    }
+    for (int i = tid; i < n; i += kSmallThreads) {
+        keysOut[i] = smallKeys[i];
+        if (WithVals) valsOut[i] = smallVals[i];
     }
 }
 
@@ -384,10 +465,10 @@ static int ensureZeroed(sphgb_ctx* c, DBuf& b, size_t need)
 }
 
 int radixSort(sphgb_ctx* c, const u64* keysIn, u64* keysOut, const uint32_t* valsIn, uint32_t* valsOut, int64_t n,
-              int endBit)
+              int endBit, int beginBit)
 {
     if (n <= 0) return SPHGB_OK;
-    if (endBit < 1 || endBit > 64 || (valsIn == nullptr) != (valsOut == nullptr)) return SPHGB_ERR_ARG;
+    if (endBit < 1 || endBit > 64 || beginBit < 0 || beginBit >= endBit || (valsIn == nullptr) != (valsOut == nullptr)) return SPHGB_ERR_ARG;
     if (n >= (int64_t(1) << 32)) return SPHGB_ERR_TOO_LARGE;  // slots and counts are 32-bit
     cudaStream_t st = c->stream;
     if (n == 1) {
@@ -396,7 +477,26 @@ int radixSort(sphgb_ctx* c, const u64* keysIn, u64* keysOut, const uint32_t* val
         return SPHGB_OK;
     }
     const bool withVals = valsIn != nullptr;
-    const int passes = (endBit + 7) / 8;
+    const int passes = (endBit - beginBit + 7) / 8;
+    if (!c->sortSmemSet) {  // the staged tile of (key, value) pairs exceeds the default 48 KB
+        SPHGB_CUDA(cudaFuncSetAttribute(onesweep<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        int(kStagePairs)));
+        SPHGB_CUDA(cudaFuncSetAttribute(onesweep<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        int(kStageKeys)));
+        SPHGB_CUDA(cudaFuncSetAttribute(smallSort<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmallBytes)));
+        SPHGB_CUDA(cudaFuncSetAttribute(smallSort<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        int(kSmallBytes)));
+        c->sortSmemSet = true;
+    }
+    if (n <= kSmallSort) {
+        if (withVals)
+            smallSort<true><<<1, kSmallThreads, kSmallBytes, st>>>(keysIn, valsIn, keysOut, valsOut, int(n), beginBit,
+                                                                   passes);
+        else
+            smallSort<false><<<1, kSmallThreads, kSmallBytes, st>>>(keysIn, nullptr, keysOut, nullptr, int(n), beginBit,
+                                                                    passes);
+        return launched(c, "smallSort");
+    }
     const int64_t tiles = (n + kTile - 1) / kTile;
     // scratch: ping-pong keys (and values), digit histograms; look-back words; sort state
     const size_t bKeys = align256(sizeof(u64) * n), bVals = withVals ? align256(sizeof(uint32_t) * n) : 0;
@@ -409,27 +509,20 @@ int radixSort(sphgb_ctx* c, const u64* keysIn, u64* keysOut, const uint32_t* val
     SPHGB_TRY(ensureZeroed(c, c->sortState, sizeof(uint32_t) * kStateWords));
     uint32_t* state = c->sortState.as<uint32_t>();
 
-    if (!c->sortSmemSet) {  // the staged tile of (key, value) pairs exceeds the default 48 KB
-        SPHGB_CUDA(cudaFuncSetAttribute(onesweep<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        int(kStagePairs)));
-        SPHGB_CUDA(cudaFuncSetAttribute(onesweep<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        int(kStageKeys)));
-        c->sortSmemSet = true;
-    }
     SPHGB_CUDA(cudaMemsetAsync(hist, 0, sizeof(uint32_t) * kMaxPasses * kRadix, st));
     const unsigned histBlocks = unsigned(tiles < 8 * 152 ? tiles : 8 * 152);
-    allDigitsHist<<<histBlocks, kThreads, 0, st>>>(keysIn, n, passes, hist);
+    allDigitsHist<<<histBlocks, kThreads, 0, st>>>(keysIn, n, beginBit, passes, hist);
     SPHGB_TRY(launched(c, "allDigitsHist"));
     digitPlan<<<1, kRadix, 0, st>>>(hist, passes, n, state);
     SPHGB_TRY(launched(c, "digitPlan"));
     for (int pass = 0; pass < passes; ++pass) {
         if (withVals)
             onesweep<true><<<unsigned(tiles), kThreads, kStagePairs, st>>>(keysIn, valsIn, keysTmp, valsTmp, keysOut,
-                                                                           valsOut, n, pass, hist, c->sortLook.as<u64>(),
-                                                                           state);
+                                                                           valsOut, n, beginBit, pass, hist,
+                                                                           c->sortLook.as<u64>(), state);
         else
             onesweep<false><<<unsigned(tiles), kThreads, kStageKeys, st>>>(keysIn, nullptr, keysTmp, nullptr, keysOut,
-                                                                           nullptr, n, pass, hist,
+                                                                           nullptr, n, beginBit, pass, hist,
                                                                            c->sortLook.as<u64>(), state);
         SPHGB_TRY(launched(c, "onesweep"));
     }
