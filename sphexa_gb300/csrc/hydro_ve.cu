@@ -1240,65 +1240,6 @@ __global__ void meVeRec64Kernel(int64_t n, MeVeArgs a, ListView lv, double* __re
     rhof[j] = float(rho);
 }
 
-// Atwood weights a_mom, b_mom of a pair (momentum_energy_kern.hpp:160-190) in FP64: the exact decision
-// of |rho_i - rho_j| / (rho_i + rho_j) against 0.1 and 0.2 and, between them, the ramp
-// xm_i^(2-s) xm_j^s = xm_i^2 q and xm_j^(2-s) xm_i^s = xm_j^2 / q, q = (xm_j / xm_i)^s.  For the pairs
-// atwoodWeights leaves open: sums near a threshold, arguments beyond the table.
-__device__ __noinline__ double2 atwoodExact(double rhoi, double rhoj, double dln, double xmi, double xmj)
-{
-    constexpr double Atmin = 0.1, Atmax = 0.2, ramp = 1.0 / (Atmax - Atmin);
-    const double dr = fabs(rhoi - rhoj), sr = rhoi + rhoj;
-    if (lessNonNeg(dr, Atmin * sr)) return make_double2(xmi * xmi, xmj * xmj);
-    if (lessNonNeg(Atmax * sr, dr)) return make_double2(xmi * xmj, xmi * xmj);
-    const double s = ramp * (dr / sr - Atmin);
-    const double q = exp(s * dln);
-    return make_double2(xmi * xmi * q, xmj * xmj / q);
-}
-
-// the same weights with few FP64 instructions: the two flat branches are taken where FP32 copies of rho
-// decide safely (1e-6 of the sum beside a threshold, and sums FP32 cannot hold, go to atwoodExact).
-// On the ramp (a quarter of the pairs of a jittered lattice or a clustered sphere, so nearly every warp
-// is there for some lane) the quotient comes from a 20-bit reciprocal by two Newton corrections, and
-// q = e^a and 1 / q = e^-a, |a| <= 1/2, together from a table of e^(+-k/1024) and the even and odd parts
-// of the series of the rest, |rest| <= 2^-11: 21 FP64 instructions instead of two divisions and an exp.
-__device__ __forceinline__ void atwoodWeights(const double* __restrict__ rho, const double* __restrict__ lnxm,
-                                              const double4* __restrict__ expTab, int64_t i, int64_t j, float rhofi,
-                                              float rhofj, double xmi, double xmj, double& am, double& bm)
-{
-    const float dr = fabsf(rhofi - rhofj), sr = rhofi + rhofj;
-    am = xmi * xmi;
-    bm = xmj * xmj;
-    if (sr > 1e-30f && dr < (0.1f - 1e-6f) * sr) return;
-    if (sr > 1e-30f && dr > (0.2f + 1e-6f) * sr && dr < 1e38f) {
-        am = bm = xmi * xmj;
-        return;
-    }
-    const double rhoi = rho[i], rhoj = __ldg(rho + j), dln = __ldg(lnxm + j) - lnxm[i];
-    const double d = fabs(rhoi - rhoj), t = rhoi + rhoj;
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(t));
-    double at = d * y;
-    at = fma(fma(-t, at, d), y, at);
-    at = fma(fma(-t, at, d), y, at);
-    const double a = fma(10.0, at, -1.0) * dln;
-    // |a| from the high word, truncated to 20 bits, as a float: the nearest table node to within 2^-20
-    const unsigned hi = unsigned(__double2hiint(a)), mag = hi & 0x7fffffffu;
-    const bool onRamp = sr > 1e-30f && dr > (0.1f + 1e-6f) * sr && dr < (0.2f - 1e-6f) * sr && mag < 0x3fe00000u;
-    if (!onRamp) {
-        const double2 ab = atwoodExact(rhoi, rhoj, dln, xmi, xmj);
-        am = ab.x;
-        bm = ab.y;
-        return;
-    }
-    int k = mag < 0x3f300000u ? 0 : __float2int_rn(__uint_as_float((mag - (896u << 20)) << 3) * 1024.f);
-    k = (hi >> 31) ? -k : k;
-    const double4 e = expTab[kExpNodes + k];  // e^(k/1024), e^(-k/1024), k/1024
-    const double r = a - e.z, r2 = r * r;
-    const double even = r2 * fma(r2, 1.0 / 24.0, 0.5), odd = fma(r * r2, 1.0 / 6.0, r);
-    am *= fma(e.x, even + odd, e.x);
-    bm *= fma(e.y, even - odd, e.y);
-}
-
 // num / den by a 20-bit reciprocal and two Newton corrections of the quotient (five FP64 instructions,
 // within an ulp); den beyond 2^+-1000 takes the division
 __device__ __forceinline__ double quotient(double num, double den)

@@ -403,6 +403,27 @@ __device__ __forceinline__ double lookupVSlope(const KTab<Smooth>& tb, double v,
     }
 }
 
+// value at x = v / dx and its derivative d/dx, in table units
+template<bool Smooth>
+__device__ __forceinline__ double lookupXSlope(const KTab<Smooth>& tb, double x, double& slope)
+{
+    const TabSlot s = tabSlot(x);
+    if (s.k < 0) {
+        slope = 0.0;
+        return 0.0;
+    }
+    if constexpr (Smooth) {
+        const double2 a = __ldg(tb.t + 2 * s.k), b = __ldg(tb.t + 2 * s.k + 1);
+        const double f = s.frac;
+        slope = fma(fma(3.0 * b.y, f, 2.0 * b.x), f, a.y);
+        return fma(fma(fma(b.y, f, b.x), f, a.y), f, a.x);
+    } else {
+        const double2 t = __ldg(tb.t + s.k);
+        slope = t.y;
+        return fma(t.y, s.frac, t.x);
+    }
+}
+
 // the context's FP64 tables of W and dW/dv in its kernel form
 inline const double2* tabW64(const sphgb_ctx* c)
 {
@@ -472,6 +493,111 @@ __device__ __forceinline__ Rec4d ldRec4d(const Rec4d* p)
     Rec4d r;
     asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.v[0]), "=d"(r.v[1]), "=d"(r.v[2]), "=d"(r.v[3]) : "l"(p));
     return r;
+}
+
+// Atwood weights a_mom, b_mom of a pair (momentum_energy_kern.hpp:160-190) in FP64: the exact decision
+// of |rho_i - rho_j| / (rho_i + rho_j) against 0.1 and 0.2 and, between them, the ramp
+// xm_i^(2-s) xm_j^s = xm_i^2 q and xm_j^(2-s) xm_i^s = xm_j^2 / q, q = (xm_j / xm_i)^s.  For the pairs
+// atwoodWeights leaves open: sums near a threshold, arguments beyond the table.
+static __device__ __noinline__ double2 atwoodExact(double rhoi, double rhoj, double dln, double xmi, double xmj)
+{
+    constexpr double Atmin = 0.1, Atmax = 0.2, ramp = 1.0 / (Atmax - Atmin);
+    const double dr = fabs(rhoi - rhoj), sr = rhoi + rhoj;
+    if (lessNonNeg(dr, Atmin * sr)) return make_double2(xmi * xmi, xmj * xmj);
+    if (lessNonNeg(Atmax * sr, dr)) return make_double2(xmi * xmj, xmi * xmj);
+    const double s = ramp * (dr / sr - Atmin);
+    const double q = exp(s * dln);
+    return make_double2(xmi * xmi * q, xmj * xmj / q);
+}
+
+// the same weights with few FP64 instructions: the two flat branches are taken where FP32 copies of rho
+// decide safely (1e-6 of the sum beside a threshold, and sums FP32 cannot hold, go to atwoodExact).
+// On the ramp (a quarter of the pairs of a jittered lattice or a clustered sphere, so nearly every warp
+// is there for some lane) the quotient comes from a 20-bit reciprocal by two Newton corrections, and
+// q = e^a and 1 / q = e^-a, |a| <= 1/2, together from a table of e^(+-k/1024) and the even and odd parts
+// of the series of the rest, |rest| <= 2^-11: 21 FP64 instructions instead of two divisions and an exp.
+__device__ __forceinline__ void atwoodWeights(const double* __restrict__ rho, const double* __restrict__ lnxm,
+                                              const double4* __restrict__ expTab, int64_t i, int64_t j, float rhofi,
+                                              float rhofj, double xmi, double xmj, double& am, double& bm)
+{
+    const float dr = fabsf(rhofi - rhofj), sr = rhofi + rhofj;
+    am = xmi * xmi;
+    bm = xmj * xmj;
+    if (sr > 1e-30f && dr < (0.1f - 1e-6f) * sr) return;
+    if (sr > 1e-30f && dr > (0.2f + 1e-6f) * sr && dr < 1e38f) {
+        am = bm = xmi * xmj;
+        return;
+    }
+    const double rhoi = rho[i], rhoj = __ldg(rho + j), dln = __ldg(lnxm + j) - lnxm[i];
+    const double d = fabs(rhoi - rhoj), t = rhoi + rhoj;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(t));
+    double at = d * y;
+    at = fma(fma(-t, at, d), y, at);
+    at = fma(fma(-t, at, d), y, at);
+    const double a = fma(10.0, at, -1.0) * dln;
+    // |a| from the high word, truncated to 20 bits, as a float: the nearest table node to within 2^-20
+    const unsigned hi = unsigned(__double2hiint(a)), mag = hi & 0x7fffffffu;
+    const bool onRamp = sr > 1e-30f && dr > (0.1f + 1e-6f) * sr && dr < (0.2f - 1e-6f) * sr && mag < 0x3fe00000u;
+    if (!onRamp) {
+        const double2 ab = atwoodExact(rhoi, rhoj, dln, xmi, xmj);
+        am = ab.x;
+        bm = ab.y;
+        return;
+    }
+    int k = mag < 0x3f300000u ? 0 : __float2int_rn(__uint_as_float((mag - (896u << 20)) << 3) * 1024.f);
+    k = (hi >> 31) ? -k : k;
+    const double4 e = expTab[kExpNodes + k];  // e^(k/1024), e^(-k/1024), k/1024
+    const double r = a - e.z, r2 = r * r;
+    const double even = r2 * fma(r2, 1.0 / 24.0, 0.5), odd = fma(r * r2, 1.0 / 6.0, r);
+    am *= fma(e.x, even + odd, e.x);
+    bm *= fma(e.y, even - odd, e.y);
+}
+
+// the weights with what their derivatives need, from FP64 rho and ln xm (the adjoint): s of the ramp (0
+// below it, 1 above), and on it At = |rho_i - rho_j| / (rho_i + rho_j) and 1 / (rho_i + rho_j)
+struct AtwoodRamp {
+    double am, bm, s, At, srInv;
+    bool ramp;
+};
+
+__device__ __forceinline__ AtwoodRamp atwoodRamp(const double4* __restrict__ expTab, double rhoi, double rhoj,
+                                                 double lnxmi, double lnxmj, double xmi, double xmj)
+{
+    const double d = fabs(rhoi - rhoj), t = rhoi + rhoj;
+    AtwoodRamp o{xmi * xmi, xmj * xmj, 0.0, 0.0, 0.0, false};
+    if (lessNonNeg(d, 0.1 * t)) return o;
+    if (lessNonNeg(0.2 * t, d)) {
+        o.am = o.bm = xmi * xmj;
+        o.s = 1.0;
+        return o;
+    }
+    o.ramp = true;
+    const unsigned e0 = (unsigned(__double2hiint(t)) >> 20) & 0x7ffu;
+    const bool table = e0 - 23u <= 2000u;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(t));
+    y = fma(fma(-t, y, 1.0), y, y);
+    y = fma(fma(-t, y, 1.0), y, y);
+    o.srInv = table ? y : 1.0 / t;
+    o.At = d * o.srInv;
+    o.s = fma(10.0, o.At, -1.0);
+    const double a = o.s * (lnxmj - lnxmi);
+    const unsigned hi = unsigned(__double2hiint(a)), mag = hi & 0x7fffffffu;
+    if (mag >= 0x3fe00000u) {
+        const double q = exp(a);
+        o.am *= q;
+        o.bm /= q;
+        return o;
+    }
+    int k = mag < 0x3f300000u ? 0 : __float2int_rn(__uint_as_float((mag - (896u << 20)) << 3) * 1024.f);
+    k = (hi >> 31) ? -k : k;
+    const double4 e = expTab[kExpNodes + k];
+    const double r = a - e.z, r2 = r * r;
+    const double even = r2 * fma(r2, 1.0 / 24.0, 0.5), odd = fma(r * r2, 1.0 / 6.0, r);
+    o.am *= fma(e.x, even + odd, e.x);
+    o.bm *= fma(e.y, even - odd, e.y);
+    return o;
 }
 
 // W and dW/dv at the same v
