@@ -108,14 +108,20 @@ struct sphgb_ctx {
     // per-particle accumulators of the pair-once passes (up to 6 x n doubles)
     bool deterministic = false;
     sphgb::DBuf pairAcc;
-    // within one sweep: |r|, w_ij and the kernel function at both ends of every owned entry, stored
-    // by the pair-once xmass pass and read by the later pair-once passes of the same sweep (PairGeo in
-    // pairs.cuh); geoRows: per warp of 32 targets its longest owned list, then its first row
+    // |r|, w_ij and the kernel function at both ends of every owned entry, stored by the pair-once xmass
+    // or density pass and read by the later pair-once passes (PairGeo in pairs.cuh); geoRows: per warp of
+    // 32 targets its first row (from the owned-list build), and the row counter
     // rho0Sum: the xmass pass's sum w m_j per particle, for gradh
     sphgb::DBuf pairGeo, geoRows, rho0Sum;
     size_t geoRowCount = 0;
     int geoArrays = 0;  // 5: with the difference and velocity-difference vectors, 2: without
     bool geoValid = false;
+    // outside a sweep the caller may change x y z v h between passes: the pass that stores the cache keeps
+    // a copy of them, and every later pass on the same lists (epoch geoSnapEpoch) compares its inputs with
+    // the copy bit by bit; where a value differs, geoStale is set and the kernels form the geometry
+    sphgb::DBuf geoSnap, geoStale;
+    int64_t geoSnapEpoch = -1, geoSnapN = 0;
+    bool geoChecked = false;  // the running pass compared its inputs with geoSnap
     // inside sphgb_sweep_passes the per-particle precomputes are built by the first pass only
     bool inSweep = false, sweepPrepared = false;
     // within one sweep: the EOS ran in the gradh epilogue / the per-particle quotients are formed

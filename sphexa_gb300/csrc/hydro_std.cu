@@ -135,10 +135,11 @@ __global__ void __launch_bounds__(kPairBlock) xmassOnceKernel(ListView lv, Owned
     atomicAdd(acc + i, rho0);
 }
 
-// sums: where the pass keeps sum w m_j for gradh (with the geometry cache), or null
+// sums: where the pass keeps sum w m_j for gradh (within a sweep, with the geometry cache), or null;
+// snap: where it keeps the inputs of the cache (outside a sweep), or null
 template<bool StoreRho>
 __global__ void xmassOnceFinish(int64_t first, int64_t last, const double* h, const double* m, double K,
-                                const double* acc, double* out, double* sums)
+                                const double* acc, double* out, double* sums, GeoInputs in, double* snap, int64_t n)
 {
     const int64_t i = first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (i >= last) return;
@@ -146,6 +147,10 @@ __global__ void xmassOnceFinish(int64_t first, int64_t last, const double* h, co
     const double hInv = 1.0 / hi, h3Inv = hInv * hInv * hInv;
     const double xm = mi / ((mi + acc[i]) * K * h3Inv);
     if (sums) sums[i] = acc[i];
+    if (snap) {
+#pragma unroll
+        for (int q = 0; q < kGeoInputs; ++q) snap[q * n + i] = in.f[q][i];
+    }
     out[i] = StoreRho ? mi / xm : xm;
 }
 
@@ -266,7 +271,7 @@ __global__ void __launch_bounds__(kPairBlock) iadKernel(ListView lv, CoordFp64 c
 // FP64 IAD with one evaluation per mutual pair over the owned lists: i adds vol_j W_i r r^T, and a mutual
 // pair gives j vol_i W_j r r^T by FP64 atomics.  Geo: arrays of the pair-geometry cache (5, 2), or 0.
 template<bool Smooth, int Geo>
-__global__ void __launch_bounds__(kPairBlock) iadStdOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf,
+__device__ __forceinline__ void iadStdOnceBody(ListView lv, OwnedView ov, CoordFp64 cf,
                                                                const double* h, const double* vol,
                                                                KTab<Smooth> tab, const double* hInv64, int64_t n,
                                                                double* acc, PairGeo geo)
@@ -319,6 +324,17 @@ __global__ void __launch_bounds__(kPairBlock) iadStdOnceKernel(ListView lv, Owne
     }
 #pragma unroll
     for (int q = 0; q < 6; ++q) atomicAdd(acc + q * n + i, tau[q]);
+}
+
+template<bool Smooth, int Geo>
+__global__ void __launch_bounds__(kPairBlock) iadStdOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf,
+                                                               const double* h, const double* vol,
+                                                               KTab<Smooth> tab, const double* hInv64, int64_t n,
+                                                               double* acc, PairGeo geo)
+{
+    if constexpr (Geo >= 0) iadStdOnceBody<Smooth, Geo>(lv, ov, cf, h, vol, tab, hInv64, n, acc, geo);
+    else if (*geo.stale) iadStdOnceBody<Smooth, 0>(lv, ov, cf, h, vol, tab, hInv64, n, acc, geo);
+    else iadStdOnceBody<Smooth, -Geo>(lv, ov, cf, h, vol, tab, hInv64, n, acc, geo);
 }
 
 __global__ void iadStdOnceFinish(int64_t n, const double* h, double K, const double* acc, IadOut o)
@@ -500,7 +516,7 @@ __global__ void meStdRec64Kernel(int64_t n, MeStdArgs a, Rec4d* __restrict__ rec
 // density 3.5 -> 2.8, which also fills the geometry cache).
 // Geo: arrays of the pair-geometry cache (5, 2), or 0 to form the geometry here.
 template<bool Smooth, int Geo>
-__global__ void __launch_bounds__(kPairBlock) meStdOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf, MeStdArgs a,
+__device__ __forceinline__ void meStdOnceBody(ListView lv, OwnedView ov, CoordFp64 cf, MeStdArgs a,
                                                               const Rec4d* __restrict__ rec, double* __restrict__ acc,
                                                               PairGeo geo)
 {
@@ -597,6 +613,16 @@ __global__ void __launch_bounds__(kPairBlock) meStdOnceKernel(ListView lv, Owned
     atomicMax(accS + i, maxvBits);
 }
 
+template<bool Smooth, int Geo>
+__global__ void __launch_bounds__(kPairBlock) meStdOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf, MeStdArgs a,
+                                                              const Rec4d* __restrict__ rec, double* __restrict__ acc,
+                                                              PairGeo geo)
+{
+    if constexpr (Geo >= 0) meStdOnceBody<Smooth, Geo>(lv, ov, cf, a, rec, acc, geo);
+    else if (*geo.stale) meStdOnceBody<Smooth, 0>(lv, ov, cf, a, rec, acc, geo);
+    else meStdOnceBody<Smooth, -Geo>(lv, ov, cf, a, rec, acc, geo);
+}
+
 __global__ void __launch_bounds__(kPairBlock) meStdOnceFinish(MeStdArgs a, const double* __restrict__ acc)
 {
     const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
@@ -628,9 +654,9 @@ int launchXmass(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, v
         SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * size_t(n)));
         SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * size_t(n), c->stream));
         PairGeo geo{};
-        if (p->vx && p->vy && p->vz) SPHGB_TRY(pairGeoStore(c, &geo));
-        double* sums = nullptr;
-        if (geo.g) {
+        SPHGB_TRY(pairGeoStore(c, p, &geo));
+        double *sums = nullptr, *snap = geo.g && !c->inSweep ? c->geoSnap.as<double>() : nullptr;
+        if (geo.g && c->inSweep) {
             SPHGB_TRY(c->rho0Sum.ensure(sizeof(double) * size_t(n)));
             sums = c->rho0Sum.as<double>();
         }
@@ -647,11 +673,13 @@ int launchXmass(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, v
         if (storeRho)
             xmassOnceFinish<true><<<eb, 256, 0, c->stream>>>(first, last, static_cast<const double*>(p->h),
                                                               static_cast<const double*>(p->m), c->K,
-                                                              c->pairAcc.as<double>(), static_cast<double*>(out), sums);
+                                                              c->pairAcc.as<double>(), static_cast<double*>(out), sums,
+                                                              geoInputs(p), snap, n);
         else
             xmassOnceFinish<false><<<eb, 256, 0, c->stream>>>(first, last, static_cast<const double*>(p->h),
                                                                static_cast<const double*>(p->m), c->K,
-                                                               c->pairAcc.as<double>(), static_cast<double*>(out), sums);
+                                                               c->pairAcc.as<double>(), static_cast<double*>(out), sums,
+                                                               geoInputs(p), snap, n);
         return launched(c, "xmassOnceFinish");
     }
     const Rec8* rec = nullptr;
@@ -695,9 +723,7 @@ int launchIad(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last)
                     lv, ownedView(c), coordFp64(c, p), h, c->aux.as<double>(), KTab<S>{tabW64(c)},
                     c->hInv64.as<double>(), n, c->pairAcc.as<double>(), geo);
             };
-            if (geo.x) run(iadStdOnceKernel<S, 5>);
-            else if (geo.g) run(iadStdOnceKernel<S, 2>);
-            else run(iadStdOnceKernel<S, 0>);
+            withPairGeo(geo, [&](auto g) { run(iadStdOnceKernel<S, decltype(g)::value>); });
             return launched(c, "iadStdOnceKernel");
         }));
         iadStdOnceFinish<<<gridFor(n, 256), 256, 0, c->stream>>>(n, h, c->K, c->pairAcc.as<double>(),
@@ -763,9 +789,7 @@ int launchMeStd(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, d
                 kernel<<<ownedGrid(n), kPairBlock, 0, c->stream>>>(lv, ownedView(c), coordFp64(c, p), a, c->pack.as<Rec4d>(),
                                                              c->pairAcc.as<double>(), geo);
             };
-            if (geo.x) run(meStdOnceKernel<S, 5>);
-            else if (geo.g) run(meStdOnceKernel<S, 2>);
-            else run(meStdOnceKernel<S, 0>);
+            withPairGeo(geo, [&](auto g) { run(meStdOnceKernel<S, decltype(g)::value>); });
             return launched(c, "meStdOnceKernel");
         }));
         meStdOnceFinish<<<blocks, kPairBlock, 0, c->stream>>>(a, c->pairAcc.as<double>());

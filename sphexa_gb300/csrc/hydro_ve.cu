@@ -872,15 +872,15 @@ __global__ void __launch_bounds__(kPairBlock) meVeKernel(ListView lv, CoordFp64 
 // FP64 gradh with one evaluation per mutual pair over the owned lists.  With x = v / dx (table units)
 // and D = x dW, the reference's dterh = -(3 w + v dW) (veDefGradhJLoop, ve_def_gradh_kern.hpp:64-78)
 // is -(3 w + dx D), so its sums follow from sum w xm_j (which kx needs), sum D xm_j, and either sum w m_j
-// of the xmass pass and sum D m_j (Geo: within a sweep, where that sum is of the same geometry), or
-// sum (3 w / dx + D) m_j.  A mutual pair also gives j its terms at v_j = d / h_j with xm_i and m_i, by
+// of the xmass pass and sum D m_j (Sums: within a sweep, where that sum is of the same geometry and
+// masses), or sum (3 w / dx + D) m_j.  A mutual pair also gives j its terms at v_j = d / h_j with xm_i and m_i, by
 // FP64 atomics.  The self terms and the epilogue (ve_def_gradh_kern.hpp:60-62, 80-88) run in the
 // finishing kernels.  FP64-pipe bound: 12 instructions per mutual pair with the cache (18 with v and
 // dterh per pair, 14.7 ms at 8M; now 11.3 ms).
 constexpr double kTabDx = 1.0 / kTabInvDx;
 
-template<bool Smooth, bool Geo>
-__global__ void __launch_bounds__(kPairBlock) gradhOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf,
+template<bool Smooth, bool Geo, bool Sums>
+__device__ __forceinline__ void gradhOnceBody(ListView lv, OwnedView ov, CoordFp64 cf,
                                                                const double* h, const double* m, const double* xm,
                                                                KTab<Smooth> tw, KTab<Smooth> tdw,
                                                                const double* hInv64, int64_t n, double* acc,
@@ -924,7 +924,7 @@ __global__ void __launch_bounds__(kPairBlock) gradhOnceKernel(ListView lv, Owned
             const double xmj = __ldg(xm + j);
             kx = fma(w, xmj, kx);
             dxm = fma(D, xmj, dxm);
-            dm = fma(Geo ? D : fma(3.0 * kTabInvDx, w, D), __ldg(m + j), dm);
+            dm = fma(Sums ? D : fma(3.0 * kTabInvDx, w, D), __ldg(m + j), dm);
         }
         if (mutual) {
             const double x = dist * __ldg(hInvDx + j);
@@ -932,12 +932,25 @@ __global__ void __launch_bounds__(kPairBlock) gradhOnceKernel(ListView lv, Owned
             const double w = Geo ? wv.y : lookupX(tw, sl), D = x * lookupX(tdw, sl);
             atomicAdd(acc + j, w * xmi);
             atomicAdd(acc + n + j, D * xmi);
-            atomicAdd(acc + 2 * n + j, (Geo ? D : fma(3.0 * kTabInvDx, w, D)) * mi);
+            atomicAdd(acc + 2 * n + j, (Sums ? D : fma(3.0 * kTabInvDx, w, D)) * mi);
         }
     }
     atomicAdd(acc + i, kx);
     atomicAdd(acc + n + i, dxm);
     atomicAdd(acc + 2 * n + i, dm);
+}
+
+// Geo: 1 the sweep's cache and xmass sums, 2 the cache subject to geo.stale, 0 neither
+template<bool Smooth, int Geo>
+__global__ void __launch_bounds__(kPairBlock) gradhOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf, const double* h,
+                                                              const double* m, const double* xm, KTab<Smooth> tw,
+                                                              KTab<Smooth> tdw, const double* hInv64, int64_t n,
+                                                              double* acc, PairGeo geo)
+{
+    if constexpr (Geo == 1) gradhOnceBody<Smooth, true, true>(lv, ov, cf, h, m, xm, tw, tdw, hInv64, n, acc, geo);
+    else if (Geo == 2 && *geo.stale == 0)
+        gradhOnceBody<Smooth, true, false>(lv, ov, cf, h, m, xm, tw, tdw, hInv64, n, acc, geo);
+    else gradhOnceBody<Smooth, false, false>(lv, ov, cf, h, m, xm, tw, tdw, hInv64, n, acc, geo);
 }
 
 // kx and gradh of particle i from the sums of gradhOnceKernel (sums: the xmass pass's sum w m_j, or
@@ -1001,6 +1014,7 @@ __global__ void __launch_bounds__(kPairBlock) iadOnceKernel(ListView lv, OwnedVi
     const int64_t i = lv.first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (i >= lv.last) return;
     const int64_t ii = i - lv.first;
+    if (geo.stale && *geo.stale) geo.g = geo.w = geo.x = nullptr;  // outside a sweep, inputs changed
     const unsigned no = ov.size(ii);
     const KTab<Smooth> tab{a.w64};
     const double* hInvDx = hInv64 + 2 * n;
@@ -1106,7 +1120,7 @@ __global__ void iadOnceFinish(int64_t first, int64_t last, int64_t n, IadDivvArg
 // Bound by the FP64 pipe (13 instructions per mutual pair with the cache's w_ij, 17 with r . v and 1/|r|:
 // 15.7 -> 12.5 ms at 8M).  Geo: arrays of the pair-geometry cache (5, 2), or 0 to form the geometry.
 template<bool Smooth, int Geo>
-__global__ void __launch_bounds__(kPairBlock) avOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf, AvArgs a,
+__device__ __forceinline__ void avOnceBody(ListView lv, OwnedView ov, CoordFp64 cf, AvArgs a,
                                                             const double* hInv64, int64_t n, double* acc, PairGeo geo)
 {
     const int64_t i = lv.first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
@@ -1179,6 +1193,15 @@ __global__ void __launch_bounds__(kPairBlock) avOnceKernel(ListView lv, OwnedVie
     atomicAdd(acc + n + i, Sy);
     atomicAdd(acc + 2 * n + i, Sz);
     atomicMax(accV + i, vsigBits);
+}
+
+template<bool Smooth, int Geo>
+__global__ void __launch_bounds__(kPairBlock) avOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf, AvArgs a,
+                                                            const double* hInv64, int64_t n, double* acc, PairGeo geo)
+{
+    if constexpr (Geo >= 0) avOnceBody<Smooth, Geo>(lv, ov, cf, a, hInv64, n, acc, geo);
+    else if (*geo.stale) avOnceBody<Smooth, 0>(lv, ov, cf, a, hInv64, n, acc, geo);
+    else avOnceBody<Smooth, -Geo>(lv, ov, cf, a, hInv64, n, acc, geo);
 }
 
 __global__ void avOnceFinish(int64_t first, int64_t last, int64_t n, AvArgs a, const double* acc)
@@ -1304,7 +1327,7 @@ __device__ __forceinline__ double avRvShared(double d1, double d2, double dist)
 // directed pair evaluated, now 4.3 ms.
 // Geo: arrays of the pair-geometry cache to read (5, 2), or 0 to form the geometry here.
 template<bool AvClean, bool Smooth, int Geo>
-__global__ void __launch_bounds__(kPairBlock) meVeOnceKernel(ListView lv, CoordFp64 cf, MeVeArgs a, PairGeo geo)
+__device__ __forceinline__ void meVeOnceBody(ListView lv, CoordFp64 cf, MeVeArgs a, PairGeo geo)
 {
     using T = double;
     const int64_t i = lv.first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
@@ -1444,6 +1467,14 @@ __global__ void __launch_bounds__(kPairBlock) meVeOnceKernel(ListView lv, CoordF
     atomicMax(accS + i, maxvBits);
 }
 
+template<bool AvClean, bool Smooth, int Geo>
+__global__ void __launch_bounds__(kPairBlock) meVeOnceKernel(ListView lv, CoordFp64 cf, MeVeArgs a, PairGeo geo)
+{
+    if constexpr (Geo >= 0) meVeOnceBody<AvClean, Smooth, Geo>(lv, cf, a, geo);
+    else if (*geo.stale) meVeOnceBody<AvClean, Smooth, 0>(lv, cf, a, geo);
+    else meVeOnceBody<AvClean, Smooth, -Geo>(lv, cf, a, geo);
+}
+
 __global__ void __launch_bounds__(kPairBlock) meVeOnceFinish(ListView lv, MeVeArgs a)
 {
     const int64_t i0 = lv.first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
@@ -1493,7 +1524,7 @@ int passGradh(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last)
         SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * 3 * size_t(n)));
         SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * 3 * size_t(n), c->stream));
         const PairGeo geo = pairGeoRead(c);
-        const double* sums = geo.g ? c->rho0Sum.as<double>() : nullptr;
+        const double* sums = geo.g && !geo.stale ? c->rho0Sum.as<double>() : nullptr;
         SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
             constexpr bool S = decltype(smooth)::value;
             auto run = [&](auto kernel) {
@@ -1502,8 +1533,9 @@ int passGradh(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last)
                     static_cast<const double*>(p->m), static_cast<const double*>(p->xm), KTab<S>{tabW64(c)},
                     KTab<S>{tabDW64(c)}, c->hInv64.as<double>(), n, c->pairAcc.as<double>(), geo);
             };
-            if (geo.g) run(gradhOnceKernel<S, true>);
-            else run(gradhOnceKernel<S, false>);
+            if (geo.stale) run(gradhOnceKernel<S, 2>);
+            else if (geo.g) run(gradhOnceKernel<S, 1>);
+            else run(gradhOnceKernel<S, 0>);
             return launched(c, "gradhOnceKernel");
         }));
         if (c->inSweep && p->u && p->prho && p->c) {  // EOS and quotients fused into the epilogue
@@ -1701,9 +1733,7 @@ int passAVswitches(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last
                 kernel<<<ownedGrid(n), kPairBlock, 0, c->stream>>>(lv, ownedView(c), coordFp64(c, p), a,
                                                              c->hInv64.as<double>(), n, c->pairAcc.as<double>(), geo);
             };
-            if (geo.x) run(avOnceKernel<S, 5>);
-            else if (geo.g) run(avOnceKernel<S, 2>);
-            else run(avOnceKernel<S, 0>);
+            withPairGeo(geo, [&](auto g) { run(avOnceKernel<S, decltype(g)::value>); });
             return launched(c, "avOnceKernel");
         }));
         avOnceFinish<<<gridFor(last - first, 256), 256, 0, c->stream>>>(first, last, n, a, c->pairAcc.as<double>());
@@ -1814,15 +1844,10 @@ int passMomentumEnergyVe(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_
             SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
                 constexpr bool S = decltype(smooth)::value;
                 auto run = [&](auto kernel) { kernel<<<ownedGrid(p->n), kPairBlock, 0, c->stream>>>(lv, cf, a, geo); };
-                if (avClean) {
-                    if (geo.x) run(meVeOnceKernel<true, S, 5>);
-                    else if (geo.g) run(meVeOnceKernel<true, S, 2>);
-                    else run(meVeOnceKernel<true, S, 0>);
-                } else {
-                    if (geo.x) run(meVeOnceKernel<false, S, 5>);
-                    else if (geo.g) run(meVeOnceKernel<false, S, 2>);
-                    else run(meVeOnceKernel<false, S, 0>);
-                }
+                withPairGeo(geo, [&](auto g) {
+                    if (avClean) run(meVeOnceKernel<true, S, decltype(g)::value>);
+                    else run(meVeOnceKernel<false, S, decltype(g)::value>);
+                });
                 return launched(c, "meVeOnceKernel");
             }));
             meVeOnceFinish<<<blocks, kPairBlock, 0, c->stream>>>(lv, a);

@@ -605,6 +605,9 @@ struct MutualArgs {
     float wrapSafe2;
     uint32_t* owned;
     uint32_t* ownedCount;
+    // rows of the pair-geometry cache: each warp's first, handed out from a counter in any order
+    uint32_t* rowOff;
+    uint32_t* rowCount;
 };
 
 __global__ void ownedRecKernel(const double* __restrict__ x, const double* __restrict__ y,
@@ -764,6 +767,8 @@ __global__ void __launch_bounds__(128) ownedListKernel(MutualArgs a)
     }
     const unsigned cnt = w.finish();
     if (valid) a.ownedCount[ii] = cnt;
+    const unsigned rows = __reduce_max_sync(0xffffffffu, valid ? cnt : 0u);
+    if (valid && (ii & 31) == 0) a.rowOff[ii >> 5] = atomicAdd(a.rowCount, rows);
 }
 
 // owned lists from list membership alone: (i, j) is mutual when i is in j's (capped, ascending)
@@ -797,14 +802,6 @@ __global__ void __launch_bounds__(128) ownedByListKernel(const uint32_t* __restr
     }
     const unsigned cnt = w.finish();
     if (valid) ownedCount[ii] = cnt;
-}
-
-// longest owned list of each warp of 32 targets
-__global__ void warpMaxKernel(const uint32_t* __restrict__ count, int64_t n, uint32_t* __restrict__ wmax)
-{
-    const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-    const uint32_t m = __reduce_max_sync(0xffffffffu, i < n ? __ldg(count + i) : 0u);
-    if ((threadIdx.x & 31) == 0 && i < n) wmax[i >> 5] = m;
 }
 
 __global__ void fillOnes(uint32_t* p, int64_t n)
@@ -902,8 +899,17 @@ int buildOwned(sphgb_ctx* c, const double* x, const double* y, const double* z, 
         if (c->box.pbc[k]) a.wrapSafe2 = std::min(a.wrapSafe2, float(0.0625 * c->box.L[k] * c->box.L[k]));
     a.owned = c->owned.as<uint32_t>();
     a.ownedCount = c->ownedCount.as<uint32_t>();
+    const int64_t nWarps = (nWork + 31) / 32;
+    SPHGB_TRY(c->geoRows.ensure(sizeof(uint32_t) * size_t(nWarps + 1)));
+    a.rowOff = c->geoRows.as<uint32_t>();
+    a.rowCount = a.rowOff + nWarps;
+    SPHGB_CUDA(cudaMemsetAsync(a.rowCount, 0, sizeof(uint32_t), c->stream));
     ownedListKernel<<<gridFor(nWork, 128), 128, 0, c->stream>>>(a);
     SPHGB_TRY(launched(c, "ownedListKernel"));
+    uint32_t rows = 0;
+    SPHGB_CUDA(cudaMemcpyAsync(&rows, a.rowCount, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
+    SPHGB_CUDA(cudaStreamSynchronize(c->stream));
+    c->geoRowCount = rows;
     c->ownedEpoch = c->nbrEpoch;
     c->ownedFromLists = false;
     return SPHGB_OK;
@@ -918,7 +924,10 @@ int prepareLists(sphgb_ctx* c, const double* x, const double* y, const double* z
     c->nbrStride = (nWork + 31) / 32 * 32;
     // lists larger than the buffers hold: the pair-geometry cache of an earlier sweep gives its
     // memory back first (the next FP64 sweep sizes it again within half of the free memory)
-    if (c->nbr.bytes < sizeof(uint32_t) * listCapacity(ngmax) * c->nbrStride) c->pairGeo.release();
+    if (c->nbr.bytes < sizeof(uint32_t) * listCapacity(ngmax) * c->nbrStride) {
+        c->pairGeo.release();
+        c->geoSnapEpoch = -1;
+    }
     SPHGB_TRY(c->nbr.ensure(sizeof(uint32_t) * listCapacity(ngmax) * c->nbrStride));
     SPHGB_TRY(c->ncount.ensure(sizeof(uint32_t) * c->nbrStride));
     SPHGB_TRY(c->active.ensure(sizeof(uint32_t) * c->nbrStride + c->nbrStride));
@@ -957,24 +966,21 @@ int finishStats(sphgb_ctx* c, int64_t hIters)
 
 }  // namespace
 
-int pairGeoStore(sphgb_ctx* c, PairGeo* out)
+int pairGeoStore(sphgb_ctx* c, const sphgb_particles* p, PairGeo* out)
 {
-    *out = PairGeo{nullptr, nullptr, nullptr, nullptr, 0};
+    *out = PairGeo{};
     c->geoValid = false;
-    if (!c->inSweep || c->ownedEpoch != c->nbrEpoch || c->ownedFromLists) return SPHGB_OK;
-    const int64_t nWork = c->nbrLast - c->nbrFirst, nWarps = (nWork + 31) / 32;
-    if (nWork <= 0) return SPHGB_OK;
-    SPHGB_TRY(c->geoRows.ensure(sizeof(uint32_t) * 2 * size_t(nWarps)));
-    uint32_t* wmax = c->geoRows.as<uint32_t>();
-    uint32_t* rowOff = wmax + nWarps;
-    warpMaxKernel<<<gridFor(nWarps * 32, 256), 256, 0, c->stream>>>(c->ownedCount.as<uint32_t>(), nWork, wmax);
-    SPHGB_TRY(launched(c, "warpMaxKernel"));
-    SPHGB_TRY(exclusiveScan(c, wmax, rowOff, nWarps));
-    uint32_t lastOff = 0, lastMax = 0;
-    SPHGB_CUDA(cudaMemcpyAsync(&lastOff, rowOff + nWarps - 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
-    SPHGB_CUDA(cudaMemcpyAsync(&lastMax, wmax + nWarps - 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
-    SPHGB_CUDA(cudaStreamSynchronize(c->stream));
-    const size_t rows = size_t(lastOff) + lastMax;
+    c->geoSnapEpoch = -1;
+    if (c->ownedEpoch != c->nbrEpoch || c->ownedFromLists || !p->vx || !p->vy || !p->vz) return SPHGB_OK;
+    const size_t rows = c->geoRowCount;
+    if (rows == 0) return SPHGB_OK;
+    if (!c->inSweep) {
+        if (c->geoSnap.ensure(sizeof(double) * kGeoInputs * size_t(p->n)) != SPHGB_OK ||
+            c->geoStale.ensure(sizeof(int)) != SPHGB_OK) {
+            (void)cudaGetLastError();
+            return SPHGB_OK;
+        }
+    }
     // five arrays (|r| and 1/|r|, the two kernel values, r and dv) or the first two, whichever fits
     // in the buffer already held or in half of the free device memory
     int arrays = 0;
@@ -994,10 +1000,13 @@ int pairGeoStore(sphgb_ctx* c, PairGeo* out)
         break;
     }
     if (arrays == 0) return SPHGB_OK;
-    c->geoRowCount = rows;
     c->geoArrays = arrays;
-    c->geoValid = true;
-    *out = pairGeoRead(c);
+    if (c->inSweep) c->geoValid = true;
+    else {
+        c->geoSnapEpoch = c->nbrEpoch;
+        c->geoSnapN = p->n;
+    }
+    *out = pairGeoView(c, nullptr);
     return SPHGB_OK;
 }
 

@@ -142,7 +142,9 @@ inline bool pairOnce(const sphgb_ctx* c, const sphgb_particles* p, int64_t first
 // its square and the reciprocal square root: about a dozen FP64-pipe instructions), the approach
 // velocity w_ij = r . v_ij / |r|, the kernel function at both ends, w(|r| / h_i) and w(|r| / h_j), and,
 // where the memory is there, the difference vector r = x_i - x_j and the velocity difference dv =
-// v_j - v_i are formed once by the xmass pass and loaded by gradh, IAD, AV and momentum-energy.  Layout: the 32 targets of a warp own
+// v_j - v_i are formed once by the xmass or density pass and loaded by the passes after it.  Outside a
+// sweep the caller may change the inputs between passes; there every pass compares them with a copy
+// (recipKernel) and its kernel takes the cache or forms the geometry by the outcome (stale).  Layout: the 32 targets of a warp own
 // rows rowOff[w] .. rowOff[w] + (their longest owned list) - 1, a row holding entry k of all 32 side
 // by side, so a warp reads 512 contiguous bytes per entry and array.
 struct PairGeo {
@@ -151,6 +153,7 @@ struct PairGeo {
     double2* w;              // {w(|r| / h_i), w(|r| / h_j)}
     double2* x;              // {rx, ry}, {rz, dvx}, {dvy, dvz} at x, x + plane, x + 2 plane; or null
     int64_t plane;           // entries per array
+    const int* stale;        // outside a sweep: 1 when the inputs changed since the cache was stored
     // entry k of target ii is at base(ii) + 32 k
     __device__ __forceinline__ int64_t base(int64_t ii) const
     {
@@ -158,17 +161,46 @@ struct PairGeo {
     }
 };
 
-// the space for the xmass pass of this sweep to fill (rows from the owned counts; null outside a
-// sweep or when it cannot be had within half of the free device memory)
-int pairGeoStore(sphgb_ctx* c, PairGeo* out);
+// the inputs of the cached geometry: x y z vx vy vz h
+constexpr int kGeoInputs = 7;
+struct GeoInputs {
+    const double* f[kGeoInputs];
+};
+inline GeoInputs geoInputs(const sphgb_particles* p)
+{
+    auto d = [](const void* q) { return static_cast<const double*>(q); };
+    return GeoInputs{{p->x, p->y, p->z, d(p->vx), d(p->vy), d(p->vz), d(p->h)}};
+}
 
-// what this sweep's xmass pass stored, or null
+// the space for the xmass or density pass to fill (null when it cannot be had within half of the free
+// device memory)
+int pairGeoStore(sphgb_ctx* c, const sphgb_particles* p, PairGeo* out);
+
+inline PairGeo pairGeoView(const sphgb_ctx* c, const int* stale)
+{
+    double2* g = c->pairGeo.as<double2>();
+    const int64_t plane = 32 * int64_t(c->geoRowCount);
+    return PairGeo{c->geoRows.as<uint32_t>(), g, g + plane, c->geoArrays == 5 ? g + 2 * plane : nullptr, plane, stale};
+}
+
+// what the xmass or density pass stored: in a sweep as it is, outside one subject to the comparison; or null
 inline PairGeo pairGeoRead(const sphgb_ctx* c)
 {
-    if (!c->inSweep || !c->geoValid) return PairGeo{nullptr, nullptr, nullptr, nullptr, 0};
-    double2* g = c->pairGeo.as<double2>();
-    const int64_t nWarps = (c->nbrLast - c->nbrFirst + 31) / 32, plane = 32 * int64_t(c->geoRowCount);
-    return PairGeo{c->geoRows.as<uint32_t>() + nWarps, g, g + plane, c->geoArrays == 5 ? g + 2 * plane : nullptr, plane};
+    if (c->inSweep && c->geoValid) return pairGeoView(c, nullptr);
+    if (!c->inSweep && c->geoChecked) return pairGeoView(c, c->geoStale.as<int>());
+    return PairGeo{};
+}
+
+// the instance of a pass's kernel for a cache: launch.template operator()<Geo>() with Geo = 5 or 2 arrays, 0
+// none, negative: the kernel looks at geo.stale and takes -Geo arrays or none
+template<class F>
+inline void withPairGeo(const PairGeo& geo, F&& launch)
+{
+    if (!geo.g) launch(std::integral_constant<int, 0>{});
+    else if (geo.x && geo.stale) launch(std::integral_constant<int, -5>{});
+    else if (geo.x) launch(std::integral_constant<int, 5>{});
+    else if (geo.stale) launch(std::integral_constant<int, -2>{});
+    else launch(std::integral_constant<int, 2>{});
 }
 
 // ---- forward tape of the VE adjoint: sections of n doubles in c->veTape ----

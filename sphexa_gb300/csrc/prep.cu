@@ -54,10 +54,19 @@ __global__ void gridHInvKernel(const void* __restrict__ h, int hIsFloat, int64_t
 
 // per particle 1/h, 1/h^3 and (1/h) / dx: the last turns a pair distance into table-interval units
 // with one multiply
-__global__ void recipKernel(const double* __restrict__ h, int64_t n, double* __restrict__ out)
+// Check: also compares h, positions and velocities with the copy the pair-geometry cache was made from
+template<bool Check>
+__global__ void recipKernel(const double* __restrict__ h, int64_t n, double* __restrict__ out, GeoInputs in,
+                            const long long* __restrict__ snap, int* __restrict__ stale)
 {
     int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (i >= n) return;
+    if constexpr (Check) {
+        bool differs = false;
+#pragma unroll
+        for (int q = 0; q < kGeoInputs; ++q) differs |= __double_as_longlong(in.f[q][i]) != snap[q * n + i];
+        if (differs) *stale = 1;
+    }
     double hi = 1.0 / h[i];
     out[i] = hi;
     out[n + i] = hi * hi * hi;
@@ -70,6 +79,7 @@ __global__ void initDtWord(unsigned long long* p) { *p = 0x7ff0000000000000ull; 
 
 int buildTables(sphgb_ctx* c)
 {
+    c->geoSnapEpoch = -1;  // cached kernel values are of the old tables
     const double n = c->prm.sincIndex;
     std::vector<double> wh(kTableSize), whd(kTableSize);
     std::vector<float> wf(kTableSize);
@@ -162,7 +172,16 @@ int prepareFp64(sphgb_ctx* c, sphgb_particles* p)
 {
     const int64_t n = p->n;
     SPHGB_TRY(c->hInv64.ensure(sizeof(double) * 3 * n));
-    recipKernel<<<gridFor(n, 256), 256, 0, c->stream>>>(static_cast<const double*>(p->h), n, c->hInv64.as<double>());
+    const double* h = static_cast<const double*>(p->h);
+    c->geoChecked = !c->inSweep && !c->deterministic && c->geoSnapEpoch == c->nbrEpoch && c->geoSnapN == n && p->vx &&
+                    p->vy && p->vz;
+    if (c->geoChecked) {
+        SPHGB_CUDA(cudaMemsetAsync(c->geoStale.p, 0, sizeof(int), c->stream));
+        recipKernel<true><<<gridFor(n, 256), 256, 0, c->stream>>>(h, n, c->hInv64.as<double>(), geoInputs(p),
+                                                                  c->geoSnap.as<long long>(), c->geoStale.as<int>());
+    } else
+        recipKernel<false><<<gridFor(n, 256), 256, 0, c->stream>>>(h, n, c->hInv64.as<double>(), GeoInputs{}, nullptr,
+                                                                   nullptr);
     return launched(c, "recipKernel");
 }
 
