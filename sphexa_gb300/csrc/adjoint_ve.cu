@@ -193,11 +193,12 @@ __device__ __forceinline__ void vsigStep(const VeAdjArgs& a, int64_t j, const do
     }
 }
 
-// vsig_i and its pair alone, when the forward passes kept the other sums of vePreKernel.  One FP32
-// walk over i's list keeps a lower bound L on vsig_i from the pairs that surely approach; a pair
-// is evaluated in FP64 (vsigStep, in list order) only when its FP32 signal velocity plus the error
-// bound reaches the current L, which every pair able to set vsig_i does, so vsig_i and its pair
-// come out as in vePreKernel.  Particles whose 2h exceeds a quarter of a periodic box edge (where
+// vsig_i and its pair alone, when the forward passes kept the other sums of vePreKernel.  An FP32
+// walk over i's list finds a lower bound L on vsig_i from the pairs that surely approach; a second one
+// picks the pairs whose FP32 signal velocity plus the error bound reaches L, which every pair able to
+// set vsig_i does, and only those (one or two) are evaluated in FP64 (vsigStep, in list order), so vsig_i
+// and its pair come out as in vePreKernel.  In one walk each new maximum ran the FP64 step, for some lane
+// of the warp in nearly every step (1M particles: 3.5 -> 0.78 ms).  Particles whose 2h exceeds a quarter of a periodic box edge (where
 // the threshold-2h image rule of the FP64 geometry need not be the minimum image) walk in FP64.
 __global__ void __launch_bounds__(kVeAdjBlock) veArgKernel(VeAdjArgs a)
 {
@@ -223,9 +224,8 @@ __global__ void __launch_bounds__(kVeAdjBlock) veArgKernel(VeAdjArgs a)
         const float4 Xi = a.xc32[i], Vi = a.v32[i];
         const float viMax = fmaxf(fabsf(Vi.x), fmaxf(fabsf(Vi.y), fabsf(Vi.z)));
         const float dr = 2.f * a.ePos;  // >= |r_f - r| (three components)
-        float L = 0.f;                  // vsig_i > 0
-        for (unsigned q = 0; q < nc; ++q) {
-            const uint32_t j = a.lv.at(i, q);
+        // FP32 signal velocity of pair j with its error bound; rv: r.v with its own
+        auto filter = [&](uint32_t j, float& rv, float& erv, float& vs, float& ev) {
             const float4 Xj = a.xc32[j], Vj = a.v32[j];
             float r[3] = {Xi.x - Xj.x, Xi.y - Xj.y, Xi.z - Xj.z};
 #pragma unroll
@@ -235,18 +235,39 @@ __global__ void __launch_bounds__(kVeAdjBlock) veArgKernel(VeAdjArgs a)
                     else if (r[k] < -0.5f * a.box.Lf[k]) r[k] += a.box.Lf[k];
                 }
             const float v[3] = {Vi.x - Vj.x, Vi.y - Vj.y, Vi.z - Vj.z};
-            const float d = sqrtf(fmaf(r[0], r[0], fmaf(r[1], r[1], r[2] * r[2])));
-            const float rv = fmaf(r[0], v[0], fmaf(r[1], v[1], r[2] * v[2]));
+            const float d2 = fmaf(r[0], r[0], fmaf(r[1], r[1], r[2] * r[2])), di = rsqrtf(d2), d = d2 * di;
+            rv = fmaf(r[0], v[0], fmaf(r[1], v[1], r[2] * v[2]));
             // bounds: |v_f - v| <= dv, |r.v error| <= erv, |signal velocity error| <= ev
             const float vn = 1.8f * (viMax + fmaxf(fabsf(Vj.x), fmaxf(fabsf(Vj.y), fabsf(Vj.z))));
             const float dv = 1e-6f * vn;
-            const float erv = dr * vn + d * (dv + 1e-6f * vn);
-            const float vs = Xi.w + Xj.w - 3.f * rv / d;
-            const float ev = 3.f * (4.f * dr * vn / d + 2.f * dv + 1e-6f * vn) +
-                             1e-6f * (Xi.w + Xj.w + 3.f * fabsf(rv) / d);
-            if (!(rv >= erv) && !(vs + ev < L)) exact(j);  // may approach and may reach L (NaN: evaluate)
-            if (rv < -erv) L = fmaxf(L, vs - ev);          // surely approaches
+            erv = dr * vn + d * (dv + 1e-6f * vn);
+            const float rd = 3.f * rv * di;  // within 4 ulp of 3 rv / d, inside the 1e-6 below
+            vs = Xi.w + Xj.w - rd;
+            ev = 3.f * (4.f * dr * vn * di + 2.f * dv + 1e-6f * vn) + 1e-6f * (Xi.w + Xj.w + fabsf(rd));
+        };
+        float L = 0.f, rv, erv, vs, ev;  // vsig_i > 0
+        for (unsigned q = 0; q < nc; ++q) {
+            filter(a.lv.at(i, q), rv, erv, vs, ev);
+            if (rv < -erv) L = fmaxf(L, vs - ev);  // surely approaches
         }
+        uint32_t c0 = 0, c1 = 0;
+        int held = 0;
+        for (unsigned q = 0; q < nc; ++q) {
+            const uint32_t j = a.lv.at(i, q);
+            filter(j, rv, erv, vs, ev);
+            if (!(rv >= erv) && !(vs + ev < L)) {  // may approach and may reach L (NaN: evaluate)
+                if (held == 2) {
+                    exact(c0);
+                    exact(c1);
+                    held = 0;
+                }
+                if (held == 0) c0 = j;
+                else c1 = j;
+                ++held;
+            }
+        }
+        if (held > 0) exact(c0);
+        if (held > 1) exact(c1);
     }
     a.vsig[i] = vsig;
     a.vsigArg[i] = arg;
@@ -1184,57 +1205,63 @@ __global__ void __launch_bounds__(kVeAdjBlock) veGradhAdjKernel(VeAdjArgs a)
     put(a.xmB, k, xm, at);
 }
 
+// scatter form over the owned lists (gradhAdj at both ends of a mutual pair).  In table units, x = v / dx
+// and slopes d/dx, an end's radial partial is B / (h dx) and its h partial -B x / h with
+// B = wb w' - dx q (wd + x wd'), q = S_om xm + S_r0 m of the other end, wb = S_kx xm - 3 q.  FP64-pipe
+// bound (1M particles: 8.2 -> 5.7 ms; xmass below 5.2 -> 3.2).
 template<bool Smooth>
 __global__ void __launch_bounds__(kVeAdjBlock) veGradhAdjOnceKernel(VeAdjArgs a, OwnedView ov)
 {
+    constexpr double dx = 1.0 / kTabInvDx;
     const KTab<Smooth> tw{a.wh};
     const KTab<Smooth> tdw{a.whd};
     const int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (k >= a.n) return;
     double x[3] = {0, 0, 0}, h = 0, xm = 0;
-    const double hInvK = a.hInv[k], skx = a.Skx[k], som = a.Som[k], sr0 = a.Sr0[k];
-    const double xmK = a.xm[k], mK = a.m[k];
+    const double hDxK = a.hDx[k], skx = a.Skx[k], som = a.Som[k], sr0 = a.Sr0[k], xmK = a.xm[k], mK = a.m[k];
+    const OwnGeom og(a, k);
     const unsigned cnt = ov.size(k);
-    for (unsigned q = 0; q < cnt; ++q) {
+    // B of one end at table coordinate xt, with that end's seeds and the other end's xm and m; xmb: the
+    // other end's xm partial
+    auto term = [&](double xt, double sk, double so, double s0, double xmo, double mo, double& xmb) {
+        const TabSlot sl = tabSlot(xt);
+        double ty = 0.0, tyd = 0.0, w = 0.0, wd = 0.0;
+        if (sl.k >= 0) {
+            w = lookupXSlope(tw, sl, ty);
+            wd = lookupXSlope(tdw, sl, tyd);
+        }
+        const double q = fma(so, xmo, s0 * mo), wb = fma(-3.0, q, sk * xmo);
+        xmb = fma(sk, w, -so * fma(xt * dx, wd, 3.0 * w));
+        return fma(wb, ty, -(dx * q) * fma(xt, tyd, wd));
+    };
+    for (unsigned q = blockIdx.y; q < cnt; q += gridDim.y) {
         bool mutual;
         const uint32_t j = ov.at(k, q, mutual);
-        double r[3], d, rinv;
-        geom(a, k, j, r, d, rinv);
-        double dw, dwd;
-        double w = lookupVS(tw, d * hInvK, dw), wd = lookupVS(tdw, d * hInvK, dwd);
-        GradhGrad o;
-        gradhAdj(r, d, rinv, hInvK, w, dw, wd, dwd, a.xm[j], a.m[j], skx, som, sr0, o);
-        double rj[3];
-#pragma unroll
-        for (int t = 0; t < 3; ++t) {
-            x[t] += o.r[t];
-            rj[t] = -o.r[t];
-        }
-        h += o.hI;
+        double r[3], d, rinv, xmb;
+        og.r(a, j, r, d, rinv);
+        const double xk = d * hDxK;
+        const double bk = term(xk, skx, som, sr0, __ldg(a.xm + j), __ldg(a.m + j), xmb);
+        h = fma(-bk, xk, h);
+        double db = bk * hDxK;
+        atomicAdd(a.xmB + j, xmb);
         if (mutual) {
-            const double hInvJ = a.hInv[j];
-            const double rm[3] = {-r[0], -r[1], -r[2]};
-            w = lookupVS(tw, d * hInvJ, dw);
-            wd = lookupVS(tdw, d * hInvJ, dwd);
-            GradhGrad p;
-            gradhAdj(rm, d, rinv, hInvJ, w, dw, wd, dwd, xmK, mK, a.Skx[j], a.Som[j], a.Sr0[j], p);
-#pragma unroll
-            for (int t = 0; t < 3; ++t) {
-                rj[t] += p.r[t];
-                x[t] -= p.r[t];
-            }
-            xm += p.xmJ;
-            atomicAdd(a.bh + j, p.hI);
+            const double hDxJ = __ldg(a.hDx + j), xj = d * hDxJ;
+            const double bj = term(xj, __ldg(a.Skx + j), __ldg(a.Som + j), __ldg(a.Sr0 + j), xmK, mK, xmb);
+            db = fma(bj, hDxJ, db);
+            xm += xmb;
+            atomicAdd(a.bh + j, -bj * xj * __ldg(a.hInv + j));
         }
-        atomicAdd(a.bx + j, rj[0]);
-        atomicAdd(a.by + j, rj[1]);
-        atomicAdd(a.bz + j, rj[2]);
-        atomicAdd(a.xmB + j, o.xmJ);
+        const double dr = db * rinv;
+#pragma unroll
+        for (int t = 0; t < 3; ++t) x[t] = fma(dr, r[t], x[t]);
+        atomicAdd(a.bx + j, -dr * r[0]);
+        atomicAdd(a.by + j, -dr * r[1]);
+        atomicAdd(a.bz + j, -dr * r[2]);
     }
     atomicAdd(a.bx + k, x[0]);
     atomicAdd(a.by + k, x[1]);
     atomicAdd(a.bz + k, x[2]);
-    atomicAdd(a.bh + k, h);
+    atomicAdd(a.bh + k, h * a.hInv[k]);
     atomicAdd(a.xmB + k, xm);
 }
 
@@ -1303,38 +1330,37 @@ __global__ void __launch_bounds__(kVeAdjBlock) veXmassAdjOnceKernel(VeAdjArgs a,
     const int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (k >= a.n) return;
     double x[3] = {0, 0, 0}, h = 0;
-    const double hInvK = a.hInv[k], r0b = a.R0b[k], mK = a.m[k];
+    const double hDxK = a.hDx[k], r0b = a.R0b[k], mK = a.m[k];
+    const OwnGeom og(a, k);
     const unsigned cnt = ov.size(k);
-    for (unsigned q = 0; q < cnt; ++q) {
+    for (unsigned q = blockIdx.y; q < cnt; q += gridDim.y) {
         bool mutual;
         const uint32_t j = ov.at(k, q, mutual);
-        double r[3], d, rinv;
-        geom(a, k, j, r, d, rinv);
-        double dw;
-        lookupVS(tw, d * hInvK, dw);
-        double rb[3], hIb;
-        xmassAdj(r, d, rinv, hInvK, dw, a.m[j], r0b, rb, hIb);
-        h += hIb;
+        double r[3], d, rinv, ty;
+        og.r(a, j, r, d, rinv);
+        const double xk = d * hDxK;
+        lookupXSlope(tw, xk, ty);
+        const double bk = r0b * __ldg(a.m + j) * ty;
+        h = fma(-bk, xk, h);
+        double db = bk * hDxK;
         if (mutual) {
-            const double hInvJ = a.hInv[j];
-            const double rm[3] = {-r[0], -r[1], -r[2]};
-            lookupVS(tw, d * hInvJ, dw);
-            double pb[3], hJb;
-            xmassAdj(rm, d, rinv, hInvJ, dw, mK, a.R0b[j], pb, hJb);
-#pragma unroll
-            for (int t = 0; t < 3; ++t) rb[t] -= pb[t];
-            atomicAdd(a.bh + j, hJb);
+            const double hDxJ = __ldg(a.hDx + j), xj = d * hDxJ;
+            lookupXSlope(tw, xj, ty);
+            const double bj = __ldg(a.R0b + j) * mK * ty;
+            db = fma(bj, hDxJ, db);
+            atomicAdd(a.bh + j, -bj * xj * __ldg(a.hInv + j));
         }
+        const double dr = db * rinv;
 #pragma unroll
-        for (int t = 0; t < 3; ++t) x[t] += rb[t];
-        atomicAdd(a.bx + j, -rb[0]);
-        atomicAdd(a.by + j, -rb[1]);
-        atomicAdd(a.bz + j, -rb[2]);
+        for (int t = 0; t < 3; ++t) x[t] = fma(dr, r[t], x[t]);
+        atomicAdd(a.bx + j, -dr * r[0]);
+        atomicAdd(a.by + j, -dr * r[1]);
+        atomicAdd(a.bz + j, -dr * r[2]);
     }
     atomicAdd(a.bx + k, x[0]);
     atomicAdd(a.by + k, x[1]);
     atomicAdd(a.bz + k, x[2]);
-    atomicAdd(a.bh + k, h);
+    atomicAdd(a.bh + k, h * a.hInv[k]);
 }
 
 }  // namespace
@@ -1555,13 +1581,13 @@ int adjointVe(sphgb_ctx* c, sphgb_particles* p, const double* alphaPrev, int avC
         veGradhSeedKernel<<<eb, 256, 0, c->stream>>>(a);
         SPHGB_TRY(launched(c, "veGradhSeedKernel"));
         if (two) veGradhAdjKernel<true, S><<<pb, kVeAdjBlock, 0, c->stream>>>(a);
-        else if (once) veGradhAdjOnceKernel<S><<<pb, kVeAdjBlock, 0, c->stream>>>(a, ownedView(c));
+        else if (once) veGradhAdjOnceKernel<S><<<ownedGrid(n), kVeAdjBlock, 0, c->stream>>>(a, ownedView(c));
         else veGradhAdjKernel<false, S><<<pb, kVeAdjBlock, 0, c->stream>>>(a);
         SPHGB_TRY(launched(c, "veGradhAdjKernel"));
         veXmassSeedKernel<<<eb, 256, 0, c->stream>>>(a);
         SPHGB_TRY(launched(c, "veXmassSeedKernel"));
         if (two) veXmassAdjKernel<true, S><<<pb, kVeAdjBlock, 0, c->stream>>>(a);
-        else if (once) veXmassAdjOnceKernel<S><<<pb, kVeAdjBlock, 0, c->stream>>>(a, ownedView(c));
+        else if (once) veXmassAdjOnceKernel<S><<<ownedGrid(n), kVeAdjBlock, 0, c->stream>>>(a, ownedView(c));
         else veXmassAdjKernel<false, S><<<pb, kVeAdjBlock, 0, c->stream>>>(a);
         SPHGB_TRY(launched(c, "veXmassAdjKernel"));
         SPHGB_CUDA(cudaStreamSynchronize(c->stream));

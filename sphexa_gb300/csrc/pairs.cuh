@@ -435,15 +435,10 @@ __device__ __forceinline__ double lookupVSlope(const KTab<Smooth>& tb, double v,
     }
 }
 
-// value at x = v / dx and its derivative d/dx, in table units
+// value and derivative d/dx, in table units x = v / dx, in the interval of a slot with s.k >= 0
 template<bool Smooth>
-__device__ __forceinline__ double lookupXSlope(const KTab<Smooth>& tb, double x, double& slope)
+__device__ __forceinline__ double lookupXSlope(const KTab<Smooth>& tb, const TabSlot& s, double& slope)
 {
-    const TabSlot s = tabSlot(x);
-    if (s.k < 0) {
-        slope = 0.0;
-        return 0.0;
-    }
     if constexpr (Smooth) {
         const double2 a = __ldg(tb.t + 2 * s.k), b = __ldg(tb.t + 2 * s.k + 1);
         const double f = s.frac;
@@ -454,6 +449,14 @@ __device__ __forceinline__ double lookupXSlope(const KTab<Smooth>& tb, double x,
         slope = t.y;
         return fma(t.y, s.frac, t.x);
     }
+}
+
+template<bool Smooth>
+__device__ __forceinline__ double lookupXSlope(const KTab<Smooth>& tb, double x, double& slope)
+{
+    const TabSlot s = tabSlot(x);
+    slope = 0.0;
+    return s.k < 0 ? 0.0 : lookupXSlope(tb, s, slope);
 }
 
 // the context's FP64 tables of W and dW/dv in its kernel form
