@@ -30,9 +30,10 @@ namespace {
 constexpr int kNbrBlock = 128;
 constexpr int kWarpsPerBlock = kNbrBlock / kWarp;
 constexpr int kStack = 192;  // 8 children x (21 levels + 3)
-// internal nodes of at most this many particles are taken whole (about eight leaves of 13-16:
-// the octree's last level when a cell of 64 + particles splits into small leaves)
-constexpr uint32_t kCoarseNode = 128;
+// internal nodes of at most this many particles are taken whole: eight leaves of 13-30, the octree's
+// last level.  With nodes pruned by their distance from the target box, fewer pops pay for the extra
+// staged candidates: 8M search stage 12.9 ms against 13.1 with 128; 64 costs the 27M set 7 ms of 28.
+constexpr uint32_t kCoarseNode = 256;
 
 struct NbrArgs {
     const double *x, *y, *z;
@@ -41,6 +42,7 @@ struct NbrArgs {
     const u64* cell;      // packed grid cell per particle
     const float4* loc;    // FP32 offset inside the cell (w unused here)
     float u[3];           // cell edge per axis
+    int sh[3];            // 32 - 21 on periodic axes, 0 on open ones (wrapShift)
     int64_t first, last;
     const uint32_t* active;  // optional: only targets with active[i - first] != 0 are searched
     const int32_t* childOffsets;
@@ -82,8 +84,11 @@ __device__ __forceinline__ void gridOffset(const NbrArgs& a, const int cj[3], fl
 {
     const float lv[3] = {lj.x - lo.x, lj.y - lo.y, lj.z - lo.z};
 #pragma unroll
-    for (int k = 0; k < 3; ++k) r[k] = fmaf(float(CoordMixed::wrap(cj[k] - co[k], a.box.pbc[k])), a.u[k], lv[k]);
+    for (int k = 0; k < 3; ++k) r[k] = fmaf(float(CoordMixed::wrapShift(cj[k] - co[k], a.sh[k])), a.u[k], lv[k]);
 }
+
+// tested candidate blocks whose decision masks wait in registers before the lanes append their neighbours
+constexpr int kHeld = 4;
 
 struct WarpSmem {
     int32_t stack[kStack];
@@ -94,17 +99,23 @@ struct WarpSmem {
     alignas(16) float ny[2 * kWarp];
     alignas(16) float nz[2 * kWarp];
     alignas(16) uint32_t idx[2 * kWarp];
-    // the second cull: box of the target positions (lo x y z, squared radius, hi x y z)
+    uint32_t self[kWarp];  // position of each target in the queue, counted from the first candidate
+    uint32_t held[kHeld][kWarp];  // indices of the tested blocks whose neighbours are still to be appended
+    // the cull: box of the target positions (lo x y z, squared radius, hi x y z)
     alignas(16) float cull[8];
 };
 
+// Bound by instruction issue (about 27k warp instructions per group of 32 targets and 620 tests per target).
+// At 27M particles the search takes 28.0 ms (37.1 with an append loop per tested block, nodes pruned per
+// axis, 6 blocks per SM and nodes of 128 particles taken whole); 8 blocks of 64 registers hide the
+// staging loads best (6: 29.6 ms, 7: 28.6, 9: 30.3).
 // Fold: groups whose pairs need a fold each do it in FP32 (launched for sets below kFoldBelow, where
 // such groups occur with ordinary h); without it they run the FP64 test for every pair, and the code of the
 // fold does not cost the large sets registers (1 % of the search at 27M).
 constexpr int64_t kFoldBelow = 100000;
 
 template<bool Fold>
-__global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
+__global__ void __launch_bounds__(kNbrBlock, Fold ? 6 : 8) nbrGroupKernel(NbrArgs a)
 {
     __shared__ WarpSmem smem[kWarpsPerBlock];
     const int lane = threadIdx.x & (kWarp - 1);
@@ -148,35 +159,41 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
     const float dxi = reli[0], dyi = reli[1], dzi = reli[2];
     const float rf = valid ? __double2float_ru(twoH) : 0.f;
 
-    // group search box relative to the origin
-    float gmin[3] = {valid ? dxi - rf : INFINITY, valid ? dyi - rf : INFINITY, valid ? dzi - rf : INFINITY};
-    float gmax[3] = {valid ? dxi + rf : -INFINITY, valid ? dyi + rf : -INFINITY, valid ? dzi + rf : -INFINITY};
+    // box of the target positions relative to the origin, and the largest radius: the search region is
+    // that box grown by rfm, with rounded edges and corners
+    float tmn[3] = {valid ? dxi : INFINITY, valid ? dyi : INFINITY, valid ? dzi : INFINITY};
+    float tmx[3] = {valid ? dxi : -INFINITY, valid ? dyi : -INFINITY, valid ? dzi : -INFINITY};
+    float rfm = rf;
+    for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k)
-        for (int o = 16; o > 0; o >>= 1) {
-            gmin[k] = fminf(gmin[k], __shfl_xor_sync(0xffffffffu, gmin[k], o));
-            gmax[k] = fmaxf(gmax[k], __shfl_xor_sync(0xffffffffu, gmax[k], o));
+        for (int k = 0; k < 3; ++k) {
+            tmn[k] = fminf(tmn[k], __shfl_xor_sync(0xffffffffu, tmn[k], o));
+            tmx[k] = fmaxf(tmx[k], __shfl_xor_sync(0xffffffffu, tmx[k], o));
         }
+        rfm = fmaxf(rfm, __shfl_xor_sync(0xffffffffu, rfm, o));
+    }
     // absolute position of the origin from its cell (FP32 suffices for pruning, see the pad).
-    // foldPairs: on some periodic axis the search box reaches half the box from the origin (sets of a
+    // foldPairs: on some periodic axis the search region reaches half the box from the origin (sets of a
     // few thousand particles).  Below that a neighbour's offset, wrapped against the origin, is also
     // the image nearest to its target (|offset| <= Rg < L/2), so differences of offsets need no fold.
     bool foldPairs = false;
-    float gc[3], gs[3], Rg = 0.f;
+    float gc[3], gt[3], Rg = 0.f;  // center and half size of the target box for the walk, padded
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        if (b.pbc[k] && fmaxf(fabsf(gmin[k]), fabsf(gmax[k])) > 0.49f * b.Lf[k]) foldPairs = true;
+        const float reach = fmaxf(fabsf(tmn[k]), fabsf(tmx[k])) + rfm;
+        if (b.pbc[k] && reach > 0.49f * b.Lf[k]) foldPairs = true;
         const float lok = (k == 0) ? lo.x : (k == 1 ? lo.y : lo.z);
-        float cAbs = float(b.lo[k]) + fmaf(float(co[k]), a.u[k], lok) + 0.5f * (gmin[k] + gmax[k]);
+        float cAbs = float(b.lo[k]) + fmaf(float(co[k]), a.u[k], lok) + 0.5f * (tmn[k] + tmx[k]);
         if (b.pbc[k]) {
             if (cAbs >= float(b.hi[k])) cAbs -= b.Lf[k];
             else if (cAbs < float(b.lo[k])) cAbs += b.Lf[k];
         }
         gc[k] = cAbs;
         const float pad = float((fabs(b.lo[k]) + fabs(b.hi[k])) * 0x1p-19);
-        gs[k] = 0.5f * (gmax[k] - gmin[k]) + pad;
-        Rg = fmaxf(Rg, fmaxf(fabsf(gmin[k]), fabsf(gmax[k])));
+        gt[k] = 0.5f * (tmx[k] - tmn[k]) + pad;
+        Rg = fmaxf(Rg, reach);
     }
+    const float gR2 = rfm * rfm * (1.f + 0x1p-18f);
     // FP32 decision margin on d2: covers the rounding of cell edge, offsets and the squared sum (and,
     // where pairs are folded, of the box length, L <= 2 Rg / 0.98 there); pairs inside the margin get the
     // exact FP64 test
@@ -209,32 +226,40 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
             ++cnt;
         }
     };
+    // Appends run for four tested blocks together.  The hits of one block of 32 lie in few lanes (17
+    // loop trips for 5 hits on average, the block being a compact cluster near some of the targets); over
+    // four blocks the lanes even out (1M particles: 341 -> 150 trips per warp and search).
+    uint32_t m0 = 0, m1 = 0, m2 = 0, m3 = 0;
+    int nHeld = 0;
+    auto appendHeld = [&]() {
+        int base = -1;
+        while (m0 | m1 | m2 | m3) {
+            const bool next = m0 == 0;
+            m0 = next ? m1 : m0;
+            m1 = next ? m2 : m1;
+            m2 = next ? m3 : m2;
+            m3 = next ? 0u : m3;
+            base += next ? kWarp : 0;
+            if (m0 != 0) {
+                out.put(cnt, (&sm.held[0][0])[base + __ffs(m0)]);
+                ++cnt;
+                m0 &= m0 - 1u;
+            }
+        }
+        nHeld = 0;
+        __syncwarp();
+    };
 
     // Candidates are staged 32 at a time (one per lane, coalesced loads of cell and offset); those
-    // outside the group's search box by more than the FP32 rounding of the offsets (cullPad) are
+    // outside the search region by more than the FP32 rounding of the offsets (cullPad) are
     // dropped and the rest appended, in ascending index order, to the warp's queue by ballot
-    // compaction.  A dropped candidate is farther than 2h from every target along one axis, so the
-    // reference's FP64 test rejects it too.  Each full queue block of 32 is tested by every target
+    // compaction.  A dropped candidate is farther than 2h from every target, so the reference's FP64
+    // test rejects it too.  Each full queue block of 32 is tested by every target
     // with a fixed trip count; the last, partial block has NaN in its empty slots.
     // Groups that fold their pairs keep every candidate.
     const float cullPad = 32.f * 0x1p-24f * (Rg + fmaxf(a.u[0], fmaxf(a.u[1], a.u[2])));
-    const float bxl = gmin[0] - cullPad, bxh = gmax[0] + cullPad;
-    const float byl = gmin[1] - cullPad, byh = gmax[1] + cullPad;
-    const float bzl = gmin[2] - cullPad, bzh = gmax[2] + cullPad;
-    // second cull: the box of the target positions grown by the largest radius with rounded
-    // edges and corners (a candidate farther than max 2h from that box is farther than 2h_i from
-    // every target i); the pad covers the offsets' FP32 rounding, the factor the squared sum's
-    float tmn[3] = {valid ? dxi : INFINITY, valid ? dyi : INFINITY, valid ? dzi : INFINITY};
-    float tmx[3] = {valid ? dxi : -INFINITY, valid ? dyi : -INFINITY, valid ? dzi : -INFINITY};
-    float rfm = rf;
-    for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            tmn[k] = fminf(tmn[k], __shfl_xor_sync(0xffffffffu, tmn[k], o));
-            tmx[k] = fmaxf(tmx[k], __shfl_xor_sync(0xffffffffu, tmx[k], o));
-        }
-        rfm = fmaxf(rfm, __shfl_xor_sync(0xffffffffu, rfm, o));
-    }
+    // the cull: a candidate farther than max 2h from the target box is farther than 2h_i from every
+    // target i; the pad covers the offsets' FP32 rounding, the factor the squared sum's
     const float cullR = rfm + cullPad;
     if (lane == 0) {
         sm.cull[0] = tmn[0];
@@ -249,7 +274,10 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
     __syncwarp();
     // 1/L of the periodic axes (0 leaves an axis unfolded)
     const float foldL[3] = {b.pbc[0] ? 1.f / b.Lf[0] : 0.f, b.pbc[1] ? 1.f / b.Lf[1] : 0.f, b.pbc[2] ? 1.f / b.Lf[2] : 0.f};
-    int qn = 0;  // candidates in the queue
+    int qn = 0;          // candidates in the queue
+    uint32_t qBase = 0;  // candidates tested before the queue's first
+    sm.self[lane] = 0xffffffffu;
+    __syncwarp();
     auto testBlock = [&](int filled) {
         if (valid) tested += unsigned(filled);
         if (!Fold && foldPairs) {
@@ -309,15 +337,30 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
                     }
                 }
             }
+            // a target is no neighbour of itself
+            const uint32_t own = sm.self[lane] - qBase;
+            if (own < unsigned(kWarp)) {
+                hit &= ~(1u << own);
+                nearm &= ~(1u << own);
+            }
             if (valid) {
                 // a pair within the FP32 margin of the radius (rare): the exact test
                 for (uint32_t band = nearm & ~hit; band != 0; band &= band - 1u) {
                     const int s = __ffs(band) - 1;
                     if (exactIn(sm.idx[s])) hit |= 1u << s;
                 }
-                for (; hit != 0; hit &= hit - 1u) take(sm.idx[__ffs(hit) - 1]);
-            }
+            } else
+                hit = 0;
+            sm.held[nHeld][lane] = sm.idx[lane];
+            if (nHeld == 0) m0 = hit;
+            else if (nHeld == 1) m1 = hit;
+            else if (nHeld == 2) m2 = hit;
+            else m3 = hit;
+            ++nHeld;
+            __syncwarp();
+            if (nHeld == kHeld) appendHeld();
         }
+        qBase += kWarp;
         __syncwarp();
     };
     auto flush = [&](int64_t ja, int m) {
@@ -333,8 +376,7 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
             const float ex = fmaxf(fmaxf(cl.x - rj[0], rj[0] - ch.x), 0.f);
             const float ey = fmaxf(fmaxf(cl.y - rj[1], rj[1] - ch.y), 0.f);
             const float ez = fmaxf(fmaxf(cl.z - rj[2], rj[2] - ch.z), 0.f);
-            keep = foldPairs || (rj[0] >= bxl && rj[0] <= bxh && rj[1] >= byl && rj[1] <= byh && rj[2] >= bzl &&
-                                 rj[2] <= bzh && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= cl.w);
+            keep = foldPairs || fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= cl.w;
         }
         const unsigned km = __ballot_sync(0xffffffffu, keep);
         if (keep) {
@@ -343,6 +385,8 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
             sm.ny[q] = -rj[1];
             sm.nz[q] = -rj[2];
             sm.idx[q] = uint32_t(ja + lane);
+            const int64_t t = ja + lane - g0;
+            if (t >= 0 && t < kWarp) sm.self[t] = qBase + q;
         }
         qn += __popc(km);
         __syncwarp();
@@ -411,15 +455,17 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
         if (lane < 8) {
             const float4 c4 = a.nodeBox[2 * child], s4 = a.nodeBox[2 * child + 1];
             const float cc[3] = {c4.x, c4.y, c4.z}, ss[3] = {s4.x, s4.y, s4.z};
-            ov = true;
             inside = true;
+            float e2 = 0.f;
 #pragma unroll
             for (int k = 0; k < 3; ++k) {
                 float dd = fabsf(cc[k] - gc[k]);
                 if (b.pbc[k]) dd = fminf(dd, b.Lf[k] - dd);
-                ov = ov && (dd <= ss[k] + gs[k]);
-                inside = inside && (dd + ss[k] <= gs[k]);
+                const float gap = fmaxf(dd - ss[k] - gt[k], 0.f);
+                e2 = fmaf(gap, gap, e2);
+                inside = inside && (dd + ss[k] <= gt[k] + rfm);
             }
+            ov = e2 <= gR2;
         }
         const unsigned m = __ballot_sync(0xffffffffu, ov);
         const int k = __popc(m);
@@ -442,6 +488,7 @@ __global__ void __launch_bounds__(kNbrBlock, 6) nbrGroupKernel(NbrArgs a)
         pa += m;
     }
     drain();
+    appendHeld();
 
     if (valid) {
         out.finish(cnt);
@@ -845,7 +892,10 @@ int runSearch(sphgb_ctx* c, const double* x, const double* y, const double* z, c
     a.hIsFloat = hIsFloat;
     a.cell = c->gridKey.as<u64>();
     a.loc = c->gridLoc.as<float4>();
-    for (int k = 0; k < 3; ++k) a.u[k] = float(c->box.L[k] / double(1 << kGridBits));
+    for (int k = 0; k < 3; ++k) {
+        a.u[k] = float(c->box.L[k] / double(1 << kGridBits));
+        a.sh[k] = c->box.pbc[k] ? 32 - kGridBits : 0;
+    }
     a.first = first;
     a.last = last;
     a.active = active;

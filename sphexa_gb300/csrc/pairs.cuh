@@ -45,30 +45,33 @@ __host__ __device__ __forceinline__ int64_t listSlot(int64_t ii, unsigned k, int
 // entries per target that the buffers reserve for a capacity of ngmax (whole granules)
 inline size_t listCapacity(uint32_t ngmax) { return (size_t(ngmax) + kListGran - 1) / kListGran * kListGran; }
 
-// writes one target's list in order: entries collect in registers, every fourth one stores the
-// granule; finish() stores the last, partial granule.  Granules at or beyond the capacity are not
+// writes one target's list in order: the last three entries stay in registers, every fourth one stores
+// the granule; finish() stores the last, partial granule.  Granules at or beyond the capacity are not
 // written (entries past ngmax of a capped list are dropped, as the reference drops them).
 struct GranuleWriter {
-    uint4* out;  // granule 0 of this target; granule g at out[g * stride]
+    uint4* out;  // the open granule of this target
     int64_t stride;
-    unsigned capG;
+    unsigned cap;  // entries, whole granules
     uint32_t b0 = 0, b1 = 0, b2 = 0;
     __device__ __forceinline__ GranuleWriter(uint32_t* base, int64_t ii, int64_t stride_, uint32_t ngmax)
-        : out(reinterpret_cast<uint4*>(base) + ii), stride(stride_), capG((ngmax + kListGran - 1) / kListGran)
+        : out(reinterpret_cast<uint4*>(base) + ii), stride(stride_), cap((ngmax + kListGran - 1) / kListGran * kListGran)
     {
     }
     __device__ __forceinline__ void put(unsigned cnt, uint32_t j)
     {
-        const unsigned s = cnt % kListGran, g = cnt / kListGran;
-        b0 = s == 0 ? j : b0;
-        b1 = s == 1 ? j : b1;
-        b2 = s == 2 ? j : b2;
-        if (s == kListGran - 1 && g < capG) out[int64_t(g) * stride] = make_uint4(b0, b1, b2, j);
+        if ((cnt & (kListGran - 1)) == kListGran - 1) {
+            if (cnt < cap) *out = make_uint4(b0, b1, b2, j);
+            out += stride;
+        }
+        b0 = b1;
+        b1 = b2;
+        b2 = j;
     }
     __device__ __forceinline__ void finish(unsigned cnt)
     {
-        const unsigned g = cnt / kListGran;
-        if (cnt % kListGran != 0 && g < capG) out[int64_t(g) * stride] = make_uint4(b0, b1, b2, 0u);
+        const unsigned s = cnt & (kListGran - 1);
+        if (s != 0 && cnt < cap)
+            *out = s == 1 ? make_uint4(b2, 0u, 0u, 0u) : s == 2 ? make_uint4(b1, b2, 0u, 0u) : make_uint4(b0, b1, b2, 0u);
     }
 };
 
