@@ -238,6 +238,10 @@ int buildOwnedFromLists(sphgb_ctx* c);
 // optional 32-bit values, out of place
 int radixSort(sphgb_ctx* c, const u64* keysIn, u64* keysOut, const uint32_t* valsIn, uint32_t* valsOut, int64_t n,
               int endBit, int beginBit = 0);
+// the same for the 63-bit SFC keys of n particles with their indices, over as many upper bits as tell most
+// particles apart
+int sortParticleKeys(sphgb_ctx* c, const u64* keysIn, u64* keysOut, const uint32_t* valsIn, uint32_t* valsOut,
+                     int64_t n);
 // the radix sort's give-up flag: queue its copy to the host before a stream sync, test it after
 // (SPHGB_ERR_TIMEOUT when a look-back wait gave up; the flag is then cleared)
 int sortStatusAsync(sphgb_ctx* c);

@@ -476,8 +476,8 @@ int domainSync(sphgb_ctx* c, sphgb_particles* p, sphgb_box* box)
     keysKernel<<<gridFor(n, kBlock), kBlock, 0, st>>>(p->x, p->y, p->z, n, c->box, c->keysAlt.as<u64>(),
                                                        c->orderAlt.as<uint32_t>());
     SPHGB_TRY(launched(c, "keysKernel"));
-    SPHGB_TRY(radixSort(c, c->keysAlt.as<u64>(), c->keys.as<u64>(), c->orderAlt.as<uint32_t>(),
-                        c->order.as<uint32_t>(), n, 63));
+    SPHGB_TRY(sortParticleKeys(c, c->keysAlt.as<u64>(), c->keys.as<u64>(), c->orderAlt.as<uint32_t>(),
+                               c->order.as<uint32_t>(), n));
 
     // permute the conserved fields in place (the reference's particleProperties of sync)
     const size_t hs = p->precision == SPHGB_MIXED ? 4 : 8;

@@ -167,3 +167,36 @@ def test_inputs_changed_between_passes(gpu_ctx, moved, variant):
     gpu_ctx.set_deterministic(False)
     check_fields(out[False], out[True], "std" if variant == "std" else "ve", fields, f"{variant} {moved}")
     assert out[False]["minDt"] == pytest.approx(out[True]["minDt"], rel=1e-12)
+
+
+@pytest.mark.parametrize("n", [4096, 4097, 6001, 70001])
+@pytest.mark.parametrize("spread", ["uniform", "cells", "cluster", "coincident"])
+def test_sync_order_of_close_keys(gpu_ctx, n, spread):
+    """The key sort by upper bits: sets without and with runs of keys that agree there (particles within
+    a few grid cells of one another), one tight cluster (sorted over all bits) and equal keys (input
+    order): order and keys against numpy's stable sort of the keys of an unsorted call."""
+    import torch
+    from sphexa_gb300 import _lib, sph, workloads as W
+    wl = W.random_cube(n, seed=99, periodic=True)
+    rng = np.random.Generator(np.random.PCG64(100))
+    for k in ("x", "y", "z"):
+        x = wl.fields[k]
+        if spread == "cells":
+            x = x[np.arange(n) // 5] + rng.uniform(0.0, 4e-6, n)
+        elif spread == "cluster":
+            x = 0.3 + rng.uniform(0.0, 1e-4, n)
+        elif spread == "coincident":
+            x = x[np.arange(n) // 7]
+        wl.fields[k] = np.clip(x, 0.0, 1.0 - 1e-9)
+    d = sph.ParticlesData.from_workload(wl, "fp64", "cuda:0")
+    keys = torch.empty(n, dtype=torch.int64, device="cuda:0")
+    box = sph.Box(wl.box.copy(), wl.bc.copy())
+    b = box.to_c()
+    assert gpu_ctx.lib.sphgb_sfc_keys_noalloc(d.x.data_ptr(), d.y.data_ptr(), d.z.data_ptr(), n, _lib.C.byref(b),
+                                              keys.data_ptr(), None) == 0
+    raw = keys.cpu().numpy().view(np.uint64)
+    dom = sph.Domain(gpu_ctx, box)
+    dom.sync(d)
+    order = np.argsort(raw, kind="stable")
+    np.testing.assert_array_equal(dom.order(n), order)
+    np.testing.assert_array_equal(d.keys.cpu().numpy().view(np.uint64), raw[order])
