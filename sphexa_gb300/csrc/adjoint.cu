@@ -804,6 +804,8 @@ __global__ void __launch_bounds__(kAdjBlock) meAdjOnceT(StdScatterArgs<T> a, Own
 }
 
 // ---- one evaluation per owned entry of the owned lists (mutual pairs give both directed terms) ----
+// Small sets launch several block rows, each on its slice of the lists (ownedGrid); the per-particle
+// terms are added by row 0.
 __device__ __forceinline__ stdad::MeSide<> stdSide(const AdjArgs& a, int64_t i)
 {
     stdad::MeSide<> s;
@@ -845,7 +847,7 @@ __global__ void __launch_bounds__(kAdjBlock) meAdjOnceKernel(AdjArgs a, OwnedVie
     double bx[3] = {0, 0, 0}, bv[3] = {0, 0, 0}, bh = 0, brho = 0, bp = 0, bc = 0, bC[6] = {0, 0, 0, 0, 0, 0};
     const stdad::MeSide<> S = stdSide(a, k);
     const unsigned cnt = ov.size(k);
-    for (unsigned q = 0; q < cnt; ++q) {
+    for (unsigned q = blockIdx.y; q < cnt; q += gridDim.y) {  // this block row's slice of the lists
         bool mutual;
         const uint32_t j = ov.at(k, q, mutual);
         double gAj[3] = {0.0, 0.0, 0.0}, gEj = 0.0;
@@ -888,7 +890,7 @@ __global__ void __launch_bounds__(kAdjBlock) meAdjOnceKernel(AdjArgs a, OwnedVie
     atomicAdd(a.bvy + k, bv[1]);
     atomicAdd(a.bvz + k, bv[2]);
     atomicAdd(a.bh + k, bh);
-    atomicAdd(a.bRho + k, brho + (a.sRho ? a.sRho[k] : 0.0));
+    atomicAdd(a.bRho + k, brho + (a.sRho && blockIdx.y == 0 ? a.sRho[k] : 0.0));
     atomicAdd(a.bP + k, bp);
     atomicAdd(a.bC + k, bc);
     for (int t = 0; t < 6; ++t) atomicAdd(a.bCij + t * a.n + k, bC[t]);
@@ -910,7 +912,7 @@ __global__ void __launch_bounds__(kAdjBlock) iadAdjOnceKernel(AdjArgs a, OwnedVi
     tauOf(a, k, tauK);
     const double hInvK = a.hInv[k], volK = a.mOverRho[k], rhoInvK = a.rhoInv[k];
     const unsigned cnt = ov.size(k);
-    for (unsigned q = 0; q < cnt; ++q) {
+    for (unsigned q = blockIdx.y; q < cnt; q += gridDim.y) {  // this block row's slice of the lists
         bool mutual;
         const uint32_t j = ov.at(k, q, mutual);
         double r[3], d, rinv, dw;
@@ -951,9 +953,9 @@ __global__ void __launch_bounds__(kAdjBlock) densityAdjOnceKernel(AdjArgs a, Own
     const int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (k >= a.n) return;
     const double rhobK = a.bRho[k], hInvK = a.hInv[k], mK = a.m[k];
-    double bx[3] = {0, 0, 0}, bh = rhobK * (-3.0 * a.rho[k] * hInvK);
+    double bx[3] = {0, 0, 0}, bh = blockIdx.y == 0 ? rhobK * (-3.0 * a.rho[k] * hInvK) : 0.0;
     const unsigned cnt = ov.size(k);
-    for (unsigned q = 0; q < cnt; ++q) {
+    for (unsigned q = blockIdx.y; q < cnt; q += gridDim.y) {  // this block row's slice of the lists
         bool mutual;
         const uint32_t j = ov.at(k, q, mutual);
         double r[3], d, rinv, dw;
@@ -1265,17 +1267,17 @@ int adjointStd(sphgb_ctx* c, sphgb_particles* p, const sphgb_seeds* s, sphgb_gra
     SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
         constexpr bool S = decltype(smooth)::value;
         if (deterministic) meAdjKernel<S><<<blocks, kAdjBlock, 0, c->stream>>>(a);
-        else meAdjOnceKernel<S><<<blocks, kAdjBlock, 0, c->stream>>>(a, ownedView(c));
+        else meAdjOnceKernel<S><<<ownedGrid(n), kAdjBlock, 0, c->stream>>>(a, ownedView(c));
         SPHGB_TRY(launched(c, "meAdjKernel"));
         iadPrepKernel<<<gridFor(n, 256), 256, 0, c->stream>>>(a);
         SPHGB_TRY(launched(c, "iadPrepKernel"));
         if (deterministic) iadAdjKernel<S><<<blocks, kAdjBlock, 0, c->stream>>>(a);
-        else iadAdjOnceKernel<S><<<blocks, kAdjBlock, 0, c->stream>>>(a, ownedView(c));
+        else iadAdjOnceKernel<S><<<ownedGrid(n), kAdjBlock, 0, c->stream>>>(a, ownedView(c));
         SPHGB_TRY(launched(c, "iadAdjKernel"));
         eosAdjKernel<<<gridFor(n, 256), 256, 0, c->stream>>>(a);
         SPHGB_TRY(launched(c, "eosAdjKernel"));
         if (deterministic) densityAdjKernel<S><<<blocks, kAdjBlock, 0, c->stream>>>(a);
-        else densityAdjOnceKernel<S><<<blocks, kAdjBlock, 0, c->stream>>>(a, ownedView(c));
+        else densityAdjOnceKernel<S><<<ownedGrid(n), kAdjBlock, 0, c->stream>>>(a, ownedView(c));
         return launched(c, "densityAdjKernel");
     }));
     SPHGB_CUDA(cudaStreamSynchronize(c->stream));

@@ -820,17 +820,20 @@ __global__ void __launch_bounds__(128) ownedListKernel(MutualArgs a)
 
 // owned lists from list membership alone: (i, j) is mutual when i is in j's (capped, ascending)
 // list, found by binary search, so the decision holds whatever the positions are now (frozen lists
-// after moved particles).  Ownership of a mutual pair as in ownedListKernel.
+// after moved particles).  A mutual pair goes by index parity: balanced lists (ownWithinWarp) gave the
+// FP32 adjoint that walks these no time back, and FP32 sums in another order move its gradients by
+// 4e-7, three times what two runs differ by.
 __global__ void __launch_bounds__(128) ownedByListKernel(const uint32_t* __restrict__ nbr,
                                                          const uint32_t* __restrict__ count, int64_t first, int64_t last,
                                                          int64_t stride, uint32_t ngmax, uint32_t* __restrict__ owned,
                                                          uint32_t* __restrict__ ownedCount)
 {
     const int64_t i = first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-    const bool valid = i < last;
+    if (i >= last) return;
     const int64_t ii = i - first;
-    const unsigned nc = valid ? min(__ldg(count + ii), ngmax) : 0u;
-    OwnedWriter w(owned, ii, first, stride, ngmax);
+    const unsigned nc = min(__ldg(count + ii), ngmax);
+    unsigned cnt = 0;
+    GranuleWriter out(owned, ii, stride, ngmax);
     for (unsigned k = 0; k < nc; ++k) {
         const uint32_t j = __ldg(nbr + listSlot(ii, k, stride));
         bool m = false;
@@ -845,10 +848,11 @@ __global__ void __launch_bounds__(128) ownedByListKernel(const uint32_t* __restr
             }
             m = lo < min(__ldg(count + jj), ngmax) && int64_t(__ldg(nbr + listSlot(jj, lo, stride))) == i;
         }
-        w.offer(j, m);
+        const bool own = !m || ((((i ^ int64_t(j)) & 1) != 0) == (i < int64_t(j)));
+        if (own) out.put(cnt++, j | (m ? 0x80000000u : 0u));
     }
-    const unsigned cnt = w.finish();
-    if (valid) ownedCount[ii] = cnt;
+    out.finish(cnt);
+    ownedCount[ii] = cnt;
 }
 
 __global__ void fillOnes(uint32_t* p, int64_t n)
