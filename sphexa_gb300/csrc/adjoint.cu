@@ -507,13 +507,86 @@ struct StdScatterArgs {
     int64_t n;
     const T *sRho, *sAx, *sAy, *sAz;
     const double* sDu;
-    // adjoints, accumulated in the pair type: the FP64 form writes the caller's gradients and FP64
-    // state, the mixed form FP32 arrays (converted to the FP64 gradients at the end)
+    // adjoints, accumulated in the pair type: the FP64 form adds to the caller's gradients and FP64
+    // state arrays, the mixed form to one record of 16 floats per particle (acc, see slot()), converted
+    // to the FP64 gradients at the end
     T *bx, *by, *bz, *bvx, *bvy, *bvz, *bh, *bu;
     T *bRho, *bP, *bC, *bCij, *tauBar;
+    T* acc;
+    T* rhoB;                              // the complete rho adjoint, read by the density adjoint
     T *hInv, *moR, *poR, *rhoInv, *poR2;  // per-particle quotients in the pair type
+    float4* side;                         // mixed form: 5 per particle, what a pair reads of it (meInOf)
     CoordMixed cm;                         // mixed form: the grid-form coordinates of the forward passes
 };
+
+// Accumulator slots.  The mixed form keeps a particle's 16 accumulators in one 64-byte record and adds
+// four at a time (a 16-byte vector reduction, each component an FP32 add of its own).  The pair kernels
+// were bound by the issue of scalar reductions and gathers, 16 reductions (momentum-energy), 4 (IAD) and
+// 3 (density) per pair; now it is 4, 1 and 1.  With the 80-byte records of meInOf, forward and gradient
+// at 125k particles went from 2368 to 2000 us.
+enum : int { kBx, kBy, kBz, kBRho, kBvx, kBvy, kBvz, kBh, kBP, kBC, kBCij, kSlots = 16 };
+
+template<int S, class T>
+__device__ __forceinline__ T* slot(const StdScatterArgs<T>& a, int64_t k)
+{
+    if constexpr (std::is_same_v<T, float>) {
+        return a.acc + kSlots * k + S;
+    } else if constexpr (S >= kBCij) {
+        return a.bCij + (S - kBCij) * a.n + k;
+    } else {
+        T* const by[kBCij] = {a.bx, a.by, a.bz, a.bRho, a.bvx, a.bvy, a.bvz, a.bh, a.bP, a.bC};
+        return by[S] + k;
+    }
+}
+
+template<int S, class T>
+__device__ __forceinline__ void add4(const StdScatterArgs<T>& a, int64_t k, T v0, T v1, T v2, T v3)
+{
+    if constexpr (std::is_same_v<T, float>) {
+        atomicAdd(reinterpret_cast<float4*>(slot<S>(a, k)), make_float4(v0, v1, v2, v3));
+    } else {
+        atomicAdd(slot<S>(a, k), v0);
+        atomicAdd(slot<S + 1>(a, k), v1);
+        atomicAdd(slot<S + 2>(a, k), v2);
+        atomicAdd(slot<S + 3>(a, k), v3);
+    }
+}
+
+// the position adjoint alone: the record's fourth word (rho) gets +0
+template<class T>
+__device__ __forceinline__ void addPos(const StdScatterArgs<T>& a, int64_t k, T v0, T v1, T v2)
+{
+    if constexpr (std::is_same_v<T, float>) {
+        add4<kBx>(a, k, v0, v1, v2, 0.0f);
+    } else {
+        atomicAdd(a.bx + k, v0);
+        atomicAdd(a.by + k, v1);
+        atomicAdd(a.bz + k, v2);
+    }
+}
+
+// all accumulators of one end of a momentum-energy pair (or of a particle's own sums)
+template<class T>
+__device__ __forceinline__ void addMe(const StdScatterArgs<T>& a, int64_t k, T rx, T ry, T rz, T vx, T vy, T vz, T h,
+                                      T rho, T p, T c, const T C[6])
+{
+    add4<kBx>(a, k, rx, ry, rz, rho);
+    add4<kBvx>(a, k, vx, vy, vz, h);
+    add4<kBP>(a, k, p, c, C[0], C[1]);
+    add4<kBCij + 2>(a, k, C[2], C[3], C[4], C[5]);
+}
+
+// seeds of particle k in the pair type: K times the acceleration seeds and -K/2 times the du seed;
+// false when they are all zero
+template<class T>
+__device__ __forceinline__ bool seedsOfT(const StdScatterArgs<T>& a, int64_t k, T gA[3], T& gE)
+{
+    gA[0] = a.sAx ? T(a.K * double(a.sAx[k])) : T(0);
+    gA[1] = a.sAy ? T(a.K * double(a.sAy[k])) : T(0);
+    gA[2] = a.sAz ? T(a.K * double(a.sAz[k])) : T(0);
+    gE = a.sDu ? T(-0.5 * a.K * a.sDu[k]) : T(0);
+    return gA[0] != T(0) || gA[1] != T(0) || gA[2] != T(0) || gE != T(0);
+}
 
 template<class T>
 __global__ void stdQuotKernel(StdScatterArgs<T> a)
@@ -526,6 +599,16 @@ __global__ void stdQuotKernel(StdScatterArgs<T> a)
     a.poR[i] = T(p / rho);
     a.rhoInv[i] = T(1.0 / rho);
     a.poR2[i] = T(p / (rho * rho));
+    if constexpr (std::is_same_v<T, float>) {
+        float gA[3], gE;
+        seedsOfT(a, i, gA, gE);
+        float4* r = a.side + 5 * i;
+        r[0] = make_float4(a.hInv[i], a.c[i], a.m[i], a.rhoInv[i]);
+        r[1] = make_float4(a.poR[i], a.poR2[i], a.C[0][i], a.C[1][i]);
+        r[2] = make_float4(a.C[2][i], a.C[3][i], a.C[4][i], a.C[5][i]);
+        r[3] = make_float4(a.vx[i], a.vy[i], a.vz[i], gA[0]);
+        r[4] = make_float4(gA[1], gA[2], gE, 0.0f);
+    }
 }
 
 template<class T>
@@ -541,6 +624,52 @@ __device__ __forceinline__ stdad::MeSide<T> stdSideT(const StdScatterArgs<T>& a,
 #pragma unroll
     for (int q = 0; q < 6; ++q) s.C[q] = a.C[q][i];
     return s;
+}
+
+// what the momentum-energy adjoint reads of one particle; the mixed form has it in 80 contiguous bytes
+// (five 16-byte loads; field by field it was 19 loads and an FP64 conversion per neighbour)
+template<class T>
+struct MeIn {
+    stdad::MeSide<T> s;
+    T v[3], gA[3], gE;
+    bool any;  // some seed is not zero
+};
+
+template<class T>
+__device__ __forceinline__ MeIn<T> meInOf(const StdScatterArgs<T>& a, int64_t i)
+{
+    MeIn<T> o;
+    if constexpr (std::is_same_v<T, float>) {
+        const float4* r = a.side + 5 * i;
+        const float4 r0 = __ldg(r), r1 = __ldg(r + 1), r2 = __ldg(r + 2), r3 = __ldg(r + 3), r4 = __ldg(r + 4);
+        o.s.hInv = r0.x;
+        o.s.c = r0.y;
+        o.s.m = r0.z;
+        o.s.rhoInv = r0.w;
+        o.s.poR = r1.x;
+        o.s.poR2 = r1.y;
+        o.s.C[0] = r1.z;
+        o.s.C[1] = r1.w;
+        o.s.C[2] = r2.x;
+        o.s.C[3] = r2.y;
+        o.s.C[4] = r2.z;
+        o.s.C[5] = r2.w;
+        o.v[0] = r3.x;
+        o.v[1] = r3.y;
+        o.v[2] = r3.z;
+        o.gA[0] = r3.w;
+        o.gA[1] = r4.x;
+        o.gA[2] = r4.y;
+        o.gE = r4.z;
+        o.any = o.gA[0] != 0.0f || o.gA[1] != 0.0f || o.gA[2] != 0.0f || o.gE != 0.0f;
+    } else {
+        o.s = stdSideT(a, i);
+        o.v[0] = a.vx[i];
+        o.v[1] = a.vy[i];
+        o.v[2] = a.vz[i];
+        o.any = seedsOfT(a, i, o.gA, o.gE);
+    }
+    return o;
 }
 
 // r = x_i - x_j as the forward passes of that form take it: FP64 differences with the legacy fold
@@ -572,24 +701,21 @@ __global__ void __launch_bounds__(kAdjBlock) meAdjScatterT(StdScatterArgs<T> a)
     const auto tab = kernelTab<Smooth>(a.wh);
     const int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (k >= a.n) return;
-    const T gA[3] = {a.sAx ? T(a.K * double(a.sAx[k])) : T(0), a.sAy ? T(a.K * double(a.sAy[k])) : T(0),
-                     a.sAz ? T(a.K * double(a.sAz[k])) : T(0)};
-    const T gE = a.sDu ? T(-0.5 * a.K * a.sDu[k]) : T(0);
+    const MeIn<T> I = meInOf(a, k);
     T bx[3] = {0, 0, 0}, bv[3] = {0, 0, 0}, bh = 0, brho = 0, bp = 0, bc = 0, bC[6] = {0, 0, 0, 0, 0, 0};
-    if (gA[0] != T(0) || gA[1] != T(0) || gA[2] != T(0) || gE != T(0)) {
-        const stdad::MeSide<T> S = stdSideT(a, k);
+    if (I.any) {
         const T zero[3] = {T(0), T(0), T(0)};
         const unsigned nc = a.lv.capped(k);
         for (unsigned q = 0; q < nc; ++q) {
             const int64_t j = a.lv.at(k, q);
-            const stdad::MeSide<T> J = stdSideT(a, j);
+            const MeIn<T> J = meInOf(a, j);
             T r[3], d, rinv;
             geomT(a, k, j, r, d, rinv);
-            const T v[3] = {a.vx[k] - a.vx[j], a.vy[k] - a.vy[j], a.vz[k] - a.vz[j]};
+            const T v[3] = {I.v[0] - J.v[0], I.v[1] - J.v[1], I.v[2] - J.v[2]};
             T dwi, dwj;
-            const T wi = lookupSlopeT(tab, d * S.hInv, dwi), wj = lookupSlopeT(tab, d * J.hInv, dwj);
+            const T wi = lookupSlopeT(tab, d * I.s.hInv, dwi), wj = lookupSlopeT(tab, d * J.s.hInv, dwj);
             stdad::MeGrad<T> o;
-            stdad::meStdAdjPair<T>(r, d, rinv, v, S, J, wi, dwi, wj, dwj, gA, gE, zero, T(0), o);
+            stdad::meStdAdjPair<T>(r, d, rinv, v, I.s, J.s, wi, dwi, wj, dwj, I.gA, I.gE, zero, T(0), o);
             for (int t = 0; t < 3; ++t) {
                 bx[t] += o.r[t];
                 bv[t] += o.v[t];
@@ -599,30 +725,10 @@ __global__ void __launch_bounds__(kAdjBlock) meAdjScatterT(StdScatterArgs<T> a)
             bp += o.pI;
             bc += o.c;
             for (int t = 0; t < 6; ++t) bC[t] += o.CI[t];
-            atomicAdd(a.bx + j, -o.r[0]);
-            atomicAdd(a.by + j, -o.r[1]);
-            atomicAdd(a.bz + j, -o.r[2]);
-            atomicAdd(a.bvx + j, -o.v[0]);
-            atomicAdd(a.bvy + j, -o.v[1]);
-            atomicAdd(a.bvz + j, -o.v[2]);
-            atomicAdd(a.bh + j, o.hJ);
-            atomicAdd(a.bRho + j, o.rhoJ);
-            atomicAdd(a.bP + j, o.pJ);
-            atomicAdd(a.bC + j, o.c);
-            for (int t = 0; t < 6; ++t) atomicAdd(a.bCij + t * a.n + j, o.CJ[t]);
+            addMe(a, j, -o.r[0], -o.r[1], -o.r[2], -o.v[0], -o.v[1], -o.v[2], o.hJ, o.rhoJ, o.pJ, o.c, o.CJ);
         }
     }
-    atomicAdd(a.bx + k, bx[0]);
-    atomicAdd(a.by + k, bx[1]);
-    atomicAdd(a.bz + k, bx[2]);
-    atomicAdd(a.bvx + k, bv[0]);
-    atomicAdd(a.bvy + k, bv[1]);
-    atomicAdd(a.bvz + k, bv[2]);
-    atomicAdd(a.bh + k, bh);
-    atomicAdd(a.bRho + k, brho + (a.sRho ? a.sRho[k] : T(0)));
-    atomicAdd(a.bP + k, bp);
-    atomicAdd(a.bC + k, bc);
-    for (int t = 0; t < 6; ++t) atomicAdd(a.bCij + t * a.n + k, bC[t]);
+    addMe(a, k, bx[0], bx[1], bx[2], bv[0], bv[1], bv[2], bh, brho + (a.sRho ? a.sRho[k] : T(0)), bp, bc, bC);
 }
 
 template<class T>
@@ -634,10 +740,10 @@ __global__ void iadPrepT(StdScatterArgs<T> a)
 #pragma unroll
     for (int q = 0; q < 6; ++q) {
         C[q] = double(a.C[q][k]);
-        Cb[q] = double(a.bCij[q * a.n + k]);
+        Cb[q] = double(slot<kBCij>(a, k)[std::is_same_v<T, float> ? int64_t(q) : q * a.n]);
     }
     stdad::iadSeed(a.K, double(a.h[k]), C, Cb, tauB, hb);
-    a.bh[k] += T(hb);
+    *slot<kBh>(a, k) += T(hb);
 #pragma unroll
     for (int q = 0; q < 6; ++q) a.tauBar[q * a.n + k] = T(tauB[q]);
 }
@@ -663,15 +769,10 @@ __global__ void __launch_bounds__(kAdjBlock) iadAdjScatterT(StdScatterArgs<T> a)
         stdad::iadAdjTerm<T>(r, d, rinv, hInv, w, dw, a.moR[j], a.rhoInv[j], tauB, rb, hIb, rhoJb);
         for (int t = 0; t < 3; ++t) bx[t] += rb[t];
         bh += hIb;
-        atomicAdd(a.bx + j, -rb[0]);
-        atomicAdd(a.by + j, -rb[1]);
-        atomicAdd(a.bz + j, -rb[2]);
-        atomicAdd(a.bRho + j, rhoJb);
+        add4<kBx>(a, j, -rb[0], -rb[1], -rb[2], rhoJb);
     }
-    atomicAdd(a.bx + k, bx[0]);
-    atomicAdd(a.by + k, bx[1]);
-    atomicAdd(a.bz + k, bx[2]);
-    atomicAdd(a.bh + k, bh);
+    addPos(a, k, bx[0], bx[1], bx[2]);
+    atomicAdd(slot<kBh>(a, k), bh);
 }
 
 // p = (gamma-1) rho u, c = sqrt(gamma (gamma-1) u)
@@ -681,20 +782,27 @@ __global__ void eosAdjT(StdScatterArgs<T> a)
     const int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (k >= a.n) return;
     const double g1 = a.gamma - 1.0;
-    const double u = a.u[k], rho = double(a.rho[k]), c = double(a.c[k]), bp = double(a.bP[k]);
-    a.bRho[k] += T(bp * g1 * u);
-    a.bu[k] = T(bp * g1 * rho + (c > 0.0 ? double(a.bC[k]) * a.gamma * g1 / (2.0 * c) : 0.0));
+    const double u = a.u[k], rho = double(a.rho[k]), c = double(a.c[k]), bp = double(*slot<kBP>(a, k));
+    a.rhoB[k] = *slot<kBRho>(a, k) + T(bp * g1 * u);
+    a.bu[k] = T(bp * g1 * rho + (c > 0.0 ? double(*slot<kBC>(a, k)) * a.gamma * g1 / (2.0 * c) : 0.0));
 }
 
 // the mixed form's FP32 gradients to the caller's FP64 arrays
-__global__ void gradsToDouble(int64_t n, const float* __restrict__ src, double* x, double* y, double* z, double* vx,
-                              double* vy, double* vz, double* h, double* u)
+__global__ void gradsToDouble(StdScatterArgs<float> a, double* x, double* y, double* z, double* vx, double* vy,
+                              double* vz, double* h, double* u)
 {
     const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-    if (i >= n) return;
-    double* dst[8] = {x, y, z, vx, vy, vz, h, u};
-#pragma unroll
-    for (int k = 0; k < 8; ++k) dst[k][i] = double(src[k * n + i]);
+    if (i >= a.n) return;
+    const float4 r = *reinterpret_cast<const float4*>(slot<kBx>(a, i));
+    const float4 v = *reinterpret_cast<const float4*>(slot<kBvx>(a, i));
+    x[i] = double(r.x);
+    y[i] = double(r.y);
+    z[i] = double(r.z);
+    vx[i] = double(v.x);
+    vy[i] = double(v.y);
+    vz[i] = double(v.z);
+    h[i] = double(v.w);
+    u[i] = double(a.bu[i]);
 }
 
 template<class T, bool Smooth>
@@ -703,7 +811,7 @@ __global__ void __launch_bounds__(kAdjBlock) densityAdjScatterT(StdScatterArgs<T
     const auto tab = kernelTab<Smooth>(a.wh);
     const int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (k >= a.n) return;
-    const T rhob = a.bRho[k];
+    const T rhob = a.rhoB[k];
     const T hInv = a.hInv[k];
     T bx[3] = {0, 0, 0}, bh = rhob * (T(-3) * a.rho[k] * hInv);
     const unsigned nc = a.lv.capped(k);
@@ -716,26 +824,10 @@ __global__ void __launch_bounds__(kAdjBlock) densityAdjScatterT(StdScatterArgs<T
         stdad::densityAdjTerm<T>(r, d, rinv, hInv, dw, a.m[j], T(a.K), rhob, rb, hIb);
         for (int t = 0; t < 3; ++t) bx[t] += rb[t];
         bh += hIb;
-        atomicAdd(a.bx + j, -rb[0]);
-        atomicAdd(a.by + j, -rb[1]);
-        atomicAdd(a.bz + j, -rb[2]);
+        addPos(a, j, -rb[0], -rb[1], -rb[2]);
     }
-    atomicAdd(a.bx + k, bx[0]);
-    atomicAdd(a.by + k, bx[1]);
-    atomicAdd(a.bz + k, bx[2]);
-    atomicAdd(a.bh + k, bh);
-}
-
-// seeds of particle k in the pair type: K times the acceleration seeds and -K/2 times the du seed;
-// false when they are all zero
-template<class T>
-__device__ __forceinline__ bool seedsOfT(const StdScatterArgs<T>& a, int64_t k, T gA[3], T& gE)
-{
-    gA[0] = a.sAx ? T(a.K * double(a.sAx[k])) : T(0);
-    gA[1] = a.sAy ? T(a.K * double(a.sAy[k])) : T(0);
-    gA[2] = a.sAz ? T(a.K * double(a.sAz[k])) : T(0);
-    gE = a.sDu ? T(-0.5 * a.K * a.sDu[k]) : T(0);
-    return gA[0] != T(0) || gA[1] != T(0) || gA[2] != T(0) || gE != T(0);
+    addPos(a, k, bx[0], bx[1], bx[2]);
+    atomicAdd(slot<kBh>(a, k), bh);
 }
 
 // the momentum-energy adjoint of the mixed form over owned lists: one evaluation per owned entry,
@@ -749,26 +841,25 @@ __global__ void __launch_bounds__(kAdjBlock) meAdjOnceT(StdScatterArgs<T> a, Own
     const auto tab = kernelTab<Smooth>(a.wh);
     const int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (k >= a.n) return;
-    T gA[3], gE;
-    const bool anyK = seedsOfT(a, k, gA, gE);
+    const MeIn<T> I = meInOf(a, k);
     T bx[3] = {0, 0, 0}, bv[3] = {0, 0, 0}, bh = 0, brho = 0, bp = 0, bc = 0, bC[6] = {0, 0, 0, 0, 0, 0};
-    const stdad::MeSide<T> S = stdSideT(a, k);
-    const T zero[3] = {T(0), T(0), T(0)};
     const unsigned cnt = ov.size(k);
     for (unsigned q = 0; q < cnt; ++q) {
         bool mutual;
         const uint32_t j = ov.at(k, q, mutual);
-        T gAj[3] = {T(0), T(0), T(0)}, gEj = T(0);
-        const bool anyJ = mutual && seedsOfT(a, j, gAj, gEj);
-        if (!anyK && !anyJ) continue;
-        const stdad::MeSide<T> J = stdSideT(a, j);
+        MeIn<T> J = meInOf(a, j);
+        if (!mutual) {
+            J.any = false;
+            J.gA[0] = J.gA[1] = J.gA[2] = J.gE = T(0);
+        }
+        if (!I.any && !J.any) continue;
         T r[3], d, rinv;
         geomT(a, k, j, r, d, rinv);
-        const T v[3] = {a.vx[k] - a.vx[j], a.vy[k] - a.vy[j], a.vz[k] - a.vz[j]};
+        const T v[3] = {I.v[0] - J.v[0], I.v[1] - J.v[1], I.v[2] - J.v[2]};
         T dwi, dwj;
-        const T wi = lookupSlopeT(tab, d * S.hInv, dwi), wj = lookupSlopeT(tab, d * J.hInv, dwj);
+        const T wi = lookupSlopeT(tab, d * I.s.hInv, dwi), wj = lookupSlopeT(tab, d * J.s.hInv, dwj);
         stdad::MeGrad<T> o;
-        stdad::meStdAdjPair<T>(r, d, rinv, v, S, J, wi, dwi, wj, dwj, anyK ? gA : zero, anyK ? gE : T(0), gAj, gEj, o);
+        stdad::meStdAdjPair<T>(r, d, rinv, v, I.s, J.s, wi, dwi, wj, dwj, I.gA, I.gE, J.gA, J.gE, o);
         for (int t = 0; t < 3; ++t) {
             bx[t] += o.r[t];
             bv[t] += o.v[t];
@@ -778,29 +869,9 @@ __global__ void __launch_bounds__(kAdjBlock) meAdjOnceT(StdScatterArgs<T> a, Own
         bp += o.pI;
         bc += o.c;
         for (int t = 0; t < 6; ++t) bC[t] += o.CI[t];
-        atomicAdd(a.bx + j, -o.r[0]);
-        atomicAdd(a.by + j, -o.r[1]);
-        atomicAdd(a.bz + j, -o.r[2]);
-        atomicAdd(a.bvx + j, -o.v[0]);
-        atomicAdd(a.bvy + j, -o.v[1]);
-        atomicAdd(a.bvz + j, -o.v[2]);
-        atomicAdd(a.bh + j, o.hJ);
-        atomicAdd(a.bRho + j, o.rhoJ);
-        atomicAdd(a.bP + j, o.pJ);
-        atomicAdd(a.bC + j, o.c);
-        for (int t = 0; t < 6; ++t) atomicAdd(a.bCij + t * a.n + j, o.CJ[t]);
+        addMe(a, j, -o.r[0], -o.r[1], -o.r[2], -o.v[0], -o.v[1], -o.v[2], o.hJ, o.rhoJ, o.pJ, o.c, o.CJ);
     }
-    atomicAdd(a.bx + k, bx[0]);
-    atomicAdd(a.by + k, bx[1]);
-    atomicAdd(a.bz + k, bx[2]);
-    atomicAdd(a.bvx + k, bv[0]);
-    atomicAdd(a.bvy + k, bv[1]);
-    atomicAdd(a.bvz + k, bv[2]);
-    atomicAdd(a.bh + k, bh);
-    atomicAdd(a.bRho + k, brho + (a.sRho ? a.sRho[k] : T(0)));
-    atomicAdd(a.bP + k, bp);
-    atomicAdd(a.bC + k, bc);
-    for (int t = 0; t < 6; ++t) atomicAdd(a.bCij + t * a.n + k, bC[t]);
+    addMe(a, k, bx[0], bx[1], bx[2], bv[0], bv[1], bv[2], bh, brho + (a.sRho ? a.sRho[k] : T(0)), bp, bc, bC);
 }
 
 // ---- one evaluation per owned entry of the owned lists (mutual pairs give both directed terms) ----
@@ -1079,9 +1150,10 @@ static int adjointStdScatter(sphgb_ctx* c, sphgb_particles* p, const sphgb_seeds
 {
     const int64_t n = p->n;
     constexpr bool fp32 = std::is_same_v<T, float>;
-    // state in T: rho, p, c adjoints, C adjoint (6), tau adjoint (6), quotients (5), and for the
-    // mixed form the 8 gradients before their conversion to FP64
-    SPHGB_TRY(c->adjState.ensure(sizeof(T) * (fp32 ? 28 : 20) * n));
+    // state in T: rho, p, c adjoints and C adjoint (9; the mixed form has its 16 accumulators and the 20
+    // words of its records instead), tau adjoint (6), quotients (5), the complete rho adjoint, and for
+    // the mixed form the u gradient before its conversion to FP64
+    SPHGB_TRY(c->adjState.ensure(sizeof(T) * (fp32 ? kSlots + 20 + 13 : 21) * n));
     T* st = c->adjState.as<T>();
     StdScatterArgs<T> a{};
     auto f = [](const void* q) { return static_cast<const T*>(q); };
@@ -1114,29 +1186,19 @@ static int adjointStdScatter(sphgb_ctx* c, sphgb_particles* p, const sphgb_seeds
         a.sAz = f(s->az);
         a.sDu = s->du;
     }
-    a.bRho = st;
-    a.bP = st + n;
-    a.bC = st + 2 * n;
-    a.bCij = st + 3 * n;
-    a.tauBar = st + 9 * n;
-    T* quot = st + 15 * n;
-    a.hInv = quot;
-    a.moR = quot + n;
-    a.poR = quot + 2 * n;
-    a.rhoInv = quot + 3 * n;
-    a.poR2 = quot + 4 * n;
     if constexpr (fp32) {
-        T* gr = st + 20 * n;
-        a.bx = gr;
-        a.by = gr + n;
-        a.bz = gr + 2 * n;
-        a.bvx = gr + 3 * n;
-        a.bvy = gr + 4 * n;
-        a.bvz = gr + 5 * n;
-        a.bh = gr + 6 * n;
-        a.bu = gr + 7 * n;
-        SPHGB_CUDA(cudaMemsetAsync(gr, 0, sizeof(T) * 8 * n, c->stream));
+        a.acc = st;  // 64-byte records first: they and the 80-byte ones stay aligned for any n
+        a.side = reinterpret_cast<float4*>(st + kSlots * n);
+        st += (kSlots + 20) * n;
+        a.bu = st + 12 * n;
+        SPHGB_CUDA(cudaMemsetAsync(a.acc, 0, sizeof(T) * kSlots * n, c->stream));
     } else {
+        a.bRho = st;
+        a.bP = st + n;
+        a.bC = st + 2 * n;
+        a.bCij = st + 3 * n;
+        SPHGB_CUDA(cudaMemsetAsync(st, 0, sizeof(T) * 9 * n, c->stream));
+        st += 9 * n;
         a.bx = g->x;
         a.by = g->y;
         a.bz = g->z;
@@ -1148,7 +1210,13 @@ static int adjointStdScatter(sphgb_ctx* c, sphgb_particles* p, const sphgb_seeds
         for (double* q : {g->x, g->y, g->z, g->vx, g->vy, g->vz, g->h})
             SPHGB_CUDA(cudaMemsetAsync(q, 0, sizeof(double) * n, c->stream));
     }
-    SPHGB_CUDA(cudaMemsetAsync(st, 0, sizeof(T) * 9 * n, c->stream));
+    a.tauBar = st;
+    a.hInv = st + 6 * n;
+    a.moR = st + 7 * n;
+    a.poR = st + 8 * n;
+    a.rhoInv = st + 9 * n;
+    a.poR2 = st + 10 * n;
+    a.rhoB = st + 11 * n;
     if (fp32 && !c->deterministic && (c->ownedEpoch != c->nbrEpoch || !c->ownedFromLists))
         SPHGB_TRY(buildOwnedFromLists(c));
     const unsigned blocks = gridFor(n, kAdjBlock), eb = gridFor(n, 256);
@@ -1173,7 +1241,7 @@ static int adjointStdScatter(sphgb_ctx* c, sphgb_particles* p, const sphgb_seeds
         return launched(c, "densityAdjScatterT");
     }));
     if constexpr (fp32) {
-        gradsToDouble<<<eb, 256, 0, c->stream>>>(n, st + 20 * n, g->x, g->y, g->z, g->vx, g->vy, g->vz, g->h, g->u);
+        gradsToDouble<<<eb, 256, 0, c->stream>>>(a, g->x, g->y, g->z, g->vx, g->vy, g->vz, g->h, g->u);
         SPHGB_TRY(launched(c, "gradsToDouble"));
     }
     SPHGB_CUDA(cudaStreamSynchronize(c->stream));
