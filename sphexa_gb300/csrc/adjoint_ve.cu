@@ -1368,6 +1368,20 @@ __global__ void __launch_bounds__(kVeAdjBlock) veXmassAdjOnceKernel(VeAdjArgs a,
 // number of n-sized double sections of the VE adjoint state
 constexpr int kVeAdjSections = 82;
 
+int anySeed(sphgb_ctx* c, const double* seed, int64_t n, bool& any)
+{
+    SPHGB_TRY(c->reduceScratch.ensure(sizeof(unsigned long long) * 4));
+    int* dev = c->reduceScratch.as<int>();
+    int got = 0;
+    SPHGB_CUDA(cudaMemsetAsync(dev, 0, sizeof(int), c->stream));
+    anySeedKernel<<<gridFor(n, 256), 256, 0, c->stream>>>(seed, n, dev);
+    SPHGB_TRY(launched(c, "anySeedKernel"));
+    SPHGB_CUDA(cudaMemcpyAsync(&got, dev, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    SPHGB_CUDA(cudaStreamSynchronize(c->stream));
+    any = got != 0;
+    return SPHGB_OK;
+}
+
 int adjointVe(sphgb_ctx* c, sphgb_particles* p, const double* alphaPrev, int avClean, const sphgb_seeds* s,
               sphgb_grads* g, int deterministic)
 {
@@ -1508,15 +1522,7 @@ int adjointVe(sphgb_ctx* c, sphgb_particles* p, const double* alphaPrev, int avC
     SPHGB_TRY(launched(c, "veQuotKernel"));
     bool withDu = a.sDu != nullptr;
     if (withDu) {  // a du seed that is zero everywhere (autograd's for an unused output) is none
-        SPHGB_TRY(c->reduceScratch.ensure(sizeof(unsigned long long) * 4));
-        int* any = c->reduceScratch.as<int>();
-        int got = 0;
-        SPHGB_CUDA(cudaMemsetAsync(any, 0, sizeof(int), c->stream));
-        anySeedKernel<<<eb, 256, 0, c->stream>>>(a.sDu, n, any);
-        SPHGB_TRY(launched(c, "anySeedKernel"));
-        SPHGB_CUDA(cudaMemcpyAsync(&got, any, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-        SPHGB_CUDA(cudaStreamSynchronize(c->stream));
-        withDu = got != 0;
+        SPHGB_TRY(anySeed(c, a.sDu, n, withDu));
         if (!withDu) a.sDu = nullptr;
     }
     // forward sums kept by the forward passes on these lists (sphgb_set_adjoint_tape) are read from

@@ -248,6 +248,7 @@ int sortStatusAsync(sphgb_ctx* c);
 int sortStatusAfterSync(sphgb_ctx* c);
 // exclusive prefix sum of n 32-bit counts (out may not alias in)
 int exclusiveScan(sphgb_ctx* c, const uint32_t* in, uint32_t* out, int64_t n);
+int anySeed(sphgb_ctx* c, const double* seed, int64_t n, bool& any);  // some seed value is not zero
 int adjointStd(sphgb_ctx* c, sphgb_particles* p, const sphgb_seeds* s, sphgb_grads* g, int deterministic);
 int adjointVe(sphgb_ctx* c, sphgb_particles* p, const double* alphaPrev, int avClean, const sphgb_seeds* s,
               sphgb_grads* g, int deterministic);

@@ -203,13 +203,14 @@ def test_sync_order_of_close_keys(gpu_ctx, n, spread):
 
 
 @pytest.mark.parametrize("precision, bar", [("fp64", 1e-11), ("mixed", 1e-5)])
+@pytest.mark.parametrize("du", [False, True])
 @pytest.mark.parametrize("side", [9, 40])
-def test_std_adjoint_over_owned_lists(side, precision, bar):
+def test_std_adjoint_over_owned_lists(side, du, precision, bar):
     """The std adjoint over owned lists (FP64: cut into 16 slices at 729 particles, 5 at 64,000; mixed:
     sums in 64-byte records, an odd count and a whole number of blocks) against the walk over the full
     lists.  Both add the same terms in different orders: about 150 terms a sum and four chained sums,
     each rounded to 1.1e-16 (6e-8) of the partial sum, so the bars leave a factor of a hundred (thirty)
-    for cancellation between terms."""
+    for cancellation between terms.  du: with and without a du seed (a kernel of its own each)."""
     import torch
     from sphexa_gb300 import autograd as AG, sph, workloads as W
     grads = {}
@@ -226,7 +227,10 @@ def test_std_adjoint_over_owned_lists(side, precision, bar):
             ctx.set_deterministic(True)
         base = [t.clone().requires_grad_(True) for t in sw.inputs()]
         out = AG.StdSweepFunction.apply(sw, *base)
-        AG.loss_rho_a(*[o.to(torch.float64) for o in out[:4]], rho_t).backward()
+        loss = AG.loss_rho_a(*[o.to(torch.float64) for o in out[:4]], rho_t)
+        if du:
+            loss = loss + (out[4].to(torch.float64) ** 2).sum()
+        loss.backward()
         grads[det] = [b.grad.detach().to(torch.float64) for b in base]
         ctx.close()
     for g1, g0 in zip(grads[False], grads[True]):
