@@ -111,8 +111,7 @@ struct sphgb_ctx {
     // |r|, w_ij and the kernel function at both ends of every owned entry, stored by the pair-once xmass
     // or density pass and read by the later pair-once passes (PairGeo in pairs.cuh); geoRows: per warp of
     // 32 targets its first row (from the owned-list build), and the row counter
-    // rho0Sum: the xmass pass's sum w m_j per particle, for gradh
-    sphgb::DBuf pairGeo, geoRows, rho0Sum;
+    sphgb::DBuf pairGeo, geoRows;
     size_t geoRowCount = 0;
     int geoArrays = 0;  // 5: with the difference and velocity-difference vectors, 2: without
     bool geoValid = false;

@@ -144,18 +144,16 @@ __global__ void __launch_bounds__(kPairBlock) xmassOnceKernel(ListView lv, Owned
     atomicAdd(acc + i, rho0);
 }
 
-// sums: where the pass keeps sum w m_j for gradh (within a sweep, with the geometry cache), or null;
 // snap: where it keeps the inputs of the cache (outside a sweep), or null
 template<bool StoreRho>
 __global__ void xmassOnceFinish(int64_t first, int64_t last, const double* h, const double* m, double K,
-                                const double* acc, double* out, double* sums, GeoInputs in, double* snap, int64_t n)
+                                const double* acc, double* out, GeoInputs in, double* snap, int64_t n)
 {
     const int64_t i = first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (i >= last) return;
     const double hi = h[i], mi = m[i];
     const double hInv = 1.0 / hi, h3Inv = hInv * hInv * hInv;
     const double xm = mi / ((mi + acc[i]) * K * h3Inv);
-    if (sums) sums[i] = acc[i];
     if (snap) {
 #pragma unroll
         for (int q = 0; q < kGeoInputs; ++q) snap[q * n + i] = in.f[q][i];
@@ -720,11 +718,7 @@ int launchXmass(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, v
         SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * size_t(n), c->stream));
         PairGeo geo{};
         SPHGB_TRY(pairGeoStore(c, p, &geo));
-        double *sums = nullptr, *snap = geo.g && !c->inSweep ? c->geoSnap.as<double>() : nullptr;
-        if (geo.g && c->inSweep) {
-            SPHGB_TRY(c->rho0Sum.ensure(sizeof(double) * size_t(n)));
-            sums = c->rho0Sum.as<double>();
-        }
+        double* snap = geo.g && !c->inSweep ? c->geoSnap.as<double>() : nullptr;
         SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
             constexpr bool S = decltype(smooth)::value;
             xmassOnceKernel<S><<<ownedGrid(n), kPairBlock, 0, c->stream>>>(
@@ -738,12 +732,12 @@ int launchXmass(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, v
         if (storeRho)
             xmassOnceFinish<true><<<eb, 256, 0, c->stream>>>(first, last, static_cast<const double*>(p->h),
                                                               static_cast<const double*>(p->m), c->K,
-                                                              c->pairAcc.as<double>(), static_cast<double*>(out), sums,
+                                                              c->pairAcc.as<double>(), static_cast<double*>(out),
                                                               geoInputs(p), snap, n);
         else
             xmassOnceFinish<false><<<eb, 256, 0, c->stream>>>(first, last, static_cast<const double*>(p->h),
                                                                static_cast<const double*>(p->m), c->K,
-                                                               c->pairAcc.as<double>(), static_cast<double*>(out), sums,
+                                                               c->pairAcc.as<double>(), static_cast<double*>(out),
                                                                geoInputs(p), snap, n);
         return launched(c, "xmassOnceFinish");
     }

@@ -871,15 +871,15 @@ __global__ void __launch_bounds__(kPairBlock) meVeKernel(ListView lv, CoordFp64 
 
 // FP64 gradh with one evaluation per mutual pair over the owned lists.  With x = v / dx (table units)
 // and D = x dW, the reference's dterh = -(3 w + v dW) (veDefGradhJLoop, ve_def_gradh_kern.hpp:64-78)
-// is -(3 w + dx D), so its sums follow from sum w xm_j (which kx needs), sum D xm_j, and either sum w m_j
-// of the xmass pass and sum D m_j (Sums: within a sweep, where that sum is of the same geometry and
-// masses), or sum (3 w / dx + D) m_j.  A mutual pair also gives j its terms at v_j = d / h_j with xm_i and m_i, by
+// is -dx (3 w / dx + D); a mutual pair also gives j its terms at v_j = d / h_j with xm_i and m_i, by
 // FP64 atomics.  The self terms and the epilogue (ve_def_gradh_kern.hpp:60-62, 80-88) run in the
-// finishing kernels.  FP64-pipe bound: 12 instructions per mutual pair with the cache (18 with v and
-// dterh per pair, 14.7 ms at 8M; now 11.3 ms).
+// finishing kernels.  The two parts of dterh are added per pair: their sums cancel to a few per cent, so
+// summed apart they cost ten times the rounding (1e-13 of the acceleration where gradh is 2e-3).
+// FP64-pipe bound: 14 instructions per mutual pair with the cache (18 with v and an unfused dterh:
+// 14.7 ms at 8M, now 10.9 ms).
 constexpr double kTabDx = 1.0 / kTabInvDx;
 
-template<bool Smooth, bool Geo, bool Sums>
+template<bool Smooth, bool Geo>
 __device__ __forceinline__ void gradhOnceBody(ListView lv, OwnedView ov, CoordFp64 cf,
                                                                const double* h, const double* m, const double* xm,
                                                                KTab<Smooth> tw, KTab<Smooth> tdw,
@@ -920,19 +920,19 @@ __device__ __forceinline__ void gradhOnceBody(ListView lv, OwnedView ov, CoordFp
         {
             const double x = dist * hiInvDx;
             const TabSlot sl = tabSlot(x);
-            const double w = Geo ? wv.x : lookupX(tw, sl), D = x * lookupX(tdw, sl);
+            const double w = Geo ? wv.x : lookupX(tw, sl), E = fma(3.0 * kTabInvDx, w, x * lookupX(tdw, sl));
             const double xmj = __ldg(xm + j);
             kx = fma(w, xmj, kx);
-            dxm = fma(D, xmj, dxm);
-            dm = fma(Sums ? D : fma(3.0 * kTabInvDx, w, D), __ldg(m + j), dm);
+            dxm = fma(E, xmj, dxm);
+            dm = fma(E, __ldg(m + j), dm);
         }
         if (mutual) {
             const double x = dist * __ldg(hInvDx + j);
             const TabSlot sl = tabSlot(x);
-            const double w = Geo ? wv.y : lookupX(tw, sl), D = x * lookupX(tdw, sl);
+            const double w = Geo ? wv.y : lookupX(tw, sl), E = fma(3.0 * kTabInvDx, w, x * lookupX(tdw, sl));
             atomicAdd(acc + j, w * xmi);
-            atomicAdd(acc + n + j, D * xmi);
-            atomicAdd(acc + 2 * n + j, (Sums ? D : fma(3.0 * kTabInvDx, w, D)) * mi);
+            atomicAdd(acc + n + j, E * xmi);
+            atomicAdd(acc + 2 * n + j, E * mi);
         }
     }
     atomicAdd(acc + i, kx);
@@ -940,30 +940,28 @@ __device__ __forceinline__ void gradhOnceBody(ListView lv, OwnedView ov, CoordFp
     atomicAdd(acc + 2 * n + i, dm);
 }
 
-// Geo: 1 the sweep's cache and xmass sums, 2 the cache subject to geo.stale, 0 neither
+// Geo: 1 the sweep's cache, 2 the cache subject to geo.stale, 0 neither
 template<bool Smooth, int Geo>
 __global__ void __launch_bounds__(kPairBlock) gradhOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf, const double* h,
                                                               const double* m, const double* xm, KTab<Smooth> tw,
                                                               KTab<Smooth> tdw, const double* hInv64, int64_t n,
                                                               double* acc, PairGeo geo)
 {
-    if constexpr (Geo == 1) gradhOnceBody<Smooth, true, true>(lv, ov, cf, h, m, xm, tw, tdw, hInv64, n, acc, geo);
+    if constexpr (Geo == 1) gradhOnceBody<Smooth, true>(lv, ov, cf, h, m, xm, tw, tdw, hInv64, n, acc, geo);
     else if (Geo == 2 && *geo.stale == 0)
-        gradhOnceBody<Smooth, true, false>(lv, ov, cf, h, m, xm, tw, tdw, hInv64, n, acc, geo);
-    else gradhOnceBody<Smooth, false, false>(lv, ov, cf, h, m, xm, tw, tdw, hInv64, n, acc, geo);
+        gradhOnceBody<Smooth, true>(lv, ov, cf, h, m, xm, tw, tdw, hInv64, n, acc, geo);
+    else gradhOnceBody<Smooth, false>(lv, ov, cf, h, m, xm, tw, tdw, hInv64, n, acc, geo);
 }
 
-// kx and gradh of particle i from the sums of gradhOnceKernel (sums: the xmass pass's sum w m_j, or
-// null where that is part of the third sum)
+// kx and gradh of particle i from the sums of gradhOnceKernel
 __device__ __forceinline__ void gradhEpilogue(int64_t i, int64_t n, double hi, double mi, double xmi, double K,
-                                              const double* acc, const double* sums, double* tapeWom, double* tapeWr0,
-                                              double& kxi, double& gradhi)
+                                              const double* acc, double* tapeWom, double* tapeWr0, double& kxi,
+                                              double& gradhi)
 {
     const double hInv = 1.0 / hi, h3Inv = hInv * hInv * hInv;
-    const double sx = acc[i], sm = sums ? sums[i] : 0.0;
-    kxi = (xmi + sx) * (K * h3Inv);
-    double whomega = fma(-kTabDx, acc[n + i], -3.0 * (xmi + sx)) * (K * h3Inv * hInv);
-    const double wrho0 = fma(-kTabDx, acc[2 * n + i], -3.0 * (mi + sm)) * (K * h3Inv * hInv);
+    kxi = (xmi + acc[i]) * (K * h3Inv);
+    double whomega = fma(-kTabDx, acc[n + i], -3.0 * xmi) * (K * h3Inv * hInv);
+    const double wrho0 = fma(-kTabDx, acc[2 * n + i], -3.0 * mi) * (K * h3Inv * hInv);
     if (tapeWom) {
         tapeWom[i] = whomega;
         tapeWr0[i] = wrho0;
@@ -975,20 +973,20 @@ __device__ __forceinline__ void gradhEpilogue(int64_t i, int64_t n, double hi, d
 }
 
 __global__ void gradhOnceFinish(int64_t first, int64_t last, int64_t n, const double* h, const double* m,
-                                const double* xm, double K, const double* acc, const double* sums, double* kxOut,
+                                const double* xm, double K, const double* acc, double* kxOut,
                                 double* gradhOut, double* tapeWom, double* tapeWr0)
 {
     const int64_t i = first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (i >= last) return;
     double kxi, gradhi;
-    gradhEpilogue(i, n, h[i], m[i], xm[i], K, acc, sums, tapeWom, tapeWr0, kxi, gradhi);
+    gradhEpilogue(i, n, h[i], m[i], xm[i], K, acc, tapeWom, tapeWr0, kxi, gradhi);
     kxOut[i] = kxi;
     gradhOut[i] = gradhi;
 }
 
 // the same epilogue fused with the EOS and the quotients of the later passes (inside a sweep)
 __global__ void gradhEosFinish(int64_t n, const double* h, const double* m, const double* xm, double K,
-                               const double* acc, const double* sums, double* kxOut, double* gradhOut, const double* u,
+                               const double* acc, double* kxOut, double* gradhOut, const double* u,
                                double gamma, void* prho, void* c, void* rho, void* p, double* aux, double* tapeWom,
                                double* tapeWr0)
 {
@@ -996,7 +994,7 @@ __global__ void gradhEosFinish(int64_t n, const double* h, const double* m, cons
     if (i >= n) return;
     const double mi = m[i], xmi = xm[i];
     double kxi, gradhi;
-    gradhEpilogue(i, n, h[i], mi, xmi, K, acc, sums, tapeWom, tapeWr0, kxi, gradhi);
+    gradhEpilogue(i, n, h[i], mi, xmi, K, acc, tapeWom, tapeWr0, kxi, gradhi);
     kxOut[i] = kxi;
     gradhOut[i] = gradhi;
     const double prhoi = eosVe<double>(i, u[i], mi, kxi, xmi, gradhi, gamma, prho, c, rho, p);
@@ -1524,7 +1522,6 @@ int passGradh(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last)
         SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * 3 * size_t(n)));
         SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * 3 * size_t(n), c->stream));
         const PairGeo geo = pairGeoRead(c);
-        const double* sums = geo.g && !geo.stale ? c->rho0Sum.as<double>() : nullptr;
         SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
             constexpr bool S = decltype(smooth)::value;
             auto run = [&](auto kernel) {
@@ -1542,14 +1539,14 @@ int passGradh(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last)
             SPHGB_TRY(c->aux.ensure(sizeof(double) * 6 * n));
             gradhEosFinish<<<gridFor(n, 256), 256, 0, c->stream>>>(
                 n, static_cast<const double*>(p->h), static_cast<const double*>(p->m), static_cast<const double*>(p->xm),
-                c->K, c->pairAcc.as<double>(), sums, static_cast<double*>(p->kx), static_cast<double*>(p->gradh), p->u,
+                c->K, c->pairAcc.as<double>(), static_cast<double*>(p->kx), static_cast<double*>(p->gradh), p->u,
                 c->prm.gamma, p->prho, p->c, p->rho, p->p, c->aux.as<double>(), tWom, tWr0);
             c->eosFused = c->auxReady = true;
             return launched(c, "gradhEosFinish");
         }
         gradhOnceFinish<<<gridFor(last - first, 256), 256, 0, c->stream>>>(
             first, last, n, static_cast<const double*>(p->h), static_cast<const double*>(p->m),
-            static_cast<const double*>(p->xm), c->K, c->pairAcc.as<double>(), sums, static_cast<double*>(p->kx),
+            static_cast<const double*>(p->xm), c->K, c->pairAcc.as<double>(), static_cast<double*>(p->kx),
             static_cast<double*>(p->gradh), tWom, tWr0);
         return launched(c, "gradhOnceFinish");
     }

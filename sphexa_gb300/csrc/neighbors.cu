@@ -1035,7 +1035,7 @@ int pairGeoStore(sphgb_ctx* c, const sphgb_particles* p, PairGeo* out)
             return SPHGB_OK;
         }
     }
-    // five arrays (|r| and 1/|r|, the two kernel values, r and dv) or the first two, whichever fits
+    // five arrays (|r| and w_ij, the two kernel values, r and dv) or the first two, whichever fits
     // in the buffer already held or in half of the free device memory
     int arrays = 0;
     for (int a : {5, 2}) {
