@@ -44,7 +44,7 @@ STD_FLOPS_PER_PAIR = {"density": 20.2, "iad": 37.6, "me": 117.3}
 # dram__bytes_write.sum, profiles/*_sedov100_jit_1M.md); traffic grows with the particle count.
 # The pair-once kernels of the default FP64 mode inside a sweep: most of it is the stream of the
 # sweep's pair-geometry cache (80 bytes per owned entry), read instead of recomputed.
-NCU_DRAM_BYTES_PER_PARTICLE = {"me": 4808.1, "iad_divv": 4823.9, "av": 4581.1}
+NCU_DRAM_BYTES_PER_PARTICLE = {"me": 4506.1, "iad_divv": 4570.1, "av": 3498.8}
 STAGES_VE = ["sync", "neighbors", "xmass", "gradh", "eos", "iad_divv", "av", "me"]
 STAGES_STD = ["sync", "neighbors", "density", "eos", "iad", "me", "-", "-"]
 # FP32 distance test of one search candidate against the target's radius: 3 coordinate differences,

@@ -876,7 +876,7 @@ __global__ void __launch_bounds__(kPairBlock) meVeKernel(ListView lv, CoordFp64 
 // finishing kernels.  The two parts of dterh are added per pair: their sums cancel to a few per cent, so
 // summed apart they cost ten times the rounding (1e-13 of the acceleration where gradh is 2e-3).
 // FP64-pipe bound: 14 instructions per mutual pair with the cache (18 with v and an unfused dterh:
-// 14.7 ms at 8M, now 10.9 ms).
+// 14.7 ms at 8M, now 12 ms).
 constexpr double kTabDx = 1.0 / kTabInvDx;
 
 template<bool Smooth, bool Geo>
