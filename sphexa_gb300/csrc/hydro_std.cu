@@ -97,12 +97,14 @@ __global__ void __launch_bounds__(kPairBlock) xmassKernel(ListView lv, CoordFp64
 
 // FP64 xmass / density with one evaluation per mutual pair over the owned lists: i adds
 // W(d / h_i) m_j, and for a mutual pair j receives W(d / h_j) m_i by an FP64 atomic.  Inside a
-// sweep it also fills the pair-geometry cache (geo) the later pair-once passes read.
-template<bool Smooth>
+// sweep it also fills the pair-geometry cache (geo) the later pair-once passes read.  Exact: acc + n holds
+// the rounding errors of the sums (exactSums).
+template<bool Smooth, bool Exact>
 __global__ void __launch_bounds__(kPairBlock) xmassOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf,
                                                                const double* h, const double* m, KTab<Smooth> tab,
                                                                const double* hInvDx, double* acc, PairGeo geo,
-                                                               const double* vx, const double* vy, const double* vz)
+                                                               const double* vx, const double* vy, const double* vz,
+                                                               int64_t n)
 {
     const int64_t i = lv.first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (i >= lv.last) return;
@@ -136,24 +138,25 @@ __global__ void __launch_bounds__(kPairBlock) xmassOnceKernel(ListView lv, Owned
                 geo.x[geo.plane + e] = make_double2(rz, dvx);
                 geo.x[2 * geo.plane + e] = make_double2(dvy, dvz);
             }
-            if (mutual) atomicAdd(acc + j, wj * mi);
+            if (mutual) sumAdd<Exact>(acc + j, acc + n + j, wj * mi);
         } else if (mutual) {
-            atomicAdd(acc + j, lookupX(tab, dist * __ldg(hInvDx + j)) * mi);
+            sumAdd<Exact>(acc + j, acc + n + j, lookupX(tab, dist * __ldg(hInvDx + j)) * mi);
         }
     }
-    atomicAdd(acc + i, rho0);
+    sumAdd<Exact>(acc + i, acc + n + i, rho0);
 }
 
 // snap: where it keeps the inputs of the cache (outside a sweep), or null
 template<bool StoreRho>
 __global__ void xmassOnceFinish(int64_t first, int64_t last, const double* h, const double* m, double K,
-                                const double* acc, double* out, GeoInputs in, double* snap, int64_t n)
+                                const double* acc, const double* lo, double* out, GeoInputs in, double* snap,
+                                int64_t n)
 {
     const int64_t i = first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (i >= last) return;
     const double hi = h[i], mi = m[i];
     const double hInv = 1.0 / hi, h3Inv = hInv * hInv * hInv;
-    const double xm = mi / ((mi + acc[i]) * K * h3Inv);
+    const double xm = mi / ((mi + (lo ? acc[i] + lo[i] : acc[i])) * K * h3Inv);
     if (snap) {
 #pragma unroll
         for (int q = 0; q < kGeoInputs; ++q) snap[q * n + i] = in.f[q][i];
@@ -714,30 +717,36 @@ int launchXmass(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, v
     unsigned blocks = gridFor(last - first, kPairBlock);
     if (std::is_same_v<P, Fp64Tag> && pairOnce(c, p, first, last)) {
         const int64_t n = p->n;
-        SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * size_t(n)));
-        SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * size_t(n), c->stream));
+        const bool exact = exactSums(n);
+        SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * (exact ? 2 : 1) * size_t(n)));
+        SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * (exact ? 2 : 1) * size_t(n), c->stream));
+        const double* lo = exact ? c->pairAcc.as<double>() + n : nullptr;
         PairGeo geo{};
         SPHGB_TRY(pairGeoStore(c, p, &geo));
         double* snap = geo.g && !c->inSweep ? c->geoSnap.as<double>() : nullptr;
         SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
             constexpr bool S = decltype(smooth)::value;
-            xmassOnceKernel<S><<<ownedGrid(n), kPairBlock, 0, c->stream>>>(
+            auto run = [&](auto kernel) {
+                kernel<<<ownedGrid(n), kPairBlock, 0, c->stream>>>(
                 lv, ownedView(c), cf, static_cast<const double*>(p->h), static_cast<const double*>(p->m),
                 KTab<S>{tabW64(c)}, c->hInv64.as<double>() + 2 * n, c->pairAcc.as<double>(), geo,
                 static_cast<const double*>(p->vx), static_cast<const double*>(p->vy),
-                static_cast<const double*>(p->vz));
+                static_cast<const double*>(p->vz), n);
+            };
+            if (exact) run(xmassOnceKernel<S, true>);
+            else run(xmassOnceKernel<S, false>);
             return launched(c, "xmassOnceKernel");
         }));
         const unsigned eb = gridFor(last - first, 256);
         if (storeRho)
             xmassOnceFinish<true><<<eb, 256, 0, c->stream>>>(first, last, static_cast<const double*>(p->h),
                                                               static_cast<const double*>(p->m), c->K,
-                                                              c->pairAcc.as<double>(), static_cast<double*>(out),
+                                                              c->pairAcc.as<double>(), lo, static_cast<double*>(out),
                                                               geoInputs(p), snap, n);
         else
             xmassOnceFinish<false><<<eb, 256, 0, c->stream>>>(first, last, static_cast<const double*>(p->h),
                                                                static_cast<const double*>(p->m), c->K,
-                                                               c->pairAcc.as<double>(), static_cast<double*>(out),
+                                                               c->pairAcc.as<double>(), lo, static_cast<double*>(out),
                                                                geoInputs(p), snap, n);
         return launched(c, "xmassOnceFinish");
     }

@@ -879,7 +879,7 @@ __global__ void __launch_bounds__(kPairBlock) meVeKernel(ListView lv, CoordFp64 
 // 14.7 ms at 8M, now 12 ms).
 constexpr double kTabDx = 1.0 / kTabInvDx;
 
-template<bool Smooth, bool Geo>
+template<bool Smooth, bool Geo, bool Exact>
 __device__ __forceinline__ void gradhOnceBody(ListView lv, OwnedView ov, CoordFp64 cf,
                                                                const double* h, const double* m, const double* xm,
                                                                KTab<Smooth> tw, KTab<Smooth> tdw,
@@ -930,38 +930,42 @@ __device__ __forceinline__ void gradhOnceBody(ListView lv, OwnedView ov, CoordFp
             const double x = dist * __ldg(hInvDx + j);
             const TabSlot sl = tabSlot(x);
             const double w = Geo ? wv.y : lookupX(tw, sl), E = fma(3.0 * kTabInvDx, w, x * lookupX(tdw, sl));
-            atomicAdd(acc + j, w * xmi);
-            atomicAdd(acc + n + j, E * xmi);
-            atomicAdd(acc + 2 * n + j, E * mi);
+            sumAdd<Exact>(acc + j, acc + 3 * n + j, w * xmi);
+            sumAdd<Exact>(acc + n + j, acc + 4 * n + j, E * xmi);
+            sumAdd<Exact>(acc + 2 * n + j, acc + 5 * n + j, E * mi);
         }
     }
-    atomicAdd(acc + i, kx);
-    atomicAdd(acc + n + i, dxm);
-    atomicAdd(acc + 2 * n + i, dm);
+    sumAdd<Exact>(acc + i, acc + 3 * n + i, kx);
+    sumAdd<Exact>(acc + n + i, acc + 4 * n + i, dxm);
+    sumAdd<Exact>(acc + 2 * n + i, acc + 5 * n + i, dm);
 }
 
-// Geo: 1 the sweep's cache, 2 the cache subject to geo.stale, 0 neither
-template<bool Smooth, int Geo>
+// Geo: 1 the sweep's cache, 2 the cache subject to geo.stale, 0 neither; Exact: acc + 3 n .. holds the
+// rounding errors of the three sums (exactSums)
+template<bool Smooth, int Geo, bool Exact>
 __global__ void __launch_bounds__(kPairBlock) gradhOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf, const double* h,
                                                               const double* m, const double* xm, KTab<Smooth> tw,
                                                               KTab<Smooth> tdw, const double* hInv64, int64_t n,
                                                               double* acc, PairGeo geo)
 {
-    if constexpr (Geo == 1) gradhOnceBody<Smooth, true>(lv, ov, cf, h, m, xm, tw, tdw, hInv64, n, acc, geo);
+    if constexpr (Geo == 1) gradhOnceBody<Smooth, true, Exact>(lv, ov, cf, h, m, xm, tw, tdw, hInv64, n, acc, geo);
     else if (Geo == 2 && *geo.stale == 0)
-        gradhOnceBody<Smooth, true>(lv, ov, cf, h, m, xm, tw, tdw, hInv64, n, acc, geo);
-    else gradhOnceBody<Smooth, false>(lv, ov, cf, h, m, xm, tw, tdw, hInv64, n, acc, geo);
+        gradhOnceBody<Smooth, true, Exact>(lv, ov, cf, h, m, xm, tw, tdw, hInv64, n, acc, geo);
+    else gradhOnceBody<Smooth, false, Exact>(lv, ov, cf, h, m, xm, tw, tdw, hInv64, n, acc, geo);
 }
 
 // kx and gradh of particle i from the sums of gradhOnceKernel
 __device__ __forceinline__ void gradhEpilogue(int64_t i, int64_t n, double hi, double mi, double xmi, double K,
-                                              const double* acc, double* tapeWom, double* tapeWr0, double& kxi,
-                                              double& gradhi)
+                                              const double* acc, bool exact, double* tapeWom, double* tapeWr0,
+                                              double& kxi, double& gradhi)
 {
     const double hInv = 1.0 / hi, h3Inv = hInv * hInv * hInv;
-    kxi = (xmi + acc[i]) * (K * h3Inv);
-    double whomega = fma(-kTabDx, acc[n + i], -3.0 * xmi) * (K * h3Inv * hInv);
-    const double wrho0 = fma(-kTabDx, acc[2 * n + i], -3.0 * mi) * (K * h3Inv * hInv);
+    double s[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) s[q] = exact ? acc[q * n + i] + acc[(3 + q) * n + i] : acc[q * n + i];
+    kxi = (xmi + s[0]) * (K * h3Inv);
+    double whomega = fma(-kTabDx, s[1], -3.0 * xmi) * (K * h3Inv * hInv);
+    const double wrho0 = fma(-kTabDx, s[2], -3.0 * mi) * (K * h3Inv * hInv);
     if (tapeWom) {
         tapeWom[i] = whomega;
         tapeWr0[i] = wrho0;
@@ -973,20 +977,20 @@ __device__ __forceinline__ void gradhEpilogue(int64_t i, int64_t n, double hi, d
 }
 
 __global__ void gradhOnceFinish(int64_t first, int64_t last, int64_t n, const double* h, const double* m,
-                                const double* xm, double K, const double* acc, double* kxOut,
+                                const double* xm, double K, const double* acc, bool exact, double* kxOut,
                                 double* gradhOut, double* tapeWom, double* tapeWr0)
 {
     const int64_t i = first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (i >= last) return;
     double kxi, gradhi;
-    gradhEpilogue(i, n, h[i], m[i], xm[i], K, acc, tapeWom, tapeWr0, kxi, gradhi);
+    gradhEpilogue(i, n, h[i], m[i], xm[i], K, acc, exact, tapeWom, tapeWr0, kxi, gradhi);
     kxOut[i] = kxi;
     gradhOut[i] = gradhi;
 }
 
 // the same epilogue fused with the EOS and the quotients of the later passes (inside a sweep)
 __global__ void gradhEosFinish(int64_t n, const double* h, const double* m, const double* xm, double K,
-                               const double* acc, double* kxOut, double* gradhOut, const double* u,
+                               const double* acc, bool exact, double* kxOut, double* gradhOut, const double* u,
                                double gamma, void* prho, void* c, void* rho, void* p, double* aux, double* tapeWom,
                                double* tapeWr0)
 {
@@ -994,7 +998,7 @@ __global__ void gradhEosFinish(int64_t n, const double* h, const double* m, cons
     if (i >= n) return;
     const double mi = m[i], xmi = xm[i];
     double kxi, gradhi;
-    gradhEpilogue(i, n, h[i], mi, xmi, K, acc, tapeWom, tapeWr0, kxi, gradhi);
+    gradhEpilogue(i, n, h[i], mi, xmi, K, acc, exact, tapeWom, tapeWr0, kxi, gradhi);
     kxOut[i] = kxi;
     gradhOut[i] = gradhi;
     const double prhoi = eosVe<double>(i, u[i], mi, kxi, xmi, gradhi, gamma, prho, c, rho, p);
@@ -1519,8 +1523,9 @@ int passGradh(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last)
     double* tWr0 = tape ? tape + int64_t(kTapeWr0) * p->n : nullptr;
     if (pairOnce(c, p, first, last)) {
         const int64_t n = p->n;
-        SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * 3 * size_t(n)));
-        SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * 3 * size_t(n), c->stream));
+        const bool exact = exactSums(n);
+        SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * (exact ? 6 : 3) * size_t(n)));
+        SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * (exact ? 6 : 3) * size_t(n), c->stream));
         const PairGeo geo = pairGeoRead(c);
         SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
             constexpr bool S = decltype(smooth)::value;
@@ -1530,23 +1535,28 @@ int passGradh(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last)
                     static_cast<const double*>(p->m), static_cast<const double*>(p->xm), KTab<S>{tabW64(c)},
                     KTab<S>{tabDW64(c)}, c->hInv64.as<double>(), n, c->pairAcc.as<double>(), geo);
             };
-            if (geo.stale) run(gradhOnceKernel<S, 2>);
-            else if (geo.g) run(gradhOnceKernel<S, 1>);
-            else run(gradhOnceKernel<S, 0>);
+            auto pick = [&](auto e) {
+                constexpr bool X = decltype(e)::value;
+                if (geo.stale) run(gradhOnceKernel<S, 2, X>);
+                else if (geo.g) run(gradhOnceKernel<S, 1, X>);
+                else run(gradhOnceKernel<S, 0, X>);
+            };
+            if (exact) pick(std::true_type{});
+            else pick(std::false_type{});
             return launched(c, "gradhOnceKernel");
         }));
         if (c->inSweep && p->u && p->prho && p->c) {  // EOS and quotients fused into the epilogue
             SPHGB_TRY(c->aux.ensure(sizeof(double) * 6 * n));
             gradhEosFinish<<<gridFor(n, 256), 256, 0, c->stream>>>(
                 n, static_cast<const double*>(p->h), static_cast<const double*>(p->m), static_cast<const double*>(p->xm),
-                c->K, c->pairAcc.as<double>(), static_cast<double*>(p->kx), static_cast<double*>(p->gradh), p->u,
+                c->K, c->pairAcc.as<double>(), exact, static_cast<double*>(p->kx), static_cast<double*>(p->gradh), p->u,
                 c->prm.gamma, p->prho, p->c, p->rho, p->p, c->aux.as<double>(), tWom, tWr0);
             c->eosFused = c->auxReady = true;
             return launched(c, "gradhEosFinish");
         }
         gradhOnceFinish<<<gridFor(last - first, 256), 256, 0, c->stream>>>(
             first, last, n, static_cast<const double*>(p->h), static_cast<const double*>(p->m),
-            static_cast<const double*>(p->xm), c->K, c->pairAcc.as<double>(), static_cast<double*>(p->kx),
+            static_cast<const double*>(p->xm), c->K, c->pairAcc.as<double>(), exact, static_cast<double*>(p->kx),
             static_cast<double*>(p->gradh), tWom, tWr0);
         return launched(c, "gradhOnceFinish");
     }

@@ -126,6 +126,32 @@ inline dim3 ownedGrid(int64_t n)
     return dim3(unsigned((n + kPairBlock - 1) / kPairBlock), unsigned(s < 1 ? 1 : s > 16 ? 16 : s));
 }
 
+// Sets in the most slices keep the rounding errors of the density-like sums (xmass, gradh) as well: their
+// atomics arrive in another order in every run, and where gradh is near 0 (2e-3 in an open set of 3000
+// particles) plain sums let the acceleration differ by 1e-13 from run to run.  Larger sets, where each
+// sum would pay for it on the FP64 pipe, do without.
+inline bool exactSums(int64_t n)
+{
+    return ownedGrid(n).y >= 16;
+}
+
+// *hi += v with the rounding error of that addition (two-sum) added to *lo: hi + lo is the sum of all
+// v to twice the precision, whatever their order
+__device__ __forceinline__ void atomicAddExact(double* hi, double* lo, double v)
+{
+    const double old = atomicAdd(hi, v);
+    const double s = __dadd_rn(old, v), b = __dsub_rn(s, old);
+    const double e = __dadd_rn(__dsub_rn(old, __dsub_rn(s, b)), __dsub_rn(v, b));
+    if (e != 0.0 && isfinite(e)) atomicAdd(lo, e);  // an infinite sum has no error to keep
+}
+
+template<bool Exact>
+__device__ __forceinline__ void sumAdd(double* hi, double* lo, double v)
+{
+    if constexpr (Exact) atomicAddExact(hi, lo, v);
+    else atomicAdd(hi, v);
+}
+
 inline OwnedView ownedView(const sphgb_ctx* c)
 {
     return OwnedView{c->owned.as<uint32_t>(), c->ownedCount.as<uint32_t>(), c->nbrStride};

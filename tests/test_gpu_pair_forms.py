@@ -235,3 +235,16 @@ def test_std_adjoint_over_owned_lists(side, du, precision, bar):
         ctx.close()
     for g1, g0 in zip(grads[False], grads[True]):
         assert float((g1 - g0).norm() / g0.norm()) <= bar
+
+
+@pytest.mark.parametrize("n", [3000, 19456])
+def test_small_set_densities_do_not_depend_on_the_order_of_atomics(gpu_ctx, n):
+    """Sets in the most slices (up to 19,456 particles) keep the rounding errors of the xmass and gradh
+    sums: hi + lo carries each sum to about 1e-32 of it in any order, so two sweeps round to the same
+    bits."""
+    from sphexa_gb300 import workloads as W
+    wl = W.random_cube(n, seed=61, periodic=False)
+    gpu_ctx.set_deterministic(False)
+    a, b = run_gpu(gpu_ctx, wl, "ve", False), run_gpu(gpu_ctx, wl, "ve", False)
+    for f in ("xm", "kx", "gradh"):
+        assert np.array_equal(a[f], b[f]), f
