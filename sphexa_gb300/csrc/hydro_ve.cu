@@ -1293,17 +1293,34 @@ __device__ __forceinline__ double expNegSmall(double x, const double4* __restric
     return en.x * fma(e.x, y, e.x);
 }
 
-// avRvCorrection (hydro_ve/momentum_energy_kern.hpp:43-63) over |r|, without d3: with d1 and d2 the
-// velocity gradients' quadratic forms at both ends and A = d1 / d2, the limiter 4 A / (1 + A)^2 lies in
-// [0, 1] for A >= 0 and is cut to 0 below, so that -phi (d1 + d2) = -d3 2 d1 d2 / (d1 + d2) where d1 and
-// d2 have one sign, else 0: one quotient instead of two divisions, shared by the two ends.
-__device__ __forceinline__ double avRvShared(double d1, double d2, double dist)
+// avRvCorrection (hydro_ve/momentum_energy_kern.hpp:43-63) over |r| without d3, as the reference writes it;
+// each end has its own A.  For gradients that avRvShared leaves open.
+static __device__ __noinline__ double2 avRvWide(double d1, double d2, double dist)
 {
-    const long long b1 = __double_as_longlong(d1), b2 = __double_as_longlong(d2);
-    constexpr long long inf = 0x7ff0000000000000LL, mag = 0x7fffffffffffffffLL;
-    const bool finite = (b1 & mag) < inf && (b2 & mag) < inf;
-    if (finite && ((b1 ^ b2) < 0 || (b1 & mag) == 0 || (b2 & mag) == 0)) return 0.0;
-    return 2.0 * d1 * quotient(d2, (d1 + d2) * dist);
+    auto share = [&](double a, double b) {
+        const double A = b != 0.0 ? a / b : 0.0, Ap1 = 1.0 + A;
+        return 0.5 * fmax(0.0, fmin(1.0, 4.0 * A / (Ap1 * Ap1))) * (d1 + d2) / dist;
+    };
+    return make_double2(share(d1, d2), share(d2, d1));
+}
+
+// the same for the owner (x) and the neighbour (y) of a pair: with d1 and d2 the velocity gradients'
+// quadratic forms at both ends and A = d1 / d2, the limiter 4 A / (1 + A)^2 lies in [0, 1] for A >= 0 and
+// is cut to 0 below, so that -phi (d1 + d2) = -d3 2 d1 d2 / (d1 + d2) where d1 and d2 have one sign, else
+// 0: one quotient instead of two divisions, shared by the two ends.  Magnitudes beyond 2^+-250 (a smooth
+// field that decays into the subnormal range has them), where the products and A itself leave the exponent
+// range, and values that are not finite take the reference's form.
+__device__ __forceinline__ double2 avRvShared(double d1, double d2, double dist)
+{
+    const unsigned h1 = unsigned(__double2hiint(d1)), h2 = unsigned(__double2hiint(d2));
+    const unsigned e1 = (h1 >> 20) & 0x7ffu, e2 = (h2 >> 20) & 0x7ffu;
+    if (e1 - 773u > 500u || e2 - 773u > 500u) {
+        if (d1 == 0.0 && d2 == 0.0) return make_double2(0.0, 0.0);  // regions at rest
+        return avRvWide(d1, d2, dist);
+    }
+    if (int(h1 ^ h2) < 0) return make_double2(0.0, 0.0);
+    const double s = 2.0 * d1 * quotient(d2, (d1 + d2) * dist);
+    return make_double2(s, s);
 }
 
 // FP64 VE momentum-energy with one evaluation per mutual pair, for lists that cover every particle.
@@ -1405,9 +1422,9 @@ __device__ __forceinline__ void meVeOnceBody(ListView lv, CoordFp64 cf, MeVeArgs
             const Rec4d j3 = ldRec4d(recj + 3), j4 = ldRec4d(recj + 4);
             const T gi[6] = {i3.v[0], i3.v[1], i3.v[2], i3.v[3], i4.v[0], i4.v[1]};
             const T gj[6] = {j3.v[0], j3.v[1], j3.v[2], j3.v[3], j4.v[0], j4.v[1]};
-            const T share = avRvShared(quadForm(rx, ry, rz, gi), quadForm(rx, ry, rz, gj), dist);
+            const double2 share = avRvShared(quadForm(rx, ry, rz, gi), quadForm(rx, ry, rz, gj), dist);
             const T eta = dist * (lessNonNeg(j4.v[2], i4.v[2]) ? j4.v[2] : i4.v[2]);  // min of |r|/h
-            T ci = share, cj = share;
+            T ci = share.x, cj = share.y;
             if (lessNonNeg(eta, i4.v[3])) {
                 const T e = 5.0 * (eta - i4.v[3]);
                 ci *= expNegSmall(e * e, a.expTab);

@@ -1,0 +1,62 @@
+"""The FP64 pass variants with inputs near the ends of their types' range: the one-evaluation form of each
+mutual pair against the order-fixed form on the same inputs, and neighbour counts against the oracle."""
+
+import numpy as np
+import pytest
+
+from test_gpu_parity import field_scale, fp64_tol, run_gpu
+
+pytestmark = pytest.mark.gpu
+
+ME_FIELDS = ("ax", "ay", "az", "du")
+
+
+def momentum_energy_both(gpu_ctx, edit, clean=False, side=12, seed=111):
+    """du, ax, ay, az and the time step of the default and the order-fixed momentum-energy pass after
+    edit(d) changed fields of a jittered lattice that went through the passes before it"""
+    from sphexa_gb300 import sph, workloads as W
+    wl = W.fourier(side, seed=seed, rho_seed=seed + 1, v_seed=seed + 2)
+    out = {}
+    for det in (True, False):
+        gpu_ctx.set_deterministic(det)
+        gpu_ctx.set_params(ng0=int(wl.params["ng0"]), ngmax=int(wl.params["ngmax"]), bucket=int(wl.params["bucket"]),
+                           minDt=float(wl.params["minDt"]))
+        d = sph.ParticlesData.from_workload(wl, "fp64", "cuda:0", av_clean=clean)
+        box = sph.Box(wl.box.copy(), wl.bc.copy())
+        sph.Domain(gpu_ctx, box).sync(d)
+        sph.find_neighbors_sfc(gpu_ctx, 0, wl.n, d)
+        gpu_ctx.set_deterministic(True)  # the same inputs of the last pass for both forms
+        sph.compute_xmass(gpu_ctx, d)
+        sph.compute_ve_def_gradh(gpu_ctx, d)
+        sph.compute_eos(gpu_ctx, d)
+        sph.compute_iad_divv_curlv(gpu_ctx, d)
+        sph.compute_av_switches(gpu_ctx, d)
+        gpu_ctx.set_deterministic(det)
+        edit(d)
+        sph.compute_momentum_energy(gpu_ctx, d, clean)
+        out[det] = {f: d.f[f].cpu().numpy() for f in ME_FIELDS}
+        out[det]["minDt"] = d.minDtCourant
+    gpu_ctx.set_deterministic(False)
+    return out[False], out[True]
+
+
+def check_me(once, fixed):
+    for f in ME_FIELDS:
+        assert np.all(np.isfinite(fixed[f])), f
+        err = np.max(np.abs(once[f] - fixed[f])) / field_scale(fixed, f)
+        assert err <= 1e-12, f"{f}: {err:.3e}"
+    assert once["minDt"] == pytest.approx(fixed["minDt"], rel=1e-12)
+
+
+@pytest.mark.parametrize("size", [1e-300, 1e-312, 1e-318, 1e-322])
+def test_viscosity_cleaning_with_subnormal_velocity_gradients(gpu_ctx, size):
+    """Velocity gradients that decay into the subnormal range (a smooth pulse far from its centre): the
+    cleaning term of such pairs is next to nothing and must not become infinite."""
+    def edit(d):
+        for k in ("dV11", "dV12", "dV13", "dV22", "dV23", "dV33"):
+            t = d.f[k]
+            half = t.shape[0] // 2
+            t[:half] = t[:half].sign() * size
+            d.f["dV11"][:half] = size
+            d.f["dV22"][:half] = size
+    check_me(*momentum_energy_both(gpu_ctx, edit, clean=True))
