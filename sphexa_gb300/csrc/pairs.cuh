@@ -575,7 +575,8 @@ static __device__ __noinline__ double2 atwoodExact(double rhoi, double rhoj, dou
 }
 
 // the same weights with few FP64 instructions: the two flat branches are taken where FP32 copies of rho
-// decide safely (1e-6 of the sum beside a threshold, and sums FP32 cannot hold, go to atwoodExact).
+// decide safely (1e-6 of the sum beside a threshold, and sums near the ends of FP32's range or beyond, where
+// they lose bits or overflow although both densities fit, go to atwoodExact).
 // On the ramp (a quarter of the pairs of a jittered lattice or a clustered sphere, so nearly every warp
 // is there for some lane) the quotient comes from a 20-bit reciprocal by two Newton corrections, and
 // q = e^a and 1 / q = e^-a, |a| <= 1/2, together from a table of e^(+-k/1024) and the even and odd parts
@@ -587,8 +588,9 @@ __device__ __forceinline__ void atwoodWeights(const double* __restrict__ rho, co
     const float dr = fabsf(rhofi - rhofj), sr = rhofi + rhofj;
     am = xmi * xmi;
     bm = xmj * xmj;
-    if (sr > 1e-30f && dr < (0.1f - 1e-6f) * sr) return;
-    if (sr > 1e-30f && dr > (0.2f + 1e-6f) * sr && dr < 1e38f) {
+    const bool held = sr > 1e-30f && sr < 1e38f;
+    if (held && dr < (0.1f - 1e-6f) * sr) return;
+    if (held && dr > (0.2f + 1e-6f) * sr) {
         am = bm = xmi * xmj;
         return;
     }
@@ -602,7 +604,7 @@ __device__ __forceinline__ void atwoodWeights(const double* __restrict__ rho, co
     const double a = fma(10.0, at, -1.0) * dln;
     // |a| from the high word, truncated to 20 bits, as a float: the nearest table node to within 2^-20
     const unsigned hi = unsigned(__double2hiint(a)), mag = hi & 0x7fffffffu;
-    const bool onRamp = sr > 1e-30f && dr > (0.1f + 1e-6f) * sr && dr < (0.2f - 1e-6f) * sr && mag < 0x3fe00000u;
+    const bool onRamp = held && dr > (0.1f + 1e-6f) * sr && dr < (0.2f - 1e-6f) * sr && mag < 0x3fe00000u;
     if (!onRamp) {
         const double2 ab = atwoodExact(rhoi, rhoj, dln, xmi, xmj);
         am = ab.x;

@@ -60,3 +60,16 @@ def test_viscosity_cleaning_with_subnormal_velocity_gradients(gpu_ctx, size):
             d.f["dV11"][:half] = size
             d.f["dV22"][:half] = size
     check_me(*momentum_energy_both(gpu_ctx, edit, clean=True))
+
+
+def test_atwood_weights_where_the_sum_of_densities_leaves_fp32(gpu_ctx):
+    """Densities that FP32 holds with sums that it does not: the decision between the flat branches and
+    the ramp is the FP64 one."""
+    import torch
+
+    def edit(d):
+        g = torch.Generator(device="cuda:0")
+        g.manual_seed(5)
+        rho = torch.empty_like(d.f["kx"]).uniform_(1.3e38, 3.3e38, generator=g)
+        d.f["kx"].copy_(rho * d.f["xm"] / d.f["m"])
+    check_me(*momentum_energy_both(gpu_ctx, edit))
