@@ -1229,8 +1229,18 @@ __global__ void avOnceFinish(int64_t first, int64_t last, int64_t n, AvArgs a, c
                avAlpha<double>(a, ld<double>(a.alpha, i), hi, ci, divvi, __longlong_as_double(vb), gx, gy, gz));
 }
 
+// the power of two that brings the first particle's mass to [1, 2): the pair sums of the pair-once
+// momentum-energy pass hold products of two masses, of which one is taken in this unit, so that they stay
+// in the exponent range wherever the masses do (a power of two changes no other bit)
+__device__ __forceinline__ double massUnit(const void* m)
+{
+    const long long b = __double_as_longlong(ld<double>(m, 0));
+    const int e = int(b >> 52) & 0x7ff;
+    return (b << 1) == 0 || e == 0x7ff ? 1.0 : __longlong_as_double((long long)(max(1, 2046 - max(1, e))) << 52);
+}
+
 // neighbour-side fields of the pair-once momentum-energy pass, 96 bytes per particle in three 32-byte
-// loads: A = m h^-3 c_ab (six entries), c, m, prho, 1/rho, xm, alpha / 8; and rho in FP32.  m and
+// loads: A = m h^-3 c_ab (six entries), c, m (in the unit of massUnit), prho, 1/rho, xm, alpha / 8; and rho in FP32.  m and
 // h^-3 enter every use of c, so they are folded in once per particle instead of per pair.  With the
 // viscosity cleaning two more: the symmetric velocity gradient (six entries), 1/h, and eta_crit of the
 // particle's neighbour count (momentum_energy_kern.hpp:43-63).
@@ -1254,7 +1264,7 @@ __global__ void meVeRec64Kernel(int64_t n, MeVeArgs a, ListView lv, double* __re
         rhoInv = aux[5 * n + j];
     }
     rec[R * j] = {f * ld<double>(a.c11, j), f * ld<double>(a.c12, j), f * ld<double>(a.c13, j), f * ld<double>(a.c22, j)};
-    rec[R * j + 1] = {f * ld<double>(a.c23, j), f * ld<double>(a.c33, j), ld<double>(a.c, j), m};
+    rec[R * j + 1] = {f * ld<double>(a.c23, j), f * ld<double>(a.c33, j), ld<double>(a.c, j), m * massUnit(a.m)};
     rec[R * j + 2] = {ld<double>(a.prho, j), rhoInv, xm, 0.125 * ld<double>(a.alpha, j)};
     if constexpr (AvClean) {
         const unsigned nc = lv.capped(j - lv.first);
@@ -1334,7 +1344,7 @@ __device__ __forceinline__ double2 avRvShared(double d1, double d2, double dist)
 //
 // Bound by the FP64 pipe (2 lanes per cycle and SM), so the pair terms are arranged for few FP64
 // instructions: 50 per mutual pair, 21 more on the Atwood ramp (atwoodWeights).  The sums are forces: with A = m h^-3 c at each end (per particle),
-// w_i' = m_j w_i and w_j' = m_i w_j, hv = visc / 2, t = hv / rho, P_i = w_i' (prho_i am + t_i) and
+// w_i' = m_j w_i and w_j' = m_i w_j (m in the unit of massUnit), hv = visc / 2, t = hv / rho, P_i = w_i' (prho_i am + t_i) and
 // P_j = w_j' (prho_j bm + t_j), both ends add the same V = P_i A_i r + P_j A_j r, with opposite signs,
 // and the same Q = t_i w_i' s_i + t_j w_j' s_j (s = v_ij . A r); the finishing kernel divides by the
 // particle's mass.  vsig is kept doubled, alpha divided by 8 (both exact).  With the per-pair exp and
@@ -1501,7 +1511,7 @@ __global__ void __launch_bounds__(kPairBlock) meVeOnceFinish(ListView lv, MeVeAr
     double dt = INFINITY;
     if (valid) {
         const int64_t i = i0;
-        const double prhoi = ld<double>(a.prho, i), mInv = 1.0 / ld<double>(a.m, i);
+        const double prhoi = ld<double>(a.prho, i), mInv = 1.0 / (ld<double>(a.m, i) * massUnit(a.m));
         const double en = a.acc[3 * a.n + i] * mInv, avSum = a.acc[4 * a.n + i] * mInv;
         if (a.tapeEn) {
             a.tapeEn[i] = en;

@@ -73,3 +73,15 @@ def test_atwood_weights_where_the_sum_of_densities_leaves_fp32(gpu_ctx):
         rho = torch.empty_like(d.f["kx"]).uniform_(1.3e38, 3.3e38, generator=g)
         d.f["kx"].copy_(rho * d.f["xm"] / d.f["m"])
     check_me(*momentum_energy_both(gpu_ctx, edit))
+
+
+@pytest.mark.parametrize("clean", [False, True])
+@pytest.mark.parametrize("scale", [1e-200, 1e-170, 1e170, 1e200])
+def test_masses_near_the_ends_of_the_exponent_range(gpu_ctx, scale, clean):
+    """Masses of 1e+-200 with prho and kx of a caller's own equation of state: products of two masses leave
+    the exponent range, the accelerations do not."""
+    def edit(d):
+        d.f["m"].mul_(scale)
+        d.f["kx"].div_(scale)
+        d.f["prho"].div_(scale)
+    check_me(*momentum_energy_both(gpu_ctx, edit, clean=clean))
