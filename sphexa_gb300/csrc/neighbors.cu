@@ -34,6 +34,10 @@ constexpr int kStack = 192;  // 8 children x (21 levels + 3)
 // last level.  With nodes pruned by their distance from the target box, fewer pops pay for the extra
 // staged candidates: 8M search stage 12.9 ms against 13.1 with 128; 64 costs the 27M set 7 ms of 28.
 constexpr uint32_t kCoarseNode = 256;
+// above the rounding of a squared FP32 distance that is subnormal (lengths below 1e-19 in the caller's units):
+// part of every margin on squares.  Below 1e-21 all squares lie inside it and all candidates take the FP64
+// test.
+constexpr float kTinySq = 0x1p-140f;
 
 struct NbrArgs {
     const double *x, *y, *z;
@@ -193,12 +197,12 @@ __global__ void __launch_bounds__(kNbrBlock, Fold ? 6 : 8) nbrGroupKernel(NbrArg
         gt[k] = 0.5f * (tmx[k] - tmn[k]) + pad;
         Rg = fmaxf(Rg, reach);
     }
-    const float gR2 = rfm * rfm * (1.f + 0x1p-18f);
+    const float gR2 = fmaf(rfm * rfm, 1.f + 0x1p-18f, kTinySq);
     // FP32 decision margin on d2: covers the rounding of cell edge, offsets and the squared sum (and,
     // where pairs are folded, of the box length, L <= 2 Rg / 0.98 there); pairs inside the margin get the
     // exact FP64 test
     const float r2f = float(r2);
-    const float margin = 64.f * 0x1p-24f * (Rg + rf) * (Rg + rf);
+    const float margin = 64.f * 0x1p-24f * (Rg + rf) * (Rg + rf) + kTinySq;
     const float inBelow = r2f - margin;   // d2f < inBelow: neighbour
     const float outAbove = r2f + margin;  // d2f > outAbove: not a neighbour
 
@@ -265,7 +269,7 @@ __global__ void __launch_bounds__(kNbrBlock, Fold ? 6 : 8) nbrGroupKernel(NbrArg
         sm.cull[0] = tmn[0];
         sm.cull[1] = tmn[1];
         sm.cull[2] = tmn[2];
-        sm.cull[3] = cullR * cullR * (1.f + 0x1p-18f);
+        sm.cull[3] = fmaf(cullR * cullR, 1.f + 0x1p-18f, kTinySq);
         sm.cull[4] = tmx[0];
         sm.cull[5] = tmx[1];
         sm.cull[6] = tmx[2];
@@ -735,7 +739,7 @@ __device__ __forceinline__ bool mutualPair(const MutualArgs& a, int64_t i, const
     // across a periodic face only a target that takes the minimum image can list i
     if (wrapped && !(R2s < 0.f)) return false;
     const float d2 = fmaf(r[0], r[0], fmaf(r[1], r[1], r[2] * r[2]));
-    const float eps = 0x1p-17f * R2j;
+    const float eps = fmaf(0x1p-17f, R2j, kTinySq);
     if (d2 < R2j - eps) return true;
     if (d2 > R2j + eps) return false;
     return mutualExact(a, i, j, loadH(a.h, a.hIsFloat, j));

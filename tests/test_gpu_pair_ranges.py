@@ -85,3 +85,20 @@ def test_masses_near_the_ends_of_the_exponent_range(gpu_ctx, scale, clean):
         d.f["kx"].div_(scale)
         d.f["prho"].div_(scale)
     check_me(*momentum_energy_both(gpu_ctx, edit, clean=clean))
+
+
+@pytest.mark.parametrize("scale", [1e-19, 1e-20, 1e-21, 1e-22, 1e-24, 1e-30])
+@pytest.mark.parametrize("n, periodic", [(600, True), (1728, True), (6000, True), (3000, False)])
+def test_neighbours_where_squared_radii_are_subnormal_in_fp32(gpu_ctx, port, n, periodic, scale):
+    """Lengths whose squares FP32 holds with a few bits or none: neighbour counts of small periodic boxes
+    (pairs folded one by one) and of an open set against the oracle."""
+    from sphexa_gb300 import workloads as W
+    wl = W.random_cube(n, seed=120 + n, periodic=periodic)
+    for k in ("x", "y", "z", "h"):
+        wl.fields[k] = wl.fields[k] * scale
+    wl.box = wl.box * scale
+    wl.fields["m"] = wl.fields["m"] * scale ** 3
+    gpu_ctx.set_deterministic(False)
+    r = run_gpu(gpu_ctx, wl, "std", False)
+    ref = port.sweep(wl, "std", False)
+    np.testing.assert_array_equal(r["nc"], ref["nc"])
