@@ -19,6 +19,7 @@
 // entries transposed per granule (listSlot), written one 16-byte granule at a time, so that the pair
 // passes read them coalesced.
 #include <algorithm>
+#include <cmath>
 
 
 #include "pairs.cuh"
@@ -55,6 +56,7 @@ struct NbrArgs {
     const float4* nodeBox;
     const uint2* nodeRange;  // particles [start, end) per node
     int64_t numNodes;
+    float pruneUnit;         // power of two: the unit of the squared distances that prune nodes
     DevBox box;
     uint32_t ngmax;
     int64_t stride;
@@ -197,7 +199,7 @@ __global__ void __launch_bounds__(kNbrBlock, Fold ? 6 : 8) nbrGroupKernel(NbrArg
         gt[k] = 0.5f * (tmx[k] - tmn[k]) + pad;
         Rg = fmaxf(Rg, reach);
     }
-    const float gR2 = fmaf(rfm * rfm, 1.f + 0x1p-18f, kTinySq);
+    const float gR = rfm * a.pruneUnit, gR2 = fmaf(gR * gR, 1.f + 0x1p-18f, kTinySq);
     // FP32 decision margin on d2: covers the rounding of cell edge, offsets and the squared sum (and,
     // where pairs are folded, of the box length, L <= 2 Rg / 0.98 there); pairs inside the margin get the
     // exact FP64 test
@@ -465,7 +467,7 @@ __global__ void __launch_bounds__(kNbrBlock, Fold ? 6 : 8) nbrGroupKernel(NbrArg
             for (int k = 0; k < 3; ++k) {
                 float dd = fabsf(cc[k] - gc[k]);
                 if (b.pbc[k]) dd = fminf(dd, b.Lf[k] - dd);
-                const float gap = fmaxf(dd - ss[k] - gt[k], 0.f);
+                const float gap = fmaxf(dd - ss[k] - gt[k], 0.f) * a.pruneUnit;
                 e2 = fmaf(gap, gap, e2);
                 inside = inside && (dd + ss[k] <= gt[k] + rfm);
             }
@@ -904,6 +906,11 @@ int runSearch(sphgb_ctx* c, const double* x, const double* y, const double* z, c
         a.u[k] = float(c->box.L[k] / double(1 << kGridBits));
         a.sh[k] = c->box.pbc[k] ? 32 - kGridBits : 0;
     }
+    // boxes beyond 2^+-30 are pruned in units of their own size: squares of lengths below 1e-19 or above 1e19
+    // would underflow or overflow, and every node would be walked
+    const double longest = std::max(c->box.L[0], std::max(c->box.L[1], c->box.L[2]));
+    const int e = longest > 0.0 && std::isfinite(longest) ? std::ilogb(longest) : 0;
+    a.pruneUnit = std::abs(e) > 30 ? float(std::ldexp(1.0, std::min(126, std::max(-126, -e)))) : 1.f;
     a.first = first;
     a.last = last;
     a.active = active;

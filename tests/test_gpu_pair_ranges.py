@@ -102,3 +102,20 @@ def test_neighbours_where_squared_radii_are_subnormal_in_fp32(gpu_ctx, port, n, 
     r = run_gpu(gpu_ctx, wl, "std", False)
     ref = port.sweep(wl, "std", False)
     np.testing.assert_array_equal(r["nc"], ref["nc"])
+
+
+@pytest.mark.parametrize("scale", [1e-30, 1e-24, 1e22, 1e28])
+def test_search_prunes_nodes_in_any_unit(gpu_ctx, scale):
+    """Lengths whose squares leave FP32: nodes are pruned as in ordinary units, single candidates are not.
+    Pairs tested then: with nodes of at most 256 particles (edge 6.4 spacings) the region of 9 spacings
+    grows to 21.7 at most, 16.5 times as many pairs as the 620 per target of ordinary units; without
+    pruning it would be every pair of the set, 97 times."""
+    from sphexa_gb300 import workloads as W
+    tested = []
+    for f in (1.0, scale):
+        wl = W.random_cube(60000, seed=140, periodic=False)
+        for k in ("x", "y", "z", "h"):
+            wl.fields[k] = wl.fields[k] * f
+        wl.box = wl.box * f
+        tested.append(run_gpu(gpu_ctx, wl, "std", False)["stats"]["candidates"])
+    assert tested[1] <= 20 * tested[0], tested
