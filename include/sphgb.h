@@ -111,6 +111,16 @@ int sphgb_set_params(sphgb_ctx* ctx, const sphgb_params* params);
  * with FP64 atomics, so the last bits of those passes' outputs can differ from run to run.
  * on = 1: every list owner sums its own pairs in list order, bitwise reproducible. */
 int sphgb_set_deterministic(sphgb_ctx* ctx, int32_t on);
+/* Pair-geometry cache of the FP64 passes with on = 0 above (no reference counterpart): the first pair pass
+ * (xmass or std density) over all particles keeps each owned pair's geometry and kernel values for the
+ * passes after it.  arrays = 5 (default): 80 bytes per owned pair, or 32 where that does not fit; 2: 32
+ * bytes; 0: none, and the memory is freed.  It takes at most half of the free device memory inside
+ * sphgb_sweep / sphgb_sweep_passes and an eighth of it in passes called one by one, and is given back when
+ * another allocation of the context needs the space.  The results do not depend on it. */
+int sphgb_set_pair_cache(sphgb_ctx* ctx, int32_t arrays);
+/* what the cache holds: arrays of the last store, bytes, allocations since the context was made (any
+ * pointer may be NULL) */
+int sphgb_get_pair_cache(sphgb_ctx* ctx, int32_t* arrays, int64_t* bytes, int64_t* allocations);
 /* Forward tape of the VE adjoint (no reference counterpart).  on = 1: the FP64 VE passes over all
  * particles (gradh, IAD + divv/curlv, AV switches, momentum-energy) keep the per-particle sums
  * that sphgb_adjoint_ve needs (16 doubles per particle, held by the context), and the adjoint

@@ -20,8 +20,12 @@ void setCudaError(cudaError_t e, const char* what)
 
 namespace {
 
+// the context of the thread's current call (reclaimPairGeo): set at every entry that may allocate
+thread_local sphgb_ctx* currentCtx = nullptr;
+
 int useDevice(sphgb_ctx* c)
 {
+    currentCtx = c;
     if (!c) return SPHGB_ERR_ARG;
     SPHGB_CUDA(cudaSetDevice(c->device));
     return SPHGB_OK;
@@ -64,6 +68,14 @@ int checkRange(const sphgb_particles* p, int64_t first, int64_t last)
 
 // for the entry points in other translation units
 int useDeviceOf(sphgb_ctx* c) { return useDevice(c); }
+
+bool reclaimPairGeo(const DBuf* wanted)
+{
+    sphgb_ctx* c = currentCtx;
+    if (!c || !c->pairGeo.p || wanted == &c->pairGeo) return false;
+    c->dropPairGeo();
+    return true;
+}
 }  // namespace sphgb
 
 using namespace sphgb;
@@ -112,6 +124,7 @@ int sphgb_create(sphgb_ctx** out, int device)
 {
     if (!out) return SPHGB_ERR_ARG;
     *out = nullptr;
+    currentCtx = nullptr;
     int count = 0;
     if (cudaGetDeviceCount(&count) != cudaSuccess || count == 0) return SPHGB_ERR_NOTFOUND;
     if (device < 0 || device >= count) return SPHGB_ERR_ARG;
@@ -140,6 +153,7 @@ int sphgb_create(sphgb_ctx** out, int device)
 int sphgb_destroy(sphgb_ctx* c)
 {
     if (!c) return SPHGB_ERR_ARG;
+    currentCtx = nullptr;
     cudaSetDevice(c->device);
     cudaStreamSynchronize(c->stream);
     DBuf* bufs[] = {&c->keys,     &c->keysAlt,      &c->order,         &c->orderAlt,      &c->sortTemp,
@@ -182,6 +196,24 @@ int sphgb_set_deterministic(sphgb_ctx* c, int32_t on)
 {
     if (!c || (on != 0 && on != 1)) return SPHGB_ERR_ARG;
     c->deterministic = on != 0;
+    return SPHGB_OK;
+}
+
+int sphgb_set_pair_cache(sphgb_ctx* c, int32_t arrays)
+{
+    SPHGB_TRY(useDevice(c));
+    if (arrays != 0 && arrays != 2 && arrays != 5) return SPHGB_ERR_ARG;
+    c->geoLimit = arrays;
+    if (c->geoArrays > arrays) c->dropPairGeo();
+    return SPHGB_OK;
+}
+
+int sphgb_get_pair_cache(sphgb_ctx* c, int32_t* arrays, int64_t* bytes, int64_t* allocations)
+{
+    if (!c) return SPHGB_ERR_ARG;
+    if (arrays) *arrays = c->pairGeo.p ? c->geoArrays : 0;
+    if (bytes) *bytes = int64_t(c->pairGeo.bytes);
+    if (allocations) *allocations = c->geoAllocs;
     return SPHGB_OK;
 }
 

@@ -30,6 +30,11 @@ void setCudaError(cudaError_t e, const char* what);
         if (s_ != SPHGB_OK) return s_;       \
     } while (0)
 
+struct DBuf;
+// frees the pair-geometry cache of the context that the calling thread is in, unless `wanted` is that buffer;
+// false when there is nothing to free
+bool reclaimPairGeo(const DBuf* wanted);
+
 // growable device buffer
 struct DBuf {
     void* p = nullptr;
@@ -42,6 +47,10 @@ struct DBuf {
         bytes = 0;
         size_t alloc = need < 256 ? 256 : need;
         cudaError_t e = cudaMalloc(&p, alloc);
+        if (e == cudaErrorMemoryAllocation && reclaimPairGeo(this)) {
+            (void)cudaGetLastError();
+            e = cudaMalloc(&p, alloc);
+        }
         if (e != cudaSuccess) {
             setCudaError(e, "cudaMalloc");
             p = nullptr;
@@ -114,6 +123,8 @@ struct sphgb_ctx {
     sphgb::DBuf pairGeo, geoRows;
     size_t geoRowCount = 0;
     int geoArrays = 0;  // 5: with the difference and velocity-difference vectors, 2: without
+    int geoLimit = 5;   // most arrays to keep (sphgb_set_pair_cache)
+    int64_t geoAllocs = 0;
     bool geoValid = false;
     // outside a sweep the caller may change x y z v h between passes: the pass that stores the cache keeps
     // a copy of them, and every later pass on the same lists (epoch geoSnapEpoch) compares its inputs with
@@ -121,6 +132,14 @@ struct sphgb_ctx {
     sphgb::DBuf geoSnap, geoStale;
     int64_t geoSnapEpoch = -1, geoSnapN = 0;
     bool geoChecked = false;  // the running pass compared its inputs with geoSnap
+    void dropPairGeo()
+    {
+        pairGeo.release();
+        geoSnap.release();
+        geoSnapEpoch = -1;
+        geoArrays = 0;
+        geoValid = geoChecked = false;
+    }
     // inside sphgb_sweep_passes the per-particle precomputes are built by the first pass only
     bool inSweep = false, sweepPrepared = false;
     // within one sweep: the EOS ran in the gradh epilogue / the per-particle quotients are formed

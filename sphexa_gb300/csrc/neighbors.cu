@@ -989,10 +989,7 @@ int prepareLists(sphgb_ctx* c, const double* x, const double* y, const double* z
     c->nbrStride = (nWork + 31) / 32 * 32;
     // lists larger than the buffers hold: the pair-geometry cache of an earlier sweep gives its
     // memory back first (the next FP64 sweep sizes it again within half of the free memory)
-    if (c->nbr.bytes < sizeof(uint32_t) * listCapacity(ngmax) * c->nbrStride) {
-        c->pairGeo.release();
-        c->geoSnapEpoch = -1;
-    }
+    if (c->nbr.bytes < sizeof(uint32_t) * listCapacity(ngmax) * c->nbrStride) c->dropPairGeo();
     SPHGB_TRY(c->nbr.ensure(sizeof(uint32_t) * listCapacity(ngmax) * c->nbrStride));
     SPHGB_TRY(c->ncount.ensure(sizeof(uint32_t) * c->nbrStride));
     SPHGB_TRY(c->active.ensure(sizeof(uint32_t) * c->nbrStride + c->nbrStride));
@@ -1038,7 +1035,7 @@ int pairGeoStore(sphgb_ctx* c, const sphgb_particles* p, PairGeo* out)
     c->geoSnapEpoch = -1;
     if (c->ownedEpoch != c->nbrEpoch || c->ownedFromLists || !p->vx || !p->vy || !p->vz) return SPHGB_OK;
     const size_t rows = c->geoRowCount;
-    if (rows == 0) return SPHGB_OK;
+    if (rows == 0 || c->geoLimit == 0) return SPHGB_OK;
     if (!c->inSweep) {
         if (c->geoSnap.ensure(sizeof(double) * kGeoInputs * size_t(p->n)) != SPHGB_OK ||
             c->geoStale.ensure(sizeof(int)) != SPHGB_OK) {
@@ -1047,20 +1044,25 @@ int pairGeoStore(sphgb_ctx* c, const sphgb_particles* p, PairGeo* out)
         }
     }
     // five arrays (|r| and w_ij, the two kernel values, r and dv) or the first two, whichever fits
-    // in the buffer already held or in half of the free device memory
+    // in the buffer already held, in half of the free device memory inside a sweep, or in an eighth of it
+    // outside (a caller that makes the passes one by one allocates more of its own between them; 8M particles
+    // take 33 GB, an eighth of an empty device)
+    const size_t share = c->inSweep ? 2 : 8;
     int arrays = 0;
     for (int a : {5, 2}) {
+        if (a > c->geoLimit) continue;
         const size_t need = size_t(a) * 32 * sizeof(double2) * rows;
         if (c->pairGeo.bytes >= need) {
             arrays = a;
             break;
         }
         size_t freeB = 0, totalB = 0;
-        if (cudaMemGetInfo(&freeB, &totalB) != cudaSuccess || need > (freeB + c->pairGeo.bytes) / 2) continue;
+        if (cudaMemGetInfo(&freeB, &totalB) != cudaSuccess || need > (freeB + c->pairGeo.bytes) / share) continue;
         if (c->pairGeo.ensure(need) != SPHGB_OK) {
             (void)cudaGetLastError();
             continue;
         }
+        ++c->geoAllocs;
         arrays = a;
         break;
     }

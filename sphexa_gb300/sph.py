@@ -81,6 +81,16 @@ class Context:
         momentum-energy) evaluate mutual pairs once and scatter with FP64 atomics."""
         check(self.lib.sphgb_set_deterministic(self.h, int(bool(on))), "sphgb_set_deterministic")
 
+    def set_pair_cache(self, arrays: int) -> None:
+        """Most arrays of the FP64 pair-geometry cache: 5 (default), 2 or 0 (none; frees the memory)."""
+        check(self.lib.sphgb_set_pair_cache(self.h, int(arrays)), "sphgb_set_pair_cache")
+
+    def pair_cache(self) -> dict:
+        """arrays, bytes and allocations of the pair-geometry cache."""
+        a, b, n = C.c_int32(), C.c_int64(), C.c_int64()
+        check(self.lib.sphgb_get_pair_cache(self.h, C.byref(a), C.byref(b), C.byref(n)), "sphgb_get_pair_cache")
+        return dict(arrays=a.value, bytes=b.value, allocations=n.value)
+
     def set_adjoint_tape(self, on: bool) -> None:
         """FP64 VE passes keep the sums the VE adjoint needs (sphgb_set_adjoint_tape)."""
         check(self.lib.sphgb_set_adjoint_tape(self.h, int(bool(on))), "sphgb_set_adjoint_tape")

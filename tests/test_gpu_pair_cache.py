@@ -1,0 +1,67 @@
+"""Memory of the FP64 pair-geometry cache: how much of the device it takes, and that it is given back."""
+
+import contextlib
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+
+
+@contextlib.contextmanager
+def free_memory(leave):
+    """all but `leave` bytes of the device held by a tensor"""
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - leave, dtype=torch.uint8, device="cuda:0")
+    try:
+        yield
+    finally:
+        del fill
+        torch.cuda.empty_cache()
+
+
+def frozen(side, ctx):
+    from sphexa_gb300 import autograd as AG, sph, workloads as W
+    wl = W.fourier(side, seed=131, rho_seed=132, v_seed=133)
+    d = sph.ParticlesData.from_workload(wl, "fp64", "cuda:0")
+    sw = AG.FrozenVeSweep(ctx, d, sph.Box(wl.box.copy(), wl.bc.copy()), tape=False)
+    sw.freeze()
+    return wl, d, sw
+
+
+def test_single_passes_take_an_eighth_of_the_free_memory():
+    """27,000 particles, 120 MB of geometry, 400 MB free: a pass called by itself takes 50 MB of it (two of the
+    five arrays, and the copy of its inputs)."""
+    import torch
+    from sphexa_gb300 import sph
+    ctx = sph.Context(0)
+    wl, d, sw = frozen(30, ctx)
+    with free_memory(400 * MB):
+        free = torch.cuda.mem_get_info()[0]
+        sph.compute_xmass(ctx, d)
+        used = free - torch.cuda.mem_get_info()[0]
+    ctx.close()
+    # an eighth, the copy of the inputs (1.5 MB), the sums (0.4 MB), and the allocator's 2 MB pages of each
+    assert used <= free // 8 + 16 * MB, used
+
+
+def test_cache_is_given_back_when_the_context_needs_the_space():
+    """After a sweep that left 1.5 GB of geometry, with 160 MB free, the adjoint's 225 MB of state are found."""
+    from sphexa_gb300 import sph
+    ctx = sph.Context(0)
+    wl, d, sw = frozen(70, ctx)
+    vals = list(sw.inputs())
+    rho, ax, ay, az, du = sw.forward(*vals)
+    seeds = (2.0 * rho, 2.0 * ax, 2.0 * ay, 2.0 * az, None)
+    with free_memory(160 * MB):
+        g = [t.cpu().numpy() for t in sw.backward(*seeds)]
+    assert all(np.all(np.isfinite(q)) for q in g)
+    rho, ax, ay, az, du = sw.forward(*vals)  # and the passes go on
+    again = [t.cpu().numpy() for t in sw.backward(*seeds)]
+    for a, b in zip(g, again):
+        assert np.max(np.abs(a - b)) <= 1e-10 * np.max(np.abs(b))
+    ctx.close()
