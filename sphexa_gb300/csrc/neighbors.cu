@@ -1056,12 +1056,14 @@ int pairGeoStore(sphgb_ctx* c, const sphgb_particles* p, PairGeo* out)
             arrays = a;
             break;
         }
+        // the rows change a little with every search of a moving set: 3 % more than asked for, where that fits
         size_t freeB = 0, totalB = 0;
-        if (cudaMemGetInfo(&freeB, &totalB) != cudaSuccess || need > (freeB + c->pairGeo.bytes) / share) continue;
-        if (c->pairGeo.ensure(need) != SPHGB_OK) {
-            (void)cudaGetLastError();
-            continue;
-        }
+        if (cudaMemGetInfo(&freeB, &totalB) != cudaSuccess) continue;
+        const size_t most = (freeB + c->pairGeo.bytes) / share, padded = need + need / 32;
+        if (need > most) continue;
+        const bool got = (padded <= most && c->pairGeo.ensure(padded) == SPHGB_OK) || c->pairGeo.ensure(need) == SPHGB_OK;
+        (void)cudaGetLastError();  // of an attempt that failed
+        if (!got) continue;
         ++c->geoAllocs;
         arrays = a;
         break;

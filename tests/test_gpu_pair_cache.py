@@ -65,3 +65,21 @@ def test_cache_is_given_back_when_the_context_needs_the_space():
     for a, b in zip(g, again):
         assert np.max(np.abs(a - b)) <= 1e-10 * np.max(np.abs(b))
     ctx.close()
+
+
+def test_small_rises_of_the_pair_count_do_not_reallocate():
+    """Twelve sweeps with h growing by 0.06 % each (2 % more pairs in all): one allocation."""
+    from sphexa_gb300 import sph, workloads as W
+    ctx = sph.Context(0)
+    wl = W.fourier(30, seed=134, rho_seed=135, v_seed=136)
+    d = sph.ParticlesData.from_workload(wl, "fp64", "cuda:0")
+    box = sph.Box(wl.box.copy(), wl.bc.copy())
+    pairs = []
+    for step in range(12):
+        sph.sweep(ctx, d, box, "ve")
+        pairs.append(ctx.stats()["nc_sum"])
+        d.f["h"].mul_(1.0006)
+    assert 1.01 * pairs[0] < pairs[-1] < 1.03 * pairs[0], pairs
+    cache = ctx.pair_cache()
+    assert cache["arrays"] == 5 and cache["allocations"] == 1, cache
+    ctx.close()
