@@ -83,3 +83,61 @@ def test_small_rises_of_the_pair_count_do_not_reallocate():
     cache = ctx.pair_cache()
     assert cache["arrays"] == 5 and cache["allocations"] == 1, cache
     ctx.close()
+
+
+FIELDS = dict(ve=("xm", "kx", "gradh", "rho", "c11", "c23", "divv", "curlv", "alpha", "ax", "ay", "az", "du"),
+              std=("rho", "c11", "c23", "ax", "ay", "az", "du"))
+
+
+@pytest.mark.parametrize("arrays", [0, 2, 5])
+@pytest.mark.parametrize("variant", ["ve", "ve_clean", "std"])
+@pytest.mark.parametrize("how", ["sweep", "passes", "passes_moved"])
+def test_every_form_of_the_cache_matches_the_order_fixed_passes(gpu_ctx, arrays, variant, how):
+    """No cache, the two arrays of scalars, and all five, filled and read inside a sweep and by passes called
+    one by one, with the same inputs and with velocities changed after the first pass."""
+    from sphexa_gb300 import sph, workloads as W
+    from test_gpu_parity import field_scale, fp64_tol
+    wl = W.fourier(13, seed=141, rho_seed=142, v_seed=143)
+    clean, chain = variant == "ve_clean", "std" if variant == "std" else "ve"
+    gpu_ctx.set_params(ng0=int(wl.params["ng0"]), ngmax=int(wl.params["ngmax"]), bucket=int(wl.params["bucket"]),
+                       minDt=float(wl.params["minDt"]))
+    out = {}
+    for det in (True, False):
+        gpu_ctx.set_deterministic(det)
+        gpu_ctx.set_pair_cache(0)
+        gpu_ctx.set_pair_cache(arrays)
+        d = sph.ParticlesData.from_workload(wl, "fp64", "cuda:0", av_clean=clean)
+        box = sph.Box(wl.box.copy(), wl.bc.copy())
+        if how == "sweep":
+            sph.sweep(gpu_ctx, d, box, chain, clean)
+        else:
+            sph.Domain(gpu_ctx, box).sync(d)
+            sph.find_neighbors_sfc(gpu_ctx, 0, wl.n, d)
+            (sph.compute_density if chain == "std" else sph.compute_xmass)(gpu_ctx, d)
+            if how == "passes_moved":
+                d.f["vy"].mul_(1.01)
+            if chain == "std":
+                sph.compute_eos_hydro_std(gpu_ctx, d)
+                sph.compute_iad(gpu_ctx, d)
+                sph.compute_momentum_energy_std(gpu_ctx, d)
+            else:
+                sph.compute_ve_def_gradh(gpu_ctx, d)
+                sph.compute_eos(gpu_ctx, d)
+                sph.compute_iad_divv_curlv(gpu_ctx, d)
+                sph.compute_av_switches(gpu_ctx, d)
+                sph.compute_momentum_energy(gpu_ctx, d, clean)
+        out[det] = {f: d.f[f].cpu().numpy() for f in FIELDS[chain]}
+        out[det]["minDt"] = d.minDtCourant
+        assert gpu_ctx.pair_cache()["arrays"] == (0 if det else arrays)
+    gpu_ctx.set_deterministic(False)
+    gpu_ctx.set_pair_cache(5)
+    for f in FIELDS[chain]:
+        err = np.max(np.abs(out[False][f] - out[True][f])) / field_scale(out[True], f)
+        assert err <= fp64_tol(out[True], f, chain), f"{f}: {err:.3e}"
+    assert out[False]["minDt"] == pytest.approx(out[True]["minDt"], rel=1e-12)
+
+
+def test_cache_limits_are_checked(gpu_ctx):
+    for bad in (-1, 1, 3, 6):
+        with pytest.raises(Exception):
+            gpu_ctx.set_pair_cache(bad)
