@@ -203,8 +203,8 @@ int sphgb_set_pair_cache(sphgb_ctx* c, int32_t arrays)
 {
     SPHGB_TRY(useDevice(c));
     if (arrays != 0 && arrays != 2 && arrays != 5) return SPHGB_ERR_ARG;
+    if (arrays < c->geoLimit) c->dropPairGeo();
     c->geoLimit = arrays;
-    if (c->geoArrays > arrays) c->dropPairGeo();
     return SPHGB_OK;
 }
 

@@ -125,6 +125,7 @@ struct sphgb_ctx {
     int geoArrays = 0;  // 5: with the difference and velocity-difference vectors, 2: without
     int geoLimit = 5;   // most arrays to keep (sphgb_set_pair_cache)
     int64_t geoAllocs = 0;
+    int geoUnread = 0;  // stores outside a sweep since a pass last asked for the cache
     bool geoValid = false;
     // outside a sweep the caller may change x y z v h between passes: the pass that stores the cache keeps
     // a copy of them, and every later pass on the same lists (epoch geoSnapEpoch) compares its inputs with

@@ -213,8 +213,9 @@ inline PairGeo pairGeoView(const sphgb_ctx* c, const int* stale)
 }
 
 // what the xmass or density pass stored: in a sweep as it is, outside one subject to the comparison; or null
-inline PairGeo pairGeoRead(const sphgb_ctx* c)
+inline PairGeo pairGeoRead(sphgb_ctx* c)
 {
+    if (!c->inSweep) c->geoUnread = 0;
     if (c->inSweep && c->geoValid) return pairGeoView(c, nullptr);
     if (!c->inSweep && c->geoChecked) return pairGeoView(c, c->geoStale.as<int>());
     return PairGeo{};

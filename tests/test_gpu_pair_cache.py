@@ -141,3 +141,22 @@ def test_cache_limits_are_checked(gpu_ctx):
     for bad in (-1, 1, 3, 6):
         with pytest.raises(Exception):
             gpu_ctx.set_pair_cache(bad)
+
+
+def test_first_pass_repeated_alone_stops_storing():
+    """xmass called again and again with no pass to read its geometry: the third call stores none, and the call
+    after a pass that asked does."""
+    from sphexa_gb300 import sph
+    ctx = sph.Context(0)
+    wl, d, sw = frozen(12, ctx)
+    held = []
+    for _ in range(4):
+        sph.compute_xmass(ctx, d)
+        held.append(ctx.pair_cache()["arrays"])
+    assert held == [5, 5, 0, 0], held
+    xm = d.f["xm"].cpu().numpy()
+    sph.compute_ve_def_gradh(ctx, d)
+    sph.compute_xmass(ctx, d)
+    assert ctx.pair_cache()["arrays"] == 5
+    np.testing.assert_allclose(d.f["xm"].cpu().numpy(), xm, rtol=1e-14)
+    ctx.close()
