@@ -143,6 +143,7 @@ struct sphgb_ctx {
     }
     // inside sphgb_sweep_passes the per-particle precomputes are built by the first pass only
     bool inSweep = false, sweepPrepared = false;
+    int sortAllBits = 0;  // syncs left that sort keys over all bits at once (sortParticleKeys)
     // within one sweep: the EOS ran in the gradh epilogue / the per-particle quotients are formed
     bool eosFused = false, auxReady = false;
     // packed neighbour-side records of the mixed pair passes and of the pair-once momentum-energy pass
