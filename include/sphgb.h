@@ -105,10 +105,13 @@ int sphgb_destroy(sphgb_ctx* ctx);
 int sphgb_set_stream(sphgb_ctx* ctx, void* cuda_stream);
 int sphgb_set_params(sphgb_ctx* ctx, const sphgb_params* params);
 /* Summation order of the FP64 passes: VE xmass, gradh, IAD + divv/curlv, AV switches and
- * momentum-energy, std density, IAD and momentum-energy (no reference counterpart; the reference's GPU passes are order-fixed, e.g.
- * hydro_ve/momentum_energy_gpu.cu:53-144).  on = 0 (default): when the lists cover every particle,
- * each pair whose two ends list each other is evaluated once and the neighbour's share is added
- * with FP64 atomics, so the last bits of those passes' outputs can differ from run to run.
+ * momentum-energy, std density, IAD and momentum-energy (no reference counterpart; the reference's GPU
+ * passes are order-fixed, e.g. hydro_ve/momentum_energy_gpu.cu:53-144).  on = 0 (default): when the lists
+ * cover every particle, each pair whose two ends list each other is evaluated once.  The VE passes add the
+ * neighbour's share with FP64 atomics, so the last bits of their outputs can differ from run to run.  The
+ * std passes keep it in a record of the pair (36 bytes per owned pair, within the shares of the free
+ * memory that sphgb_set_pair_cache names; else they walk whole lists as with on = 1) and add the records
+ * in a fixed order: the same bits in every run.
  * on = 1: every list owner sums its own pairs in list order, bitwise reproducible. */
 int sphgb_set_deterministic(sphgb_ctx* ctx, int32_t on);
 /* Pair-geometry cache of the FP64 passes with on = 0 above (no reference counterpart): the first pair pass

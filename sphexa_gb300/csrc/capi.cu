@@ -20,7 +20,7 @@ void setCudaError(cudaError_t e, const char* what)
 
 namespace {
 
-// the context of the thread's current call (reclaimPairGeo): set at every entry that may allocate
+// the context of the thread's current call (reclaimPairMemory): set at every entry that may allocate
 thread_local sphgb_ctx* currentCtx = nullptr;
 
 int useDevice(sphgb_ctx* c)
@@ -69,11 +69,14 @@ int checkRange(const sphgb_particles* p, int64_t first, int64_t last)
 // for the entry points in other translation units
 int useDeviceOf(sphgb_ctx* c) { return useDevice(c); }
 
-bool reclaimPairGeo(const DBuf* wanted)
+bool reclaimPairMemory(const DBuf* wanted)
 {
     sphgb_ctx* c = currentCtx;
-    if (!c || !c->pairGeo.p || wanted == &c->pairGeo) return false;
+    if (!c || (!c->pairGeo.p && !c->pairRec.p)) return false;
+    for (const DBuf* b : {&c->pairGeo, &c->geoSnap, &c->geoStale, &c->pairRec, &c->inbox})
+        if (b == wanted) return false;  // one of them never takes the place of another, which the pass may hold
     c->dropPairGeo();
+    c->dropPairRec();
     return true;
 }
 }  // namespace sphgb
@@ -164,7 +167,7 @@ int sphgb_destroy(sphgb_ctx* c)
                     &c->gridKey,
                     &c->gridLoc,  &c->hInv64,       &c->reduceScratch, &c->aux,         &c->adjKeys,
                     &c->adjKeysAlt, &c->tOff,       &c->tIdx,          &c->adjState,      &c->whx64,
-                    &c->whdx64,     &c->owned,      &c->ownedCount, &c->pairAcc,    &c->pairGeo,    &c->geoRows,    &c->geoSnap,    &c->geoStale,   &c->pack,       &c->rhof,       &c->expTab,     &c->whx32,     &c->whH32, &c->whdH32,    &c->refMask,
+                    &c->whdx64,     &c->owned,      &c->ownedCount, &c->pairAcc,    &c->pairGeo,    &c->geoRows,    &c->geoSnap,    &c->geoStale,   &c->pairRec,  &c->inbox,  &c->inboxOff, &c->inboxCount, &c->pack,       &c->rhof,       &c->expTab,     &c->whx32,     &c->whH32, &c->whdH32,    &c->refMask,
                     &c->refFp64,    &c->divvBound,  &c->intScratch, &c->scanTemp, &c->veTape,
                     &c->checkWord,  &c->whS64,      &c->whdS64,     &c->sortLook,   &c->sortState};
     for (DBuf* b : bufs) b->release();
@@ -203,7 +206,10 @@ int sphgb_set_pair_cache(sphgb_ctx* c, int32_t arrays)
 {
     SPHGB_TRY(useDevice(c));
     if (arrays != 0 && arrays != 2 && arrays != 5) return SPHGB_ERR_ARG;
-    if (arrays < c->geoLimit) c->dropPairGeo();
+    if (arrays < c->geoLimit) {
+        c->dropPairGeo();
+        c->dropPairRec();
+    }
     c->geoLimit = arrays;
     return SPHGB_OK;
 }

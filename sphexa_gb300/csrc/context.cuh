@@ -31,9 +31,10 @@ void setCudaError(cudaError_t e, const char* what);
     } while (0)
 
 struct DBuf;
-// frees the pair-geometry cache of the context that the calling thread is in, unless `wanted` is that buffer;
-// false when there is nothing to free
-bool reclaimPairGeo(const DBuf* wanted);
+// frees the pair-geometry cache and the pair records of the context that the calling thread is in, unless
+// `wanted` belongs to them; false when there is nothing to free.  A pass takes its other buffers before it looks
+// at either.
+bool reclaimPairMemory(const DBuf* wanted);
 
 // growable device buffer
 struct DBuf {
@@ -47,7 +48,7 @@ struct DBuf {
         bytes = 0;
         size_t alloc = need < 256 ? 256 : need;
         cudaError_t e = cudaMalloc(&p, alloc);
-        if (e == cudaErrorMemoryAllocation && reclaimPairGeo(this)) {
+        if (e == cudaErrorMemoryAllocation && reclaimPairMemory(this)) {
             (void)cudaGetLastError();
             e = cudaMalloc(&p, alloc);
         }
@@ -141,6 +142,16 @@ struct sphgb_ctx {
         geoArrays = 0;
         geoValid = geoChecked = false;
     }
+    void dropPairRec()
+    {
+        pairRec.release();
+        inbox.release();
+        inboxEpoch = -1;
+    }
+    // std passes: one 32-byte record per owned pair for its other end, and each particle's mutual pairs that
+    // others own, by owner (PairRec in pairs.cuh); inboxOff, inbox: of the owned lists of epoch inboxEpoch
+    sphgb::DBuf pairRec, inbox, inboxOff, inboxCount;
+    int64_t inboxEpoch = -1;
     // inside sphgb_sweep_passes the per-particle precomputes are built by the first pass only
     bool inSweep = false, sweepPrepared = false;
     int sortAllBits = 0;  // syncs left that sort keys over all bits at once (sortParticleKeys)

@@ -9,10 +9,10 @@
 //               momentum_energy.hpp:41-101)
 // FP64 form: per-particle quotients (m/rho, p/rho, p/rho^2, 1/h, 1/h^3) are formed once per
 // particle, 1/|r| comes from rsqrt, periodic wrap tests run only where they can fire; where the lists
-// cover every particle a mutual pair is evaluated once (owned lists, FP64 atomics; set_deterministic
-// selects the order-fixed walks), and inside a sweep IAD and momentum-energy read the pair geometry
-// that the density pass stored.  Results agree with the reference to rounding.  Mixed form: FP32 pair arithmetic on grid-local
-// offsets, Kahan sums, per-particle epilogues (normalisation, 3x3 inverse factor) in FP64.
+// cover every particle a mutual pair is evaluated once, its other end's share passing through a record that
+// is gathered in a fixed order (PairRec: the same bits in every run; set_deterministic selects the walks over
+// whole lists), and IAD and momentum-energy read the pair geometry that the density pass stored.  Results
+// agree with the reference to rounding.  Mixed form: FP32 pair arithmetic on grid-local offsets, Kahan sums, per-particle epilogues (normalisation, 3x3 inverse factor) in FP64.
 #include "pairs.cuh"
 
 namespace sphgb {
@@ -96,16 +96,19 @@ __global__ void __launch_bounds__(kPairBlock) xmassKernel(ListView lv, CoordFp64
 }
 
 // FP64 xmass / density with one evaluation per mutual pair over the owned lists: i adds
-// W(d / h_i) m_j, and for a mutual pair j receives W(d / h_j) m_i by an FP64 atomic.  Inside a
-// sweep it also fills the pair-geometry cache (geo) the later pair-once passes read.  Exact: acc + n holds
-// the rounding errors of the sums (exactSums).
-template<bool Smooth, bool Exact>
+// W(d / h_i) m_j, and for a mutual pair j receives W(d / h_j) m_i.  It also fills the pair-geometry cache
+// (geo) that the later pair-once passes read.  Mode: j's share by FP64 atomics, with the rounding errors of the
+// sums in acc + n (exactSums) or without (xmass), or by the pair's record (PairRec, std density).
+enum XmassMode { kXmassSum, kXmassExact, kXmassRecords };
+
+template<bool Smooth, XmassMode Mode>
 __global__ void __launch_bounds__(kPairBlock) xmassOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf,
                                                                const double* h, const double* m, KTab<Smooth> tab,
                                                                const double* hInvDx, double* acc, PairGeo geo,
                                                                const double* vx, const double* vy, const double* vz,
-                                                               int64_t n)
+                                                               int64_t n, PairRec pr)
 {
+    constexpr bool Exact = Mode == kXmassExact;
     const int64_t i = lv.first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (i >= lv.last) return;
     const int64_t ii = i - lv.first;
@@ -113,9 +116,13 @@ __global__ void __launch_bounds__(kPairBlock) xmassOnceKernel(ListView lv, Owned
     auto t = cf.target(i);
     const double hi = h[i], mi = m[i], twoH = 2.0 * hi, hiInvDx = hInvDx[i];
     const bool wrap = cf.needsWrap(t, twoH);
-    const int64_t gb = geo.base(ii);
+    const int64_t gb = geo.g ? geo.base(ii) : 0, rb = Mode == kXmassRecords ? pr.base(ii) : 0;
     const double vxi = geo.g ? vx[i] : 0.0, vyi = geo.g ? vy[i] : 0.0, vzi = geo.g ? vz[i] : 0.0;
     double rho0 = 0.0;
+    auto give = [&](uint32_t j, unsigned k, double v) {
+        if constexpr (Mode == kXmassRecords) reinterpret_cast<double*>(pr.rec)[rb + 32 * int64_t(k)] = v;
+        else sumAdd<Exact>(acc + j, acc + n + j, v);
+    };
     for (unsigned k = blockIdx.y; k < no; k += gridDim.y) {
         bool mutual;
         const uint32_t j = ov.at(ii, k, mutual);
@@ -138,12 +145,13 @@ __global__ void __launch_bounds__(kPairBlock) xmassOnceKernel(ListView lv, Owned
                 geo.x[geo.plane + e] = make_double2(rz, dvx);
                 geo.x[2 * geo.plane + e] = make_double2(dvy, dvz);
             }
-            if (mutual) sumAdd<Exact>(acc + j, acc + n + j, wj * mi);
+            if (mutual) give(j, k, wj * mi);
         } else if (mutual) {
-            sumAdd<Exact>(acc + j, acc + n + j, lookupX(tab, dist * __ldg(hInvDx + j)) * mi);
+            give(j, k, lookupX(tab, dist * __ldg(hInvDx + j)) * mi);
         }
     }
-    sumAdd<Exact>(acc + i, acc + n + i, rho0);
+    if constexpr (Mode == kXmassRecords) pr.part[blockIdx.y * n + i] = rho0;
+    else sumAdd<Exact>(acc + i, acc + n + i, rho0);
 }
 
 // snap: where it keeps the inputs of the cache (outside a sweep), or null
@@ -291,12 +299,13 @@ __global__ void __launch_bounds__(kPairBlock) iadKernel(ListView lv, CoordFp64 c
 }
 
 // FP64 IAD with one evaluation per mutual pair over the owned lists: i adds vol_j W_i r r^T, and a mutual
-// pair gives j vol_i W_j r r^T by FP64 atomics.  Geo: arrays of the pair-geometry cache (5, 2), or 0.
+// pair gives j vol_i W_j r r^T by its record (r and the factor).  Geo: arrays of the pair-geometry cache (5, 2),
+// or 0.
 template<bool Smooth, int Geo>
 __device__ __forceinline__ void iadStdOnceBody(ListView lv, OwnedView ov, CoordFp64 cf,
                                                                const double* h, const double* vol,
                                                                KTab<Smooth> tab, const double* hInv64, int64_t n,
-                                                               double* acc, PairGeo geo)
+                                                               PairRec pr, PairGeo geo)
 {
     const int64_t i = lv.first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (i >= lv.last) return;
@@ -315,6 +324,7 @@ __device__ __forceinline__ void iadStdOnceBody(ListView lv, OwnedView ov, CoordF
         wrap = cf.needsWrap(t, twoH);
         hiInvDx = hInvDx[i];
     }
+    const int64_t rb = pr.base(ii);
     double tau[6] = {0, 0, 0, 0, 0, 0};
     for (unsigned k = blockIdx.y; k < no; k += gridDim.y, g += 32 * gridDim.y) {
         bool mutual;
@@ -338,25 +348,21 @@ __device__ __forceinline__ void iadStdOnceBody(ListView lv, OwnedView ov, CoordF
         const double vw = __ldg(vol + j) * wv.x;
 #pragma unroll
         for (int q = 0; q < 6; ++q) tau[q] = fma(vw, s[q], tau[q]);
-        if (mutual) {
-            const double vwj = voli * wv.y;
-#pragma unroll
-            for (int q = 0; q < 6; ++q) atomicAdd(acc + q * n + j, vwj * s[q]);
-        }
+        if (mutual) pr.rec[rb + 32 * int64_t(k)] = {rx, ry, rz, voli * wv.y};
     }
 #pragma unroll
-    for (int q = 0; q < 6; ++q) atomicAdd(acc + q * n + i, tau[q]);
+    for (int q = 0; q < 6; ++q) pr.part[(blockIdx.y * int64_t(6) + q) * n + i] = tau[q];
 }
 
 template<bool Smooth, int Geo>
 __global__ void __launch_bounds__(kPairBlock) iadStdOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf,
                                                                const double* h, const double* vol,
                                                                KTab<Smooth> tab, const double* hInv64, int64_t n,
-                                                               double* acc, PairGeo geo)
+                                                               PairRec pr, PairGeo geo)
 {
-    if constexpr (Geo >= 0) iadStdOnceBody<Smooth, Geo>(lv, ov, cf, h, vol, tab, hInv64, n, acc, geo);
-    else if (*geo.stale) iadStdOnceBody<Smooth, 0>(lv, ov, cf, h, vol, tab, hInv64, n, acc, geo);
-    else iadStdOnceBody<Smooth, -Geo>(lv, ov, cf, h, vol, tab, hInv64, n, acc, geo);
+    if constexpr (Geo >= 0) iadStdOnceBody<Smooth, Geo>(lv, ov, cf, h, vol, tab, hInv64, n, pr, geo);
+    else if (*geo.stale) iadStdOnceBody<Smooth, 0>(lv, ov, cf, h, vol, tab, hInv64, n, pr, geo);
+    else iadStdOnceBody<Smooth, -Geo>(lv, ov, cf, h, vol, tab, hInv64, n, pr, geo);
 }
 
 __global__ void iadStdOnceFinish(int64_t n, const double* h, double K, const double* acc, IadOut o)
@@ -578,13 +584,15 @@ __global__ void meStdRec64Kernel(int64_t n, MeStdArgs a, Rec4d* __restrict__ rec
 // V_i = w_i (m_j q_i + t_i) A_i r + w_j (m_j q_j + t_j) A_j r, since m_j / rho_j (p_j / rho_j) = m_j q_j;
 // j's is -V_j with m_i in place of m_j (the same where the masses are equal).  Energy: 2 m_j q_i w_i s_i +
 // Q with s = v_ij . A r and Q = t_i w_i s_i + t_j w_j s_j; j's is 2 m_i q_j w_j s_j + Q.  Bound by the
-// FP64 pipe: 1M particles 15.3 ms with every directed pair evaluated, now 5.4 ms (IAD 5.7 -> 2.1,
-// density 3.5 -> 2.8, which also fills the geometry cache).
+// FP64 pipe: 1M particles 15.3 ms with every directed pair evaluated, now 5.3 ms and 0.6 for the gather of
+// the records (IAD 5.7 -> 1.3 + 0.9, density 3.5 -> 2.6 + 0.2, which also fills the geometry cache; the inbox
+// 1.2 ms once per neighbour search).  With atomics in place of the records the sweep took 12.5 ms, with them
+// 14.7, and its bits differed from run to run.
 // Geo: arrays of the pair-geometry cache (5, 2), or 0 to form the geometry here.
 template<bool Smooth, int Geo>
 __device__ __forceinline__ void meStdOnceBody(ListView lv, OwnedView ov, CoordFp64 cf, MeStdArgs a,
-                                                              const Rec4d* __restrict__ rec, double* __restrict__ acc,
-                                                              PairGeo geo)
+                                                              const Rec4d* __restrict__ rec, PairRec pr,
+                                              long long* __restrict__ accS, PairGeo geo)
 {
     using T = double;
     const int64_t i = lv.first + blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
@@ -610,7 +618,7 @@ __device__ __forceinline__ void meStdOnceBody(ListView lv, OwnedView ov, CoordFp
     }
     T mx = 0, my = 0, mz = 0, en = 0;
     long long maxvBits = 0;
-    long long* accS = reinterpret_cast<long long*>(acc + 4 * n);
+    const int64_t rb = pr.base(ii);
     for (unsigned k = blockIdx.y; k < no; k += gridDim.y, g += 32 * gridDim.y) {
         bool mutual;
         const uint32_t j = ov.at(ii, k, mutual);
@@ -637,16 +645,18 @@ __device__ __forceinline__ void meStdOnceBody(ListView lv, OwnedView ov, CoordFp
             wv.x = lookupX(tabX, dist * hiInvDx);
             wv.y = lookupX(tabX, dist * __ldg(hInvDx + j));
         }
-        const T gix = i0.v[0] * rx + i0.v[1] * ry + i0.v[2] * rz;
-        const T giy = i0.v[1] * rx + i0.v[3] * ry + i1.v[0] * rz;
-        const T giz = i0.v[2] * rx + i1.v[0] * ry + i1.v[1] * rz;
-        const T gjx = j0.v[0] * rx + j0.v[1] * ry + j0.v[2] * rz;
-        const T gjy = j0.v[1] * rx + j0.v[3] * ry + j1.v[0] * rz;
-        const T gjz = j0.v[2] * rx + j1.v[0] * ry + j1.v[1] * rz;
+        // sums of products written out: every form of the cache gives the same bits
+        const T gix = fma(i0.v[2], rz, fma(i0.v[1], ry, i0.v[0] * rx));
+        const T giy = fma(i1.v[0], rz, fma(i0.v[3], ry, i0.v[1] * rx));
+        const T giz = fma(i1.v[1], rz, fma(i1.v[0], ry, i0.v[2] * rx));
+        const T gjx = fma(j0.v[2], rz, fma(j0.v[1], ry, j0.v[0] * rx));
+        const T gjy = fma(j1.v[0], rz, fma(j0.v[3], ry, j0.v[1] * rx));
+        const T gjz = fma(j1.v[1], rz, fma(j1.v[0], ry, j0.v[2] * rx));
         const T cs = i1.v[2] + j1.v[2], mj = j1.v[3];
         const T vsig = fma(T(-3), wij, cs);
         maxvBits = maxBitsNonNeg(maxvBits, vsig);
-        const T wsi = wv.x * (vxij * gix + vyij * giy + vzij * giz), wsj = wv.y * (vxij * gjx + vyij * gjy + vzij * gjz);
+        const T wsi = wv.x * fma(vzij, giz, fma(vyij, giy, vxij * gix));
+        const T wsj = wv.y * fma(vzij, gjz, fma(vyij, gjy, vxij * gjx));
         T ti = 0, tj = 0, Q = 0;
         if (negative(wij)) {  // approaching: half of artificial_viscosity(1, 1, c_i, c_j, w_ij)
             const T visc = fma(T(0.25), cs, -wij) * -wij;
@@ -665,28 +675,26 @@ __device__ __forceinline__ void meStdOnceBody(ListView lv, OwnedView ov, CoordFp
                 Pi = wv.x * fma(mi, i2.v[0], ti), Pj = wv.y * fma(mi, j2.v[0], tj);
                 Vx = fma(Pi, gix, Pj * gjx), Vy = fma(Pi, giy, Pj * gjy), Vz = fma(Pi, giz, Pj * gjz);
             }
-            atomicAdd(acc + j, -Vx);
-            atomicAdd(acc + n + j, -Vy);
-            atomicAdd(acc + 2 * n + j, -Vz);
-            atomicAdd(acc + 3 * n + j, fma(mi * (2.0 * j2.v[0]), wsj, Q));
+            pr.rec[rb + 32 * int64_t(k)] = {-Vx, -Vy, -Vz, fma(mi * (2.0 * j2.v[0]), wsj, Q)};
             atomicMax(accS + j, __double_as_longlong(vsig));
         }
     }
-    atomicAdd(acc + i, mx);
-    atomicAdd(acc + n + i, my);
-    atomicAdd(acc + 2 * n + i, mz);
-    atomicAdd(acc + 3 * n + i, en);
+    double* part = pr.part + blockIdx.y * int64_t(4) * n + i;
+    part[0] = mx;
+    part[n] = my;
+    part[2 * n] = mz;
+    part[3 * n] = en;
     atomicMax(accS + i, maxvBits);
 }
 
 template<bool Smooth, int Geo>
 __global__ void __launch_bounds__(kPairBlock) meStdOnceKernel(ListView lv, OwnedView ov, CoordFp64 cf, MeStdArgs a,
-                                                              const Rec4d* __restrict__ rec, double* __restrict__ acc,
-                                                              PairGeo geo)
+                                                              const Rec4d* __restrict__ rec, PairRec pr,
+                                                              long long* __restrict__ accS, PairGeo geo)
 {
-    if constexpr (Geo >= 0) meStdOnceBody<Smooth, Geo>(lv, ov, cf, a, rec, acc, geo);
-    else if (*geo.stale) meStdOnceBody<Smooth, 0>(lv, ov, cf, a, rec, acc, geo);
-    else meStdOnceBody<Smooth, -Geo>(lv, ov, cf, a, rec, acc, geo);
+    if constexpr (Geo >= 0) meStdOnceBody<Smooth, Geo>(lv, ov, cf, a, rec, pr, accS, geo);
+    else if (*geo.stale) meStdOnceBody<Smooth, 0>(lv, ov, cf, a, rec, pr, accS, geo);
+    else meStdOnceBody<Smooth, -Geo>(lv, ov, cf, a, rec, pr, accS, geo);
 }
 
 __global__ void __launch_bounds__(kPairBlock) meStdOnceFinish(MeStdArgs a, const double* __restrict__ acc)
@@ -715,11 +723,21 @@ int launchXmass(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, v
     CoordMixed cm = coordMixed(c);
     const void* wh = std::is_same_v<P, Fp64Tag> ? c->whx64.p : c->whH32.p;
     unsigned blocks = gridFor(last - first, kPairBlock);
-    if (std::is_same_v<P, Fp64Tag> && pairOnce(c, p, first, last)) {
+    bool once = std::is_same_v<P, Fp64Tag> && pairOnce(c, p, first, last);
+    const bool exact = once && !storeRho && exactSums(p->n);
+    const int slices = int(ownedGrid(p->n).y);
+    PairRec pr{};
+    if (once) {  // sums, then their rounding errors or the own partial sums
+        const size_t doubles = size_t(storeRho ? 1 + slices : exact ? 2 : 1) * size_t(p->n);
+        SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * doubles));
+        if (storeRho) {
+            SPHGB_TRY(pairRecords(c, c->pairAcc.as<double>() + p->n, &pr));
+            once = pr.rec != nullptr;
+        } else
+            SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * doubles, c->stream));
+    }
+    if (once) {
         const int64_t n = p->n;
-        const bool exact = exactSums(n);
-        SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * (exact ? 2 : 1) * size_t(n)));
-        SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * (exact ? 2 : 1) * size_t(n), c->stream));
         const double* lo = exact ? c->pairAcc.as<double>() + n : nullptr;
         PairGeo geo{};
         SPHGB_TRY(pairGeoStore(c, p, &geo));
@@ -731,12 +749,14 @@ int launchXmass(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, v
                 lv, ownedView(c), cf, static_cast<const double*>(p->h), static_cast<const double*>(p->m),
                 KTab<S>{tabW64(c)}, c->hInv64.as<double>() + 2 * n, c->pairAcc.as<double>(), geo,
                 static_cast<const double*>(p->vx), static_cast<const double*>(p->vy),
-                static_cast<const double*>(p->vz), n);
+                static_cast<const double*>(p->vz), n, pr);
             };
-            if (exact) run(xmassOnceKernel<S, true>);
-            else run(xmassOnceKernel<S, false>);
+            if (storeRho) run(xmassOnceKernel<S, kXmassRecords>);
+            else if (exact) run(xmassOnceKernel<S, kXmassExact>);
+            else run(xmassOnceKernel<S, kXmassSum>);
             return launched(c, "xmassOnceKernel");
         }));
+        if (storeRho) SPHGB_TRY(gatherRecords(c, pr, n, 1, slices, c->pairAcc.as<double>()));
         const unsigned eb = gridFor(last - first, 256);
         if (storeRho)
             xmassOnceFinish<true><<<eb, 256, 0, c->stream>>>(first, last, static_cast<const double*>(p->h),
@@ -785,10 +805,14 @@ int launchIad(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last)
     lv.first = first;
     lv.last = last;
     const void* wh = std::is_same_v<P, Fp64Tag> ? c->whx64.p : c->whH32.p;
+    PairRec pr{};
+    const int slices = int(ownedGrid(p->n).y);
     if (std::is_same_v<P, Fp64Tag> && pairOnce(c, p, first, last)) {
+        SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * 6 * size_t(1 + slices) * size_t(p->n)));
+        SPHGB_TRY(pairRecords(c, c->pairAcc.as<double>() + 6 * p->n, &pr));
+    }
+    if (pr.rec) {
         const int64_t n = p->n;
-        SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * 6 * size_t(n)));
-        SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * 6 * size_t(n), c->stream));
         const PairGeo geo = pairGeoRead(c);
         const double* h = static_cast<const double*>(p->h);
         SPHGB_TRY(withKernelForm(c, [&](auto smooth) {
@@ -796,11 +820,12 @@ int launchIad(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last)
             auto run = [&](auto kernel) {
                 kernel<<<ownedGrid(n), kPairBlock, 0, c->stream>>>(
                     lv, ownedView(c), coordFp64(c, p), h, c->aux.as<double>(), KTab<S>{tabW64(c)},
-                    c->hInv64.as<double>(), n, c->pairAcc.as<double>(), geo);
+                    c->hInv64.as<double>(), n, pr, geo);
             };
             withPairGeo(geo, [&](auto g) { run(iadStdOnceKernel<S, decltype(g)::value>); });
             return launched(c, "iadStdOnceKernel");
         }));
+        SPHGB_TRY(gatherRecords(c, pr, n, 6, slices, c->pairAcc.as<double>()));
         iadStdOnceFinish<<<gridFor(n, 256), 256, 0, c->stream>>>(n, h, c->K, c->pairAcc.as<double>(),
                                                                  IadOut{p->c11, p->c12, p->c13, p->c22, p->c23, p->c33});
         return launched(c, "iadStdOnceFinish");
@@ -817,7 +842,17 @@ int launchIad(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last)
 template<class P>
 int launchMeStd(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, double* minDt)
 {
-    const bool once = std::is_same_v<P, Fp64Tag> && pairOnce(c, p, first, last);
+    unsigned long long* minDtWord = nullptr;
+    SPHGB_TRY(beginDtReduction(c, &minDtWord));
+    PairRec pr{};
+    const int slices = int(ownedGrid(p->n).y);
+    if (std::is_same_v<P, Fp64Tag> && pairOnce(c, p, first, last)) {
+        const size_t n = size_t(p->n);  // four sums and the signal velocity, then the own partial sums
+        SPHGB_TRY(c->pack.ensure(sizeof(Rec4d) * 3 * n));
+        SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * (5 + 4 * size_t(slices)) * n));
+        SPHGB_TRY(pairRecords(c, c->pairAcc.as<double>() + 5 * n, &pr));
+    }
+    const bool once = pr.rec != nullptr;
     if (std::is_same_v<P, Fp64Tag> && !once) SPHGB_TRY(launchStdAux<P>(c, p, true));
     if (std::is_same_v<P, MixedTag>) SPHGB_TRY(c->aux.ensure(sizeof(float) * 3 * size_t(p->n)));
     ListView lv = listView(c);
@@ -849,12 +884,11 @@ int launchMeStd(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, d
     a.ay = p->ay;
     a.az = p->az;
     a.du = p->du;
-    SPHGB_TRY(beginDtReduction(c, &a.minDt));
+    a.minDt = minDtWord;
     if (once) {
         const int64_t n = p->n;
-        SPHGB_TRY(c->pairAcc.ensure(sizeof(double) * 5 * size_t(n)));
-        SPHGB_CUDA(cudaMemsetAsync(c->pairAcc.p, 0, sizeof(double) * 5 * size_t(n), c->stream));
-        SPHGB_TRY(c->pack.ensure(sizeof(Rec4d) * 3 * size_t(n)));
+        long long* accS = c->pairAcc.as<long long>() + 4 * n;
+        SPHGB_CUDA(cudaMemsetAsync(accS, 0, sizeof(long long) * size_t(n), c->stream));
         meStdRec64Kernel<<<gridFor(n, 256), 256, 0, c->stream>>>(n, a, c->pack.as<Rec4d>());
         SPHGB_TRY(launched(c, "meStdRec64Kernel"));
         const PairGeo geo = pairGeoRead(c);
@@ -863,11 +897,12 @@ int launchMeStd(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, d
             constexpr bool S = decltype(smooth)::value;
             auto run = [&](auto kernel) {
                 kernel<<<ownedGrid(n), kPairBlock, 0, c->stream>>>(lv, ownedView(c), coordFp64(c, p), a, c->pack.as<Rec4d>(),
-                                                             c->pairAcc.as<double>(), geo);
+                                                             pr, accS, geo);
             };
             withPairGeo(geo, [&](auto g) { run(meStdOnceKernel<S, decltype(g)::value>); });
             return launched(c, "meStdOnceKernel");
         }));
+        SPHGB_TRY(gatherRecords(c, pr, n, 4, slices, c->pairAcc.as<double>()));
         meStdOnceFinish<<<blocks, kPairBlock, 0, c->stream>>>(a, c->pairAcc.as<double>());
         SPHGB_TRY(launched(c, "meStdOnceFinish"));
         return endDtReduction(c, a.minDt, minDt);

@@ -861,6 +861,131 @@ __global__ void __launch_bounds__(128) ownedByListKernel(const uint32_t* __restr
     ownedCount[ii] = cnt;
 }
 
+// ---- records of the std passes (PairRec) ----
+// how many mutual pairs of each particle others own
+__global__ void __launch_bounds__(128) inboxCountKernel(OwnedView ov, int64_t n, uint32_t* __restrict__ count)
+{
+    const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (i >= n) return;
+    const unsigned no = ov.size(i);
+    for (unsigned k = 0; k < no; ++k) {
+        bool mutual;
+        const uint32_t j = ov.at(i, k, mutual);
+        if (mutual) atomicAdd(count + j, 1u);
+    }
+}
+
+// owner and record index of each of them, in any order (count runs down to 0)
+__global__ void __launch_bounds__(128) inboxFillKernel(OwnedView ov, const uint32_t* __restrict__ rowOff, int64_t n,
+                                                       const uint32_t* __restrict__ off, uint32_t* __restrict__ count,
+                                                       uint2* __restrict__ entries)
+{
+    const int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (i >= n) return;
+    const unsigned no = ov.size(i);
+    const uint32_t base = 32u * __ldg(rowOff + (i >> 5)) + unsigned(i & 31);
+    for (unsigned k = 0; k < no; ++k) {
+        bool mutual;
+        const uint32_t j = ov.at(i, k, mutual);
+        if (mutual) entries[__ldg(off + j) + atomicSub(count + j, 1u) - 1u] = make_uint2(uint32_t(i), base + 32u * k);
+    }
+}
+
+// the record indices by owner: one warp per particle, each entry's place is the number of smaller owners
+__global__ void __launch_bounds__(128) inboxOrderKernel(int64_t n, const uint32_t* __restrict__ off,
+                                                        const uint2* __restrict__ entries, uint32_t* __restrict__ inbox)
+{
+    const int64_t j = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) / kWarp;
+    if (j >= n) return;
+    const unsigned lane = threadIdx.x % kWarp;
+    const uint32_t o = off[j], m = off[j + 1] - o;
+    if (m <= 2 * kWarp) {
+        const uint2 none = make_uint2(0xffffffffu, 0u);
+        const uint2 e0 = lane < m ? entries[o + lane] : none, e1 = lane + kWarp < m ? entries[o + lane + kWarp] : none;
+        uint32_t b0 = 0, b1 = 0;
+        const int m0 = int(min(m, uint32_t(kWarp))), m1 = int(m) - m0;
+#pragma unroll 4
+        for (int s = 0; s < m0; ++s) {
+            const uint32_t q = __shfl_sync(0xffffffffu, e0.x, s);
+            b0 += q < e0.x;
+            b1 += q < e1.x;
+        }
+#pragma unroll 4
+        for (int s = 0; s < m1; ++s) {
+            const uint32_t q = __shfl_sync(0xffffffffu, e1.x, s);
+            b0 += q < e0.x;
+            b1 += q < e1.x;
+        }
+        if (lane < m) inbox[o + b0] = e0.y;
+        if (lane + kWarp < m) inbox[o + b1] = e1.y;
+        return;
+    }
+    for (uint32_t a0 = 0; a0 < m; a0 += kWarp) {
+        const bool valid = a0 + lane < m;
+        const uint2 e = valid ? entries[o + a0 + lane] : make_uint2(0u, 0u);
+        uint32_t before = 0;
+        for (uint32_t b0 = 0; b0 < m; b0 += kWarp) {
+            const uint32_t other = b0 + lane < m ? entries[o + b0 + lane].x : 0xffffffffu;
+            const int cnt = int(min(uint32_t(kWarp), m - b0));
+            for (int s = 0; s < cnt; ++s) before += __shfl_sync(0xffffffffu, other, s) < e.x;
+        }
+        if (valid) inbox[o + before] = e.y;
+    }
+}
+
+// Lanes lanes per particle share its records (g, g + Lanes, ...), their sums combined by shuffles; the lanes then
+// add the own partial sums of one sum each.  Reads about 48 records per particle from anywhere: 32 bytes
+// each, one sector.  Eight lanes in small sets, whose lists are serial chains; in large ones the adds of the shuffles
+// cost more than the chains (1M particles: six sums 1.35 ms with eight lanes, 0.94 with two; four sums 0.75, and
+// 0.56 with four).
+template<int Sums, int Lanes>
+__global__ void __launch_bounds__(256) gatherKernel(PairRec pr, int64_t n, const uint32_t* __restrict__ off,
+                                                    const uint32_t* __restrict__ inbox, int slices,
+                                                    double* __restrict__ acc)
+{
+    const int64_t t = (blockIdx.x * int64_t(blockDim.x) + threadIdx.x) / Lanes;
+    const unsigned g = threadIdx.x % Lanes;
+    const bool valid = t < n;
+    const int64_t j = valid ? t : 0;
+    const uint32_t to = valid ? off[j + 1] : 0u;
+    double s[Sums];
+#pragma unroll
+    for (int q = 0; q < Sums; ++q) s[q] = 0.0;
+#pragma unroll 2
+    for (uint32_t k = (valid ? off[j] : 0u) + g; k < to; k += Lanes) {
+        const uint32_t e = __ldg(inbox + k);
+        if constexpr (Sums == 1) {
+            s[0] += __ldg(reinterpret_cast<const double*>(pr.rec) + e);
+        } else {
+            const Rec4d r = ldRec4d(pr.rec + e);
+            if constexpr (Sums == 4) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q) s[q] += r.v[q];
+            } else {
+                const double x = r.v[0], y = r.v[1], z = r.v[2], fx = r.v[3] * x, fy = r.v[3] * y, fz = r.v[3] * z;
+                s[0] = fma(fx, x, s[0]);
+                s[1] = fma(fx, y, s[1]);
+                s[2] = fma(fx, z, s[2]);
+                s[3] = fma(fy, y, s[3]);
+                s[4] = fma(fy, z, s[4]);
+                s[5] = fma(fz, z, s[5]);
+            }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < Sums; ++q)
+#pragma unroll
+        for (int o = Lanes / 2; o > 0; o >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+    if (!valid) return;
+#pragma unroll
+    for (int q = 0; q < Sums; ++q)
+        if (g == unsigned(q % Lanes)) {
+            double v = 0.0;
+            for (int l = 0; l < slices; ++l) v += pr.part[(int64_t(l) * Sums + q) * n + j];
+            acc[int64_t(q) * n + j] = v + s[q];
+        }
+}
+
 __global__ void fillOnes(uint32_t* p, int64_t n)
 {
     int64_t k = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
@@ -989,7 +1114,10 @@ int prepareLists(sphgb_ctx* c, const double* x, const double* y, const double* z
     c->nbrStride = (nWork + 31) / 32 * 32;
     // lists larger than the buffers hold: the pair-geometry cache of an earlier sweep gives its
     // memory back first (the next FP64 sweep sizes it again within half of the free memory)
-    if (c->nbr.bytes < sizeof(uint32_t) * listCapacity(ngmax) * c->nbrStride) c->dropPairGeo();
+    if (c->nbr.bytes < sizeof(uint32_t) * listCapacity(ngmax) * c->nbrStride) {
+        c->dropPairGeo();
+        c->dropPairRec();
+    }
     SPHGB_TRY(c->nbr.ensure(sizeof(uint32_t) * listCapacity(ngmax) * c->nbrStride));
     SPHGB_TRY(c->ncount.ensure(sizeof(uint32_t) * c->nbrStride));
     SPHGB_TRY(c->active.ensure(sizeof(uint32_t) * c->nbrStride + c->nbrStride));
@@ -1083,6 +1211,59 @@ int pairGeoStore(sphgb_ctx* c, const sphgb_particles* p, PairGeo* out)
     }
     *out = pairGeoView(c, nullptr);
     return SPHGB_OK;
+}
+
+int pairRecords(sphgb_ctx* c, double* part, PairRec* out)
+{
+    *out = PairRec{};
+    const size_t rows = c->geoRowCount, slots = 32 * rows;
+    const int64_t n = c->nbrLast - c->nbrFirst;
+    if (rows == 0 || rows >= (size_t(1) << 27)) return SPHGB_OK;
+    if (c->inboxEpoch != c->nbrEpoch) {
+        SPHGB_TRY(c->inboxCount.ensure(sizeof(uint32_t) * size_t(n + 1)));
+        SPHGB_TRY(c->inboxOff.ensure(sizeof(uint32_t) * size_t(n + 1)));
+        uint32_t *count = c->inboxCount.as<uint32_t>(), *off = c->inboxOff.as<uint32_t>();
+        SPHGB_CUDA(cudaMemsetAsync(count, 0, sizeof(uint32_t) * size_t(n + 1), c->stream));
+        const OwnedView ov = ownedView(c);
+        inboxCountKernel<<<gridFor(n, 128), 128, 0, c->stream>>>(ov, n, count);
+        SPHGB_TRY(launched(c, "inboxCountKernel"));
+        SPHGB_TRY(exclusiveScan(c, count, off, n + 1));
+        // the space after everything that may take it back; 3 % more than asked for, as for the cache
+        if (c->pairRec.bytes < sizeof(Rec4d) * slots || c->inbox.bytes < sizeof(uint32_t) * slots) {
+            const size_t padded = slots + slots / 32, need = (sizeof(Rec4d) + sizeof(uint32_t)) * padded;
+            size_t freeB = 0, totalB = 0;
+            if (cudaMemGetInfo(&freeB, &totalB) != cudaSuccess ||
+                need > (freeB + c->pairRec.bytes + c->inbox.bytes) / (c->inSweep ? 2 : 8) ||
+                c->pairRec.ensure(sizeof(Rec4d) * padded) != SPHGB_OK ||
+                c->inbox.ensure(sizeof(uint32_t) * padded) != SPHGB_OK) {
+                (void)cudaGetLastError();
+                c->dropPairRec();
+                return SPHGB_OK;
+            }
+        }
+        inboxFillKernel<<<gridFor(n, 128), 128, 0, c->stream>>>(ov, c->geoRows.as<uint32_t>(), n, off, count,
+                                                                c->pairRec.as<uint2>());
+        SPHGB_TRY(launched(c, "inboxFillKernel"));
+        inboxOrderKernel<<<gridFor(n * kWarp, 128), 128, 0, c->stream>>>(n, off, c->pairRec.as<uint2>(),
+                                                                         c->inbox.as<uint32_t>());
+        SPHGB_TRY(launched(c, "inboxOrderKernel"));
+        c->inboxEpoch = c->nbrEpoch;
+    }
+    *out = PairRec{c->geoRows.as<uint32_t>(), c->pairRec.as<Rec4d>(), part};
+    return SPHGB_OK;
+}
+
+int gatherRecords(sphgb_ctx* c, const PairRec& pr, int64_t n, int sums, int slices, double* acc)
+{
+    const uint32_t *off = c->inboxOff.as<uint32_t>(), *inbox = c->inbox.as<uint32_t>();
+    auto run = [&](auto kernel, int lanes) {
+        kernel<<<gridFor(n * lanes, 256), 256, 0, c->stream>>>(pr, n, off, inbox, slices, acc);
+    };
+    const bool small = slices > 1;
+    if (sums == 1) small ? run(gatherKernel<1, 8>, 8) : run(gatherKernel<1, 4>, 4);
+    else if (sums == 4) small ? run(gatherKernel<4, 8>, 8) : run(gatherKernel<4, 4>, 4);
+    else small ? run(gatherKernel<6, 8>, 8) : run(gatherKernel<6, 2>, 2);
+    return launched(c, "gatherKernel");
 }
 
 int buildOwnedFromLists(sphgb_ctx* c)

@@ -100,7 +100,8 @@ inline ListView listView(const sphgb_ctx* c)
 // ---- owned lists: the pairs particle i evaluates in the pair-once FP64 passes ----
 // entry k < count[i - first] of i's owned list (granule layout) = j | mutual << 31: every pair of i's list
 // that j does not list back, and half of the mutual pairs (the other half sits in the owned lists
-// of the other ends).  A mutual pair's evaluation also produces j's terms, added with FP64 atomics.
+// of the other ends).  A mutual pair's evaluation also produces j's terms, added with FP64 atomics (VE)
+// or from a record (std, PairRec).
 struct OwnedView {
     const uint32_t* owned;
     const uint32_t* count;
@@ -116,7 +117,8 @@ struct OwnedView {
 
 // Grid of a pass over owned lists.  Small sets do not fill the chip with one thread per particle, and a
 // thread's list is a serial chain, so the lists are cut into up to 16 interleaved slices (blockIdx.y
-// walks entries y, y + S, ...; every slice adds its sums to the accumulators with the same atomics).
+// walks entries y, y + S, ...; every slice adds its sums to the accumulators with the same atomics, or keeps
+// them as partial sums, PairRec).
 // Slices are added until about four waves of warps are in flight (152 SMs x 16 resident warps each);
 // from 311k particles on there is one.
 inline dim3 ownedGrid(int64_t n)
@@ -166,6 +168,32 @@ inline bool pairOnce(const sphgb_ctx* c, const sphgb_particles* p, int64_t first
            last == p->n && c->nbrFirst == 0 && c->nbrLast == p->n;
 }
 
+// ---- reproducible sums of the std passes ----
+// The VE passes add a mutual pair's share of its other end with FP64 atomics, in any order.  The std passes
+// evaluate a mutual pair once as well, but their sums do not depend on the order of execution: the owner writes
+// the other end's share to the pair's record, and a gather adds each particle's records in the order of
+// their owners (inbox), after the partial sums of its own pairs, slice by slice.
+// The records lie in the rows of the pair-geometry cache's layout (PairGeo), so a warp writes whole lines.
+struct Rec4d;
+struct PairRec {
+    const uint32_t* rowOff;  // first row of each warp of 32 owners
+    Rec4d* rec;              // the density's records are single doubles in the same space
+    double* part;            // own sums: [slice][sum][particle]
+    __device__ __forceinline__ int64_t base(int64_t ii) const
+    {
+        return 32 * int64_t(__ldg(rowOff + (ii >> 5))) + (ii & 31);
+    }
+};
+
+// records and inbox of the current owned lists; null rec where the memory is not there (32 + 4 bytes per owned
+// pair within the cache's share of the free memory) or an index leaves 32 bits: the passes then walk whole
+// lists.  Called after a pass's other allocations, one of which may have taken the space.
+int pairRecords(sphgb_ctx* c, double* part, PairRec* out);
+
+// adds the `sums` own partial sums of `slices` slices and the records into acc[sum][particle]; sums: 1 (density),
+// 6 (IAD: records r, f stand for f r r^T) or 4 (momentum-energy)
+int gatherRecords(sphgb_ctx* c, const PairRec& pr, int64_t n, int sums, int slices, double* acc);
+
 // ---- pair geometry shared by the pair-once passes of one sweep ----
 // Inside one sweep positions, velocities and h stay put, so an owned entry's |r| (the FP64 difference,
 // its square and the reciprocal square root: about a dozen FP64-pipe instructions), the approach
@@ -173,9 +201,9 @@ inline bool pairOnce(const sphgb_ctx* c, const sphgb_particles* p, int64_t first
 // where the memory is there, the difference vector r = x_i - x_j and the velocity difference dv =
 // v_j - v_i are formed once by the xmass or density pass and loaded by the passes after it.  Outside a
 // sweep the caller may change the inputs between passes; there every pass compares them with a copy
-// (recipKernel) and its kernel takes the cache or forms the geometry by the outcome (stale).  Layout: the 32 targets of a warp own
-// rows rowOff[w] .. rowOff[w] + (their longest owned list) - 1, a row holding entry k of all 32 side
-// by side, so a warp reads 512 contiguous bytes per entry and array.
+// (recipKernel) and its kernel takes the cache or forms the geometry by the outcome (stale).  Layout: the
+// 32 targets of a warp own rows rowOff[w] .. rowOff[w] + (their longest owned list) - 1, a row holding entry
+// k of all 32 side by side, so a warp reads 512 contiguous bytes per entry and array.
 struct PairGeo {
     const uint32_t* rowOff;  // first row of each warp of 32 targets
     double2* g;              // {|r|, w_ij}; null: the pass forms the geometry itself

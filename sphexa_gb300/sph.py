@@ -76,9 +76,9 @@ class Context:
         check(self.lib.sphgb_set_params(self.h, C.byref(self.params)), "sphgb_set_params")
 
     def set_deterministic(self, on: bool) -> None:
-        """True: every pass sums in list order (bitwise reproducible); False (default): the FP64
-        passes (VE: xmass, gradh, IAD + divv/curlv, AV, momentum-energy; std: density, IAD,
-        momentum-energy) evaluate mutual pairs once and scatter with FP64 atomics."""
+        """True: every pass sums in list order (bitwise reproducible); False (default): the FP64 passes
+        evaluate mutual pairs once, the VE passes (xmass, gradh, IAD + divv/curlv, AV, momentum-energy)
+        with FP64 atomics, the std passes (density, IAD, momentum-energy) in a fixed order."""
         check(self.lib.sphgb_set_deterministic(self.h, int(bool(on))), "sphgb_set_deterministic")
 
     def set_pair_cache(self, arrays: int) -> None:
