@@ -588,6 +588,34 @@ __device__ __forceinline__ Rec4d ldRec4d(const Rec4d* p)
     return r;
 }
 
+// num / den by a 20-bit reciprocal and two Newton corrections of the quotient (five FP64 instructions,
+// within an ulp); den beyond 2^+-1000 takes the division
+__device__ __forceinline__ double quotient(double num, double den)
+{
+    const unsigned e = (unsigned(__double2hiint(den)) >> 20) & 0x7ffu;
+    if (e - 23u > 2000u) return num / den;
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(den));
+    double q = num * y;
+    q = fma(fma(-den, q, num), y, q);
+    return fma(fma(-den, q, num), y, q);
+}
+
+// e^-x for x >= 0: below 16 from e^-n, n = round(x), and the table of e^(k/1024) (x reaches 16 only with
+// a handful of neighbours)
+__device__ __forceinline__ double expNegSmall(double x, const double4* __restrict__ expTab)
+{
+    if (!(x < 16.0)) return exp(-x);
+    const int n = __float2int_rn(float(x));
+    const double4 en = expTab[2 * kExpNodes + 1 + n];  // e^-n, -, n
+    const double a = en.z - x;                         // |a| <= 1/2
+    const int k = __float2int_rn(float(a) * 1024.f);
+    const double4 e = expTab[kExpNodes + k];
+    const double r = a - e.z, r2 = r * r;
+    const double y = fma(r2, fma(r2, 1.0 / 24.0, fma(r, 1.0 / 6.0, 0.5)), r);
+    return en.x * fma(e.x, y, e.x);
+}
+
 // Atwood weights a_mom, b_mom of a pair (momentum_energy_kern.hpp:160-190) in FP64: the exact decision
 // of |rho_i - rho_j| / (rho_i + rho_j) against 0.1 and 0.2 and, between them, the ramp
 // xm_i^(2-s) xm_j^s = xm_i^2 q and xm_j^(2-s) xm_i^s = xm_j^2 / q, q = (xm_j / xm_i)^s.  For the pairs
