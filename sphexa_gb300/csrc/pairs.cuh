@@ -128,7 +128,7 @@ inline dim3 ownedGrid(int64_t n)
     return dim3(unsigned((n + kPairBlock - 1) / kPairBlock), unsigned(s < 1 ? 1 : s > 16 ? 16 : s));
 }
 
-// Sets in the most slices keep the rounding errors of the density-like sums (xmass, gradh) as well: their
+// Sets in the most slices (up to 648 warps, 20,736 particles) keep the rounding errors of the density-like sums (xmass, gradh) as well: their
 // atomics arrive in another order in every run, and where gradh is near 0 (2e-3 in an open set of 3000
 // particles) plain sums let the acceleration differ by 1e-13 from run to run.  Larger sets, where each
 // sum would pay for it on the FP64 pipe, do without.
@@ -137,8 +137,9 @@ inline bool exactSums(int64_t n)
     return ownedGrid(n).y >= 16;
 }
 
-// *hi += v with the rounding error of that addition (two-sum) added to *lo: hi + lo is the sum of all
-// v to twice the precision, whatever their order
+// *hi += v with the rounding error of that addition (two-sum) added to *lo: hi + lo is the sum of all v to about
+// 1e-32 of it in any order (lo is rounded too), so the rounded sum depends on the order only where it lies that
+// close to the middle of two numbers
 __device__ __forceinline__ void atomicAddExact(double* hi, double* lo, double v)
 {
     const double old = atomicAdd(hi, v);
