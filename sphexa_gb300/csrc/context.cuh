@@ -158,7 +158,7 @@ struct sphgb_ctx {
     // within one sweep: the EOS ran in the gradh epilogue / the per-particle quotients are formed
     bool eosFused = false, auxReady = false;
     // packed neighbour-side records of the mixed pair passes and of the pair-once momentum-energy pass
-    // (96 bytes per particle), and that pass's FP32 copy of rho
+    // (96 bytes per particle, 160 with viscosity cleaning), and that pass's FP32 copy of rho
     sphgb::DBuf pack, rhof;
     // forward tape of the VE adjoint: with tapeOn the FP64 VE passes over all particles keep the
     // per-particle sums the adjoint needs (kTape* sections x n doubles); tapeMask tells which passes

@@ -188,28 +188,26 @@ __global__ void eosStdKernel(int64_t first, int64_t last, const double* u, const
 
 // ---------------------------------------------------------------- per-particle quotients
 // aux[0,n) m/rho, [n,2n) p/rho, [2n,3n) p/rho^2
-template<class T>
-__global__ void stdAuxKernel(int64_t n, const void* m, const void* rho, const void* p, T* aux)
+// (FP64; the mixed passes have them in their records)
+__global__ void stdAuxKernel(int64_t n, const void* m, const void* rho, const void* p, double* aux)
 {
     int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (i >= n) return;
-    T ri = ld<T>(rho, i);
-    aux[i] = ld<T>(m, i) / ri;
+    const double ri = ld<double>(rho, i);
+    aux[i] = ld<double>(m, i) / ri;
     if (p) {
-        T pi = ld<T>(p, i);
-        aux[n + i] = pi / (ri * T(1));
-        aux[2 * n + i] = pi / (T(1) * ri * ri);
+        const double pi = ld<double>(p, i);
+        aux[n + i] = pi / ri;
+        aux[2 * n + i] = pi / (ri * ri);
     }
 }
 
-template<class P>
 int launchStdAux(sphgb_ctx* c, const sphgb_particles* p, bool withPressure)
 {
-    using T = typename P::T;
     const int64_t n = p->n;
-    SPHGB_TRY(c->aux.ensure(sizeof(T) * 3 * n));
-    stdAuxKernel<T><<<gridFor(n, 256), 256, 0, c->stream>>>(n, p->m, p->rho, withPressure ? p->p : nullptr,
-                                                            c->aux.as<T>());
+    SPHGB_TRY(c->aux.ensure(sizeof(double) * 3 * n));
+    stdAuxKernel<<<gridFor(n, 256), 256, 0, c->stream>>>(n, p->m, p->rho, withPressure ? p->p : nullptr,
+                                                         c->aux.as<double>());
     return launched(c, "stdAuxKernel");
 }
 
@@ -398,7 +396,7 @@ struct MeStdArgs {
 
 // neighbour-side fields of the mixed momentum-energy pass as three 32-byte blocks per particle, each read
 // by one 256-bit load: {cell (2 words) xl yl zl 1/h vx vy} {vz c c11 c12 c13 c22 c23 c33} {m m/rho p/rho};
-// aux (m/rho, p/rho, p/rho^2) is filled for the targets.  Fifteen gathers per pair before: 298k particles
+// aux (m/rho at 0, p/rho^2 at 2 n) is filled for the targets.  Fifteen gathers per pair before: 298k particles
 // 0.42 -> 0.35 ms, and IAD, with one block, 0.17 -> 0.14.
 __global__ void meStdPackKernel(int64_t n, MeStdArgs a, const u64* __restrict__ cell, const float4* __restrict__ loc,
                                 float* __restrict__ aux, float4* __restrict__ pack)
@@ -408,7 +406,6 @@ __global__ void meStdPackKernel(int64_t n, MeStdArgs a, const u64* __restrict__ 
     const float rho = ld<float>(a.rho, j), m = ld<float>(a.m, j), p = ld<float>(a.p, j);
     const float moR = m / rho, poR = p / (rho * 1.f);
     aux[j] = moR;
-    aux[n + j] = poR;
     aux[2 * n + j] = p / (1.f * rho * rho);
     const u64 cj = cell[j];
     const float4 l = loc[j];
@@ -417,8 +414,7 @@ __global__ void meStdPackKernel(int64_t n, MeStdArgs a, const u64* __restrict__ 
     q[1] = make_float4(l.z, l.w, ld<float>(a.vx, j), ld<float>(a.vy, j));
     q[2] = make_float4(ld<float>(a.vz, j), ld<float>(a.c, j), ld<float>(a.c11, j), ld<float>(a.c12, j));
     q[3] = make_float4(ld<float>(a.c13, j), ld<float>(a.c22, j), ld<float>(a.c23, j), ld<float>(a.c33, j));
-    q[4] = make_float4(m, moR, poR, 0.f);
-    q[5] = make_float4(0.f, 0.f, 0.f, 0.f);
+    q[4] = make_float4(m, moR, poR, 0.f);  // the block's second half is not read
 }
 
 template<class P, bool Smooth = false>
@@ -800,7 +796,7 @@ int launchIad(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last)
                                                                     c->gridLoc.as<float4>(), c->pack.as<float4>());
         SPHGB_TRY(launched(c, "packIadStdKernel"));
         rec = c->pack.as<Rec8>();
-    } else SPHGB_TRY(launchStdAux<P>(c, p, false));
+    } else SPHGB_TRY(launchStdAux(c, p, false));
     ListView lv = listView(c);
     lv.first = first;
     lv.last = last;
@@ -853,7 +849,7 @@ int launchMeStd(sphgb_ctx* c, sphgb_particles* p, int64_t first, int64_t last, d
         SPHGB_TRY(pairRecords(c, c->pairAcc.as<double>() + 5 * n, &pr));
     }
     const bool once = pr.rec != nullptr;
-    if (std::is_same_v<P, Fp64Tag> && !once) SPHGB_TRY(launchStdAux<P>(c, p, true));
+    if (std::is_same_v<P, Fp64Tag> && !once) SPHGB_TRY(launchStdAux(c, p, true));
     if (std::is_same_v<P, MixedTag>) SPHGB_TRY(c->aux.ensure(sizeof(float) * 3 * size_t(p->n)));
     ListView lv = listView(c);
     lv.first = first;

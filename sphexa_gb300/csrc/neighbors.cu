@@ -51,11 +51,8 @@ struct NbrArgs {
     int64_t first, last;
     const uint32_t* active;  // optional: only targets with active[i - first] != 0 are searched
     const int32_t* childOffsets;
-    const int32_t* internalToLeaf;
-    const uint32_t* layout;
     const float4* nodeBox;
     const uint2* nodeRange;  // particles [start, end) per node
-    int64_t numNodes;
     float pruneUnit;         // power of two: the unit of the squared distances that prune nodes
     DevBox box;
     uint32_t ngmax;
@@ -1040,11 +1037,8 @@ int runSearch(sphgb_ctx* c, const double* x, const double* y, const double* z, c
     a.last = last;
     a.active = active;
     a.childOffsets = c->childOffsets.as<int32_t>();
-    a.internalToLeaf = c->internalToLeaf.as<int32_t>();
-    a.layout = c->layout.as<uint32_t>();
     a.nodeBox = c->nodeBoxF.as<float4>();
     a.nodeRange = c->nodeRange.as<uint2>();
-    a.numNodes = c->numNodes;
     a.box = c->box;
     a.ngmax = ngmax;
     a.stride = c->nbrStride;
