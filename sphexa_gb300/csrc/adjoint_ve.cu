@@ -563,7 +563,7 @@ struct OwnGeom {
 // bound by the FP64 pipe.  With s = m_j abar_i - m_i abar_j both ends' Abar are multiples of s, so with
 // e = C s per end every projection follows from z = r . e, the position partial from e, and both C
 // partials from one symmetric s r^T; K h^-3 and K h^-4 come per particle, table slopes stay in table
-// units, the ramp's exp and quotient as in the forward pass.  About 185 FP64 instructions per pair
+// units, the ramp's exp and quotient as in the forward pass.  About 218 FP64 instructions per warp step
 // against 379 (1M particles: 40.2 -> 20.9 ms).
 template<bool Smooth>
 __global__ void __launch_bounds__(kVeAdjBlock) meVeAdjOnceAKernel(VeAdjArgs a, OwnedView ov)

@@ -13,8 +13,9 @@
 // xm_j/kx_j, m_j*prho_j) are formed once per particle; 1/|r| comes from rsqrt and serves both
 // |r| and rv/|r|; the Atwood-number branches are decided by comparison, and the ramp's four
 // pow() calls become one exp() of the precomputed ln xm difference; the periodic wrap tests run
-// only for targets whose 2h box touches a periodic face; inside a sweep the pair-once passes read
-// r, v_j - v_i, |r|, w_ij and both kernel values from the cache the xmass pass fills (PairGeo).
+// only for targets whose 2h box touches a periodic face; the pair-once passes read r, v_j - v_i, |r|,
+// w_ij and both kernel values from the cache that the xmass pass fills (PairGeo), outside a sweep where
+// the inputs are still those of the fill.
 // Results agree with the reference to rounding (<= 1e-12 relative).  The mixed form runs the same
 // loops in FP32 on grid-local offsets with Kahan sums.
 #include "pairs.cuh"
@@ -1315,13 +1316,15 @@ __device__ __forceinline__ double2 avRvShared(double d1, double d2, double dist)
 // integer maximum of non-negative bit patterns).
 //
 // Bound by the FP64 pipe (2 lanes per cycle and SM), so the pair terms are arranged for few FP64
-// instructions: 50 per mutual pair, 21 more on the Atwood ramp (atwoodWeights).  The sums are forces: with A = m h^-3 c at each end (per particle),
-// w_i' = m_j w_i and w_j' = m_i w_j (m in the unit of massUnit), hv = visc / 2, t = hv / rho, P_i = w_i' (prho_i am + t_i) and
-// P_j = w_j' (prho_j bm + t_j), both ends add the same V = P_i A_i r + P_j A_j r, with opposite signs,
-// and the same Q = t_i w_i' s_i + t_j w_j' s_j (s = v_ij . A r); the finishing kernel divides by the
-// particle's mass.  vsig is kept doubled, alpha divided by 8 (both exact).  With the per-pair exp and
-// divisions of the ramp and the terms factored by m_j and m_i the kernel ran 109 FP64 instructions per
-// pair: 89.8 ms at 8M (jittered Sedov), now 78 and 62.1 ms, the FP64 pipe 87 % busy.
+// instructions: about 50 per mutual pair and 21 more on the Atwood ramp (atwoodWeights), where some lane of
+// nearly every warp step is; the profile counts 77 per warp step.  The sums are forces: with A = m h^-3 c at
+// each end (per particle), w_i' = m_j w_i and w_j' = m_i w_j (m in the unit of massUnit), hv = visc / 2,
+// t = hv / rho, P_i = w_i' (prho_i am + t_i) and P_j = w_j' (prho_j bm + t_j), both ends add the same
+// V = P_i A_i r + P_j A_j r, with opposite signs, and the same Q = t_i w_i' s_i + t_j w_j' s_j
+// (s = v_ij . A r); the finishing kernel divides by the particle's mass.  vsig is kept doubled, alpha divided
+// by 8 (both exact).  With the per-pair exp and divisions of the ramp and the terms factored by m_j and m_i
+// the kernel ran 109 FP64 instructions per warp step: 89.8 ms at 8M (jittered Sedov), now 58.6 ms, the FP64
+// pipe 88 % busy.
 // AvClean: the cleaned approach velocity differs between the ends by d3, the cut-off of close pairs at
 // the owner's eta_crit (a few per cent of the pairs), so the viscous terms of the neighbour's end are
 // formed again where it does; everything else is shared.  300k-particle sphere: 12.1 ms with every

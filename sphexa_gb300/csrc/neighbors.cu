@@ -112,9 +112,11 @@ struct WarpSmem {
 // At 27M particles the search takes 28.0 ms (37.1 with an append loop per tested block, nodes pruned per
 // axis, 6 blocks per SM and nodes of 128 particles taken whole); 8 blocks of 64 registers hide the
 // staging loads best (6: 29.6 ms, 7: 28.6, 9: 30.3).
-// Fold: groups whose pairs need a fold each do it in FP32 (launched for sets below kFoldBelow, where
-// such groups occur with ordinary h); without it they run the FP64 test for every pair, and the code of the
-// fold does not cost the large sets registers (1 % of the search at 27M).
+// Fold: groups whose pairs need a fold each do it in FP32; without it they run the FP64 test for every pair,
+// and the code of the fold does not cost registers (1 % of the search at 27M).  What decides is geometry, a search
+// region beyond half a periodic box, which the launch does not know; below kFoldBelow particles a cubic box
+// with ordinary h reaches it (12^3: a sweep of 2.42 ms with the FP64 tests, 1.33 with the fold), and larger
+// sets do only in a box that is thin on a periodic axis, where they take the FP64 test as they always did.
 constexpr int64_t kFoldBelow = 100000;
 
 template<bool Fold>
