@@ -653,13 +653,10 @@ __device__ __forceinline__ void meStdOnceBody(ListView lv, OwnedView ov, CoordFp
         maxvBits = maxBitsNonNeg(maxvBits, vsig);
         const T wsi = wv.x * fma(vzij, giz, fma(vyij, giy, vxij * gix));
         const T wsj = wv.y * fma(vzij, gjz, fma(vyij, gjy, vxij * gjx));
-        T ti = 0, tj = 0, Q = 0;
-        if (negative(wij)) {  // approaching: half of artificial_viscosity(1, 1, c_i, c_j, w_ij)
-            const T visc = fma(T(0.25), cs, -wij) * -wij;
-            ti = i2.v[1] * visc;
-            tj = j2.v[1] * visc;
-            Q = fma(ti, wsi, tj * wsj);
-        }
+        T visc = 0;  // its products are formed for receding pairs too: 0 times an undefined density is NaN, as in
+                     // the reference
+        if (negative(wij)) visc = fma(T(0.25), cs, -wij) * -wij;  // half of artificial_viscosity(1, 1, ...)
+        const T ti = i2.v[1] * visc, tj = j2.v[1] * visc, Q = fma(ti, wsi, tj * wsj);
         T Pi = wv.x * fma(mj, i2.v[0], ti), Pj = wv.y * fma(mj, j2.v[0], tj);
         T Vx = fma(Pi, gix, Pj * gjx), Vy = fma(Pi, giy, Pj * gjy), Vz = fma(Pi, giz, Pj * gjz);
         mx += Vx;

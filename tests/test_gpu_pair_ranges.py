@@ -119,3 +119,37 @@ def test_search_prunes_nodes_in_any_unit(gpu_ctx, scale):
         wl.box = wl.box * f
         tested.append(run_gpu(gpu_ctx, wl, "std", False)["stats"]["candidates"])
     assert tested[1] <= 20 * tested[0], tested
+
+
+@pytest.mark.parametrize("how", ["sweep", "passes"])
+def test_undefined_std_results_show_where_the_order_fixed_form_has_them(gpu_ctx, how):
+    """A pair of particles at one point has no distance, and what its densities reach is NaN in every output that
+    takes them, du of receding neighbours included."""
+    from sphexa_gb300 import sph, workloads as W
+    wl = W.random_cube(1500, seed=201, periodic=False)
+    rng = np.random.Generator(np.random.PCG64(202))
+    for k in ("x", "y", "z"):
+        wl.fields[k][1] = wl.fields[k][0]
+    for k in ("vx", "vy", "vz"):
+        wl.fields[k] = rng.normal(0.0, 0.2, wl.n).astype(np.float32).astype(np.float64)
+    gpu_ctx.set_params(ng0=int(wl.params["ng0"]), ngmax=int(wl.params["ngmax"]), bucket=int(wl.params["bucket"]),
+                       minDt=float(wl.params["minDt"]))
+    out = {}
+    for det in (True, False):
+        gpu_ctx.set_deterministic(det)
+        d = sph.ParticlesData.from_workload(wl, "fp64", "cuda:0")
+        box = sph.Box(wl.box.copy(), wl.bc.copy())
+        if how == "sweep":
+            sph.sweep(gpu_ctx, d, box, "std")
+        else:
+            sph.Domain(gpu_ctx, box).sync(d)
+            sph.find_neighbors_sfc(gpu_ctx, 0, wl.n, d)
+            sph.compute_density(gpu_ctx, d)
+            sph.compute_eos_hydro_std(gpu_ctx, d)
+            sph.compute_iad(gpu_ctx, d)
+            sph.compute_momentum_energy_std(gpu_ctx, d)
+        out[det] = {f: np.isnan(d.f[f].cpu().numpy()) for f in ("rho", "c11", "ax", "ay", "az", "du")}
+    gpu_ctx.set_deterministic(False)
+    assert out[True]["du"].any()
+    for f in out[True]:
+        np.testing.assert_array_equal(out[False][f], out[True][f], f)
