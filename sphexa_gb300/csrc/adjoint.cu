@@ -897,16 +897,22 @@ __device__ __forceinline__ stdad::MeSide<> stdSide(const AdjArgs& a, int64_t i)
 }
 
 // r = x_i - x_j with the legacy periodic fold at 2 h_i, d = |r|
-__device__ __forceinline__ void pairGeom(const AdjArgs& a, int64_t i, int64_t j, double r[3], double& d, double& rinv)
-{
-    const long long twoHBits = __double_as_longlong(2.0 * a.h[i]);
-    const double dd[3] = {a.x[i] - a.x[j], a.y[i] - a.y[j], a.z[i] - a.z[j]};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) r[k] = a.box.pbc[k] ? CoordFp64::wrapLegacy(dd[k], twoHBits, a.box.L[k]) : dd[k];
-    const double r2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
-    rinv = rsqrt(r2);
-    d = r2 * rinv;
-}
+// Geometry of a particle's owned pairs as the FP64 passes form it (diffOwned)
+struct StdOwnGeom {
+    CoordFp64::Target t;
+    CoordFp64::Fold fold;
+    __device__ __forceinline__ StdOwnGeom(const AdjArgs& a, int64_t k)
+        : t(a.cf.target(k)), fold(a.cf.fold(t, 2.0 * a.h[k]))
+    {
+    }
+    __device__ __forceinline__ void r(const AdjArgs& a, int64_t j, bool mutual, double o[3], double& d, double& rinv) const
+    {
+        a.cf.diffOwned(t, j, mutual, fold, o[0], o[1], o[2]);
+        const double r2 = dist2(o[0], o[1], o[2]);
+        rinv = invDist(r2);
+        d = r2 * rinv;
+    }
+};
 
 template<bool Smooth>
 __global__ void __launch_bounds__(kAdjBlock) meAdjOnceKernel(AdjArgs a, OwnedView ov)
@@ -918,6 +924,7 @@ __global__ void __launch_bounds__(kAdjBlock) meAdjOnceKernel(AdjArgs a, OwnedVie
     const bool anyK = seedsOf(a, k, gA, gE);
     double bx[3] = {0, 0, 0}, bv[3] = {0, 0, 0}, bh = 0, brho = 0, bp = 0, bc = 0, bC[6] = {0, 0, 0, 0, 0, 0};
     const stdad::MeSide<> S = stdSide(a, k);
+    const StdOwnGeom og(a, k);
     const unsigned cnt = ov.size(k);
     for (unsigned q = blockIdx.y; q < cnt; q += gridDim.y) {  // this block row's slice of the lists
         bool mutual;
@@ -927,7 +934,7 @@ __global__ void __launch_bounds__(kAdjBlock) meAdjOnceKernel(AdjArgs a, OwnedVie
         if (!anyK && !anyJ) continue;
         const stdad::MeSide<> J = stdSide(a, j);
         double r[3], d, rinv;
-        pairGeom(a, k, j, r, d, rinv);
+        og.r(a, j, mutual, r, d, rinv);
         const double v[3] = {a.vx[k] - a.vx[j], a.vy[k] - a.vy[j], a.vz[k] - a.vz[j]};
         double dwi, dwj;
         const double wi = lookupSlope(tab, d * S.hInv, dwi), wj = lookupSlope(tab, d * J.hInv, dwj);
@@ -968,25 +975,6 @@ __global__ void __launch_bounds__(kAdjBlock) meAdjOnceKernel(AdjArgs a, OwnedVie
     for (int t = 0; t < 6; ++t) atomicAdd(a.bCij + t * a.n + k, bC[t]);
 }
 
-// Geometry of a particle's pairs as the FP64 passes form it (legacy fold at 2 h_i where the particle's
-// 2h box leaves the periodic box)
-struct StdOwnGeom {
-    CoordFp64::Target t;
-    double twoH;
-    bool wrap;
-    __device__ __forceinline__ StdOwnGeom(const AdjArgs& a, int64_t k)
-        : t(a.cf.target(k)), twoH(2.0 * a.h[k]), wrap(a.cf.needsWrap(t, twoH))
-    {
-    }
-    __device__ __forceinline__ void r(const AdjArgs& a, int64_t j, double o[3], double& d, double& rinv) const
-    {
-        a.cf.diffFast(t, j, twoH, wrap, o[0], o[1], o[2]);
-        const double r2 = dist2(o[0], o[1], o[2]);
-        rinv = invDist(r2);
-        d = r2 * rinv;
-    }
-};
-
 // Momentum-energy without a du seed, arranged for few FP64 instructions (the FP64 pipe bounds it).  As
 // u_j t_j = m_j p_j / rho_j^2, both ends' seed vectors are W (q S + visc s D) with the same
 // S = m_j gA_i - m_i gA_j and D = gA_i - gA_j (q = p / rho^2, s = m / rho of the end), so every
@@ -1018,7 +1006,7 @@ __global__ void __launch_bounds__(kAdjBlock) meAdjOnceAKernel(AdjArgs a, OwnedVi
         const bool anyJ = mutual && seedsOf(a, j, gJ, gEj);
         if (!anyK && !anyJ) continue;
         double r[3], d, rinv;
-        og.r(a, j, r, d, rinv);
+        og.r(a, j, mutual, r, d, rinv);
         const double v[3] = {vI[0] - __ldg(a.vx + j), vI[1] - __ldg(a.vy + j), vI[2] - __ldg(a.vz + j)};
         const double hInvJ = __ldg(a.hInv + j), hDxJ = __ldg(a.hDx + j), mJ = __ldg(a.m + j),
                      qJ = __ldg(a.pOverRho2 + j), sJ = __ldg(a.mOverRho + j);
@@ -1130,7 +1118,7 @@ __global__ void __launch_bounds__(kAdjBlock) iadAdjOnceKernel(AdjArgs a, OwnedVi
         bool mutual;
         const uint32_t j = ov.at(k, q, mutual);
         double r[3], d, rinv, ty, T[3];
-        og.r(a, j, r, d, rinv);
+        og.r(a, j, mutual, r, d, rinv);
         const double volJ = __ldg(a.mOverRho + j), xk = d * hDxK;
         double w = lookupXSlope(tab, xk, ty);
         stdad::symv<double>(tauK, r, T);
@@ -1188,7 +1176,7 @@ __global__ void __launch_bounds__(kAdjBlock) densityAdjOnceKernel(AdjArgs a, Own
         bool mutual;
         const uint32_t j = ov.at(k, q, mutual);
         double r[3], d, rinv, ty;
-        og.r(a, j, r, d, rinv);
+        og.r(a, j, mutual, r, d, rinv);
         const double xk = d * hDxK;
         lookupXSlope(tab, xk, ty);
         const double bk = fK * __ldg(a.m + j) * ty;

@@ -485,6 +485,30 @@ __global__ void __launch_bounds__(kVeAdjBlock) meVeAdjKernel(VeAdjArgs a)
     meFlush<AvClean>(a, k, s, !TwoSided);
 }
 
+// the geometry of an owned pair, in the forward passes' arithmetic
+struct OwnGeom {
+    CoordFp64::Target t;
+    CoordFp64::Fold fold;
+    double vx, vy, vz;
+    __device__ __forceinline__ OwnGeom(const VeAdjArgs& a, int64_t k)
+        : t(a.cf.target(k)), fold(a.cf.fold(t, 2.0 * a.h[k])), vx(a.vx[k]), vy(a.vy[k]), vz(a.vz[k])
+    {
+    }
+    __device__ __forceinline__ void r(const VeAdjArgs& a, int64_t j, bool mutual, double o[3], double& d, double& rinv) const
+    {
+        a.cf.diffOwned(t, j, mutual, fold, o[0], o[1], o[2]);
+        const double r2 = dist2(o[0], o[1], o[2]);
+        rinv = invDist(r2);
+        d = r2 * rinv;
+    }
+    __device__ __forceinline__ void v(const VeAdjArgs& a, int64_t j, double o[3]) const
+    {
+        o[0] = vx - __ldg(a.vx + j);
+        o[1] = vy - __ldg(a.vy + j);
+        o[2] = vz - __ldg(a.vz + j);
+    }
+};
+
 // one evaluation per owned entry of the owned lists built with the neighbour lists: a mutual pair
 // gives both particles' terms (meAdjMutual), a one-sided entry its owner's (the same function with
 // the neighbour's seeds zero); the neighbour's partials are added with FP64 atomics.  No avClean.
@@ -501,6 +525,7 @@ __global__ void __launch_bounds__(kVeAdjBlock) meVeAdjOnceKernel(VeAdjArgs a, Ow
     const MeSeed sd = meSeed<WithDu>(a, k);
     s.prho = WithDu ? a.K * a.en[k] * a.sDu[k] : 0.0;
     s.rho = a.sRho ? a.sRho[k] : 0.0;
+    const OwnGeom og(a, k);
     const unsigned cnt = ov.size(k);
     for (unsigned q = 0; q < cnt; ++q) {
         bool mutual;
@@ -510,8 +535,8 @@ __global__ void __launch_bounds__(kVeAdjBlock) meVeAdjOnceKernel(VeAdjArgs a, Ow
         if (!sd.any && !sj.any) continue;
         const MeSide J = meSide(a, j);
         double r[3], d, rinv, v[3];
-        geom(a, k, j, r, d, rinv);
-        vdiff(a, k, j, v);
+        og.r(a, j, mutual, r, d, rinv);
+        og.v(a, j, v);
         double dwi, dwj;
         const double wi = lookupVS(tw, d * S.hInv, dwi), wj = lookupVS(tw, d * J.hInv, dwj);
         MeGrad o;
@@ -534,30 +559,6 @@ __global__ void __launch_bounds__(kVeAdjBlock) meVeAdjOnceKernel(VeAdjArgs a, Ow
     }
     meFlush<false>(a, k, s, true);
 }
-
-// the geometry of an owned pair, in the forward passes' arithmetic
-struct OwnGeom {
-    CoordFp64::Target t;
-    double vx, vy, vz, twoH;
-    bool wrap;
-    __device__ __forceinline__ OwnGeom(const VeAdjArgs& a, int64_t k)
-        : t(a.cf.target(k)), vx(a.vx[k]), vy(a.vy[k]), vz(a.vz[k]), twoH(2.0 * a.h[k]), wrap(a.cf.needsWrap(t, twoH))
-    {
-    }
-    __device__ __forceinline__ void r(const VeAdjArgs& a, int64_t j, double o[3], double& d, double& rinv) const
-    {
-        a.cf.diffFast(t, j, twoH, wrap, o[0], o[1], o[2]);
-        const double r2 = dist2(o[0], o[1], o[2]);
-        rinv = invDist(r2);
-        d = r2 * rinv;
-    }
-    __device__ __forceinline__ void v(const VeAdjArgs& a, int64_t j, double o[3]) const
-    {
-        o[0] = vx - __ldg(a.vx + j);
-        o[1] = vy - __ldg(a.vy + j);
-        o[2] = vz - __ldg(a.vz + j);
-    }
-};
 
 // The same without a du seed (meAdjMutual<false>), arranged for few FP64 instructions: the kernel is
 // bound by the FP64 pipe.  With s = m_j abar_i - m_i abar_j both ends' Abar are multiples of s, so with
@@ -595,7 +596,7 @@ __global__ void __launch_bounds__(kVeAdjBlock) meVeAdjOnceAKernel(VeAdjArgs a, O
         const double mJ = __ldg(a.m + j);
         const double sv[3] = {fma(mJ, ax, -mI * bx), fma(mJ, ay, -mI * by), fma(mJ, az, -mI * bz)};
         double r[3], d, rinv, v[3];
-        og.r(a, j, r, d, rinv);
+        og.r(a, j, mutual, r, d, rinv);
         og.v(a, j, v);
         const double xi = d * hDxI, xj = d * __ldg(a.hDx + j);
         double tyi, tyj;
@@ -844,7 +845,7 @@ __global__ void __launch_bounds__(kVeAdjBlock) veAvAdjOnceKernel(VeAdjArgs a, Ow
         if (mutual && sj.any && uint32_t(k) == sj.arg) vsigb += sj.vsigb;
         if (!sk.gAny && !sj.gAny && vsigb == 0.0) continue;
         double r[3], d, rinv, g[3] = {0.0, 0.0, 0.0}, db = 0.0, divvb = 0.0;
-        og.r(a, j, r, d, rinv);
+        og.r(a, j, mutual, r, d, rinv);
         const double ddiv = divvK - __ldg(a.divv + j);
         if (sk.gAny) {
             const double xi = d * hDxK;
@@ -1057,7 +1058,7 @@ __global__ void __launch_bounds__(kVeAdjBlock) veIadAdjOnceKernel(VeAdjArgs a, O
         bool mutual;
         const uint32_t j = ov.at(k, q, mutual);
         double r[3], d, rinv, vv[3], g[3], vb[3], db;
-        og.r(a, j, r, d, rinv);
+        og.r(a, j, mutual, r, d, rinv);
         og.v(a, j, vv);
         // one end's term: weights of the other end, table coordinate x = |r| / (h dx) of this end
         auto term = [&](const double tau[6], const double PB[9], double vol, double xmo, double kxInv, double kxv, double xt,
@@ -1238,7 +1239,7 @@ __global__ void __launch_bounds__(kVeAdjBlock) veGradhAdjOnceKernel(VeAdjArgs a,
         bool mutual;
         const uint32_t j = ov.at(k, q, mutual);
         double r[3], d, rinv, xmb;
-        og.r(a, j, r, d, rinv);
+        og.r(a, j, mutual, r, d, rinv);
         const double xk = d * hDxK;
         const double bk = term(xk, skx, som, sr0, __ldg(a.xm + j), __ldg(a.m + j), xmb);
         h = fma(-bk, xk, h);
@@ -1337,7 +1338,7 @@ __global__ void __launch_bounds__(kVeAdjBlock) veXmassAdjOnceKernel(VeAdjArgs a,
         bool mutual;
         const uint32_t j = ov.at(k, q, mutual);
         double r[3], d, rinv, ty;
-        og.r(a, j, r, d, rinv);
+        og.r(a, j, mutual, r, d, rinv);
         const double xk = d * hDxK;
         lookupXSlope(tw, xk, ty);
         const double bk = r0b * __ldg(a.m + j) * ty;

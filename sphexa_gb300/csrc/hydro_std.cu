@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(kPairBlock) xmassOnceKernel(ListView lv, Owned
     const unsigned no = ov.size(ii);
     auto t = cf.target(i);
     const double hi = h[i], mi = m[i], twoH = 2.0 * hi, hiInvDx = hInvDx[i];
-    const bool wrap = cf.needsWrap(t, twoH);
+    const auto fold = cf.fold(t, twoH);
     const int64_t gb = geo.g ? geo.base(ii) : 0, rb = Mode == kXmassRecords ? pr.base(ii) : 0;
     const double vxi = geo.g ? vx[i] : 0.0, vyi = geo.g ? vy[i] : 0.0, vzi = geo.g ? vz[i] : 0.0;
     double rho0 = 0.0;
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(kPairBlock) xmassOnceKernel(ListView lv, Owned
         bool mutual;
         const uint32_t j = ov.at(ii, k, mutual);
         double rx, ry, rz;
-        cf.diffFast(t, j, twoH, wrap, rx, ry, rz);
+        cf.diffOwned(t, j, mutual, fold, rx, ry, rz);
         const double r2 = dist2(rx, ry, rz);
         const double rinv = invDist(r2);
         const double dist = r2 * rinv;
@@ -313,13 +313,13 @@ __device__ __forceinline__ void iadStdOnceBody(ListView lv, OwnedView ov, CoordF
     const double voli = vol[i];
     typename CoordFp64::Target t{};
     double twoH = 0, hiInvDx = 0;
-    bool wrap = false;
+    CoordFp64::Fold fold{};
     int64_t g = 0;
     if constexpr (Geo != 0) g = geo.base(ii) + 32 * blockIdx.y;
     if constexpr (Geo != 5) {
         t = cf.target(i);
         twoH = 2.0 * h[i];
-        wrap = cf.needsWrap(t, twoH);
+        fold = cf.fold(t, twoH);
         hiInvDx = hInvDx[i];
     }
     const int64_t rb = pr.base(ii);
@@ -334,7 +334,7 @@ __device__ __forceinline__ void iadStdOnceBody(ListView lv, OwnedView ov, CoordF
             const double2 a0 = __ldg(geo.x + g);
             rx = a0.x, ry = a0.y, rz = __ldg(geo.x + geo.plane + g).x;
         } else {
-            cf.diffFast(t, j, twoH, wrap, rx, ry, rz);
+            cf.diffOwned(t, j, mutual, fold, rx, ry, rz);
         }
         if constexpr (Geo == 0) {
             const double r2 = dist2(rx, ry, rz);
@@ -602,13 +602,13 @@ __device__ __forceinline__ void meStdOnceBody(ListView lv, OwnedView ov, CoordFp
     const T mi = i1.v[3];
     typename CoordFp64::Target t{};
     T vxi = 0, vyi = 0, vzi = 0, twoH = 0, hiInvDx = 0;
-    bool wrap = false;
+    CoordFp64::Fold fold{};
     int64_t g = 0;
     if constexpr (Geo != 0) g = geo.base(ii) + 32 * blockIdx.y;
     if constexpr (Geo != 5) {
         t = cf.target(i);
         twoH = 2.0 * ld<T>(a.h, i);
-        wrap = cf.needsWrap(t, twoH);
+        fold = cf.fold(t, twoH);
         vxi = vxA[i], vyi = vyA[i], vzi = vzA[i];
         hiInvDx = hInvDx[i];
     }
@@ -631,7 +631,7 @@ __device__ __forceinline__ void meStdOnceBody(ListView lv, OwnedView ov, CoordFp
             rx = a0.x, ry = a0.y, rz = a1.x;
             vxij = -a1.y, vyij = -a2.x, vzij = -a2.y;
         } else {
-            cf.diffFast(t, j, twoH, wrap, rx, ry, rz);
+            cf.diffOwned(t, j, mutual, fold, rx, ry, rz);
             vxij = vxi - vxA[j], vyij = vyi - vyA[j], vzij = vzi - vzA[j];
         }
         if constexpr (Geo == 0) {

@@ -895,13 +895,13 @@ __device__ __forceinline__ void gradhOnceBody(ListView lv, OwnedView ov, CoordFp
     const double mi = m[i], xmi = xm[i], hiInvDx = hInvDx[i];
     typename CoordFp64::Target t{};
     double twoH = 0.0;
-    bool wrap = false;
+    CoordFp64::Fold fold{};
     int64_t g = 0;
     if constexpr (Geo) g = geo.base(ii) + 32 * blockIdx.y;
     else {
         t = cf.target(i);
         twoH = 2.0 * h[i];
-        wrap = cf.needsWrap(t, twoH);
+        fold = cf.fold(t, twoH);
     }
     double kx = 0.0, dxm = 0.0, dm = 0.0;
     for (unsigned k = blockIdx.y; k < no; k += gridDim.y, g += 32 * gridDim.y) {
@@ -914,7 +914,7 @@ __device__ __forceinline__ void gradhOnceBody(ListView lv, OwnedView ov, CoordFp
             wv = __ldg(geo.w + g);
         } else {
             double rx, ry, rz;
-            cf.diffFast(t, j, twoH, wrap, rx, ry, rz);
+            cf.diffOwned(t, j, mutual, fold, rx, ry, rz);
             const double r2 = dist2(rx, ry, rz);
             dist = r2 * invDist(r2);
         }
@@ -1026,7 +1026,7 @@ __global__ void __launch_bounds__(kPairBlock) iadOnceKernel(ListView lv, OwnedVi
                  *vol = static_cast<const double*>(a.vol);
     auto t = cf.target(i);
     const double hi = ld<double>(a.h, i), twoH = 2.0 * hi, hiInvDx = hInvDx[i];
-    const bool wrap = cf.needsWrap(t, twoH);
+    const auto fold = cf.fold(t, twoH);
     const double vxi = vx[i], vyi = vy[i], vzi = vz[i], voli = vol[i], xmi = xm[i];
     const int64_t gb = geo.base(ii);
     double tau[6] = {0, 0, 0, 0, 0, 0}, M[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -1043,7 +1043,7 @@ __global__ void __launch_bounds__(kPairBlock) iadOnceKernel(ListView lv, OwnedVi
             dist = __ldg(geo.g + e).x;
             wv = __ldg(geo.w + e);
         } else {
-            cf.diffFast(t, j, twoH, wrap, rx, ry, rz);
+            cf.diffOwned(t, j, mutual, fold, rx, ry, rz);
             if (geo.g) {
                 const int64_t e = gb + 32 * int64_t(k);
                 dist = __ldg(geo.g + e).x;
@@ -1138,13 +1138,13 @@ __device__ __forceinline__ void avOnceBody(ListView lv, OwnedView ov, CoordFp64 
     const double ci = c[i], divvi = divv[i], voli = vol[i];
     typename CoordFp64::Target t{};
     double vxi = 0, vyi = 0, vzi = 0, twoH = 0, hiInvDx = 0;
-    bool wrap = false;
+    CoordFp64::Fold fold{};
     int64_t g = 0;
     if constexpr (Geo != 0) g = geo.base(ii) + 32 * blockIdx.y;
     if constexpr (Geo != 5) {
         t = cf.target(i);
         twoH = 2.0 * ld<double>(a.h, i);
-        wrap = cf.needsWrap(t, twoH);
+        fold = cf.fold(t, twoH);
         vxi = vx[i], vyi = vy[i], vzi = vz[i];
         hiInvDx = hInvDx[i];
     }
@@ -1164,7 +1164,7 @@ __device__ __forceinline__ void avOnceBody(ListView lv, OwnedView ov, CoordFp64 
             const double2 a0 = __ldg(geo.x + g);
             rx = a0.x, ry = a0.y, rz = __ldg(geo.x + geo.plane + g).x;
         } else {
-            cf.diffFast(t, j, twoH, wrap, rx, ry, rz);
+            cf.diffOwned(t, j, mutual, fold, rx, ry, rz);
         }
         if constexpr (Geo == 0) {
             const double r2 = dist2(rx, ry, rz);
@@ -1350,11 +1350,11 @@ __device__ __forceinline__ void meVeOnceBody(ListView lv, CoordFp64 cf, MeVeArgs
     const float rhofi = a.rhof[i];
     typename CoordFp64::Target t{};
     T vxi = 0, vyi = 0, vzi = 0, hiInvDx = 0, twoH = 0;
-    bool wrap = false;
+    CoordFp64::Fold fold{};
     if constexpr (Geo != 5) {
         t = cf.target(i);
         twoH = 2.0 * ld<T>(a.h, i);
-        wrap = cf.needsWrap(t, twoH);
+        fold = cf.fold(t, twoH);
         vxi = vxA[i], vyi = vyA[i], vzi = vzA[i];
         hiInvDx = hInvDx[i];
     }
@@ -1385,7 +1385,7 @@ __device__ __forceinline__ void meVeOnceBody(ListView lv, CoordFp64 cf, MeVeArgs
             rx = a0.x, ry = a0.y, rz = a1.x;
             vxij = -a1.y, vyij = -a2.x, vzij = -a2.y;
         } else {
-            cf.diffFast(t, j, twoH, wrap, rx, ry, rz);
+            cf.diffOwned(t, j, mutual, fold, rx, ry, rz);
             vxij = vxi - vxA[j], vyij = vyi - vyA[j], vzij = vzi - vzA[j];
         }
         if constexpr (Geo == 0) {

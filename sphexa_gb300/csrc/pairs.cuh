@@ -12,6 +12,7 @@
 //           rounding.  Sums that the error budget needs are Kahan-compensated.
 #pragma once
 
+#include <algorithm>
 #include <type_traits>
 
 #include "context.cuh"
@@ -296,6 +297,8 @@ struct CoordFp64 {
     const double *x, *y, *z;
     double L[3], lo[3], hi[3];
     int pbc[3];
+    long long half[3];  // bits of L / 2
+    unsigned halfHigh;  // smallest high word of L / 2 over the periodic axes
     struct Target {
         double x, y, z;
     };
@@ -340,6 +343,35 @@ struct CoordFp64 {
             rz = t.z - z[j];
         }
     }
+    // The difference of an owned pair.  A one-sided entry is the owner's alone: diffFast.  A mutual pair serves
+    // both ends, whose own rules (threshold 2h_i, 2h_j; fold or not by the ends' distances from the faces) agree
+    // while both list the other, but not once particles have moved on frozen lists: it takes the nearest
+    // image, which is what each end's rule gives wherever its kernel function is not 0 (2h <= L/4 for both
+    // ends when the lists were built).  Thresholds and comparisons on bit patterns, as in wrapLegacy.
+    // One integer test of the largest component's high word against the smallest threshold keeps the folds out of
+    // the loop but near a face.
+    struct Fold {
+        long long twoH;
+        unsigned high;
+    };
+    __device__ __forceinline__ Fold fold(const Target& t, double twoH) const
+    {
+        return {__double_as_longlong(twoH), needsWrap(t, twoH) ? unsigned(__double2hiint(twoH)) : 0x80000000u};
+    }
+    __device__ __forceinline__ void diffOwned(const Target& t, int64_t j, bool mutual, const Fold& f, double& rx,
+                                              double& ry, double& rz) const
+    {
+        rx = t.x - x[j];
+        ry = t.y - y[j];
+        rz = t.z - z[j];
+        const unsigned m = max(unsigned(__double2hiint(rx)) & 0x7fffffffu,
+                               max(unsigned(__double2hiint(ry)) & 0x7fffffffu, unsigned(__double2hiint(rz)) & 0x7fffffffu));
+        if (m >= (mutual ? halfHigh : f.high)) {
+            if (pbc[0]) rx = wrapLegacy(rx, mutual ? half[0] : f.twoH, L[0]);
+            if (pbc[1]) ry = wrapLegacy(ry, mutual ? half[1] : f.twoH, L[1]);
+            if (pbc[2]) rz = wrapLegacy(rz, mutual ? half[2] : f.twoH, L[2]);
+        }
+    }
 };
 
 inline CoordFp64 coordFp64(const sphgb_ctx* c, const sphgb_particles* p)
@@ -348,11 +380,15 @@ inline CoordFp64 coordFp64(const sphgb_ctx* c, const sphgb_particles* p)
     r.x = p->x;
     r.y = p->y;
     r.z = p->z;
+    r.halfHigh = 0x80000000u;  // no difference reaches it
     for (int k = 0; k < 3; ++k) {
         r.L[k] = c->box.L[k];
         r.lo[k] = c->box.lo[k];
         r.hi[k] = c->box.hi[k];
         r.pbc[k] = c->box.pbc[k];
+        const double halfL = 0.5 * c->box.L[k];
+        std::memcpy(&r.half[k], &halfL, sizeof(halfL));
+        if (r.pbc[k]) r.halfHigh = std::min(r.halfHigh, unsigned(r.half[k] >> 32));
     }
     return r;
 }
