@@ -583,7 +583,7 @@ __global__ void meStdRec64Kernel(int64_t n, MeStdArgs a, Rec4d* __restrict__ rec
 // FP64 pipe: 1M particles 15.3 ms with every directed pair evaluated, now 5.3 ms and 0.6 for the gather of
 // the records (IAD 5.7 -> 1.3 + 0.9, density 3.5 -> 2.6 + 0.2, which also fills the geometry cache; the inbox
 // 1.2 ms once per neighbour search).  With atomics in place of the records the sweep took 12.5 ms, with them
-// 14.7, and its bits differed from run to run.
+// 14.5, but its bits differed from run to run.
 // Geo: arrays of the pair-geometry cache (5, 2), or 0 to form the geometry here.
 template<bool Smooth, int Geo>
 __device__ __forceinline__ void meStdOnceBody(ListView lv, OwnedView ov, CoordFp64 cf, MeStdArgs a,
