@@ -273,7 +273,7 @@ __global__ void __launch_bounds__(kPairBlock) iadKernel(ListView lv, CoordFp64 c
                 Bn = ldRec8(rec + pick(G, s));
             }
             float rx, ry, rz;
-            cm.diffBlock(t, B, rx, ry, rz);
+            cm.diffBlock<true>(t, B, rx, ry, rz);
             float dist = sqrtf(fmaf(rx, rx, fmaf(ry, ry, rz * rz)));
             float w = lookupH32(tab, dist * t.hInv);
             float vw = B.v[5] * w;
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(kPairBlock) meStdKernel(ListView lv, CoordFp64
                 n2 = __ldg(reinterpret_cast<const float4*>(a.pack + 3 * int64_t(jn) + 2));
             }
             T rx, ry, rz;
-            cm.diffBlock(t, b0, rx, ry, rz);
+            cm.diffBlock<true>(t, b0, rx, ry, rz);
             const T hjInv = b0.v[5];
             T r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
             T rinv = rsqrtf(r2);
@@ -582,8 +582,8 @@ __global__ void meStdRec64Kernel(int64_t n, MeStdArgs a, Rec4d* __restrict__ rec
 // Q with s = v_ij . A r and Q = t_i w_i s_i + t_j w_j s_j; j's is 2 m_i q_j w_j s_j + Q.  Bound by the
 // FP64 pipe: 1M particles 15.3 ms with every directed pair evaluated, now 5.3 ms and 0.6 for the gather of
 // the records (IAD 5.7 -> 1.3 + 0.9, density 3.5 -> 2.6 + 0.2, which also fills the geometry cache; the inbox
-// 1.2 ms once per neighbour search).  With atomics in place of the records the sweep took 12.5 ms, with them
-// 14.5, but its bits differed from run to run.
+// 1.2 ms once per neighbour search).  With atomics in place of the records the sweep took 12.5 ms and its bits
+// differed from run to run; with them 14.5.
 // Geo: arrays of the pair-geometry cache (5, 2), or 0 to form the geometry here.
 template<bool Smooth, int Geo>
 __device__ __forceinline__ void meStdOnceBody(ListView lv, OwnedView ov, CoordFp64 cf, MeStdArgs a,

@@ -823,13 +823,20 @@ struct CoordMixed {
     // 11): d itself when |d| < 2^20, d -/+ 2^21 beyond; s = 0 leaves d unchanged.  The same
     // image as wrap() except at exactly half the box, where both images are equally near.
     __device__ __forceinline__ static int wrapShift(int d, int s) { return int(unsigned(d) << s) >> s; }
-    // the same difference from a neighbour block written by packGridBlock
+    // the same difference from a neighbour block written by packGridBlock; Odd: with the image
+    // of wrap() at half the box, odd in d, r_ij = -r_ji (the std IAD and momentum-energy passes, where a lattice of a few
+    // particles a side has pairs there)
+    template<bool Odd = false>
     __device__ __forceinline__ void diffBlock(const Target& t, const Rec8& b, float& rx, float& ry, float& rz) const
     {
         const u64 k = u64(__float_as_uint(b.v[0])) | (u64(__float_as_uint(b.v[1])) << 32);
-        int dx = wrapShift(t.ix - int(k & kGridMask), sh[0]);
-        int dy = wrapShift(t.iy - int((k >> kGridBits) & kGridMask), sh[1]);
-        int dz = wrapShift(t.iz - int(k >> (2 * kGridBits)), sh[2]);
+        int dx = t.ix - int(k & kGridMask);
+        int dy = t.iy - int((k >> kGridBits) & kGridMask);
+        int dz = t.iz - int(k >> (2 * kGridBits));
+        constexpr int half = 1 << (kGridBits - 1);
+        dx = Odd && dx == half ? half : wrapShift(dx, sh[0]);
+        dy = Odd && dy == half ? half : wrapShift(dy, sh[1]);
+        dz = Odd && dz == half ? half : wrapShift(dz, sh[2]);
         rx = fmaf(float(dx), u[0], t.xl - b.v[2]);
         ry = fmaf(float(dy), u[1], t.yl - b.v[3]);
         rz = fmaf(float(dz), u[2], t.zl - b.v[4]);
